@@ -43,13 +43,19 @@ struct BoxSrc {
 // Per-insertion record: dE_intra, dE_inter (without reciprocal), dE_frag, ln_pbias.
 using WRec = double4_32a;
 
-// Widom cell edge rcut_cbmc / cells-per-cutoff, measured on the 64-box butane
-// batch: with row-trimmed stencils, cells of a third of the cutoff visit 2.4x
-// fewer candidates and the FP64 kernel runs 22 % faster than with cells of the
-// cutoff; the FP32 kernel is fastest with cells of the cutoff (its time goes
-// to set-up and divergence more than to candidates: 22.5 ms at 1, 26.0 ms at 2).
+// Widom cell edge rcut_cbmc / cells-per-cutoff, measured on the 64-box butane batch:
+// with row-trimmed stencils, cells of a third of the cutoff visit 2.4x fewer
+// candidates and the FP64 kernel runs 22 % faster than with cells of the cutoff.  The
+// FP32 kernel searches cells only in boxes without voxel lists and while the lists are
+// built: 15.2 ms at 1.25, 17.6 ms at 1.
 constexpr double kCellsPerCutoffFP64 = 3.0;
-constexpr double kCellsPerCutoffMixed = 1.0;
+constexpr double kCellsPerCutoffMixed = 1.25;
+constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory of a CTA
+// voxels per cutoff of the neighbour lists: 2.6, 3.25 and 4 for the CBMC radius took
+// 15.4, 15.2 and 15.8 ms, 3, 4 and 5 for the full one 15.2, 15.2 and 15.5 ms
+constexpr double kVoxPerCutoffCbmc = 3.25;
+constexpr double kVoxPerCutoffFull = 4.0;
+constexpr double kVoxMaxBytes = 4.0e9;      // most device memory for them
 
 __device__ __forceinline__ int wrapc(int c, int n) {
   c %= n;
@@ -786,21 +792,8 @@ struct QueryAcc {
   KahanF e;
   float eabs = 0.0f;
   unsigned long long visited = 0, in_cut = 0;
-  int nband = 0, atom = 0;      // kQDetect: band pairs met, the current test atom
-  BandPair* band = nullptr;     // kQDetect: the first kMaxBand of them
+  int nband = 0;
 };
-
-// Query modes.  kQPlain: FP32 decisions.  kQDetect (the full-cutoff pass of
-// the FP32 growth): FP32 decisions, every pair within a band noted in A (a
-// pair in the band of rcut_low^2 counts as no overlap and adds its energy;
-// only an FP32 r^2 below the band is a certain overlap).  kQExact: decisions
-// inside a band made in FP64 from the FP64 coordinates p64.
-constexpr int kQPlain = 0, kQDetect = 1, kQExact = 2;
-
-__device__ __forceinline__ void band_note(QueryAcc& A, int j, float r2, int kind) {
-  if (A.nband < kMaxBand) A.band[A.nband] = BandPair{j, r2, (unsigned char)A.atom, (unsigned char)kind, 0, 0};
-  ++A.nband;
-}
 
 // r^2 to a stored atom, through the row's image shift (folded in full dimensions)
 __device__ __forceinline__ float pair_r2(const BoxF& f, const bool (&full)[3], bool fold_any, float qx, float qy,
@@ -817,9 +810,10 @@ __device__ __forceinline__ float pair_r2(const BoxF& f, const bool (&full)[3], b
 // r^2 of two stored atoms at once on the packed FP32x2 pipe (FFMA2, sm_100 and
 // later): the same operations and rounding as pair_r2 without a fold,
 // qx - a.x formed as fma(a.x, -1, qx)
-__device__ __forceinline__ float2 pair_r2_x2(float qx, float qy, float qz, const float4& a0, const float4& a1) {
+__device__ __forceinline__ float2 pair_r2_x2(float qx0, float qx1, float qy, float qz, const float4& a0,
+                                             const float4& a1) {
   const float2 m1 = make_float2(-1.0f, -1.0f);
-  const float2 dx = __ffma2_rn(make_float2(a0.x, a1.x), m1, make_float2(qx, qx));
+  const float2 dx = __ffma2_rn(make_float2(a0.x, a1.x), m1, make_float2(qx0, qx1));
   const float2 dy = __ffma2_rn(make_float2(a0.y, a1.y), m1, make_float2(qy, qy));
   const float2 dz = __ffma2_rn(make_float2(a0.z, a1.z), m1, make_float2(qz, qz));
   return __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
@@ -866,27 +860,20 @@ __device__ __forceinline__ bool overlap_exact(const BoxViewF& V, float r2, int j
   return exact_r2(f, V.p64, j, p64) < f.low2d;
 }
 
-// LJ and real-space Ewald energy of one pair inside the selection radius.
-// kQDetect flags a pair at or above the lower edge rlo of the cutoff bands;
-// kQExact compares an FP32 r^2 within a band of the vdW or Coulomb cutoff with
-// the cutoff in FP64, from the FP64 coordinates, so that the pair counts
-// exactly when the FP64 energy counts it.
-template <bool COUNT, int MODE = kQPlain>
-__device__ __forceinline__ void pair_energy(const BoxViewF& V, QueryAcc& A, const float4& a, int j, float r2,
-                                            const float2* lrow, bool vdw_on, bool qq_on, float rv2, float rq2,
-                                            float qa, float rlo = 0.0f, const double* p64 = nullptr) {
+// LJ and real-space Ewald energy of one pair inside the selection radius.  An
+// FP32 r^2 within a band of the vdW or Coulomb cutoff is compared with the cutoff
+// in FP64, from the FP64 coordinates, so that the pair counts exactly when the
+// FP64 energy counts it.
+__device__ __forceinline__ void pair_energy_exact(const BoxViewF& V, QueryAcc& A, const float4& a, int j, float r2,
+                                                  const float2* lrow, bool vdw_on, bool qq_on, float rv2, float rq2,
+                                                  float qa, const double* p64) {
+  const BoxF& f = *V.f;
   bool in_v = r2 <= rv2, in_q = r2 <= rq2;
-  if (MODE == kQDetect && r2 >= rlo) band_note(A, j, r2, 0);
-  if (MODE == kQExact) {
-    const BoxF& f = *V.f;
-    if (fabsf(r2 - rv2) <= f.band_v || fabsf(r2 - rq2) <= f.band_q) {
-      const double d2 = exact_r2(f, V.p64, j, p64);
-      in_v = d2 <= f.rv2d;
-      in_q = d2 <= f.rq2d;
-    }
-    if (!in_v && !in_q) return;
+  if (fabsf(r2 - rv2) <= f.band_v || fabsf(r2 - rq2) <= f.band_q) {
+    const double d2 = exact_r2(f, V.p64, j, p64);
+    in_v = d2 <= f.rv2d;
+    in_q = d2 <= f.rq2d;
   }
-  if (COUNT) ++A.in_cut;
   const int tj = __float_as_int(a.w);
   if (vdw_on && tj >= 0 && in_v) {
     const float2 es = lrow[tj];
@@ -895,21 +882,20 @@ __device__ __forceinline__ void pair_energy(const BoxViewF& V, QueryAcc& A, cons
     A.eabs += fabsf(ev);
   }
   if (qq_on && in_q) {
-    const float eq = qq_ewald_inter_f(V.f->alpha, qa * V.q32[j], r2);
+    const float eq = qq_ewald_inter_f(f.alpha, qa * V.q32[j], r2);
     A.e.add(eq);
     A.eabs += fabsf(eq);
   }
 }
 
-// FP32 energy of one test atom at p against the box atoms within the cutoff,
-// added to A.  Returns true on core overlap (r^2 < rcut_low^2), as
-// Compute_MoleculePair_Energy (energy_routines.f90:1676-1679) does.
-// A CBMC query with the CBMC options: check_overlap against r_min^2 of the
-// type pair and, with the energy table, Estimate_MoleculePair_Energy per pair
-// (FP32 table; a pair's bin can differ from FP64 within rounding of a bin edge)
-__device__ bool query_f_opt(const BoxViewF& V, QueryAcc& A, float px, float py, float pz, int ta, float qa) {
+// FP32 energy of one test atom at p against the box atoms within the full cutoff,
+// added to A, the cutoff decisions within a band made in FP64 from the FP64
+// coordinates p64 of the query atom.  Returns true on core overlap (r^2 <
+// rcut_low^2), as Compute_MoleculePair_Energy (energy_routines.f90:1676-1679) does.
+__device__ bool query_f_exact(const BoxViewF& V, QueryAcc& A, float px, float py, float pz, int ta, float qa,
+                              const double* p64) {
   const BoxF& f = *V.f;
-  const float rc = f.rc_cbmc;
+  const float rc = f.rc_full;
   const float p[3] = {px, py, pz};
   int lo[3], hi[3];
   bool full[3];
@@ -923,13 +909,16 @@ __device__ bool query_f_opt(const BoxViewF& V, QueryAcc& A, float px, float py, 
     lo[d] = full[d] ? 0 : l;
     hi[d] = full[d] ? f.nc[d] - 1 : h;
   }
+  const float rv2 = f.rv2;
+  const float rq2 = f.rq2;
   const bool vdw_on = ta >= 0;
   const bool qq_on = f.charge_on && qa != 0.0f;
-  const float rsel2 = f.rcb2;
+  // the selection and overlap radii, widened by the FP32 bands
+  const float band = fmaxf(vdw_on ? f.band_v : 0.0f, qq_on ? f.band_q : 0.0f);
+  const float rsel2 = fmaxf(vdw_on ? rv2 : -1.0f, qq_on ? rq2 : -1.0f) + band;
+  const float low2q = f.low2 + f.band_low;
   const float rc2 = rc * rc;
   const float2* lrow = V.ljp + (vdw_on ? ta : 0) * kMaxTypes;
-  const float* rmrow = f.rmin2 + (vdw_on ? ta : 0) * kMaxTypes;
-  const float qicf = qa * (float)kCHARGE_FACTOR;
   const int nc0 = f.nc[0], nc1 = f.nc[1], nc2 = f.nc[2];
   for (int cz = lo[2]; cz <= hi[2]; ++cz) {
     const int sz = cell_image(cz, nc2);
@@ -958,21 +947,8 @@ __device__ bool query_f_opt(const BoxViewF& V, QueryAcc& A, float px, float py, 
         for (int j = j0; j < j1; ++j) {
           const float4 a = V.p32[j];
           const float r2 = pair_r2(f, fl, fold_any, qx, qy, qz, a);
-          const int tj = __float_as_int(a.w);
-          if (f.sector && r2 < (vdw_on && tj >= 0 ? rmrow[tj] : f.low2)) return true;
-          if (f.tab_res > 0) {
-            float e = 0.0f;
-            const int k = table_pair_f(f.tab_v, f.tab_f2, f.tab_res, f.tab_shift, f.tab_rcs, f.tab_step,
-                                       f.tab_inv_step, f.ntypes, r2, ta, tj, qicf, qq_on ? V.q32[j] : 0.0f, e);
-            if (k == 2) return true;
-            if (k == 1) {
-              A.e.add(e);
-              A.eabs += fabsf(e);
-            }
-          } else {
-            if (r2 < f.low2) return true;
-            if (r2 <= rsel2) pair_energy<false>(V, A, a, j, r2, lrow, vdw_on, qq_on, f.rcb2, f.rcb2, qa);
-          }
+          if (r2 < low2q && overlap_exact(V, r2, j, p64)) return true;
+          if (r2 <= rsel2) pair_energy_exact(V, A, a, j, r2, lrow, vdw_on, qq_on, rv2, rq2, qa, p64);
         }
         cx += run;
       }
@@ -981,111 +957,530 @@ __device__ bool query_f_opt(const BoxViewF& V, QueryAcc& A, float px, float py, 
   return false;
 }
 
-// MODE: kQPlain, kQDetect or kQExact (then p64 holds the FP64 coordinates of
-// the query atom).
-template <bool COUNT, bool OPT = false, int MODE = kQPlain>
-__device__ bool query_f(const BoxViewF& V, QueryAcc& A, float px, float py, float pz, int ta, float qa, bool cbmc,
-                        bool want_qq, const double* p64 = nullptr) {
-  if (OPT && cbmc) return query_f_opt(V, A, px, py, pz, ta, qa);
-  const BoxF& f = *V.f;
-  const float rc = cbmc ? f.rc_cbmc : f.rc_full;
-  const float p[3] = {px, py, pz};
-  int lo[3], hi[3];
-  bool full[3];
+// ---------------------------------------------------------------------------
+// Warp-wide neighbour queries of the mixed Widom kernel.
+//
+// A lane owns an insertion and does its serial steps (draws, geometry, weights);
+// the queries of all lanes are put in a queue in shared memory and the warp
+// works through them together, one (query, stencil row) per lane.  Rows of
+// different queries fill the 32 lanes whatever the insertions' own states are:
+// with a query per lane a warp instruction did the work of 7.6 lanes, because
+// the insertions end their queries at different candidates.  A row's pairs
+// within the selection radius are listed first and their energies formed
+// afterwards, so that the energy code runs for full lists and not for the odd
+// lane whose candidate happens to be near.
+constexpr int kCoopItems = 128;  // rows of one batch of queries
+constexpr int kCoopHits = 8;     // listed pairs per lane
+constexpr int kCoopBand = 64;    // band pairs of a warp's insertions
+
+// Scratch of one warp
+struct CoopWarp {
+  float4 pos[32];            // query point and type; then its sum (s, c, sum of |terms|)
+  int2 st[32];               // first row (cy | cz << 16), rows per slab | slabs << 8 | full y, z << 16
+  float q[32];               // charge of the query atom
+  int own[32];               // owner lane | atom << 8
+  int ov[32];                // core overlap met
+  float2 part[kCoopItems];   // partial sum (s, c) of a (query, row)
+  float pabs[kCoopItems];    // its sum of |terms|
+  float2 hit[kCoopHits][32]; // r^2 and box atom of the listed pairs of a lane
+  int nband[32];             // band pairs met by an owner's full-cutoff pass
+  BandPair band[kCoopBand];  // the noted ones; pad0: owner lane
+  int nnote;
+};
+
+// cells of dimension d within rc of p, as a query's stencil spans them
+__device__ __forceinline__ void stencil_f(const BoxF& f, int d, float p, float rc, int& lo, int& n, bool& full) {
+  const float w = fminf(rc * f.cinv[d], 1.0e5f);
+  const float ul = fminf(fmaxf((p + f.hL[d]) * f.cinv[d] - w - 1e-3f, -1.0e6f), 1.0e6f);
+  const float uh = fminf(fmaxf((p + f.hL[d]) * f.cinv[d] + w + 1e-3f, -1.0e6f), 1.0e6f);
+  const int l = (int)floorf(ul), h = (int)floorf(uh);
+  full = h - l + 1 >= f.nc[d];
+  lo = full ? 0 : l;
+  n = full ? f.nc[d] : h - l + 1;
+}
+
+// Neighbour lists on a grid of voxels: the atoms within the query radius plus half
+// a voxel diagonal of a voxel's centre, so every query point in the voxel reads one
+// contiguous list instead of the rows of a cell stencil (27 entries for 13 atoms
+// within 6.5 A of the benchmark's fluid, against 65 visited through the cells).  An
+// entry holds the atom and its periodic image.  The atoms that may lie within
+// rcut_low come first.
+struct VoxGrid {
+  int nv[3];
+  float inv[3];    // voxels per A
+  float edge[3];
+  float R2;        // list radius squared, about the voxel centre
+  float near2;     // squared radius of the atoms that come first
+  int off;         // first record of the box
+  int on;
+};
+constexpr unsigned kVoxAtomBits = 17;
+constexpr unsigned kVoxAtomMask = (1u << kVoxAtomBits) - 1u;
+
+// Dynamic shared memory of a CTA: the head, one CoopWarp per warp, then (with
+// SMEM) the box's cell starts and atoms at the offsets of its CoopBox.
+struct CoopHead {
+  BoxF f;
+  VoxGrid vox[2];                     // neighbour lists of the CBMC and the full-cutoff radius
+  float4 shift[125];                  // (sx Lx, sy Ly, sz Lz) at 62 + sx + 5 sy + 25 sz
+  float2 ljp[kMaxTypes * kMaxTypes];  // (eps, sigma^2)
+  double ec;
+  int atom_off, cell_off, natoms;
+  int rows_cbmc, rows_full;  // row slots of a query of either radius
+};
+struct CoopBox {
+  const uint4* vrec;    // voxel records of the batch: first word of the list, near entries, entries
+  const uint4* vlist;   // their entries, four to a word
+  const float4* p32;  // global (SMEM false)
+  const float* q32;
+  const int* cstart;
+  unsigned off_cells, off_atoms;
+};
+extern __shared__ __align__(32) unsigned char smem[];
+__device__ __forceinline__ CoopHead& coop_head() { return *reinterpret_cast<CoopHead*>(smem); }
+constexpr unsigned kCoopHeadBytes = (sizeof(CoopHead) + 31) & ~31u;
+__device__ __forceinline__ CoopWarp& coop_warp() {
+  return reinterpret_cast<CoopWarp*>(smem + kCoopHeadBytes)[threadIdx.x >> 5];
+}
+
+// most cells a stencil of radius rc spans in dimension d
+__device__ __forceinline__ int stencil_max(const BoxF& f, int d, float rc) {
+  return min(f.nc[d], (int)floorf(fminf(2.0f * rc * f.cinv[d], 1.0e5f) + 4.0e-3f) + 2);
+}
+
+// a band pair of owner lane `own`, atom `atom` noted in W (all lanes of a warp may call it at once)
+__device__ __forceinline__ void coop_note(CoopWarp& W, int own, int j, float r2, int kind) {
+  const int lane = own & 0xff;
+  if (atomicAdd(&W.nband[lane], 1) >= kMaxBand) return;
+  const int s = atomicAdd(&W.nnote, 1);
+  if (s < kCoopBand) W.band[s] = BandPair{j, r2, (unsigned char)(own >> 8), (unsigned char)kind, (unsigned char)lane, 0};
+  else atomicAdd(&W.nband[lane], kMaxBand);  // no room: k_widom_fix redoes the pass
+}
+
+// The energies of the nq queries of W (pos, q, own, st filled, ov cleared): sums
+// left in pos, overlaps in ov.  rows: row slots per query.  DETECT: the
+// full-cutoff pass with its band notes; OPT: a CBMC query with the CBMC options.
+template <bool SMEM, bool COUNT, bool OPT, bool DETECT>
+__device__ __noinline__ void coop_eval(const CoopBox B, int nq, bool want_qq, QueryAcc& cnt) {
+  const CoopHead& H = coop_head();
+  const BoxF& f = H.f;
+  CoopWarp& W = coop_warp();
+  const float4* p32;
+  const int* cstart;
+  if constexpr (SMEM) {
+    p32 = reinterpret_cast<const float4*>(smem + B.off_atoms);
+    cstart = reinterpret_cast<const int*>(smem + B.off_cells);
+  } else {
+    p32 = B.p32;
+    cstart = B.cstart;
+  }
+  const int rows = DETECT ? H.rows_full : H.rows_cbmc;
+  const int lane = threadIdx.x & 31;
+  const float rc = DETECT ? f.rc_full : f.rc_cbmc;
+  const float rv2 = DETECT ? f.rv2 : f.rcb2;
+  const float rq2 = DETECT ? f.rq2 : f.rcb2;
+  const float rc2 = rc * rc;
+  const int nc0 = f.nc[0], nc1 = f.nc[1], nc2 = f.nc[2];
+  const int rs = min(rows, kCoopItems);
+  const int nbatch = kCoopItems / rs;  // queries of a batch
+  const float inv_rs = 1.0f / (float)rs;
+  for (int q0 = 0; q0 < nq; q0 += nbatch) {
+    const int nb = min(nbatch, nq - q0);
+    for (int base = 0; base < nb * rs; base += 32) {
+      const int item = base + lane;
+      const bool valid = item < nb * rs;
+      const int ql = valid ? (int)(((float)item + 0.5f) * inv_rs) : 0;
+      const int qi = q0 + ql, slot = item - ql * rs;
+      const float4 p = W.pos[qi];
+      const int2 st = W.st[qi];
+      const int ta = __float_as_int(p.w);
+      const float qa = W.q[qi];
+      const bool vdw_on = ta >= 0;
+      const bool qq_on = want_qq && f.charge_on && qa != 0.0f;
+      const float band = DETECT ? fmaxf(vdw_on ? f.band_v : 0.0f, qq_on ? f.band_q : 0.0f) : 0.0f;
+      const float rsel2 = fmaxf(vdw_on ? rv2 : -1.0f, qq_on ? rq2 : -1.0f) + band;
+      const float low2q = DETECT ? f.low2 + f.band_low : f.low2;
+      const float rlo = fminf(vdw_on ? rv2 : 3.0e38f, qq_on ? rq2 : 3.0e38f) - band;
+      const float2* lrow = H.ljp + (vdw_on ? ta : 0) * kMaxTypes;
+      const float* rmrow = f.rmin2 + (vdw_on ? ta : 0) * kMaxTypes;
+      const float qicf = qa * (float)kCHARGE_FACTOR;
+      const int ny = st.y & 0xff, nrow = ny * ((st.y >> 8) & 0xff);
+      const bool fully = (st.y >> 16) & 1, fullz = (st.y >> 17) & 1;
+      const int lo1 = (int)(short)(st.x & 0xffff), lo2 = st.x >> 16;
+      KahanF e;
+      float eabs = 0.0f;
+      bool ov = false;
+      int nh = 0;
+      // energies of the listed pairs
+      auto drain = [&]() {
+        const int most = __reduce_max_sync(0xffffffffu, nh);
+        for (int h = 0; h < most; ++h)
+          if (h < nh) {
+            const float2 hv = W.hit[h][lane];
+            const int j = __float_as_int(hv.y);
+            const float r2 = hv.x;
+            if (DETECT && r2 >= rlo) coop_note(W, W.own[qi], j, r2, 0);
+            if (COUNT) ++cnt.in_cut;
+            const int tj = __float_as_int(p32[j].w);
+            if (vdw_on && tj >= 0 && r2 <= rv2) {
+              const float2 es = lrow[tj];
+              const float ev = lj_pair_f(es.x, es.y, r2);
+              e.add(ev);
+              eabs += fabsf(ev);
+            }
+            if (qq_on && r2 <= rq2) {
+              const float eq = qq_ewald_inter_f(f.alpha, qa * B.q32[j], r2);
+              e.add(eq);
+              eabs += fabsf(eq);
+            }
+          }
+        nh = 0;
+      };
+      const int turns = (rows + rs - 1) / rs;  // one, but for stencils of more rows than a batch holds
+      for (int turn = 0; turn < turns; ++turn) {
+        const int rr = slot + turn * rs;
+        // the row's candidates: up to two runs of cells, the second beyond the box edge
+        int ja = 0, na = 0, jb = 0, n = 0;
+        float qxa = 0.0f, qxb = 0.0f, qy = 0.0f, qz = 0.0f;
+        bool fl[3] = {false, fully, fullz};
+        if (valid && rr < nrow && !ov && !W.ov[qi]) {
+          const int iz = (int)(((float)rr + 0.5f) * (1.0f / (float)ny));
+          const int cz = lo2 + iz, cy = lo1 + rr - iz * ny;
+          const float dz2 = fullz ? 0.0f : slab_d2_f(cz, f.ch[2], f.hL[2], p.z);
+          const float d2 = fully ? dz2 : dz2 + slab_d2_f(cy, f.ch[1], f.hL[1], p.y);
+          if (dz2 <= rc2 && d2 <= rc2) {
+            const int sz = cell_image(cz, nc2), sy = cell_image(cy, nc1);
+            qz = p.z + (float)sz * f.L[2];
+            qy = p.y + (float)sy * f.L[1];
+            int xlo, xhi;
+            row_x_cells_f(f, p.x, rc2 - d2, xlo, xhi, fl[0]);
+            const int* cs = cstart + ((cz + sz * nc2) * nc1 + cy + sy * nc1) * nc0;
+            const int sx = cell_image(xlo, nc0);
+            const int wx = xlo + sx * nc0;
+            const int run = min(xhi - xlo, nc0 - 1 - wx) + 1;
+            qxa = p.x + (float)sx * f.L[0];
+            ja = cs[wx];
+            n = na = cs[wx + run] - ja;
+            if (xlo + run <= xhi) {
+              qxb = p.x + (float)(sx - 1) * f.L[0];
+              jb = cs[0];
+              n += cs[xhi + (sx - 1) * nc0 + 1] - jb;
+            }
+            if (COUNT) cnt.visited += (unsigned long long)n;
+          }
+        }
+        const bool fold_any = fl[0] || fl[1] || fl[2];
+        const int most = __reduce_max_sync(0xffffffffu, n);
+        jb -= na;
+        for (int t = 0; t < most; t += 2) {
+          if (t < n) {
+            const bool two = t + 1 < n;
+            const int j0 = t < na ? ja + t : jb + t, j1 = two ? (t + 1 < na ? ja + t + 1 : jb + t + 1) : j0;
+            const float4 a0 = p32[j0], a1 = p32[j1];
+            const float qx0 = t < na ? qxa : qxb, qx1 = t + 1 < na ? qxa : qxb;
+            float r20, r21;
+            if (!fold_any) {
+              const float2 r2 = pair_r2_x2(qx0, qx1, qy, qz, a0, a1);
+              r20 = r2.x;
+              r21 = r2.y;
+            } else {
+              r20 = pair_r2(f, fl, fold_any, qx0, qy, qz, a0);
+              r21 = pair_r2(f, fl, fold_any, qx1, qy, qz, a1);
+            }
+            if (!two) r21 = 3.0e38f;
+            if (OPT) {
+              for (int s = 0; s < 2 && !ov; ++s) {
+                if (s == 1 && !two) break;
+                const float r2 = s ? r21 : r20;
+                const int j = s ? j1 : j0, tj = __float_as_int(s ? a1.w : a0.w);
+                if (f.sector && r2 < (vdw_on && tj >= 0 ? rmrow[tj] : f.low2)) {
+                  ov = true;
+                } else if (f.tab_res > 0) {
+                  float et = 0.0f;
+                  const int k = table_pair_f(f.tab_v, f.tab_f2, f.tab_res, f.tab_shift, f.tab_rcs, f.tab_step,
+                                             f.tab_inv_step, f.ntypes, r2, ta, tj, qicf, qq_on ? B.q32[j] : 0.0f, et);
+                  if (k == 2) ov = true;
+                  if (k == 1) {
+                    e.add(et);
+                    eabs += fabsf(et);
+                  }
+                } else if (r2 < f.low2) {
+                  ov = true;
+                } else if (r2 <= rsel2) {
+                  W.hit[nh++][lane] = make_float2(r2, __int_as_float(j));
+                }
+              }
+            } else {
+              if (fminf(r20, r21) < low2q) {
+                if (!DETECT || fminf(r20, r21) < f.low2 - f.band_low) {
+                  ov = true;
+                } else {
+                  if (r20 < low2q) coop_note(W, W.own[qi], j0, r20, 1);
+                  if (r21 < low2q) coop_note(W, W.own[qi], j1, r21, 1);
+                }
+              }
+              if (r20 <= rsel2) W.hit[nh++][lane] = make_float2(r20, __int_as_float(j0));
+              if (r21 <= rsel2) W.hit[nh++][lane] = make_float2(r21, __int_as_float(j1));
+            }
+            if (ov) {  // the query's energy is not asked for any more
+              n = 0;
+              nh = 0;
+            }
+          }
+          if (__any_sync(0xffffffffu, nh > kCoopHits - 2)) drain();
+        }
+      }
+      if (ov) W.ov[qi] = 1;
+      __syncwarp();
+      if (W.ov[qi]) nh = 0;
+      drain();
+      if (valid) {
+        W.part[item] = make_float2(e.s, e.c);
+        if (DETECT) W.pabs[item] = eabs;
+      }
+    }
+    __syncwarp();
+    if (lane < nb) {  // the rows of a query added in their order
+      KahanF e;
+      float ea = 0.0f;
+      for (int s = 0; s < rs; ++s) {
+        const float2 v = W.part[lane * rs + s];
+        e.add(v.x);
+        e.c += v.y;
+        if (DETECT) ea += W.pabs[lane * rs + s];
+      }
+      W.pos[q0 + lane] = make_float4(e.s, e.c, ea, 0.0f);
+    }
+    __syncwarp();
+  }
+}
+
+// the voxel record of point (x, y, z), which is moved by whole box edges where it
+// lies beyond the neighbouring images; code: its own image shift as an entry has it
+__device__ __forceinline__ uint4 vox_record(const BoxF& f, const VoxGrid& g, const uint4* vrec, float& x, float& y,
+                                            float& z, int& code) {
+  float p[3] = {x, y, z};
+  int w[3], s[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const float w = fminf(rc * f.cinv[d], 1.0e5f);
-    const float ul = fminf(fmaxf((p[d] + f.hL[d]) * f.cinv[d] - w - 1e-3f, -1.0e6f), 1.0e6f);
-    const float uh = fminf(fmaxf((p[d] + f.hL[d]) * f.cinv[d] + w + 1e-3f, -1.0e6f), 1.0e6f);
-    const int l = (int)floorf(ul), h = (int)floorf(uh);
-    full[d] = h - l + 1 >= f.nc[d];
-    lo[d] = full[d] ? 0 : l;
-    hi[d] = full[d] ? f.nc[d] - 1 : h;
+    const int i = (int)floorf(fminf(fmaxf((p[d] + f.hL[d]) * g.inv[d], -1.0e6f), 1.0e6f));
+    s[d] = cell_image(i, g.nv[d]);
+    w[d] = i + s[d] * g.nv[d];
+    if (s[d] > 1 || s[d] < -1) {
+      p[d] += (float)s[d] * f.L[d];
+      s[d] = 0;
+    }
   }
-  const float rv2 = cbmc ? f.rcb2 : f.rv2;
-  const float rq2 = cbmc ? f.rcb2 : f.rq2;
-  const float low2 = f.low2;
+  x = p[0];
+  y = p[1];
+  z = p[2];
+  code = s[0] + 5 * s[1] + 25 * s[2];
+  return __ldg(&vrec[g.off + (w[2] * g.nv[1] + w[1]) * g.nv[0] + w[0]]);
+}
+
+// Core overlap of a CBMC query point: only the first entries of its list can be that near
+template <bool SMEM>
+__device__ __forceinline__ bool vox_overlap(const CoopBox& B, const CoopHead& H, float x, float y, float z) {
+  const float4* p32;
+  if constexpr (SMEM) p32 = reinterpret_cast<const float4*>(smem + B.off_atoms);
+  else p32 = B.p32;
+  int code;
+  const uint4 rec = vox_record(H.f, H.vox[0], B.vrec, x, y, z, code);
+  const unsigned* list = reinterpret_cast<const unsigned*>(B.vlist + rec.x);
+  const int nnear = (int)rec.y;
+  bool ov = false;
+  for (int t = 0; t < nnear && !ov; ++t) {
+    const unsigned e = __ldg(&list[t]);
+    const float4 a = p32[e & kVoxAtomMask], sh = H.shift[(int)(e >> kVoxAtomBits) + code];
+    const float dx = (x + sh.x) - a.x, dy = (y + sh.y) - a.y, dz = (z + sh.z) - a.z;
+    ov = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < H.f.low2;
+  }
+  return ov;
+}
+
+// coop_eval through the voxel lists: a query per lane, or per 2, 4 ... 32 lanes where
+// the queue is short.  CBMC queries (not DETECT) come without an overlap.
+template <bool SMEM, bool COUNT, bool DETECT>
+__device__ __noinline__ void coop_eval_list(const CoopBox B, int nq, bool want_qq, QueryAcc& cnt) {
+  const CoopHead& H = coop_head();
+  const BoxF& f = H.f;
+  CoopWarp& W = coop_warp();
+  const float4* p32;
+  if constexpr (SMEM) p32 = reinterpret_cast<const float4*>(smem + B.off_atoms);
+  else p32 = B.p32;
+  const int lane = threadIdx.x & 31;
+  const int lb = 5 - (32 - __clz(nq - 1));  // log2 of the lanes per query (nq = 1: 5)
+  const int qi = lane >> lb, sub = lane & ((1 << lb) - 1);
+  const float rv2 = DETECT ? f.rv2 : f.rcb2;
+  const float rq2 = DETECT ? f.rq2 : f.rcb2;
+  const bool valid = qi < nq;
+  const float4 p = W.pos[valid ? qi : 0];
+  const int ta = __float_as_int(p.w);
+  const float qa = W.q[valid ? qi : 0];
   const bool vdw_on = ta >= 0;
   const bool qq_on = want_qq && f.charge_on && qa != 0.0f;
-  // the selection and overlap radii, widened by the FP32 bands in the
-  // kQDetect and kQExact modes; rlo: the lower edge of the cutoff bands
-  const float band = MODE != kQPlain ? fmaxf(vdw_on ? f.band_v : 0.0f, qq_on ? f.band_q : 0.0f) : 0.0f;
+  const float band = DETECT ? fmaxf(vdw_on ? f.band_v : 0.0f, qq_on ? f.band_q : 0.0f) : 0.0f;
   const float rsel2 = fmaxf(vdw_on ? rv2 : -1.0f, qq_on ? rq2 : -1.0f) + band;
-  const float low2q = MODE != kQPlain ? low2 + f.band_low : low2;
+  const float low2q = f.low2 + f.band_low;
   const float rlo = fminf(vdw_on ? rv2 : 3.0e38f, qq_on ? rq2 : 3.0e38f) - band;
-  const float rc2 = rc * rc;
-  const float2* lrow = V.ljp + (vdw_on ? ta : 0) * kMaxTypes;
-  const int nc0 = f.nc[0], nc1 = f.nc[1], nc2 = f.nc[2];
-  for (int cz = lo[2]; cz <= hi[2]; ++cz) {
-    const int sz = cell_image(cz, nc2);
-    const int wz = cz + sz * nc2;
-    const float qz = pz + (float)sz * f.L[2];
-    const float dz2 = full[2] ? 0.0f : slab_d2_f(cz, f.ch[2], f.hL[2], pz);
-    if (dz2 > rc2) continue;
-    for (int cy = lo[1]; cy <= hi[1]; ++cy) {
-      const float d2 = full[1] ? dz2 : dz2 + slab_d2_f(cy, f.ch[1], f.hL[1], py);
-      if (d2 > rc2) continue;
-      int xlo, xhi;
-      bool fl[3] = {false, full[1], full[2]};
-      row_x_cells_f(f, px, rc2 - d2, xlo, xhi, fl[0]);
-      const bool fold_any = fl[0] || fl[1] || fl[2];
-      const int sy = cell_image(cy, nc1);
-      const int wy = cy + sy * nc1;
-      const float qy = py + (float)sy * f.L[1];
-      const int row = (wz * nc1 + wy) * nc0;
-      int cx = xlo;
-      while (cx <= xhi) {
-        const int sx = cell_image(cx, nc0);
-        const int wx = cx + sx * nc0;
-        const int run = min(xhi - cx, nc0 - 1 - wx) + 1;
-        const float qx = px + (float)sx * f.L[0];
-        const int j0 = V.cstart[row + wx], j1 = V.cstart[row + wx + run];
-        if (COUNT) A.visited += (unsigned long long)(j1 - j0);
-        // two candidates per iteration: independent distance chains
-        int j = j0;
-        for (; j + 1 < j1; j += 2) {
-          const float4 a0 = V.p32[j], a1 = V.p32[j + 1];
-          float r20, r21;
-          if (!fold_any) {
-            const float2 r2 = pair_r2_x2(qx, qy, qz, a0, a1);
-            r20 = r2.x;
-            r21 = r2.y;
+  const float2* lrow = H.ljp + (vdw_on ? ta : 0) * kMaxTypes;
+  float x = p.x, y = p.y, z = p.z;
+  int code = 0, n = 0;
+  const uint4* list = B.vlist;
+  if (valid && W.st[qi].y != 1) {  // a slot without an atom has no rows
+    const uint4 rec = vox_record(f, H.vox[DETECT ? 1 : 0], B.vrec, x, y, z, code);
+    list += rec.x;
+    n = (int)rec.z;
+  }
+  // half of the entries lie within the cutoff, so every entry's energy is formed, two
+  // at a time on the packed FP32 pipe, and those outside add zero
+  float2 es = make_float2(0.0f, 0.0f), ec = es;  // compensated sums of the even and the odd entries
+  float eabs = 0.0f;
+  bool ov = false;
+  auto add2 = [&](float2 v) {  // TwoSum: the rounding error of the addition, exactly
+    const float2 t = __fadd2_rn(es, v);
+    const float2 m1 = make_float2(-1.0f, -1.0f);
+    const float2 w = __ffma2_rn(es, m1, t);                      // t - es
+    const float2 d = __fadd2_rn(__ffma2_rn(__ffma2_rn(w, m1, t), m1, es), __ffma2_rn(w, m1, v));
+    ec = __fadd2_rn(ec, d);
+    es = t;
+  };
+  if (COUNT && sub == 0) cnt.visited += (unsigned long long)n;
+  for (int g = sub; 4 * g < n && !ov; g += 1 << lb) {
+    const uint4 E = __ldg(&list[g]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int left = n - 4 * g - 2 * k;
+      if (left <= 0) break;
+      const unsigned e0 = k ? E.z : E.x, e1 = left > 1 ? (k ? E.w : E.y) : e0;
+      const int j0 = (int)(e0 & kVoxAtomMask), j1 = (int)(e1 & kVoxAtomMask);
+      const float4 a0 = p32[j0], a1 = p32[j1];
+      const float4 s0 = H.shift[(int)(e0 >> kVoxAtomBits) + code], s1 = H.shift[(int)(e1 >> kVoxAtomBits) + code];
+      const float2 m1 = make_float2(-1.0f, -1.0f);
+      const float2 dx = __ffma2_rn(make_float2(a0.x, a1.x), m1, __fadd2_rn(make_float2(x, x), make_float2(s0.x, s1.x)));
+      const float2 dy = __ffma2_rn(make_float2(a0.y, a1.y), m1, __fadd2_rn(make_float2(y, y), make_float2(s0.y, s1.y)));
+      const float2 dz = __ffma2_rn(make_float2(a0.z, a1.z), m1, __fadd2_rn(make_float2(z, z), make_float2(s0.z, s1.z)));
+      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+      const bool in0 = r2.x <= rsel2, in1 = left > 1 && r2.y <= rsel2;
+      if (COUNT) cnt.in_cut += (int)in0 + (int)in1;
+      if (DETECT) {
+        const float rmin = fminf(r2.x, left > 1 ? r2.y : r2.x);
+        if (rmin < low2q) {
+          if (rmin < f.low2 - f.band_low) {
+            ov = true;  // a certain overlap
           } else {
-            r20 = pair_r2(f, fl, fold_any, qx, qy, qz, a0);
-            r21 = pair_r2(f, fl, fold_any, qx, qy, qz, a1);
+            if (r2.x < low2q) coop_note(W, W.own[qi], j0, r2.x, 1);
+            if (left > 1 && r2.y < low2q) coop_note(W, W.own[qi], j1, r2.y, 1);
           }
-          if (fminf(r20, r21) < low2q) {
-            if (MODE == kQPlain) return true;
-            if (MODE == kQDetect) {
-              if (fminf(r20, r21) < low2 - f.band_low) return true;  // a certain overlap
-              if (r20 < low2q) band_note(A, j, r20, 1);
-              if (r21 < low2q) band_note(A, j + 1, r21, 1);
-            } else if (overlap_exact(V, r20, j, p64) || overlap_exact(V, r21, j + 1, p64)) {
-              return true;
-            }
-          }
-          if (r20 <= rsel2) pair_energy<COUNT, MODE>(V, A, a0, j, r20, lrow, vdw_on, qq_on, rv2, rq2, qa, rlo, p64);
-          if (r21 <= rsel2) pair_energy<COUNT, MODE>(V, A, a1, j + 1, r21, lrow, vdw_on, qq_on, rv2, rq2, qa, rlo, p64);
         }
-        if (j < j1) {
-          const float4 a0 = V.p32[j];
-          const float r20 = pair_r2(f, fl, fold_any, qx, qy, qz, a0);
-          if (r20 < low2q) {
-            if (MODE == kQPlain) return true;
-            if (MODE == kQDetect) {
-              if (r20 < low2 - f.band_low) return true;
-              band_note(A, j, r20, 1);
-            } else if (overlap_exact(V, r20, j, p64)) {
-              return true;
-            }
-          }
-          if (r20 <= rsel2) pair_energy<COUNT, MODE>(V, A, a0, j, r20, lrow, vdw_on, qq_on, rv2, rq2, qa, rlo, p64);
-        }
-        cx += run;
+        if (in0 && r2.x >= rlo) coop_note(W, W.own[qi], j0, r2.x, 0);
+        if (in1 && r2.y >= rlo) coop_note(W, W.own[qi], j1, r2.y, 0);
+      }
+      if (vdw_on) {
+        const int t0 = __float_as_int(a0.w), t1 = __float_as_int(a1.w);
+        const float2 l0 = lrow[max(t0, 0)], l1 = lrow[max(t1, 0)];
+        float2 ev = make_float2(lj_pair_f(l0.x, l0.y, r2.x), lj_pair_f(l1.x, l1.y, r2.y));
+        if (!(t0 >= 0 && r2.x <= rv2)) ev.x = 0.0f;
+        if (!(t1 >= 0 && left > 1 && r2.y <= rv2)) ev.y = 0.0f;
+        add2(ev);
+        if (DETECT) eabs += fabsf(ev.x) + fabsf(ev.y);
+      }
+      if (qq_on) {
+        float2 eq = make_float2(0.0f, 0.0f);
+        if (r2.x <= rq2) eq.x = qq_ewald_inter_f(f.alpha, qa * B.q32[j0], r2.x);
+        if (left > 1 && r2.y <= rq2) eq.y = qq_ewald_inter_f(f.alpha, qa * B.q32[j1], r2.y);
+        add2(eq);
+        if (DETECT) eabs += fabsf(eq.x) + fabsf(eq.y);
       }
     }
   }
-  return false;
+  KahanF e;
+  e.s = es.x;
+  e.c = ec.x;
+  e.add(es.y);
+  e.c += ec.y;
+  __syncwarp();
+  for (int o = 1 << lb >> 1; o > 0; o >>= 1) {
+    const float s = __shfl_down_sync(0xffffffffu, e.s, o), c = __shfl_down_sync(0xffffffffu, e.c, o);
+    e.add(s);
+    e.c += c;
+    if (DETECT) {
+      eabs += __shfl_down_sync(0xffffffffu, eabs, o);
+      const int other = __shfl_down_sync(0xffffffffu, (int)ov, o);
+      ov = ov || other;
+    }
+  }
+  __syncwarp();
+  if (valid && sub == 0) {
+    W.pos[qi] = make_float4(e.s, e.c, eabs, 0.0f);
+    if (DETECT && ov) W.ov[qi] = 1;
+  }
+  __syncwarp();
+}
+
+// Energy of the atoms ids[0..nat) (own numbers and positions per lane: r, shifted
+// by sx, sy, sz) against the box for every lane that is `on`: added to A, ov set
+// on core overlap.  The lanes' first atoms are queried together, then the next
+// ones of the lanes without an overlap; with few lanes on, several atoms at once.
+template <bool SMEM, bool COUNT, bool OPT, bool DETECT>
+__device__ __forceinline__ void coop_atoms(const CoopBox& B, const SpeciesF& S, bool on, const float* r,
+                                           const int* ids, int nat, float sx, float sy, float sz, bool want_qq,
+                                           QueryAcc& A, bool& ov, QueryAcc& cnt) {
+  const BoxF& f = coop_head().f;
+  CoopWarp& W = coop_warp();
+  const int lane = threadIdx.x & 31;
+  const float rc = DETECT ? f.rc_full : f.rc_cbmc;
+  const bool lists = !OPT && coop_head().vox[DETECT ? 1 : 0].on;
+  on = on && !ov;
+  if (lists && !DETECT && on)  // the trials with a core overlap end here, before their energies
+    for (int i = 0; i < nat && !ov; ++i) {
+      const int at = ids[i];
+      ov = vox_overlap<SMEM>(B, coop_head(), r[3 * at] + sx, r[3 * at + 1] + sy, r[3 * at + 2] + sz);
+    }
+  const int most = __reduce_max_sync(0xffffffffu, on ? nat : 0);
+  for (int i0 = 0; i0 < most;) {
+    const bool mine = on && !ov && i0 < nat;
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (!m) break;
+    const int per = min(32 / __popc(m), most - i0);  // atoms of a lane in this batch
+    const int s0 = __popc(m & ((1u << lane) - 1u)) * per;
+    if (mine)
+      for (int a = 0; a < per; ++a) {
+        const int s = s0 + a;
+        W.ov[s] = 0;
+        W.st[s] = make_int2(0, 1);  // no rows
+        W.pos[s] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(-1));
+        W.q[s] = 0.0f;
+        if (i0 + a < nat) {
+          const int at = DETECT ? i0 + a : ids[i0 + a];
+          const float x = r[3 * at] + sx, y = r[3 * at + 1] + sy, z = r[3 * at + 2] + sz;
+          int lo1 = 0, ny = 0, lo2 = 0, nz = 0;
+          bool fy = false, fz = false;
+          if (!lists) {
+            stencil_f(f, 1, y, rc, lo1, ny, fy);
+            stencil_f(f, 2, z, rc, lo2, nz, fz);
+          }
+          W.pos[s] = make_float4(x, y, z, __int_as_float(S.type[at]));
+          W.st[s] = make_int2((lo1 & 0xffff) | (int)((unsigned)lo2 << 16), ny | nz << 8 | (int)fy << 16 | (int)fz << 17);
+          W.q[s] = S.q[at];
+          W.own[s] = lane | at << 8;
+        }
+      }
+    __syncwarp();
+    if (lists) coop_eval_list<SMEM, COUNT, DETECT>(B, __popc(m) * per, want_qq, cnt);
+    else coop_eval<SMEM, COUNT, OPT, DETECT>(B, __popc(m) * per, want_qq, cnt);
+    if (mine)
+      for (int a = 0; a < per && i0 + a < nat; ++a) {
+        const int s = s0 + a;
+        if (W.ov[s]) ov = true;
+        const float4 v = W.pos[s];
+        A.e.add(v.x);
+        A.e.c += v.y;
+        A.eabs += v.z;
+      }
+    __syncwarp();
+    i0 += per;
+  }
 }
 
 // Record of one insertion (FP32 parts; the full-cutoff energy as a two-term sum)
@@ -1271,27 +1666,16 @@ __device__ inline void replay_molecule_f64(const WidomSpecies& S, const BoxF& f,
   }
 }
 
-// Energy of atoms `ids` against the box: sum into e, true on overlap
-template <bool COUNT, bool OPT>
-__device__ __forceinline__ bool query_atoms_f(const BoxViewF& V, QueryAcc& A, const SpeciesF& S, const float* r,
-                                              const int* ids, int n, float sx, float sy, float sz, bool cbmc,
-                                              bool want_qq) {
-  for (int i = 0; i < n; ++i) {
-    const int a = ids[i];
-    if (query_f<COUNT, OPT>(V, A, r[3 * a] + sx, r[3 * a + 1] + sy, r[3 * a + 2] + sz, S.type[a], S.q[a], cbmc, want_qq))
-      return true;
-  }
-  return false;
-}
-
-// One Widom insertion: Widom_Insert (widom_insert.f90:250-447) with the CBMC
-// growth of Build_Molecule (fragment_growth.f90:120-900) and
-// Fragment_Placement (:1449-2132), in FP32
-template <bool COUNT, bool OPT>
-__device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const BoxViewF& V,
+// One Widom insertion per lane that is `on`: Widom_Insert (widom_insert.f90:
+// 250-447) with the CBMC growth of Build_Molecule (fragment_growth.f90:120-900)
+// and Fragment_Placement (:1449-2132), in FP32.  The whole warp calls it; the
+// neighbour queries are the warp's, everything else is a lane's own.
+template <bool SMEM, bool COUNT, bool OPT>
+__device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const CoopBox& B, bool on,
                                 const float* __restrict__ lib, Lfsr rng, double* xyz_out, QueryAcc& cnt,
                                 FixEntry& fe) {
-  const BoxF& f = *V.f;
+  const CoopHead& H = coop_head();
+  const BoxF& f = H.f;
   const int n = S.natoms;
   RecF out{0, 0, 0, 0, 0, 0.0, 0, 0, false};
   int sel_first = 0;
@@ -1299,7 +1683,7 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
   float r[3 * kMaxAtoms];
   unsigned exist = 0u;
   float ln_pbias = 0.0f;
-  bool cbmc_overlap = false;
+  bool cbmc_overlap = !on;
 
   // Step 1: first fragment and growth order (fragment_growth.f90:218-253, 1317-1446)
   const unsigned v0 = draw_u32(rng);
@@ -1391,9 +1775,8 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
     const float ay = centre_of(draw_u32(rng), f.L[1], f.Llo[1]);
     const float az = centre_of(draw_u32(rng), f.L[2], f.Llo[2]);
     QueryAcc A;
-    bool ov = query_atoms_f<COUNT, OPT>(V, A, SF, r, fa_ids, nfa, ax, ay, az, true, cbmc_qq);
-    cnt.visited += A.visited;
-    cnt.in_cut += A.in_cut;
+    bool ov = false;
+    coop_atoms<SMEM, COUNT, OPT, false>(B, SF, on, r, fa_ids, nfa, ax, ay, az, cbmc_qq, A, ov, cnt);
     const float e = A.e.s + A.e.c;
     ov = ov || e >= f.kmaxE;
     nrg[it] = e;
@@ -1403,7 +1786,7 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
   {
     float lnw = 0.0f;
     const int sel = select_trial_f(ki, nrg, ovm, f.beta, unit_of(draw_u32(rng)), &lnw);
-    if (sel < 0) {
+    if (sel < 0 || !on) {
       cbmc_overlap = true;
     } else {
       ln_pbias = ln_pbias - f.beta * nrg[sel] - lnw;
@@ -1428,23 +1811,25 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
     }
   }
   // Step 5: Fragment_Placement, kappa_dih dihedral trials per fragment
-  if (!cbmc_overlap && norder > 1) {
-    float e_prev = dihedral_f(SF, r, exist);
+  if (S.nfrag > 1) {
+    float e_prev = cbmc_overlap ? 0.0f : dihedral_f(SF, r, exist);
     unsigned placed = 1u << fstart;
     const int kd = S.kappa_dih;
     float dn[kMaxKappa], dd[kMaxKappa];
-    for (int oi = 1; oi < norder && !cbmc_overlap; ++oi) {
-      const int fr = order[oi];
+    for (int oi = 1; oi < S.nfrag; ++oi) {
+      bool grow = !cbmc_overlap && oi < norder;  // this lane places a fragment
+      if (!__any_sync(0xffffffffu, grow)) break;
+      const int fr = order[grow ? oi : 0];
       const int nf = S.frag_natoms[fr];
       const unsigned grown = exist;
       const int nconf = S.nconfig[fr];
-      draw_u32(rng);  // the duplicated draw of fragment_growth.f90:1578,1584
-      const int cf = index_of(draw_u32(rng), nconf);
+      if (grow) draw_u32(rng);  // the duplicated draw of fragment_growth.f90:1578,1584
+      const int cf = grow ? index_of(draw_u32(rng), nconf) : 0;
       float cfg[3 * kMaxAtoms];
       const float* Lf = lib + S.lib_off[fr] + (size_t)cf * nf * 3;
       for (int j = 0; j < nf; ++j) {
         const int a = S.frag_atoms[fr][j];
-        exist |= 1u << a;
+        if (grow) exist |= 1u << a;
         cfg[3 * a] = Lf[3 * j];
         cfg[3 * a + 1] = Lf[3 * j + 1];
         cfg[3 * a + 2] = Lf[3 * j + 2];
@@ -1459,8 +1844,9 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
         }
       }
       if (fc < 0) {  // no placed neighbour: the fragment graph is not connected
-        cbmc_overlap = true;
-        break;
+        if (grow) cbmc_overlap = true;
+        grow = false;
+        fc = fr;
       }
       const int anc_i = S.frag_atoms[fr][0], anc_c = S.frag_atoms[fc][0];
       int ids[kMaxAtoms], nid = 0;
@@ -1501,13 +1887,13 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
         cfg[3 * a + 1] = x * al_i[3] + y * al_i[4] + z * al_i[5];
         cfg[3 * a + 2] = x * al_i[6] + y * al_i[7] + z * al_i[8];
       }
-      const float theta0 = (float)kTWOPI * unit_of(draw_u32(rng));
+      const float theta0 = grow ? (float)kTWOPI * unit_of(draw_u32(rng)) : 0.0f;
       const float dtheta = (float)kTWOPI / (float)kd;
       unsigned dov = 0u;
       for (int ii = 0; ii < kd; ++ii) {
         float sth, cth;
         sincosf(theta0 + (float)ii * dtheta, &sth, &cth);
-        for (int j = 0; j < nid; ++j) {
+        for (int j = 0; grow && j < nid; ++j) {
           const int a = ids[j];
           const float x = cfg[3 * a], y = cfg[3 * a + 1], z = cfg[3 * a + 2];
           const float yr = cth * y + sth * z, zr = -sth * y + cth * z;
@@ -1517,27 +1903,20 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
         }
         dn[ii] = 0.0f;
         dd[ii] = 0.0f;
-        exist &= ~idmask;
         float niv = 0.0f, niq = 0.0f, noq = 0.0f;
-        bool ov = false;
+        bool ov = !grow;
+        if (grow) exist &= ~idmask;
         for (int j = 0; j < nid && !ov; ++j) {
           exist |= 1u << ids[j];
           float eiv, eiq, eoq;
-          ov = atom_intra_f(SF, f, V.ljp, ids[j], r, exist, eiv, eiq, eoq);
+          ov = atom_intra_f(SF, f, H.ljp, ids[j], r, exist, eiv, eiq, eoq);
           niv += eiv;
           niq += eiq;
           noq += eoq;
         }
-        if (ov) {
-          exist = combined;
-          dov |= 1u << ii;
-          continue;
-        }
-        QueryAcc A;
-        ov = query_atoms_f<COUNT, OPT>(V, A, SF, r, newids, nnew, 0.0f, 0.0f, 0.0f, true, cbmc_qq);
-        cnt.visited += A.visited;
-        cnt.in_cut += A.in_cut;
         exist = combined;
+        QueryAcc A;
+        coop_atoms<SMEM, COUNT, OPT, false>(B, SF, grow, r, newids, nnew, 0.0f, 0.0f, 0.0f, cbmc_qq, A, ov, cnt);
         if (!ov) {
           const float ed = dihedral_f(SF, r, exist);
           dd[ii] = ed;
@@ -1547,10 +1926,11 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
         if (ov) dov |= 1u << ii;
       }
       float lnw = 0.0f;
+      if (!grow) continue;
       const int trl = select_trial_f(kd, dn, dov, f.beta, unit_of(draw_u32(rng)), &lnw);
       if (trl < 0) {
         cbmc_overlap = true;
-        break;
+        continue;
       }
       ln_pbias = ln_pbias - f.beta * dn[trl] - lnw;
       float sth, cth;
@@ -1572,30 +1952,38 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
   // widom_insert.f90:350-447
   ln_pbias = ln_pbias + ln_pseq + (float)S.ln_kappa_ins + (float)S.ln_kappa_dih_term;
   out.ln_pbias = ln_pbias;
-  if (cbmc_overlap) {
-    out.status = 1;
-    return out;
-  }
-  if (S.nfrag > 1) {  // Fold_Molecule, orthorhombic branch
+  if (!cbmc_overlap && S.nfrag > 1) {  // Fold_Molecule, orthorhombic branch
     for (int d = 0; d < 3; ++d) {
       const float sh = com[d] > f.hL[d] ? -f.L[d] : (com[d] < -f.hL[d] ? f.L[d] : 0.0f);
       if (sh != 0.0f)
         for (int a = 0; a < n; ++a) r[3 * a + d] += sh;
     }
   }
+  CoopWarp& W = coop_warp();
+  const int lane = threadIdx.x & 31;
+  W.nband[lane] = 0;
+  if (lane == 0) W.nnote = 0;
+  __syncwarp();
   QueryAcc A;
-  A.band = fe.band;
   bool ov = false;
-  for (int a = 0; a < n && !ov; ++a) {
-    A.atom = a;
-    ov = query_f<COUNT, false, kQDetect>(V, A, r[3 * a], r[3 * a + 1], r[3 * a + 2], SF.type[a], SF.q[a], false,
-                                         true);
+  coop_atoms<SMEM, COUNT, false, true>(B, SF, !cbmc_overlap, r, nullptr, n, 0.0f, 0.0f, 0.0f, true, A, ov, cnt);
+  if (cbmc_overlap) {
+    out.status = 1;
+    return out;
   }
-  cnt.visited += A.visited;
-  cnt.in_cut += A.in_cut;
+  A.nband = W.nband[lane];
   if (!ov && A.nband > 0) {  // pairs within FP32 rounding of a cutoff: k_widom_fix decides them in FP64
     out.fix = true;
     fe.nband = A.nband;
+    int nn = 0;  // this insertion's notes, by atom and box atom
+    for (int q = 0; q < min(W.nnote, kCoopBand) && A.nband <= kMaxBand; ++q) {
+      if (W.band[q].pad0 != lane) continue;
+      const BandPair bp = W.band[q];
+      int at = nn++;
+      for (; at > 0 && (fe.band[at - 1].atom > bp.atom || (fe.band[at - 1].atom == bp.atom && fe.band[at - 1].j > bp.j)); --at)
+        fe.band[at] = fe.band[at - 1];
+      fe.band[at] = bp;
+    }
     fe.sel = (unsigned char)sel_first;
     fe.norder = (unsigned char)norder;
     for (int k = 0; k < norder; ++k) {
@@ -1607,7 +1995,7 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
     out.status = 2;
     return out;
   }
-  const IntraF io = molecule_intra_f(SF, f, V.ljp, r);
+  const IntraF io = molecule_intra_f(SF, f, H.ljp, r);
   if (io.overlap) {
     out.status = 3;
     return out;
@@ -1622,12 +2010,11 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
   return out;
 }
 
-// 16 warps per staged box and two CTAs per SM (64 registers): the kernel is
-// latency-bound, and warps per scheduler matter more than the few spills.  The
-// launch autotuner may choose 256-thread CTAs instead (four per SM by
-// registers, fewer by shared memory for large boxes; more CTAs per box).
-constexpr int kF32Threads = 512;
-constexpr int kF32Waves = 8;  // CTAs per resident slot: many short waves even out uneven boxes
+// 24 warps per CTA and one CTA per SM (80 registers), fewer where the staged box and
+// the warps' scratch do not fit together.  On the 64-box butane batch 16, 24 and 32
+// warps take 11.6, 11.5 and 11.3 ms, on 3,000 waters 1.33, 0.81 and 0.85 ms.
+constexpr int kF32Threads = 768;
+constexpr int kF32Waves = 64;  // at most this many CTAs per SM
 
 // FP32 constants of box b (thread 0), the FP64 edges and squared cutoffs
 // and the FP32 error bands of the full-cutoff pass
@@ -1678,60 +2065,165 @@ __device__ inline void widom_ljp(float2* s_ljp, const PairTable& T) {
   }
 }
 
-template <bool SMEM, bool COUNT, bool OPT, int NT = kF32Threads>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_widom_f32(WidomSpecies S, SpeciesF SF, PairTable T, const BoxDev* boxes,
+// The voxel lists of grid `which` (0 CBMC, 1 full) of every box of the batch: a thread
+// per voxel counts its atoms through the cell lists, the CTA takes the room for its
+// voxels' lists in one piece from the cursor, and each thread writes its own (padded
+// to whole words).  Lists stand in no fixed order, the entries of each one do.
+__global__ void __launch_bounds__(128) k_vox_lists(const BoxDev* boxes, const VoxGrid* vox, int which, const float4* c32,
+                                                   const int* cstart, uint4* vrec, unsigned* vlist,
+                                                   unsigned long long* cursor) {
+  __shared__ int warp_sum[4];
+  __shared__ unsigned long long base;
+  const int k = blockIdx.y;
+  const VoxGrid g = vox[2 * k + which];
+  const int nvox = g.nv[0] * g.nv[1] * g.nv[2];
+  if (!g.on || (int)(blockIdx.x * blockDim.x) >= nvox) return;
+  const BoxDev& b = boxes[k];
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = v < nvox;
+  const float R = sqrtf(g.R2);
+  const float4* p32 = c32 + b.atom_off;
+  const int* cs = cstart + b.cell_off + k;
+  float c[3], L[3], hL[3], ci[3], h[3];
+  int lo[3], hi[3], nc[3];
+  const int iv[3] = {v % g.nv[0], v / g.nv[0] % g.nv[1], v / (g.nv[0] * g.nv[1])};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    L[d] = b.Lf[d];
+    nc[d] = b.nc[d];
+    hL[d] = b.hLf[d];
+    ci[d] = (float)b.cell_inv[d];
+    h[d] = L[d] / (float)nc[d];
+    c[d] = ((float)iv[d] + 0.5f) * g.edge[d] - hL[d];
+    lo[d] = (int)floorf((c[d] - R + hL[d]) * ci[d] - 1e-3f);
+    hi[d] = (int)floorf((c[d] + R + hL[d]) * ci[d] + 1e-3f);
+  }
+  int total = 0, nnear = 0;
+  unsigned* out = nullptr;
+  // visits the atoms of the list: fn(atom, code, is near)
+  auto visit = [&](auto fn) {
+    for (int cz = lo[2]; cz <= hi[2]; ++cz) {
+      const int sz = cell_image(cz, nc[2]);
+      const float qz = c[2] + (float)sz * L[2];
+      const float z0 = (float)cz * h[2] - hL[2];
+      const float ez = fmaxf(fmaxf(z0 - c[2], c[2] - (z0 + h[2])) - 1e-3f * h[2], 0.0f);
+      for (int cy = lo[1]; cy <= hi[1]; ++cy) {
+        const float y0 = (float)cy * h[1] - hL[1];
+        const float ey = fmaxf(fmaxf(y0 - c[1], c[1] - (y0 + h[1])) - 1e-3f * h[1], 0.0f);
+        const float rem = g.R2 - ez * ez - ey * ey;
+        if (rem < 0.0f) continue;
+        const int sy = cell_image(cy, nc[1]);
+        const float qy = c[1] + (float)sy * L[1];
+        const int row = ((cz + sz * nc[2]) * nc[1] + cy + sy * nc[1]) * nc[0];
+        const float w = sqrtf(rem);
+        const int xlo = (int)floorf((c[0] - w + hL[0]) * ci[0] - 1e-3f);
+        const int xhi = (int)floorf((c[0] + w + hL[0]) * ci[0] + 1e-3f);
+        for (int cx = xlo; cx <= xhi;) {
+          const int sx = cell_image(cx, nc[0]);
+          const int wx = cx + sx * nc[0], run = min(xhi - cx, nc[0] - 1 - wx) + 1;
+          const float qx = c[0] + (float)sx * L[0];
+          const int code = 62 + sx + 5 * sy + 25 * sz;
+          for (int j = cs[row + wx]; j < cs[row + wx + run]; ++j) {
+            const float4 a = p32[j];
+            const float dx = qx - a.x, dy = qy - a.y, dz = qz - a.z;
+            const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            if (r2 <= g.R2) fn(j, code, r2 <= g.near2);
+          }
+          cx += run;
+        }
+      }
+    }
+  };
+  if (live) visit([&](int, int, bool near) {
+    ++total;
+    nnear += near ? 1 : 0;
+  });
+  const int need = live ? (total + 3) & ~3 : 0;
+  int incl = need;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) warp_sum[w] = incl;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long t = 0;
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += warp_sum[q];
+    base = atomicAdd(cursor, t);
+  }
+  __syncthreads();
+  unsigned long long at = base + (incl - need);
+  for (int q = 0; q < w; ++q) at += warp_sum[q];
+  if (!live) return;
+  vrec[g.off + v] = make_uint4((unsigned)(at >> 2), (unsigned)nnear, (unsigned)total, 0u);
+  out = vlist + at;
+  int first = 0, last = total - 1;
+  visit([&](int j, int code, bool near) { out[near ? first++ : last--] = (unsigned)j | (unsigned)code << kVoxAtomBits; });
+}
+
+// per_warp: insertions a warp works on at a time (a power of two up to 32)
+template <bool SMEM, bool COUNT, bool OPT>
+__global__ void __launch_bounds__(kF32Threads, 1) k_widom_f32(WidomSpecies S, SpeciesF SF, PairTable T, const BoxDev* boxes,
                                                    const int* box_ids, const float4* c32, const float* cq32,
                                                    const int* cstart, const float* __restrict__ libf, long long n_ins,
                                                    uint64_t seed, WRec* rec, signed char* status, double* xyz,
                                                    int want_xyz, CassWidomTrace* trace, FixEntry* fix_q,
-                                                   int* fix_n, double band_scale,
+                                                   int* fix_n, int per_warp,
+                                                   const VoxGrid* vox, const uint4* vrec, const uint4* vlist,
+                                                   double band_scale,
                                                    unsigned long long* pair_counts) {
-  extern __shared__ __align__(32) unsigned char smem[];
-  __shared__ BoxF sf;
-  __shared__ float2 s_ljp[kMaxTypes * kMaxTypes];
-  __shared__ int s_atom_off, s_cell_off, s_natoms;
-  __shared__ double s_ec;
+  CoopHead& H = coop_head();
   const int k = blockIdx.y;
+  const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     const BoxDev& b = boxes[k];
-    widom_boxf(sf, b, band_scale);
-    s_atom_off = b.atom_off;
-    s_cell_off = b.cell_off;
-    s_natoms = b.natoms;
-    s_ec = b.e_inter_constant;
+    widom_boxf(H.f, b, band_scale);
+    H.atom_off = b.atom_off;
+    H.cell_off = b.cell_off;
+    H.natoms = b.natoms;
+    H.ec = b.e_inter_constant;
+    H.rows_cbmc = stencil_max(H.f, 1, H.f.rc_cbmc) * stencil_max(H.f, 2, H.f.rc_cbmc);
+    H.rows_full = stencil_max(H.f, 1, H.f.rc_full) * stencil_max(H.f, 2, H.f.rc_full);
   }
-  if (OPT) boxf_options(sf, boxes[k], T.ntypes);
-  widom_ljp(s_ljp, T);
+  if (OPT) boxf_options(H.f, boxes[k], T.ntypes);
+  widom_ljp(H.ljp, T);
+  if (threadIdx.x < 2) H.vox[threadIdx.x] = vox[2 * k + threadIdx.x];
+  for (int q = threadIdx.x; q < 125; q += blockDim.x)
+    H.shift[q] = make_float4((float)(q % 5 - 2) * (float)boxes[k].L[0], (float)(q / 5 % 5 - 2) * (float)boxes[k].L[1],
+                             (float)(q / 25 - 2) * (float)boxes[k].L[2], 0.0f);
   __syncthreads();
-  const int ncell = sf.nc[0] * sf.nc[1] * sf.nc[2];
-  BoxViewF V;
-  V.f = &sf;
-  V.q32 = cq32 + s_atom_off;
-  V.p64 = nullptr;
-  V.ljp = s_ljp;
+  const int ncell = H.f.nc[0] * H.f.nc[1] * H.f.nc[2];
+  CoopBox B;
+  B.vrec = vrec;
+  B.vlist = vlist;
+  B.q32 = cq32 + H.atom_off;
+  B.p32 = c32 + H.atom_off;
+  B.cstart = cstart + H.cell_off + k;
+  B.off_cells = kCoopHeadBytes + (blockDim.x >> 5) * (unsigned)sizeof(CoopWarp);
+  B.off_atoms = B.off_cells + (((ncell + 1) * (unsigned)sizeof(int) + 31) & ~31u);
   if (SMEM) {
-    int* cs = reinterpret_cast<int*>(smem);
-    for (int c = threadIdx.x; c <= ncell; c += blockDim.x) cs[c] = cstart[s_cell_off + k + c];
-    const size_t off = ((size_t)(ncell + 1) * sizeof(int) + 31) & ~(size_t)31;
-    float4* s32 = reinterpret_cast<float4*>(smem + off);
-    for (int j = threadIdx.x; j < s_natoms; j += blockDim.x) s32[j] = c32[s_atom_off + j];
-    V.p32 = s32;
-    V.cstart = cs;
+    int* cs = reinterpret_cast<int*>(smem + B.off_cells);
+    for (int c = threadIdx.x; c <= ncell; c += blockDim.x) cs[c] = B.cstart[c];
+    float4* s32 = reinterpret_cast<float4*>(smem + B.off_atoms);
+    for (int j = threadIdx.x; j < H.natoms; j += blockDim.x) s32[j] = B.p32[j];
     __syncthreads();
-  } else {
-    V.p32 = c32 + s_atom_off;
-    V.cstart = cstart + s_cell_off + k;
   }
-  const long long stride = (long long)gridDim.x * blockDim.x;
   QueryAcc cnt;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_ins; i += stride) {
+  const long long warps = blockDim.x >> 5;
+  for (long long first = (blockIdx.x * warps + (threadIdx.x >> 5)) * per_warp; first < n_ins;
+       first += gridDim.x * warps * per_warp) {
+    const long long i = first + lane;
+    const bool on = lane < per_warp && i < n_ins;
     const size_t g = (size_t)k * n_ins + i;
     const Lfsr rng = seed_stream(seed, box_ids[k], i);
     FixEntry fe;
-    const RecF o = run_insertion_f<COUNT, OPT>(S, SF, V, libf, rng, want_xyz ? xyz + g * 3 * S.natoms : nullptr,
-                                               cnt, fe);
+    const RecF o = run_insertion_f<SMEM, COUNT, OPT>(S, SF, B, on, libf, rng,
+                                                     want_xyz && on ? xyz + g * 3 * S.natoms : nullptr, cnt, fe);
+    __syncwarp();
+    if (!on) continue;
     const double e_int = o.e_inter;
-    rec[g] = make_double4_32a((double)o.dE_intra, e_int + s_ec, (double)o.dE_frag, (double)o.ln_pbias);
+    rec[g] = make_double4_32a((double)o.dE_intra, e_int + H.ec, (double)o.dE_frag, (double)o.ln_pbias);
     status[g] = (signed char)o.status;
     if (trace) {
       CassWidomTrace& t = trace[g];
@@ -1812,8 +2304,7 @@ __global__ void __launch_bounds__(128) k_widom_fix(WidomSpecies S, SpeciesF SF, 
       QueryAcc A;
       bool ov = false;
       for (int a = 0; a < n && !ov; ++a)
-        ov = query_f<false, false, kQExact>(V, A, r[3 * a], r[3 * a + 1], r[3 * a + 2], SF.type[a], SF.q[a], false,
-                                            true, r64 + 3 * a);
+        ov = query_f_exact(V, A, r[3 * a], r[3 * a + 1], r[3 * a + 2], SF.type[a], SF.q[a], r64 + 3 * a);
       int st = 2;
       double e_int = 0.0, e_abs = 0.0, dE_intra = 0.0, dE_frag = 0.0;
       if (!ov) {
@@ -1888,7 +2379,6 @@ __global__ void __launch_bounds__(128) k_widom(WidomSpecies S, PairTable T, Spec
                                                const double* __restrict__ lib, long long n_ins,
                                                uint64_t seed, WRec* rec, signed char* status, double* xyz,
                                                int want_xyz, CassWidomTrace* trace, unsigned long long* pair_counts) {
-  extern __shared__ __align__(32) unsigned char smem[];
   __shared__ BoxDev sb;
   const int k = blockIdx.y;
   if (threadIdx.x == 0) sb = boxes[k];
@@ -2268,7 +2758,7 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     src[k].p32 = B.d_p32.as<float4>();
     src[k].meta = B.d_meta.as<int4>();
     const size_t sm_cells = ((size_t)(ncell + 1) * sizeof(int) + 31) & ~(size_t)31;
-    max_smem32 = std::max(max_smem32, sm_cells + (size_t)B.npacked * sizeof(float4));
+    max_smem32 = std::max(max_smem32, sm_cells + (size_t)B.npacked * sizeof(float4));  // and the warps' scratch
     max_smem64 = std::max(max_smem64, sm_cells + (size_t)B.npacked * (sizeof(double4_32a) + sizeof(int)));
     max_na = std::max(max_na, B.npacked);
     atom_off += B.npacked;
@@ -2344,7 +2834,7 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   // the box is staged in shared memory when it fits
   SpeciesF SF;
   const bool f32 = mixed && fast_mixed && species_f(s, SF);
-  const size_t max_smem = f32 ? max_smem32 : max_smem64;
+  const size_t max_smem = max_smem64;
   const bool use_smem = max_smem <= (size_t)200 * 1024;
   int dev_sms = 0;
   CASS_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
@@ -2375,31 +2865,119 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   // queued (both inside the kernel timing)
   int* d_fixn = nullptr;
   FixEntry* d_fixq = nullptr;
-  auto launch_f32 = [&](auto kern, const SpeciesF& SF, int nthreads) -> int {
-    int rc2 = c->d_widom_fix.reserve((size_t)nboxes * sizeof(int) + 64 + nrec * sizeof(FixEntry));
+  // Voxel lists: per box and radius, where the query's stencil never spans the box (the
+  // cell search then sees every pair through one image shift, as an entry does) and the
+  // insertions' queries are worth the lists: a list costs about as much as the cell
+  // search of a query, and 32 of an insertion's queries (4 full-cutoff ones) use them
+  std::vector<VoxGrid> vox(2 * nboxes);
+  size_t vox_records = 0;
+  double vox_entries = 0.0;
+  int vox_most[2] = {0, 0};
+  const bool opt_cbmc = c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap;
+  if (f32 && !opt_cbmc && n_ins > 0)
+    for (int k = 0; k < nboxes; ++k) {
+      const BoxDev& b = bd[k];
+      const double rfull2 = std::max(b.rcut_vdwsq, b.rcut_coulsq);
+      // the full-cutoff pass also looks at the pairs of the bands (widom_boxf) outside its cutoffs
+      const double band = 3.5 * std::sqrt(rfull2) * 5.0e-7 * (std::max(b.L[0], std::max(b.L[1], b.L[2])) + 20.0) *
+                              c->widom_band + 1.0e-6 * rfull2;
+      const double rcs[2] = {std::sqrt(b.rcut_cbmcsq), std::sqrt(rfull2 + band)};
+      for (int w = 0; w < 2; ++w) {
+        VoxGrid& g = vox[2 * k + w];
+        memset(&g, 0, sizeof(g));
+        if (b.natoms < 1 || b.natoms > (int)kVoxAtomMask || !(rcs[w] > 0.0)) continue;
+        const double edge = rcs[w] / (w ? kVoxPerCutoffFull : kVoxPerCutoffCbmc);
+        bool open = true;
+        double diag2 = 0.0, nvox = 1.0, most = 1.0;
+        for (int d = 0; d < 3; ++d) {
+          g.nv[d] = (int)std::min(1024.0, std::ceil(b.L[d] / edge));
+          g.inv[d] = (float)(g.nv[d] / b.L[d]);
+          g.edge[d] = (float)(b.L[d] / g.nv[d]);
+          diag2 += (double)g.edge[d] * g.edge[d];
+          nvox *= g.nv[d];
+          open = open && std::floor(2.0 * rcs[w] * b.cell_inv[d] + 8.0e-3) + 2.0 < b.nc[d];
+        }
+        // half a diagonal, with a margin above the FP32 rounding of the coordinates
+        const double lmax = std::max(b.L[0], std::max(b.L[1], b.L[2]));
+        const double half = 0.5 * std::sqrt(diag2) + 2.0e-3 + 4.0e-6 * lmax, R = rcs[w] + half;
+        for (int d = 0; d < 3; ++d) {
+          open = open && R < 0.5 * b.L[d] + 0.25 * rcs[w];
+          most *= 2.0 * (R + half) / g.edge[d] + 1.0;
+        }
+        // entries of an atom: at most the voxels in the sphere of R and another half diagonal
+        const double per_atom = std::min(most, 4.18879021 * std::pow(R + half, 3.0) * nvox / b.volume);
+        const double room = b.natoms * per_atom + 3.0 * nvox;
+        const double rho_list = 4.18879021 * R * R * R * b.natoms / b.volume;
+        if (!open || nvox > 1.0e8 || rho_list > 2.0e4 || (double)n_ins * (w ? 2.0 : 32.0) < nvox ||
+            (vox_entries + room) * sizeof(unsigned) > kVoxMaxBytes)
+          continue;
+        g.R2 = (float)(R * R);
+        const double near = std::sqrt(b.rcut_lowsq) + half;
+        g.near2 = (float)(near * near);
+        g.off = (int)vox_records;
+        g.on = 1;
+        vox_records += (size_t)nvox;
+        vox_entries += room;
+        vox_most[w] = std::max(vox_most[w], (int)nvox);
+      }
+    }
+  // warps per CTA: as many as fit beside the staged box
+  auto smem_f32 = [&](int warps, bool box) { return kCoopHeadBytes + warps * sizeof(CoopWarp) + (box ? max_smem32 : 0); };
+  int warps32 = kF32Threads / 32;
+  while (warps32 > 4 && smem_f32(warps32, true) > kSmemMax) warps32 /= 2;
+  const bool smem32 = smem_f32(warps32, true) <= kSmemMax;
+  if (!smem32) warps32 = kF32Threads / 32;
+  auto launch_f32 = [&](auto kern, const SpeciesF& SF) -> int {
+    const size_t fix_off = ((size_t)nboxes * sizeof(int) + 63) & ~(size_t)63;
+    int rc2 = c->d_widom_fix.reserve(fix_off + 64 + nrec * sizeof(FixEntry));
     if (rc2) return rc2;
     d_fixn = c->d_widom_fix.as<int>();
-    d_fixq = reinterpret_cast<FixEntry*>(c->d_widom_fix.as<unsigned char>() +
-                                         (((size_t)nboxes * sizeof(int) + 63) & ~(size_t)63));
+    d_fixq = reinterpret_cast<FixEntry*>(c->d_widom_fix.as<unsigned char>() + fix_off);
     CASS_CUDA(cudaMemsetAsync(d_fixn, 0, (size_t)nboxes * sizeof(int), c->stream));
-    if (use_smem) CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem));
-    int per_sm = 1;
-    CASS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nthreads, use_smem ? max_smem : 0));
-    per_sm = std::max(per_sm, 1);
-    const int waves = c->widom_waves > 0 ? c->widom_waves : kF32Waves;
-    long long want = ((long long)dev_sms * per_sm * waves + nboxes - 1) / nboxes;
-    long long need = (n_ins + nthreads - 1) / nthreads;
-    int chunks = (int)std::max<long long>(1, std::min(want, need));
+    const size_t vox_head = ((2 * (size_t)nboxes * sizeof(VoxGrid) + sizeof(unsigned long long) + 255) & ~(size_t)255);
+    const size_t vox_rec = (vox_records * sizeof(uint4) + 255) & ~(size_t)255;
+    if (c->d_vox.reserve(vox_head + vox_rec + (size_t)vox_entries * sizeof(unsigned) + 256)) {
+      cudaGetLastError();  // no room for the lists: the cell search serves every query
+      for (VoxGrid& g : vox) g.on = 0;
+      vox_most[0] = vox_most[1] = 0;
+      if ((rc2 = c->d_vox.reserve(vox_head))) return rc2;
+    }
+    unsigned char* vb = c->d_vox.as<unsigned char>();
+    VoxGrid* d_vox = reinterpret_cast<VoxGrid*>(vb);
+    unsigned long long* d_cursor = reinterpret_cast<unsigned long long*>(vb + 2 * (size_t)nboxes * sizeof(VoxGrid));
+    uint4* d_vrec = reinterpret_cast<uint4*>(vb + vox_head);
+    unsigned* d_vlist = reinterpret_cast<unsigned*>(vb + vox_head + vox_rec);
+    CASS_CUDA(h2d(c, d_vox, vox.data(), vox.size() * sizeof(VoxGrid)));
+    CASS_CUDA(cudaMemsetAsync(d_cursor, 0, sizeof(unsigned long long), c->stream));
+    CASS_CUDA(cudaEventRecord(c->ev[1], c->stream));
+    for (int w = 0; w < 2; ++w)
+      if (vox_most[w] > 0) {
+        k_vox_lists<<<dim3((vox_most[w] + 127) / 128, nboxes), 128, 0, c->stream>>>(
+            d_bd, d_vox, w, d_c32, c->d_cell_start.as<int>(), d_vrec, d_vlist, d_cursor);
+        CASS_CUDA(cudaGetLastError());
+        count_launch(c);
+      }
+    const size_t dyn = smem_f32(warps32, smem32);
+    CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    // insertions per warp: as few as give every warp of the GPU work at once, up to one per lane
+    int per_warp = 1;
+    while (per_warp < 32 && (n_ins + per_warp - 1) / per_warp * nboxes > (long long)dev_sms * warps32) per_warp *= 2;
+    // one group of insertions per warp: a CTA is as long as its slowest warp, and the
+    // hardware hands out the CTAs; in very large calls several, to stage the box less often
+    const long long groups = (n_ins + per_warp - 1) / per_warp;
+    const int nthreads = 32 * (int)std::min<long long>(warps32, std::max<long long>(1, (groups * nboxes + dev_sms - 1) / dev_sms));
+    const long long need = (groups + nthreads / 32 - 1) / (nthreads / 32);
+    const long long most = std::max<long long>(1, (long long)dev_sms * kF32Waves / nboxes);
+    const int chunks = (int)std::max<long long>(1, (need + (need + most - 1) / most - 1) / ((need + most - 1) / most));
     dim3 g(chunks, nboxes);
     c->stats.widom_grid_x = chunks;
     c->stats.widom_grid_y = nboxes;
     c->stats.widom_block = nthreads;
-    c->stats.widom_smem_bytes = use_smem ? (int)max_smem : 0;
-    CASS_CUDA(cudaEventRecord(c->ev[1], c->stream));
-    kern<<<g, nthreads, use_smem ? max_smem : 0, c->stream>>>(
+    c->stats.widom_smem_bytes = (int)dyn;
+    kern<<<g, nthreads, dyn, c->stream>>>(
         S, SF, c->pt, d_bd, d_ids, d_c32, c->d_cq32.as<float>(), c->d_cell_start.as<int>(), s.d_library_f.as<float>(),
-        (long long)n_ins, seed, d_rec, d_status, d_xyz, any_recip ? 1 : 0, d_trace, d_fixq, d_fixn, c->widom_band,
-        d_pairs);
+        (long long)n_ins, seed, d_rec, d_status, d_xyz, any_recip ? 1 : 0, d_trace, d_fixq, d_fixn, per_warp,
+        d_vox, d_vrec, reinterpret_cast<const uint4*>(d_vlist), c->widom_band, d_pairs);
     CASS_CUDA(cudaGetLastError());
     // one thread per queued insertion, the grid sized for 3 % of the
     // insertions (one to two per cent are queued; a longer queue is strided)
@@ -2415,12 +2993,9 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   };
   if (n_ins > 0) {
     const bool opt = c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap;  // no pair counts with options
-    const int nt = opt || d_pairs ? kF32Threads : (c->widom_threads == 256 ? 256 : kF32Threads);
-    if (f32 && opt) rc = use_smem ? launch_f32(k_widom_f32<true, false, true>, SF, nt) : launch_f32(k_widom_f32<false, false, true>, SF, nt);
-    else if (f32 && d_pairs) rc = use_smem ? launch_f32(k_widom_f32<true, true, false>, SF, nt) : launch_f32(k_widom_f32<false, true, false>, SF, nt);
-    else if (f32 && nt == 256)
-      rc = use_smem ? launch_f32(k_widom_f32<true, false, false, 256>, SF, nt) : launch_f32(k_widom_f32<false, false, false, 256>, SF, nt);
-    else if (f32) rc = use_smem ? launch_f32(k_widom_f32<true, false, false>, SF, nt) : launch_f32(k_widom_f32<false, false, false>, SF, nt);
+    if (f32 && opt) rc = smem32 ? launch_f32(k_widom_f32<true, false, true>, SF) : launch_f32(k_widom_f32<false, false, true>, SF);
+    else if (f32 && d_pairs) rc = smem32 ? launch_f32(k_widom_f32<true, true, false>, SF) : launch_f32(k_widom_f32<false, true, false>, SF);
+    else if (f32) rc = smem32 ? launch_f32(k_widom_f32<true, false, false>, SF) : launch_f32(k_widom_f32<false, false, false>, SF);
     else rc = use_smem ? launch(k_widom<true>) : launch(k_widom<false>);
     if (rc) return rc;
     if (any_recip) {
@@ -2481,52 +3056,37 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   return CASS_OK;
 }
 
-// The launch-shape autotuner: the first call with a new batch signature
-// (species, boxes, precision, CBMC options, order of magnitude of the insertion
-// count) times the Widom kernel with each candidate cell edge on a sample of the
-// insertions with its own seed (the faster of two runs after a first that sizes
-// the buffers), keeps the fastest
-// for the context, and then runs the call.  A shape changes neither the
-// insertions' random streams nor the per-box sums (fixed order over
-// insertions); the cell edge changes only the order of each query's pair sum.
+// The cell-edge autotuner of the FP64 kernel: the first call with a new batch
+// signature (species, boxes, CBMC options, order of magnitude of the insertion count)
+// times the kernel with each candidate edge on a sample of the insertions with its own
+// seed (the faster of two runs after a first that sizes the buffers), keeps the faster
+// one for the context, and then runs the call.  The edge changes neither the
+// insertions' random streams nor the per-box sums (fixed order over insertions), only
+// the order of each query's pair sum.  The mixed kernel has one shape: its queries
+// hardly use the cells, and the lists' own edge does not matter within a tenth.
 extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
                                  int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
                                  CassWidomTrace* trace) {
-  if (!c || !iboxes || nboxes < 1 || !out || n_ins < 64 || !c->widom_autotune || c->widom_cells > 0.0 ||
-      c->widom_waves > 0 || c->widom_threads > 0)
+  if (!c || c->precision == CASS_PREC_MIXED || !iboxes || nboxes < 1 || !out || n_ins < 64 || !c->widom_autotune ||
+      c->widom_cells > 0.0)
     return widom_insert_impl(c, is1, nboxes, iboxes, n_ins, kappa_ins, kappa_dih, seed, out, trace);
   std::vector<long long> key = {is1, c->precision, kappa_ins, kappa_dih, c->cbmc_opt.energy_table_res,
                                 c->cbmc_opt.sector_overlap, (long long)std::log2((double)n_ins)};
   for (int k = 0; k < nboxes; ++k) key.push_back(iboxes[k]);
-  auto run_with = [&](const cass_ctx_impl::WidomShape& sh, int64_t n, uint64_t sd, CassWidomResult* o,
-                      CassWidomTrace* tr) {
-    c->widom_cells = sh.cells;
-    c->widom_waves = sh.waves;
-    c->widom_threads = sh.threads;
+  auto run_with = [&](double cells, int64_t n, uint64_t sd, CassWidomResult* o, CassWidomTrace* tr) {
+    c->widom_cells = cells;
     const int rc = widom_insert_impl(c, is1, nboxes, iboxes, n, kappa_ins, kappa_dih, seed ^ sd, o, tr);
     c->widom_cells = 0.0;
-    c->widom_waves = 0;
-    c->widom_threads = 0;
     return rc;
   };
   for (const auto& e : c->widom_tuned)
     if (e.first == key) return run_with(e.second, n_ins, 0, out, trace);
-  const bool mixed = c->precision == CASS_PREC_MIXED;
-  // candidate shapes: the cell edge (cells per rcut_cbmc) and, for the FP32
-  // kernel, the CTA size (512 threads two per SM, or 256 threads)
-  std::vector<cass_ctx_impl::WidomShape> shapes;
-  if (mixed)
-    for (int nt : {512, 256})
-      for (double cc : {1.0, 1.25}) shapes.push_back({cc, kF32Waves, nt});
-  else
-    for (double cc : {3.0, 4.0}) shapes.push_back({cc, kF32Waves, 512});
-  // the CTAs per box follow the insertion count, so the mixed kernel is timed at
-  // the call's own count (up to 32,768 per box); the FP64 kernel on 4,096
-  const int64_t sample = std::min<int64_t>(n_ins, mixed ? 32768 : 4096);
+  const double shapes[] = {3.0, 4.0};  // cells per rcut_cbmc
+  const int64_t sample = std::min<int64_t>(n_ins, 4096);
   std::vector<CassWidomResult> tmp(nboxes);
-  cass_ctx_impl::WidomShape best = shapes[0];
+  double best = shapes[0];
   float best_ms = -1.0f;
-  for (const auto& sh : shapes) {
+  for (double sh : shapes) {
     float ms = 0.0f;
     for (int rep = 0; rep < 3; ++rep) {  // the first run of a shape also sizes its buffers
       const int rc = run_with(sh, sample, 0x5bd1e995ULL, tmp.data(), nullptr);

@@ -94,35 +94,57 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return v;  // valid in thread 0
 }
 
+// NV block sums at once (their chains overlap), valid in thread 0
+template <int NV>
+__device__ __forceinline__ void block_sums(double (&v)[NV], double (*sh)[NV]) {
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+  __syncthreads();
+  if (l == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh[w][k] = v[k];
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = l < nw ? sh[l][k] : 0.0;
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+  }
+}
+
 // Writes NV partial sums of this block, then the last block to finish sums
 // all partials (fixed order) into out[0..NV).  counter must start at 0 and is
 // reset by the last block.
 template <int NV>
-__device__ void reduce_partials(double (&v)[NV], double* partial, unsigned* counter, double* out, int* flag_in,
-                                int flag_val) {
-  __shared__ double sh[32];
+__device__ void reduce_partials(double (&v)[NV], double* partial, unsigned* counter, double* out) {
+  __shared__ double sh[32][NV];
   __shared__ bool last;
-  int nb = gridDim.x * gridDim.y;
-  int bid = blockIdx.y * gridDim.x + blockIdx.x;
-  for (int k = 0; k < NV; ++k) {
-    double s = block_sum(v[k], sh);
-    if (threadIdx.x == 0) partial[(size_t)bid * NV + k] = s;
+  const int nb = gridDim.x * gridDim.y;
+  const int bid = blockIdx.y * gridDim.x + blockIdx.x;
+  block_sums<NV>(v, sh);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) partial[(size_t)bid * NV + k] = v[k];
+    __threadfence();
+    last = (atomicAdd(counter, 1u) == (unsigned)(nb - 1));
   }
-  (void)flag_in;
-  (void)flag_val;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(counter, 1u) == (unsigned)(nb - 1));
   __syncthreads();
   if (!last) return;
   __threadfence();
-  for (int k = 0; k < NV; ++k) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) s += __ldcg(&partial[(size_t)b * NV + k]);
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) out[k] = s;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  for (int b = threadIdx.x; b < nb; b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] += __ldcg(&partial[(size_t)b * NV + k]);
+  block_sums<NV>(v, sh);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = v[k];
+    *counter = 0u;
   }
-  if (threadIdx.x == 0) *counter = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -182,7 +204,7 @@ __global__ void __launch_bounds__(kBlock) k_mol_inter(BoxDev b, PairTable t, con
   }
   if (ov) atomicOr(ovflag, 1);
   double v[2] = {ev + fv.value(), eq + fq.value()};
-  reduce_partials<2>(v, partial, counter, out, nullptr, 0);
+  reduce_partials<2>(v, partial, counter, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -264,30 +286,22 @@ __global__ void __launch_bounds__(kBlock) k_trial_energy(BoxDev b, PairTable t, 
 
 // ---------------------------------------------------------------------------
 // K6a: all inter-molecular pairs of a box (pairs (i,j), j > i, different
-// molecules).  Block (x, y) takes atoms i of row block x against the j tile y,
-// staged in shared memory.  FAST (mixed precision, LJ cut / cut_tail with no
-// charges or Ewald): FP32 minimum image, r^2 and pair energies with
-// compensated FP32 sums; otherwise the FP64 pair functions.
+// molecules).
+//
+// k_pair_total (mixed precision, LJ cut / cut_tail with no charges or Ewald):
+// block (x, y) takes atoms i of row block x against the j tile y, staged in shared
+// memory, with FP32 minimum image, r^2 and pair energies and compensated FP32 sums.
 constexpr int kTileJ = 512;
 
-template <bool FAST>
-// pre2 (FP64 kernel): an FP32 bound on r^2 beyond every cutoff of the box with
-// a margin far above FP32 rounding; pairs past it skip the FP64 arithmetic,
-// which decides every cutoff exactly (FLT_MAX where a style has no cutoff)
-// com (FP64 kernel, may be NULL): per-atom molecule COM records for
-// Check_MoleculePair_Cutoff with radius rmax
 __global__ void __launch_bounds__(kBlock) k_pair_total(BoxDev b, PairTable t, const double4_32a* __restrict__ p64,
-                                                       const int4* __restrict__ meta, int n, float pre2,
-                                                       const double4_32a* __restrict__ com, double rmax,
-                                                       double* partial, unsigned* counter, double* out, int* ovflag) {
-  __shared__ double4_32a sj[FAST ? 1 : kBlock];
+                                                       const int4* __restrict__ meta, int n, double* partial,
+                                                       unsigned* counter, double* out, int* ovflag) {
   __shared__ float4 sf[kBlock];
   __shared__ int2 sm[kBlock];  // molecule slot, type
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const double4_32a pi = i < n ? p64[i] : make_double4_32a(0, 0, 0, 0);
   const int4 mi = i < n ? meta[i] : make_int4(-1, -1, -1, -1);
   const float4 pif = make_float4((float)pi.x, (float)pi.y, (float)pi.z, (float)pi.w);
-  double ev = 0.0, eq = 0.0;
   KahanF fv, fq;
   bool ov = false;
   const int j0 = blockIdx.y * kTileJ;
@@ -297,13 +311,12 @@ __global__ void __launch_bounds__(kBlock) k_pair_total(BoxDev b, PairTable t, co
   const float alphaf = (float)b.alpha;
   const bool qq_on = b.charge_style == CASS_CHARGE_COUL;
   float eps_row[kMaxTypes], sig_row[kMaxTypes];
-  if (FAST)
 #pragma unroll
-    for (int q = 0; q < kMaxTypes; ++q) {
-      const bool ok = mi.y >= 0 && q < t.ntypes;
-      eps_row[q] = ok ? t.epsf[pidx(mi.y, q, t.ntypes)] : 0.0f;
-      sig_row[q] = ok ? t.sig2f[pidx(mi.y, q, t.ntypes)] : 0.0f;
-    }
+  for (int q = 0; q < kMaxTypes; ++q) {
+    const bool ok = mi.y >= 0 && q < t.ntypes;
+    eps_row[q] = ok ? t.epsf[pidx(mi.y, q, t.ntypes)] : 0.0f;
+    sig_row[q] = ok ? t.sig2f[pidx(mi.y, q, t.ntypes)] : 0.0f;
+  }
   if (j1 > ilo + 1) {
     for (int jt = max(j0, ilo); jt < j1; jt += kBlock) {
       __syncthreads();
@@ -312,7 +325,6 @@ __global__ void __launch_bounds__(kBlock) k_pair_total(BoxDev b, PairTable t, co
         const double4_32a pj = p64[jj];
         const int4 mj = meta[jj];
         sf[threadIdx.x] = make_float4((float)pj.x, (float)pj.y, (float)pj.z, (float)pj.w);
-        if (!FAST) sj[threadIdx.x] = pj;
         sm[threadIdx.x] = make_int2(mj.x, mj.y);
       }
       __syncthreads();
@@ -323,54 +335,140 @@ __global__ void __launch_bounds__(kBlock) k_pair_total(BoxDev b, PairTable t, co
         if (j <= i) continue;
         const int2 mj = sm[k];
         if (mj.x == mi.x) continue;
-        if (FAST) {
-          const float4 pj = sf[k];
-          const float dx = fold(pif.x - pj.x, b.hLf[0], b.Lf[0]);
-          const float dy = fold(pif.y - pj.y, b.hLf[1], b.Lf[1]);
-          const float dz = fold(pif.z - pj.z, b.hLf[2], b.Lf[2]);
-          const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-          if (r2 < low2f) {
-            ov = true;
-            continue;
-          }
-          if (r2 <= rv2f && mj.y >= 0) {
-            float e = 0.0f, s2 = 0.0f;
-#pragma unroll
-            for (int q = 0; q < kMaxTypes; ++q)
-              if (q == mj.y) {
-                e = eps_row[q];
-                s2 = sig_row[q];
-              }
-            fv.add(lj_pair_f(e, s2, r2));
-          }
-          if (qq_on && r2 <= rq2f) fq.add(qq_ewald_inter_f(alphaf, pif.w * pj.w, r2));
-        } else {
-          {
-            const float4 q = sf[k];
-            const float ex = fold(pif.x - q.x, b.hLf[0], b.Lf[0]), ey = fold(pif.y - q.y, b.hLf[1], b.Lf[1]),
-                        ez = fold(pif.z - q.z, b.hLf[2], b.Lf[2]);
-            if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > pre2) continue;
-          }
-          if (com && !molpair_in(b, rmax, com[i], com[j])) continue;
-          const double4_32a pj = sj[k];
-          const double dx = fold(pi.x - pj.x, b.hL[0], b.L[0]);
-          const double dy = fold(pi.y - pj.y, b.hL[1], b.L[1]);
-          const double dz = fold(pi.z - pj.z, b.hL[2], b.L[2]);
-          const double r2 = dx * dx + dy * dy + dz * dz;
-          if (r2 < b.rcut_lowsq) {
-            ov = true;
-            continue;
-          }
-          const int m = cutoff_mask(b, r2, false);
-          if (m & 1) ev += vdw_pair(t, b, mi.y, mj.y, r2, 1.0);
-          if (m & 2) eq += qq_pair_inter(b, pi.w * pj.w, r2);
+        const float4 pj = sf[k];
+        const float dx = fold(pif.x - pj.x, b.hLf[0], b.Lf[0]);
+        const float dy = fold(pif.y - pj.y, b.hLf[1], b.Lf[1]);
+        const float dz = fold(pif.z - pj.z, b.hLf[2], b.Lf[2]);
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        if (r2 < low2f) {
+          ov = true;
+          continue;
         }
+        if (r2 <= rv2f && mj.y >= 0) {
+          float e = 0.0f, s2 = 0.0f;
+#pragma unroll
+          for (int q = 0; q < kMaxTypes; ++q)
+            if (q == mj.y) {
+              e = eps_row[q];
+              s2 = sig_row[q];
+            }
+          fv.add(lj_pair_f(e, s2, r2));
+        }
+        if (qq_on && r2 <= rq2f) fq.add(qq_ewald_inter_f(alphaf, pif.w * pj.w, r2));
       }
     }
   }
   if (ov) atomicOr(ovflag, 1);
-  double v[2] = {ev + fv.value(), eq + fq.value()};
-  reduce_partials<2>(v, partial, counter, out, nullptr, 0);
+  double v[2] = {fv.value(), fq.value()};
+  reduce_partials<2>(v, partial, counter, out);
+}
+
+// k_pair_hits: the same in FP64.  GB300 runs a warp's FP64 instruction in 16 cycles of
+// the SM's unit however many lanes need it, so the FP64 work is done for full warps:
+// lane i of a warp compares its atom with one j after the other in FP32 (pre2: beyond
+// every cutoff by far more than FP32 rounds), the pairs that pass go to a queue, and
+// 32 of them at a time are decided and evaluated in FP64.  Pairs with and without a
+// Lennard-Jones term have a queue each (in water 8 of 9 pairs have none).  A warp takes
+// 32 atoms i against `tiles` tiles of 32 atoms j >= i.
+// 2,250 atoms of water: 2.83 ms with a thread per i and its pairs as they came, 0.14 ms
+// now; 12,288 atoms: 6.3 ms and 0.74 ms.
+constexpr int kPairWarps = 4;
+constexpr int kPairSms = 152;  // the SMs a launch is sized for
+
+__global__ void __launch_bounds__(32 * kPairWarps) k_pair_hits(BoxDev b, PairTable t, const double4_32a* __restrict__ p64,
+                                                               const float4* __restrict__ p32,
+                                                               const int4* __restrict__ meta, int n, int tiles, float pre2,
+                                                               float pre2_none, const double4_32a* __restrict__ com,
+                                                               double rmax, double* partial, unsigned* counter,
+                                                               double* out, int* ovflag) {
+  __shared__ float4 sf[kPairWarps][32];
+  __shared__ unsigned queue[kPairWarps][2][64];  // lane of i << 27 | j, without and with a vdW term
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * 32, i = i0 + lane;
+  const float4 pi = p32[min(i, n - 1)];
+  const int ti = __float_as_int(pi.w);
+  unsigned vdw = 0u;  // types with which this atom has a vdW term
+  if (ti >= 0)
+    for (int q = 0; q < t.ntypes; ++q) vdw |= (t.eps[pidx(ti, q, t.ntypes)] != 0.0) ? 1u << q : 0u;
+  const bool lj = lj_plain_style(b), ewald = b.charge_style == CASS_CHARGE_COUL && b.charge_sum_style == CASS_QQ_EWALD;
+  double ev = 0.0, eq = 0.0;
+  bool ov = false;
+  int cnt[2] = {0, 0};
+  // pair `e` in FP64; V: it may have a vdW term
+  auto pair = [&](unsigned e, bool V) {
+    const int a = i0 + (int)(e >> 27), j = (int)(e & 0x7ffffffu);
+    const int4 ma = meta[a], mj = meta[j];
+    if (ma.x == mj.x) return;
+    if (com && !molpair_in(b, rmax, com[a], com[j])) return;
+    const double4_32a A = p64[a], P = p64[j];
+    const float4 fa = p32[a], fj = p32[j];
+    double d[3] = {A.x - P.x, A.y - P.y, A.z - P.z};
+    const float f[3] = {fa.x - fj.x, fa.y - fj.y, fa.z - fj.z};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // the image as FP32 sees it, unless that is too near to call
+      if (fabsf(fabsf(f[k]) - b.hLf[k]) < 1.0e-5f * b.Lf[k]) d[k] = fold(d[k], b.hL[k], b.L[k]);
+      else if (fabsf(f[k]) > b.hLf[k]) d[k] += f[k] > 0.0f ? -b.L[k] : b.L[k];
+    }
+    const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    if (r2 < b.rcut_lowsq) {
+      ov = true;
+      return;
+    }
+    const int m = cutoff_mask(b, r2, false);
+    if (ewald) {
+      const double ri = rsqrt(r2);
+      if (V && (m & 1)) {
+        if (lj) {
+          const int k = pidx(ma.y, mj.y, t.ntypes);
+          const double s2 = t.sig2[k] * (ri * ri), s6 = s2 * s2 * s2;
+          ev += 4.0 * t.eps[k] * (s6 * s6 - s6);
+        } else {
+          ev += vdw_pair(t, b, ma.y, mj.y, r2, 1.0);
+        }
+      }
+      if (m & 2) eq += A.w * P.w * kCHARGE_FACTOR * ri * erfc_as(b.alpha * (r2 * ri));
+    } else {
+      if (V && (m & 1)) ev += vdw_pair(t, b, ma.y, mj.y, r2, 1.0);
+      if (m & 2) eq += qq_pair_inter(b, A.w * P.w, r2);
+    }
+  };
+  const int nt = (n + 31) >> 5;
+  const int jt0 = blockIdx.x + (blockIdx.y * kPairWarps + w) * tiles, jt1 = min(nt, jt0 + tiles);
+  for (int jt = jt0; jt < jt1; ++jt) {
+    __syncwarp();
+    if (jt * 32 + lane < n) sf[w][lane] = p32[jt * 32 + lane];
+    __syncwarp();
+    const int most = min(32, n - jt * 32);
+    for (int k = 0; k < most; ++k) {
+      const float4 q = sf[w][k];
+      const float ex = fold(pi.x - q.x, b.hLf[0], b.Lf[0]), ey = fold(pi.y - q.y, b.hLf[1], b.Lf[1]),
+                  ez = fold(pi.z - q.z, b.hLf[2], b.Lf[2]);
+      const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+      const int tj = __float_as_int(q.w), j = jt * 32 + k;
+      const bool V = tj >= 0 && ((vdw >> tj) & 1u);
+      const bool hit = i < j && !(r2 > (V ? pre2 : pre2_none));
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const unsigned m = __ballot_sync(0xffffffffu, hit && V == (c == 1));
+        if (!m) continue;
+        if ((m >> lane) & 1u) queue[w][c][cnt[c] + __popc(m & ((1u << lane) - 1u))] = (unsigned)lane << 27 | (unsigned)j;
+        cnt[c] += __popc(m);
+        if (cnt[c] >= 32) {
+          __syncwarp();
+          cnt[c] -= 32;
+          pair(queue[w][c][cnt[c] + lane], c == 1);
+          __syncwarp();
+        }
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+    if (lane < cnt[c]) pair(queue[w][c][lane], c == 1);
+  if (ov) atomicOr(ovflag, 1);
+  double v[2] = {ev, eq};
+  reduce_partials<2>(v, partial, counter, out);
 }
 
 __global__ void __launch_bounds__(kBlock) k_intra_total(BoxDev b, PairTable t, SpeciesPools P,
@@ -401,7 +499,7 @@ __global__ void __launch_bounds__(kBlock) k_intra_total(BoxDev b, PairTable t, S
     v[5] += o.iqq;
     v[6] += o.pqq;
   }
-  reduce_partials<7>(v, partial, counter, out, nullptr, 0);
+  reduce_partials<7>(v, partial, counter, out);
 }
 
 // ---------------------------------------------------------------------------
@@ -452,50 +550,73 @@ __global__ void __launch_bounds__(128) k_sfac(const double4_32a* __restrict__ kv
   part[(size_t)blockIdx.y * nv + k] = make_double2(cs, sn);
 }
 
-// FP64 rebuild of the molecule rows along k-vector rows: thread per (row,
-// molecule); a sincos per atom at the row's start and for its step
-// e^{i 2 pi x / Lx}, then one complex product per k-vector and atom
-constexpr int kSfacRowAtoms = 4;  // molecules of up to this many atoms
-__global__ void __launch_bounds__(128) k_sfac_rows(const double4_32a* __restrict__ kvec, const int2* __restrict__ rows,
-                                                   int nrows, double hx1, const double4_32a* __restrict__ p64,
-                                                   const MolInfo* __restrict__ mols, int nm,
-                                                   const int* __restrict__ charged, double* cos_mol, double* sin_mol,
-                                                   int stride) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrows) return;
-  const int2 rw = rows[r];
-  const double4_32a h0 = kvec[rw.x];
-  for (int m = blockIdx.y; m < nm; m += gridDim.y) {
-    const MolInfo mi = mols[m];
-    if (!charged[mi.y]) continue;
-    double c[kSfacRowAtoms], s[kSfacRowAtoms], uc[kSfacRowAtoms], us[kSfacRowAtoms], q[kSfacRowAtoms];
+// FP64 rebuild of the molecule rows: a CTA per molecule and group of k-vector rows.
+// e^{i k r} = X[nx] Y[ny] Z[nz]: tables of the powers of e^{i 2 pi x / Lx} and of the
+// other two, per atom, then q Y Z per row of equal (ny, nz), all in shared memory, so that
+// a k-vector costs one complex product and sum per atom (4 FP64 operations) and no phase
+// of its own; threads take consecutive k, so the rows are written in whole lines.  12,288
+// atoms of water and 13,190 k-vectors: 4.25 ms with a thread per (row, molecule), which
+// spent most of its FP64 time on the two sincos that started each row, 3.53 ms now.
+constexpr int kSfacRowAtoms = 4;   // molecules of up to this many atoms
+constexpr int kSfacRows = 480;     // k-vector rows of a CTA
+__global__ void __launch_bounds__(kBlock) k_sfac_rows(const double4_32a* __restrict__ kvec, const int2* __restrict__ rows,
+                                                      int nrows, int rows_per_cta, double hx1, double hy1, double hz1,
+                                                      const double4_32a* __restrict__ p64,
+                                                      const MolInfo* __restrict__ mols, const int* __restrict__ charged,
+                                                      double* cos_mol, double* sin_mol, int stride) {
+  __shared__ double2 T[3][kSfacRowAtoms][kMaxKRow];
+  __shared__ double2 YZ[kSfacRowAtoms][kSfacRows];
+  __shared__ int2 srow[kSfacRows];
+  const MolInfo mi = mols[blockIdx.x];
+  if (!charged[mi.y]) return;
+  const int r0 = blockIdx.y * rows_per_cta, nr = min(rows_per_cta, nrows - r0);
+  for (int e = threadIdx.x; e < 3 * mi.w * kMaxKRow; e += blockDim.x) {
+    const int k = e % kMaxKRow, a = e / kMaxKRow % mi.w, d = e / (kMaxKRow * mi.w);
+    const double4_32a p = p64[mi.z + a];
+    const double h = (double)k * (d == 0 ? hx1 : d == 1 ? hy1 : hz1);
+    double s, c;
+    sincos(h * (d == 0 ? p.x : d == 1 ? p.y : p.z), &s, &c);
+    T[d][a][k] = make_double2(c, s);
+  }
+  for (int r = threadIdx.x; r < nr; r += blockDim.x) srow[r] = rows[r0 + r];
+  __syncthreads();
+  for (int e = threadIdx.x; e < nr * mi.w; e += blockDim.x) {
+    const int a = e / nr, r = e - a * nr;
+    const double4_32a h = kvec[srow[r].x], p = p64[mi.z + a];
+    const int nx = (int)rint(h.x / hx1), ny = (int)rint(h.y / hy1), nz = (int)rint(h.z / hz1);  // of the row's first k
+    double c, s;
+    if (nx == 0 && abs(ny) < kMaxKRow && abs(nz) < kMaxKRow) {
+      const double2 y = T[1][a][abs(ny)], z = T[2][a][abs(nz)];
+      const double ys = ny < 0 ? -y.y : y.y, zs = nz < 0 ? -z.y : z.y;
+      c = y.x * z.x - ys * zs;
+      s = y.x * zs + ys * z.x;
+    } else {
+      sincos(h.x * p.x + h.y * p.y + h.z * p.z, &s, &c);
+    }
+    YZ[a][r] = make_double2(p.w * c, p.w * s);
+  }
+  __syncthreads();
+  double* cm = cos_mol + (size_t)mi.x * stride;
+  double* sm = sin_mol + (size_t)mi.x * stride;
+  const int k1 = srow[nr - 1].x + srow[nr - 1].y;
+  for (int k = srow[0].x + threadIdx.x; k < k1; k += blockDim.x) {
+    int r = 0;  // the row of k
+    for (int hi = nr; hi - r > 1;) {
+      const int mid = (r + hi) >> 1;
+      if (srow[mid].x <= k) r = mid;
+      else hi = mid;
+    }
+    const int j = k - srow[r].x;
+    double c = 0.0, s = 0.0;
 #pragma unroll
-    for (int a = 0; a < kSfacRowAtoms; ++a) {
-      c[a] = s[a] = us[a] = q[a] = 0.0;
-      uc[a] = 1.0;
+    for (int a = 0; a < kSfacRowAtoms; ++a)
       if (a < mi.w) {
-        const double4_32a p = p64[mi.z + a];
-        sincos(h0.x * p.x + h0.y * p.y + h0.z * p.z, &s[a], &c[a]);
-        sincos(hx1 * p.x, &us[a], &uc[a]);
-        q[a] = p.w;
+        const double2 x = T[0][a][j], q = YZ[a][r];
+        c += q.x * x.x - q.y * x.y;
+        s += q.x * x.y + q.y * x.x;
       }
-    }
-    double* cm = cos_mol + (size_t)mi.x * stride + rw.x;
-    double* sm = sin_mol + (size_t)mi.x * stride + rw.x;
-    for (int j = 0; j < rw.y; ++j) {
-      double cs = 0.0, sn = 0.0;
-#pragma unroll
-      for (int a = 0; a < kSfacRowAtoms; ++a)
-        if (a < mi.w) {
-          cs = cs + q[a] * c[a];
-          sn = sn + q[a] * s[a];
-          const double c1 = c[a] * uc[a] - s[a] * us[a];
-          s[a] = s[a] * uc[a] + c[a] * us[a];
-          c[a] = c1;
-        }
-      cm[j] = cs;
-      sm[j] = sn;
-    }
+    cm[k] = c;
+    sm[k] = s;
   }
 }
 
@@ -533,7 +654,7 @@ __global__ void __launch_bounds__(kBlock) k_sfac_reduce(const double4_32a* __res
     e += kvec[k].w * (c * c + s * s);
   }
   double v[1] = {e};
-  reduce_partials<1>(v, partial, counter, out, nullptr, 0);
+  reduce_partials<1>(v, partial, counter, out);
 }
 
 // Update_System_Ewald_Reciprocal_Energy: thread per k-vector.
@@ -574,7 +695,7 @@ __global__ void __launch_bounds__(kBlock) k_ewald_update(const double4_32a* __re
     e = e + h.w * (c * c + s * s);
   }
   double v[1] = {e};
-  reduce_partials<1>(v, partial, counter, out, nullptr, 0);
+  reduce_partials<1>(v, partial, counter, out);
 }
 
 // Update_System_Ewald_Reciprocal_Energy_Widom: block per test molecule.
@@ -1486,7 +1607,7 @@ int cass_set_box(cass_ctx* c, int32_t ibox, const CassBoxDesc* d) {
     B.krow.clear();
     for (int k = 0; k < B.nvecs; ++k) {
       const double* h = &B.kvec[4 * (size_t)k];
-      const bool cont = k > 0 && h[1] == h[-3] && h[2] == h[-2] &&
+      const bool cont = k > 0 && B.krow.back().y < kMaxKRow && h[1] == h[-3] && h[2] == h[-2] &&
                         std::fabs(h[0] - (h[-4] + kTWOPI / v.L[0])) <= 1e-9 * (kTWOPI / v.L[0]);
       if (cont) ++B.krow.back().y;
       else B.krow.push_back(make_int2(k, 1));
@@ -1915,11 +2036,11 @@ static int box_reciprocal(cass_ctx* c, int ibox, double* e_recip) {
     if (c->sp[is].defined && c->sp[is].has_charge) max_na = std::max(max_na, c->sp[is].natoms);
   if (c->precision != CASS_PREC_MIXED && !B.krow.empty() && max_na <= kSfacRowAtoms && B.npacked_mols > 0) {
     const int nrows = (int)B.krow.size();
-    dim3 g((nrows + 127) / 128, std::min(B.npacked_mols, 65535));
-    k_sfac_rows<<<g, 128, 0, c->stream>>>(B.d_kvec.as<double4_32a>(), B.d_krow.as<int2>(), nrows, kTWOPI / B.dev.L[0],
-                                          B.d_p64.as<double4_32a>(), B.d_molinfo.as<int4>(), B.npacked_mols,
-                                          dch.as<int>(), c->d_cos_mol.as<double>(), c->d_sin_mol.as<double>(),
-                                          c->cos_mol_stride);
+    const int groups = (nrows + kSfacRows - 1) / kSfacRows, per = (nrows + groups - 1) / groups;
+    k_sfac_rows<<<dim3(B.npacked_mols, (nrows + per - 1) / per), kBlock, 0, c->stream>>>(
+        B.d_kvec.as<double4_32a>(), B.d_krow.as<int2>(), nrows, per, kTWOPI / B.dev.L[0], kTWOPI / B.dev.L[1],
+        kTWOPI / B.dev.L[2], B.d_p64.as<double4_32a>(), B.d_molinfo.as<int4>(), dch.as<int>(),
+        c->d_cos_mol.as<double>(), c->d_sin_mol.as<double>(), c->cos_mol_stride);
     CASS_CUDA(cudaGetLastError());
     count_launch(c);
     k_sfac_sum<<<dim3((nv + kBlock - 1) / kBlock, nchunks), kBlock, 0, c->stream>>>(
@@ -1964,38 +2085,35 @@ int cass_system_total_energy(cass_ctx* c, int32_t ibox1, int32_t intra_flag, Cas
   CassEnergy keep = E;
   E = CassEnergy{};
   *overlap = 0;
-  if ((rc = c->d_query.reserve(16))) return rc;
-  CASS_CUDA(cudaMemsetAsync(c->d_query.p, 0, sizeof(int), c->stream));
-  int n = B.npacked;
-  std::vector<double> res;
-  if (intra_flag && B.npacked_mols > 0) {
-    int nblk = std::max(1, std::min(296, (B.npacked_mols + kBlock - 1) / kBlock));
-    if ((rc = ensure_scratch(c, nblk, 7))) return rc;
-    k_intra_total<<<nblk, kBlock, 0, c->stream>>>(B.dev, c->pt, c->pools, B.d_p64.as<double4_32a>(), B.d_molinfo.as<int4>(),
-                                                   B.npacked_mols, c->d_partial.as<double>(),
-                                                   c->d_counter.as<unsigned>(), c->d_result.as<double>(),
-                                                   c->d_query.as<int>());
+  const int n = B.npacked;
+  // The intramolecular and the pair sums are launched together and read back in one
+  // copy with the overlap flag: result[0..7) intra, [8..10) pairs, the flag at [10].
+  // Boxes of single atoms have no intramolecular part.
+  const bool intra = intra_flag && B.npacked_mols > 0 && n > B.npacked_mols;
+  const int nblk_intra = std::max(1, std::min(296, (B.npacked_mols + kBlock - 1) / kBlock));
+  const bool fast = c->precision == CASS_PREC_MIXED && B.desc.vdw_style == CASS_VDW_LJ &&
+                    (B.desc.vdw_sum_style == CASS_VDW_SUM_CUT || B.desc.vdw_sum_style == CASS_VDW_SUM_CUT_TAIL) &&
+                    (B.desc.charge_style == CASS_CHARGE_NONE || B.desc.charge_sum_style == CASS_QQ_EWALD);
+  // FP64 pairs: tiles of j per warp so that about 24 warps per SM share the box's tile pairs
+  const int nt = (n + 31) / 32;
+  const long long tile_pairs = (long long)nt * (nt + 1) / 2;
+  const int tiles = (int)std::max<long long>(1, std::min<long long>(16, tile_pairs / (24LL * kPairSms)));
+  const dim3 grid = fast ? dim3((n + kBlock - 1) / kBlock, (n + kTileJ - 1) / kTileJ)
+                         : dim3(nt, (nt + kPairWarps * tiles - 1) / (kPairWarps * tiles));
+  if ((rc = ensure_scratch(c, std::max(7 * nblk_intra, n > 1 ? 2 * (int)(grid.x * grid.y) : 1), 1))) return rc;
+  if ((rc = c->h_read.reserve(16 * sizeof(double)))) return rc;
+  double* d_res = c->d_result.as<double>();
+  int* d_ov = reinterpret_cast<int*>(d_res + 10);
+  CASS_CUDA(cudaMemsetAsync(d_res, 0, 11 * sizeof(double), c->stream));
+  if (intra) {
+    k_intra_total<<<nblk_intra, kBlock, 0, c->stream>>>(B.dev, c->pt, c->pools, B.d_p64.as<double4_32a>(),
+                                                        B.d_molinfo.as<int4>(), B.npacked_mols,
+                                                        c->d_partial.as<double>(), c->d_counter.as<unsigned>(), d_res,
+                                                        d_ov);
     CASS_CUDA(cudaGetLastError());
-  count_launch(c);
-    if ((rc = sync_result(c, 7))) return rc;
-    E.bond = c->h_result[0];
-    E.angle = c->h_result[1];
-    E.dihedral = c->h_result[2];
-    E.improper = c->h_result[3];
-    E.intra_vdw = c->h_result[4];
-    E.intra_q = c->h_result[5];
-    E.inter_q = c->h_result[6];
-    E.intra = E.bond + E.angle + E.dihedral + E.improper + E.intra_q + E.intra_vdw;
-  } else if (!intra_flag) {
-    E.intra = keep.intra; E.bond = keep.bond; E.angle = keep.angle; E.dihedral = keep.dihedral;
-    E.improper = keep.improper; E.intra_vdw = keep.intra_vdw; E.intra_q = keep.intra_q;
+    count_launch(c);
   }
   if (n > 1) {
-    dim3 grid((n + kBlock - 1) / kBlock, (n + kTileJ - 1) / kTileJ);
-    if ((rc = ensure_scratch(c, grid.x * grid.y, 2))) return rc;
-    const bool fast = c->precision == CASS_PREC_MIXED && B.desc.vdw_style == CASS_VDW_LJ &&
-                      (B.desc.vdw_sum_style == CASS_VDW_SUM_CUT || B.desc.vdw_sum_style == CASS_VDW_SUM_CUT_TAIL) &&
-                      (B.desc.charge_style == CASS_CHARGE_NONE || B.desc.charge_sum_style == CASS_QQ_EWALD);
     // the largest cutoff cutoff_mask applies outside CBMC (none for the minimum-image styles)
     double rmax2 = B.dev.rcut_lowsq;
     bool bounded = true;
@@ -2009,33 +2127,48 @@ int cass_system_total_energy(cass_ctx* c, int32_t ibox1, int32_t intra_flag, Cas
       if (B.desc.charge_sum_style == CASS_QQ_MINIMUM) bounded = false;
       else rmax2 = std::max(rmax2, B.dev.rcut_coulsq);
     }
-    const float pre2 = bounded ? (float)(rmax2 * (1.0 + 1.0e-4) + 1.0e-3) : FLT_MAX;
+    auto pre = [](double r2) { return (float)(r2 * (1.0 + 1.0e-4) + 1.0e-3); };
+    const float pre2 = bounded ? pre(rmax2) : FLT_MAX;
+    // pairs without a vdW term and without charges only have their overlap test
+    const float pre2_none = B.desc.charge_style == CASS_CHARGE_COUL ? pre2 : pre(B.dev.rcut_lowsq);
     if (fast)
-      k_pair_total<true><<<grid, kBlock, 0, c->stream>>>(B.dev, c->pt, B.d_p64.as<double4_32a>(), B.d_meta.as<int4>(), n,
-                                                        pre2, nullptr, 0.0, c->d_partial.as<double>(),
-                                                        c->d_counter.as<unsigned>(), c->d_result.as<double>(),
-                                                        c->d_query.as<int>());
+      k_pair_total<<<grid, kBlock, 0, c->stream>>>(B.dev, c->pt, B.d_p64.as<double4_32a>(), B.d_meta.as<int4>(), n,
+                                                   c->d_partial.as<double>(), c->d_counter.as<unsigned>(), d_res + 8,
+                                                   d_ov);
     else
-      k_pair_total<false><<<grid, kBlock, 0, c->stream>>>(B.dev, c->pt, B.d_p64.as<double4_32a>(), B.d_meta.as<int4>(), n,
-                                                         pre2, B.comcut ? B.d_com.as<double4_32a>() : nullptr,
-                                                         B.rcut_max, c->d_partial.as<double>(),
-                                                         c->d_counter.as<unsigned>(), c->d_result.as<double>(),
-                                                         c->d_query.as<int>());
+      k_pair_hits<<<grid, 32 * kPairWarps, 0, c->stream>>>(
+          B.dev, c->pt, B.d_p64.as<double4_32a>(), B.d_p32.as<float4>(), B.d_meta.as<int4>(), n, tiles, pre2, pre2_none,
+          B.comcut ? B.d_com.as<double4_32a>() : nullptr, B.rcut_max, c->d_partial.as<double>(),
+          c->d_counter.as<unsigned>(), d_res + 8, d_ov);
     CASS_CUDA(cudaGetLastError());
-  count_launch(c);
-    if ((rc = sync_result(c, 2))) return rc;
-    E.inter_vdw += c->h_result[0];
-    E.inter_q += c->h_result[1];
+    count_launch(c);
   }
-  int hov = 0;
-  CASS_CUDA(d2h(c, &hov, c->d_query.p, sizeof(int)));
+  double* r = c->h_read.as<double>();
+  CASS_CUDA(d2h(c, r, d_res, 11 * sizeof(double)));
   CASS_CUDA(cudaStreamSynchronize(c->stream));
+  int hov = 0;
+  memcpy(&hov, r + 10, sizeof(int));
   if (hov) {
     *overlap = 1;
     B.energy_valid = false;
     B.frame_ready = false;
     return CASS_OK;
   }
+  if (intra_flag) {
+    E.bond = r[0];
+    E.angle = r[1];
+    E.dihedral = r[2];
+    E.improper = r[3];
+    E.intra_vdw = r[4];
+    E.intra_q = r[5];
+    E.inter_q = r[6];
+    E.intra = E.bond + E.angle + E.dihedral + E.improper + E.intra_q + E.intra_vdw;
+  } else {
+    E.intra = keep.intra; E.bond = keep.bond; E.angle = keep.angle; E.dihedral = keep.dihedral;
+    E.improper = keep.improper; E.intra_vdw = keep.intra_vdw; E.intra_q = keep.intra_q;
+  }
+  E.inter_vdw += r[8];
+  E.inter_q += r[9];
   E.inter = E.inter_q + E.inter_vdw;
   if (B.desc.charge_style == CASS_CHARGE_COUL) {
     if (box_has_ewald(B) && B.nvecs > 0) {

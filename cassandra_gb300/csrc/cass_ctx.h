@@ -128,6 +128,8 @@ struct SpeciesH {
   std::vector<double> pos;
 };
 
+constexpr int kMaxKRow = 64;
+
 struct BoxH {
   bool defined = false;
   CassBoxDesc desc{};
@@ -148,7 +150,7 @@ struct BoxH {
   DevBuf d_p64, d_p32, d_meta, d_molinfo;
   DevBuf d_kvec, d_cos_sum, d_sin_sum, d_cos_old, d_sin_old;
   // rows of the k-vector list: (first k, count) of runs of equal (ny, nz) with
-  // nx rising by one, for the phase recurrence of the FP64 rebuild
+  // nx rising by one, at most kMaxKRow long, for the FP64 rebuild and the adjoint
   std::vector<int2> krow;
   DevBuf d_krow;
   bool cell_dirty = true;
@@ -227,6 +229,7 @@ struct cass_ctx_impl {
   DevBuf d_cbmc_tab;
   // pinned staging of the packed-box uploads
   PinnedBuf h_pack;
+  PinnedBuf h_read;  // small results read back
   DevBuf d_stage;  // device copy of a frame load's staging area
 };
 

@@ -11,19 +11,18 @@
 // derivative of the computed energy (away from cutoff crossings, where the
 // truncated energy is discontinuous).  FP64 throughout.
 //
-//   k_grad_pairs  thread per atom i, a chunk of the atoms j per grid row in
-//                 shared-memory tiles: the force on i, sum_j q_j dE/d(q_i q_j),
-//                 and, for j > i, the per-type-pair parameter derivatives (each
-//                 pair counted once); one partial per (chunk, i)
-//   k_grad_recip  thread per atom i, a chunk of the k-vectors per grid row:
+//   k_grad_pairs  warp per atom i: the force on i, sum_j q_j dE/d(q_i q_j), and,
+//                 for j > i, the per-type-pair parameter derivatives (each pair
+//                 counted once)
+//   k_grad_recip  thread per atom i, a chunk of the k-vector rows per grid row:
 //                 2 CF q_i sum_k Cn k (S_s cos - S_c sin) and
 //                 2 CF sum_k Cn (S_c cos + S_s sin); one partial per (chunk, i)
 //   k_grad_reduce thread per atom: the chunks' partials added in chunk order
 //   k_grad_types  fixed-order tree reduction of the per-atom parameter
 //                 derivatives per type
-// The chunks spread the FP64 work of a box of a few thousand atoms over every
-// SM (a grid of atom blocks alone fills fewer SMs than GB300 has); the partial
-// buffers keep every sum in a fixed order, so repeated calls give equal bits.
+// The row chunks spread the FP64 work of a box of a few thousand atoms over every
+// SM; the partial buffers keep every sum in a fixed order, so repeated calls give
+// equal bits.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -54,11 +53,6 @@ __device__ __forceinline__ void erfc_as_d(double x, double& f, double& df) {
   // d(t poly)/dx = (poly + t dpoly) dt/dx, dt/dx = -P t^2
   df = e * ((poly + t * dpoly) * (-P * t * t) - 2.0 * x * tp);
 }
-
-struct GradAtom {
-  double4_32a p;  // x, y, z, q
-  int mol, type, species, atom;
-};
 
 // The vdW pair energy of Compute_AtomPair_Energy (energy_routines.f90:1907-2000)
 // in the box's style, differentiated: dE/d(r^2), dE/d(eps) and dE/d(sigma) of
@@ -257,162 +251,259 @@ __global__ void k_grad_bonded(SpeciesPools P, const int4* __restrict__ molinfo, 
     for (int d = 0; d < 3; ++d) grad[3 * (size_t)(mi.z + a) + d] += g[3 * a + d];
 }
 
-// pre2: an FP32 bound on r^2 beyond every cutoff of the box (with a margin far
-// above FP32 rounding of the coordinates): pairs beyond it are skipped before
-// the FP64 arithmetic, which then decides every cutoff exactly
-__global__ void __launch_bounds__(kGradBlock) k_grad_pairs(BoxDev b, PairTable T, SpeciesPools P,
-                                                           const double4_32a* __restrict__ p64,
-                                                           const float4* __restrict__ p32,
-                                                           const int4* __restrict__ meta, int n, int jchunk,
-                                                           float pre2, double* part, int* ovflag) {
-  __shared__ double4_32a sp[kGradBlock];
-  __shared__ float4 spf[kGradBlock];
-  __shared__ int4 sm[kGradBlock];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp's FP64 instruction takes 16 cycles of the SM's FP64 unit however many lanes
+// need it.  So a warp takes one atom i, compares it with 32 atoms j at a time in FP32
+// (pre2: a bound on r^2 beyond every cutoff, by far more than FP32 rounds; the FP64
+// arithmetic then decides every cutoff exactly), queues the pairs that pass and forms
+// 32 of them at a time in FP64, all lanes at work, with the sums of atom i spread over
+// the lanes and added once at the end.  Pairs with and without a vdW term have a queue
+// each.  With a lane per atom i and its pairs as they came, 14.5 of 32 lanes worked:
+// 14.7 ms for 12,288 atoms of water against 1.82 ms.
+constexpr int kGradWarps = 8;
+__global__ void __launch_bounds__(32 * kGradWarps) k_grad_pairs(BoxDev b, PairTable T, SpeciesPools P,
+                                                                const double4_32a* __restrict__ p64,
+                                                                const float4* __restrict__ p32,
+                                                                const int4* __restrict__ meta, int n, float pre2,
+                                                                float pre2_none, double* part, int* ovflag) {
+  __shared__ float4 tile[32 * kGradWarps];
+  __shared__ int queue[kGradWarps][2][64];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kGradWarps + w;
   const bool live = i < n;
-  const double4_32a pi = live ? p64[i] : make_double4_32a(0, 0, 0, 0);
-  const float4 pif = live ? p32[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const int4 mi = live ? meta[i] : make_int4(-1, -1, -1, -1);
-  const bool vdw = b.vdw_style == CASS_VDW_LJ || b.vdw_style == CASS_VDW_MIE;
+  const double4_32a pi = p64[live ? i : 0];
+  const float4 pif = p32[live ? i : 0];
+  const int4 mi = meta[live ? i : 0];
+  const SpeciesDevHdr* hi = &P.hdr[mi.z];
   const bool coul = b.charge_style == CASS_CHARGE_COUL;
+  unsigned vdw = 0u;  // types with which this atom has a vdW term
+  if (mi.y >= 0 && (b.vdw_style == CASS_VDW_LJ || b.vdw_style == CASS_VDW_MIE))
+    for (int q = 0; q < T.ntypes; ++q) vdw |= (T.eps[pidx(mi.y, q, T.ntypes)] != 0.0) ? 1u << q : 0u;
   double gx = 0, gy = 0, gz = 0, dqi = 0;
   double de[kMaxTypes], ds[kMaxTypes];
 #pragma unroll
   for (int t = 0; t < kMaxTypes; ++t) de[t] = ds[t] = 0.0;
   bool ov = false;
-  const SpeciesDevHdr* hi = live ? &P.hdr[mi.z] : nullptr;
-  const int jbeg = blockIdx.y * jchunk, jend = min(n, jbeg + jchunk);
-  for (int j0 = jbeg; j0 < jend; j0 += kGradBlock) {
-    __syncthreads();
-    if (j0 + threadIdx.x < jend) {
-      sp[threadIdx.x] = p64[j0 + threadIdx.x];
-      spf[threadIdx.x] = p32[j0 + threadIdx.x];
-      sm[threadIdx.x] = meta[j0 + threadIdx.x];
-    }
-    __syncthreads();
-    if (!live) continue;
-    const int cnt = min(kGradBlock, jend - j0);
-    for (int k = 0; k < cnt; ++k) {
-      const int j = j0 + k;
-      if (j == i) continue;
-      {
-        const float4 q = spf[k];
-        const float ex = fold(pif.x - q.x, b.hLf[0], b.Lf[0]), ey = fold(pif.y - q.y, b.hLf[1], b.Lf[1]),
-                    ez = fold(pif.z - q.z, b.hLf[2], b.Lf[2]);
-        if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > pre2) continue;
-      }
-      const double4_32a pj = sp[k];
-      const int4 mj = sm[k];
+  int cnt[2] = {0, 0};
+  // `on`: the lane has pair (i, j); V: it may have a vdW term
+  auto pair = [&](bool on, int j, bool V) {
+    double dEde = 0.0, dEds = 0.0;
+    int tj = -1;
+    if (on) {
+      const double4_32a pj = p64[j];
+      const float4 fj = p32[j];
+      const int4 mj = meta[j];
       const bool intra = mj.x == mi.x;
-      double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+      double d[3] = {pi.x - pj.x, pi.y - pj.y, pi.z - pj.z};
       double vs = 1.0, qs = 1.0;
       if (intra) {  // Compute_Molecule_Nonbond_Intra_Energy: no periodic image
         const int na = hi->natoms;
         vs = P.dp[hi->vs_off + mi.w * na + mj.w];
         qs = P.dp[hi->qs_off + mi.w * na + mj.w];
       } else {
-        dx = fold(dx, b.hL[0], b.L[0]);
-        dy = fold(dy, b.hL[1], b.L[1]);
-        dz = fold(dz, b.hL[2], b.L[2]);
+        const float f[3] = {pif.x - fj.x, pif.y - fj.y, pif.z - fj.z};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {  // the image as FP32 sees it, unless that is too near to call
+          if (fabsf(fabsf(f[k]) - b.hLf[k]) < 1.0e-5f * b.Lf[k]) d[k] = fold(d[k], b.hL[k], b.L[k]);
+          else if (fabsf(f[k]) > b.hLf[k]) d[k] += f[k] > 0.0f ? -b.L[k] : b.L[k];
+        }
       }
-      const double r2 = dx * dx + dy * dy + dz * dz;
+      const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
       if (intra) {
         if (r2 <= b.rcut_lowsq && !P.ip[hi->bonded_off + mi.w * hi->natoms + mj.w]) ov = true;
       } else if (r2 < b.rcut_lowsq) {
         ov = true;
       }
       double dEdr2 = 0.0;  // dE/d(r^2) of this pair
-      if (vdw && (cutoff_mask(b, r2, false) & 1) && mi.y >= 0 && mj.y >= 0) {
-        const int kk = pidx(mi.y, mj.y, T.ntypes);
-        if (T.eps[kk] != 0.0 && vs != 0.0) {
-          double er, ee, es;
-          vdw_pair_grad(T, b, kk, r2, vs, er, ee, es);
-          dEdr2 += er;
-          if (j > i) {
-            de[mj.y] += ee;
-            ds[mj.y] += es;
-          }
-        }
+      if (V && vs != 0.0 && (cutoff_mask(b, r2, false) & 1)) {
+        double er;
+        vdw_pair_grad(T, b, pidx(mi.y, mj.y, T.ntypes), r2, vs, er, dEde, dEds);
+        dEdr2 += er;
+        if (j > i) tj = mj.y;
       }
       // Ewald real space: inter q q CF erfc(ar)/r; intra q q CF (qscale - erf(ar))/r
       if (coul && r2 <= b.rcut_coulsq) {
-        const double r = sqrt(r2);
+        const double ri = rsqrt(r2), r = r2 * ri;
         double f, df;
         erfc_as_d(b.alpha * r, f, df);
         const double g = intra ? (qs - (1.0 - f)) : f;  // erf = 1 - erfc
-        const double phi = kCHARGE_FACTOR * g / r;      // dE/d(q_i q_j)
-        const double dphi_dr = kCHARGE_FACTOR * (b.alpha * df / r - g / r2);
+        const double phi = kCHARGE_FACTOR * g * ri;     // dE/d(q_i q_j)
         dqi += pj.w * phi;
-        dEdr2 += pi.w * pj.w * dphi_dr / (2.0 * r);
+        // dphi/dr = CF (alpha df / r - g / r^2), dE/d(r^2) = q q dphi/dr / (2 r)
+        dEdr2 += 0.5 * pi.w * pj.w * kCHARGE_FACTOR * (b.alpha * df - g * ri) * (ri * ri);
       }
-      gx += 2.0 * dEdr2 * dx;
-      gy += 2.0 * dEdr2 * dy;
-      gz += 2.0 * dEdr2 * dz;
+      gx += 2.0 * dEdr2 * d[0];
+      gy += 2.0 * dEdr2 * d[1];
+      gz += 2.0 * dEdr2 * d[2];
+    }
+    if (V)
+#pragma unroll
+      for (int t = 0; t < kMaxTypes; ++t)
+        if ((vdw >> t) & 1u) {  // the same in all lanes
+          de[t] += tj == t ? dEde : 0.0;
+          ds[t] += tj == t ? dEds : 0.0;
+        }
+  };
+  for (int j0 = 0; j0 < n; j0 += 32 * kGradWarps) {
+    __syncthreads();
+    if (j0 + (int)threadIdx.x < n) tile[threadIdx.x] = p32[j0 + threadIdx.x];
+    __syncthreads();
+    if (!live) continue;
+    for (int k0 = 0; k0 < min(32 * kGradWarps, n - j0); k0 += 32) {
+      const int j = j0 + k0 + lane;
+      const float4 q = tile[k0 + lane];
+      const float ex = fold(pif.x - q.x, b.hLf[0], b.Lf[0]), ey = fold(pif.y - q.y, b.hLf[1], b.Lf[1]),
+                  ez = fold(pif.z - q.z, b.hLf[2], b.Lf[2]);
+      const int tj = __float_as_int(q.w);
+      const bool V = tj >= 0 && ((vdw >> tj) & 1u);
+      const bool hit = j < n && j != i && !(fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > (V ? pre2 : pre2_none));
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const unsigned m = __ballot_sync(0xffffffffu, hit && V == (c == 1));
+        if (!m) continue;
+        if ((m >> lane) & 1u) queue[w][c][cnt[c] + __popc(m & ((1u << lane) - 1u))] = j;
+        cnt[c] += __popc(m);
+        if (cnt[c] >= 32) {
+          __syncwarp();
+          cnt[c] -= 32;
+          pair(true, queue[w][c][cnt[c] + lane], c == 1);
+          __syncwarp();
+        }
+      }
     }
   }
   if (!live) return;
+  __syncwarp();
+#pragma unroll
+  for (int c = 0; c < 2; ++c) pair(lane < cnt[c], lane < cnt[c] ? queue[w][c][lane] : 0, c == 1);
   if (ov) atomicOr(ovflag, 1);
-  // partial of (chunk, i): component-major so that the reduction reads coalesced
-  const size_t stride = (size_t)gridDim.y * n;
-  double* o = part + (size_t)blockIdx.y * n + i;
+  for (int o = 16; o > 0; o >>= 1) {
+    gx += __shfl_down_sync(0xffffffffu, gx, o);
+    gy += __shfl_down_sync(0xffffffffu, gy, o);
+    gz += __shfl_down_sync(0xffffffffu, gz, o);
+    dqi += __shfl_down_sync(0xffffffffu, dqi, o);
+#pragma unroll
+    for (int t = 0; t < kMaxTypes; ++t)
+      if ((vdw >> t) & 1u) {
+        de[t] += __shfl_down_sync(0xffffffffu, de[t], o);
+        ds[t] += __shfl_down_sync(0xffffffffu, ds[t], o);
+      }
+  }
+  if (lane) return;
+  double* o = part + i;
   o[0] = gx;
-  o[stride] = gy;
-  o[2 * stride] = gz;
-  o[3 * stride] = dqi;
+  o[(size_t)n] = gy;
+  o[2 * (size_t)n] = gz;
+  o[3 * (size_t)n] = dqi;
 #pragma unroll
   for (int t = 0; t < kMaxTypes; ++t) {
-    o[(4 + t) * stride] = de[t];
-    o[(4 + kMaxTypes + t) * stride] = ds[t];
+    o[(4 + t) * (size_t)n] = de[t];
+    o[(4 + kMaxTypes + t) * (size_t)n] = ds[t];
   }
 }
 
 // The k-vectors come in rows of equal (ny, nz) with nx = n0, n0+1, ... (the
 // loop order of Ewald_Reciprocal_Lattice_Vector_Setup, energy_routines.f90:
-// 2260-2311), so along a row the phase advances by the factor e^{i 2 pi x / Lx}:
-// one complex product per k-vector, a sincos at the start of each row.
+// 2260-2311), so a row's sum over nx is e^{i k0 r} times a polynomial in
+// z = e^{i 2 pi x / Lx} with the coefficients b_k = Cn (S_c - i S_s): Horner's rule
+// gives it and its derivative (the factor nx of the x force) in eight FP64
+// operations per k-vector and atom, without a phase per k-vector.  From row to row of
+// equal nz the factor e^{i ky y} advances by one complex product; a sincos starts each
+// plane.  6.7 ms before (a phase product and the four sums per k-vector, 19 FP64
+// operations with the tests for a row's end), 3.10 ms now on 12,288 atoms
+// and 13,190 k-vectors; FP64 pipe bound.
+constexpr int kGradRows = 32;       // rows of a tile
+constexpr int kGradRowVecs = 1024;  // k-vectors of a tile, and most of a row
+static_assert(kGradRowVecs >= kMaxKRow, "a row fits a tile");
 __global__ void __launch_bounds__(kGradBlock) k_grad_recip(const double4_32a* __restrict__ kvec,
+                                                           const int2* __restrict__ rows, int nrows,
                                                            const double* __restrict__ cos_sum,
-                                                           const double* __restrict__ sin_sum, int nv, int kchunk,
-                                                           double hx1, const double4_32a* __restrict__ p64, int n,
-                                                           double* part) {
-  __shared__ double4_32a sk[kGradBlock];
-  __shared__ double2 ss[kGradBlock];
+                                                           const double* __restrict__ sin_sum, double hx1, double hy1,
+                                                           const double4_32a* __restrict__ p64, int n, double* part) {
+  __shared__ double2 sb[kGradRowVecs];
+  __shared__ double4_32a sh0[kGradRows];
+  __shared__ int2 srow[kGradRows];  // first coefficient in sb, count
+  __shared__ int s_next;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = i < n;
   const double4_32a pi = live ? p64[i] : make_double4_32a(0, 0, 0, 0);
   double gx = 0, gy = 0, gz = 0, dqi = 0;
-  const int kbeg = blockIdx.y * kchunk, kend = min(nv, kbeg + kchunk);
-  double us, uc;  // e^{i hx1 x}
-  sincos(hx1 * pi.x, &us, &uc);
-  double c = 1.0, s = 0.0, py = 0.0, pz = 0.0, pxh = 0.0;
+  double zc, zs, yc, ys;  // e^{i hx1 x}, e^{i hy1 y}
+  sincos(hx1 * pi.x, &zs, &zc);
+  sincos(hy1 * pi.y, &ys, &yc);
+  double qc = 1.0, qs = 0.0, py = 0.0, pz = 0.0;  // e^{i (hy y + hz z)} of the last row
   bool have = false;
-  for (int k0 = kbeg; k0 < kend; k0 += kGradBlock) {
+  // groups of kGradRows rows, dealt to the grid's rows in turn
+  int r0 = blockIdx.y * kGradRows, rend = min(nrows, r0 + kGradRows);
+  while (r0 < nrows) {
+    // as many rows as the tile holds (the list has no row of more than kGradRowVecs)
     __syncthreads();
-    if (k0 + threadIdx.x < kend) {
-      sk[threadIdx.x] = kvec[k0 + threadIdx.x];
-      ss[threadIdx.x] = make_double2(cos_sum[k0 + threadIdx.x], sin_sum[k0 + threadIdx.x]);
+    const int base = rows[r0].x;
+    if (threadIdx.x < kGradRows && r0 + (int)threadIdx.x < rend) {
+      const int2 rw = rows[r0 + threadIdx.x];
+      srow[threadIdx.x] = make_int2(rw.x - base, rw.y);
+      sh0[threadIdx.x] = kvec[rw.x];
     }
     __syncthreads();
+    if (threadIdx.x == 0) {
+      int m = 0;
+      while (m < kGradRows && r0 + m < rend && srow[m].x + srow[m].y <= kGradRowVecs) ++m;
+      s_next = m;
+    }
+    __syncthreads();
+    const int m = s_next, nk = srow[m - 1].x + srow[m - 1].y;
+    for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+      const double cn = kvec[base + k].w;
+      sb[k] = make_double2(cn * cos_sum[base + k], -cn * sin_sum[base + k]);
+    }
+    __syncthreads();
+    r0 += m;
+    if (r0 == rend) {
+      r0 += (gridDim.y - 1) * kGradRows;
+      rend = min(nrows, r0 + kGradRows);
+    }
     if (!live) continue;
-    const int cnt = min(kGradBlock, kend - k0);
-    for (int k = 0; k < cnt; ++k) {
-      const double4_32a h = sk[k];
-      if (have && h.y == py && h.z == pz && fabs(h.x - (pxh + hx1)) <= 1e-9 * fabs(hx1)) {
-        const double c1 = c * uc - s * us;  // next nx of the row
-        s = s * uc + c * us;
-        c = c1;
+    for (int q = 0; q < m; ++q) {
+      const double4_32a h = sh0[q];
+      const int2 rw = srow[q];
+      if (have && h.z == pz && h.y == py) {
+        // a long row in pieces: the same factor
+      } else if (have && h.z == pz && fabs(h.y - (py + hy1)) <= 1e-9 * hy1) {
+        const double c1 = qc * yc - qs * ys;
+        qs = qs * yc + qc * ys;
+        qc = c1;
       } else {
-        sincos(h.x * pi.x + h.y * pi.y + h.z * pi.z, &s, &c);
-        py = h.y;
-        pz = h.z;
+        sincos(h.y * pi.y + h.z * pi.z, &qs, &qc);
         have = true;
       }
-      pxh = h.x;
-      const double w = h.w * (ss[k].y * c - ss[k].x * s);
-      gx += w * h.x;
-      gy += w * h.y;
-      gz += w * h.z;
-      dqi += h.w * (ss[k].x * c + ss[k].y * s);
+      py = h.y;
+      pz = h.z;
+      // P = sum_n b_n z^n and D = dP/dz by Horner's rule
+      double pr = 0.0, pq = 0.0, dr = 0.0, dq = 0.0;
+      for (int k = rw.y - 1; k >= 0; --k) {
+        const double2 c = sb[rw.x + k];
+        const double d1 = fma(dr, zc, fma(-dq, zs, pr));
+        dq = fma(dr, zs, fma(dq, zc, pq));
+        dr = d1;
+        const double p1 = fma(pr, zc, fma(-pq, zs, c.x));
+        pq = fma(pr, zs, fma(pq, zc, c.y));
+        pr = p1;
+      }
+      // times e^{i k0 r}; k0 has nx = 0, 1 in the row without the zero vector, or more in a later piece
+      double fc = qc, fs = qs;
+      if (h.x != 0.0) {
+        double xc = zc, xs = zs;
+        if (h.x > 1.5 * hx1) sincos(h.x * pi.x, &xs, &xc);
+        fc = qc * xc - qs * xs;
+        fs = qs * xc + qc * xs;
+      }
+      const double re = pr * fc - pq * fs, im = pr * fs + pq * fc;  // sum_k b_k e^{i k r} of the row
+      // z dP/dz e^{i k0 r}: its imaginary part carries the factor n of the x force
+      const double ec = fc * zc - fs * zs, es = fc * zs + fs * zc;
+      const double im1 = dr * es + dq * ec;
+      dqi += re;
+      gx -= h.x * im + hx1 * im1;
+      gy -= h.y * im;
+      gz -= h.z * im;
     }
   }
   if (!live) return;
@@ -424,30 +515,21 @@ __global__ void __launch_bounds__(kGradBlock) k_grad_recip(const double4_32a* __
   o[3 * stride] = dqi;
 }
 
-// the chunks' partials of atom i added in chunk order: the pair terms, then
-// 2 CF q_i times the reciprocal sums (no reciprocal part when nkc = 0)
-__global__ void k_grad_reduce(const double* __restrict__ ppart, int npc, const double* __restrict__ rpart, int nkc,
-                              const double4_32a* __restrict__ p64, int n, double* grad, double* dq,
-                              double* deps_atom, double* dsig_atom) {
+// the pair terms of atom i and 2 CF q_i times the reciprocal chunks' partials, added in
+// chunk order (no reciprocal part when nkc = 0)
+__global__ void k_grad_reduce(const double* __restrict__ ppart, const double* __restrict__ rpart, int nkc,
+                              const double4_32a* __restrict__ p64, int n, double* grad, double* dq) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const size_t ps = (size_t)npc * n;
-  double v[kGradPairVals];
+  double v[4];
 #pragma unroll
-  for (int c = 0; c < kGradPairVals; ++c) {
-    double a = 0.0;
-    for (int k = 0; k < npc; ++k) a += ppart[c * ps + (size_t)k * n + i];
-    v[c] = a;
-  }
+  for (int c = 0; c < 4; ++c) v[c] = ppart[c * (size_t)n + i];
   if (nkc > 0) {
     const size_t rs = (size_t)nkc * n;
-    double r[4];
+    double r[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int k = 0; k < nkc; ++k)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      double a = 0.0;
-      for (int k = 0; k < nkc; ++k) a += rpart[c * rs + (size_t)k * n + i];
-      r[c] = a;
-    }
+      for (int c = 0; c < 4; ++c) r[c] += rpart[c * rs + (size_t)k * n + i];
     const double f = 2.0 * kCHARGE_FACTOR, qi = p64[i].w;
     v[0] += f * qi * r[0];
     v[1] += f * qi * r[1];
@@ -458,52 +540,38 @@ __global__ void k_grad_reduce(const double* __restrict__ ppart, int npc, const d
   grad[3 * i + 1] = v[1];
   grad[3 * i + 2] = v[2];
   dq[i] = v[3];
-#pragma unroll
-  for (int t = 0; t < kMaxTypes; ++t) {
-    deps_atom[(size_t)i * kMaxTypes + t] = v[4 + t];
-    dsig_atom[(size_t)i * kMaxTypes + t] = v[4 + kMaxTypes + t];
-  }
 }
 
 constexpr int kTypeBlock = 256;
 
-// out[ti*kMaxTypes+tj] = sum over atoms of type ti of the per-atom values: one
-// block per type, each thread a fixed stride of atoms, then a fixed tree
-__global__ void __launch_bounds__(kTypeBlock) k_grad_types(const int4* __restrict__ meta, int n,
-                                                           const double* __restrict__ deps_atom,
-                                                           const double* __restrict__ dsig_atom, double* out_eps,
+// out[ti*kMaxTypes+tj] = sum over atoms of type ti of the per-atom values of tj: one
+// block per pair of types, each thread a fixed stride of atoms, then a fixed tree
+__global__ void __launch_bounds__(kTypeBlock) k_grad_types(const int4* __restrict__ meta, int n, PairTable T,
+                                                           const double* __restrict__ part, double* out_eps,
                                                            double* out_sig) {
-  __shared__ double se[kTypeBlock][kMaxTypes + 1], ssg[kTypeBlock][kMaxTypes + 1];
-  const int ti = blockIdx.x;
-  double e[kMaxTypes], s[kMaxTypes];
-#pragma unroll
-  for (int t = 0; t < kMaxTypes; ++t) e[t] = s[t] = 0.0;
-  for (int i = threadIdx.x; i < n; i += kTypeBlock) {
-    if (meta[i].y != ti) continue;
-#pragma unroll
-    for (int t = 0; t < kMaxTypes; ++t) {
-      e[t] += deps_atom[(size_t)i * kMaxTypes + t];
-      s[t] += dsig_atom[(size_t)i * kMaxTypes + t];
+  __shared__ double se[kTypeBlock], ss[kTypeBlock];
+  const int ti = blockIdx.x, tj = blockIdx.y;
+  double e = 0.0, s = 0.0;
+  const bool any = ti < T.ntypes && tj < T.ntypes && T.eps[pidx(ti, tj, T.ntypes)] != 0.0;
+  if (any)
+    for (int i = threadIdx.x; i < n; i += kTypeBlock) {
+      if (meta[i].y != ti) continue;
+      e += part[(4 + tj) * (size_t)n + i];
+      s += part[(4 + kMaxTypes + tj) * (size_t)n + i];
     }
-  }
-#pragma unroll
-  for (int t = 0; t < kMaxTypes; ++t) {
-    se[threadIdx.x][t] = e[t];
-    ssg[threadIdx.x][t] = s[t];
-  }
+  se[threadIdx.x] = e;
+  ss[threadIdx.x] = s;
   __syncthreads();
   for (int h = kTypeBlock / 2; h > 0; h >>= 1) {
-    if (threadIdx.x < h)
-#pragma unroll
-      for (int t = 0; t < kMaxTypes; ++t) {
-        se[threadIdx.x][t] += se[threadIdx.x + h][t];
-        ssg[threadIdx.x][t] += ssg[threadIdx.x + h][t];
-      }
+    if (threadIdx.x < h) {
+      se[threadIdx.x] += se[threadIdx.x + h];
+      ss[threadIdx.x] += ss[threadIdx.x + h];
+    }
     __syncthreads();
   }
-  if (threadIdx.x < kMaxTypes) {
-    out_eps[ti * kMaxTypes + threadIdx.x] = se[0][threadIdx.x];
-    out_sig[ti * kMaxTypes + threadIdx.x] = ssg[0][threadIdx.x];
+  if (threadIdx.x == 0) {
+    out_eps[ti * kMaxTypes + tj] = se[0];
+    out_sig[ti * kMaxTypes + tj] = ss[0];
   }
 }
 
@@ -551,36 +619,26 @@ extern "C" int cass_system_gradient(cass_ctx* c, int32_t ibox1, CassEnergy* ener
   if (energy) *energy = E;
   const int n = B.npacked;
   const int nt = c->ntypes;
-  // chunks of j atoms / k-vectors per grid row: about four CTAs per SM in all
+  // k-vector row groups per grid row: about six CTAs per SM in all
   int dev_sms = 0;
   CASS_CUDA(cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c->device));
   const int nb = std::max(1, (n + kGradBlock - 1) / kGradBlock);
-  const int want_rows = std::max(1, (4 * dev_sms + nb - 1) / nb);
-  auto chunking = [&](int total, int& rows) {  // chunk length, a multiple of the tile
-    rows = std::max(1, std::min(want_rows, (total + kGradBlock - 1) / kGradBlock));
-    int len = (total + rows - 1) / rows;
-    len = ((len + kGradBlock - 1) / kGradBlock) * kGradBlock;
-    rows = std::max(1, (total + len - 1) / len);
-    return len;
-  };
-  int npc = 1, nkc = 0;
-  const int jchunk = n > 0 ? chunking(n, npc) : 1;
   const bool recip = d.charge_style == CASS_CHARGE_COUL && B.nvecs > 0;
-  int kchunk = 1;
-  if (recip) kchunk = chunking(B.nvecs, nkc);
-  const size_t bytes = (size_t)n * (3 + 1 + 2 * kMaxTypes) * sizeof(double) + 2 * kMaxTypes * kMaxTypes * sizeof(double) +
-                       (size_t)n * ((size_t)npc * kGradPairVals + (size_t)nkc * 4) * sizeof(double) + 64;
-  if ((rc = c->d_grad.reserve(bytes))) return rc;
+  const int nrows = (int)B.krow.size();
+  int nkc = 0;
+  if (recip) nkc = std::max(1, std::min((6 * dev_sms + nb - 1) / nb, (nrows + kGradRows - 1) / kGradRows));
+  // results in one piece: dU/dr, dU/dq per atom, dU/deps, dU/dsig, the overlap flag
+  const size_t nout = 4 * (size_t)n + 2 * kMaxTypes * kMaxTypes + 1;
+  const size_t bytes = (nout + (size_t)n * ((size_t)kGradPairVals + (size_t)nkc * 4)) * sizeof(double) + 64;
+  if ((rc = c->d_grad.reserve(bytes)) || (rc = c->h_read.reserve(nout * sizeof(double)))) return rc;
   double* d_g = c->d_grad.as<double>();
   double* d_dq = d_g + 3 * (size_t)n;
-  double* d_de = d_dq + n;
-  double* d_ds = d_de + (size_t)n * kMaxTypes;
-  double* d_te = d_ds + (size_t)n * kMaxTypes;
+  double* d_te = d_dq + n;
   double* d_ts = d_te + kMaxTypes * kMaxTypes;
-  double* d_pp = d_ts + kMaxTypes * kMaxTypes;
-  double* d_rp = d_pp + (size_t)n * npc * kGradPairVals;
-  if ((rc = c->d_query.reserve(16))) return rc;
-  CASS_CUDA(cudaMemsetAsync(c->d_query.p, 0, sizeof(int), c->stream));
+  int* d_ov = reinterpret_cast<int*>(d_ts + kMaxTypes * kMaxTypes);
+  double* d_pp = d_g + nout;
+  double* d_rp = d_pp + (size_t)n * kGradPairVals;
+  CASS_CUDA(cudaMemsetAsync(d_ov, 0, sizeof(double), c->stream));
   if (n > 0) {
     // beyond every cutoff the kernel tests: pairs past it add nothing
     double rmax2 = 0.0;
@@ -591,24 +649,27 @@ extern "C" int cass_system_gradient(cass_ctx* c, int32_t ibox1, CassEnergy* ener
     }
     if (d.charge_style == CASS_CHARGE_COUL) rmax2 = std::max(rmax2, B.dev.rcut_coulsq);
     rmax2 = std::max(rmax2, B.dev.rcut_lowsq);
-    const float pre2 = (float)(rmax2 * (1.0 + 1.0e-4) + 1.0e-3);
-    k_grad_pairs<<<dim3(nb, npc), kGradBlock, 0, c->stream>>>(B.dev, c->pt, c->pools, B.d_p64.as<double4_32a>(),
-                                                              B.d_p32.as<float4>(), B.d_meta.as<int4>(), n, jchunk,
-                                                              pre2, d_pp, c->d_query.as<int>());
+    auto pre = [](double r2) { return (float)(r2 * (1.0 + 1.0e-4) + 1.0e-3); };
+    // pairs without a vdW term: the charges' cutoff, or only the overlap test (an
+    // intramolecular pair without a term has none of the two beyond it either)
+    const double none2 = std::max(B.dev.rcut_lowsq, d.charge_style == CASS_CHARGE_COUL ? B.dev.rcut_coulsq : 0.0);
+    k_grad_pairs<<<(n + kGradWarps - 1) / kGradWarps, 32 * kGradWarps, 0, c->stream>>>(
+        B.dev, c->pt, c->pools, B.d_p64.as<double4_32a>(), B.d_p32.as<float4>(), B.d_meta.as<int4>(), n, pre(rmax2),
+        pre(none2), d_pp, d_ov);
     CASS_CUDA(cudaGetLastError());
     count_launch(c);
     if (recip) {
-      k_grad_recip<<<dim3(nb, nkc), kGradBlock, 0, c->stream>>>(B.d_kvec.as<double4_32a>(), B.d_cos_sum.as<double>(),
-                                                                B.d_sin_sum.as<double>(), B.nvecs, kchunk,
-                                                                kTWOPI / B.dev.L[0], B.d_p64.as<double4_32a>(), n, d_rp);
+      k_grad_recip<<<dim3(nb, nkc), kGradBlock, 0, c->stream>>>(
+          B.d_kvec.as<double4_32a>(), B.d_krow.as<int2>(), nrows, B.d_cos_sum.as<double>(), B.d_sin_sum.as<double>(),
+          kTWOPI / B.dev.L[0], kTWOPI / B.dev.L[1], B.d_p64.as<double4_32a>(), n, d_rp);
       CASS_CUDA(cudaGetLastError());
       count_launch(c);
     }
-    k_grad_reduce<<<nb, kGradBlock, 0, c->stream>>>(d_pp, npc, d_rp, recip ? nkc : 0, B.d_p64.as<double4_32a>(), n, d_g,
-                                                    d_dq, d_de, d_ds);
+    k_grad_reduce<<<nb, kGradBlock, 0, c->stream>>>(d_pp, d_rp, nkc, B.d_p64.as<double4_32a>(), n, d_g, d_dq);
     CASS_CUDA(cudaGetLastError());
     count_launch(c);
-    k_grad_types<<<kMaxTypes, kTypeBlock, 0, c->stream>>>(B.d_meta.as<int4>(), n, d_de, d_ds, d_te, d_ts);
+    k_grad_types<<<dim3(kMaxTypes, kMaxTypes), kTypeBlock, 0, c->stream>>>(B.d_meta.as<int4>(), n, c->pt, d_pp, d_te,
+                                                                           d_ts);
     CASS_CUDA(cudaGetLastError());
     count_launch(c);
     if (flexible && B.npacked_mols > 0) {
@@ -618,19 +679,19 @@ extern "C" int cass_system_gradient(cass_ctx* c, int32_t ibox1, CassEnergy* ener
       count_launch(c);
     }
   }
-  std::vector<double> g(3 * (size_t)n), q(n), te(kMaxTypes * kMaxTypes, 0.0), ts(kMaxTypes * kMaxTypes, 0.0);
+  const double* g = c->h_read.as<double>();
+  const double *q = g + 3 * (size_t)n, *te = q + n, *ts = te + kMaxTypes * kMaxTypes;
   int hov = 0;
   if (n > 0) {
-    CASS_CUDA(d2h(c, g.data(), d_g, g.size() * sizeof(double)));
-    CASS_CUDA(d2h(c, q.data(), d_dq, q.size() * sizeof(double)));
-    CASS_CUDA(d2h(c, te.data(), d_te, te.size() * sizeof(double)));
-    CASS_CUDA(d2h(c, ts.data(), d_ts, ts.size() * sizeof(double)));
+    CASS_CUDA(d2h(c, c->h_read.p, d_g, nout * sizeof(double)));
+    CASS_CUDA(cudaStreamSynchronize(c->stream));
+    memcpy(&hov, ts + kMaxTypes * kMaxTypes, sizeof(int));
+  } else {
+    memset(c->h_read.p, 0, nout * sizeof(double));
   }
-  CASS_CUDA(d2h(c, &hov, c->d_query.p, sizeof(int)));
-  CASS_CUDA(cudaStreamSynchronize(c->stream));
   if (hov) return set_error(CASS_ESTATE, "gradient: the configuration has a core overlap");
   // the packed order is species-major, locate order: the order of dU_dr
-  if (dU_dr) memcpy(dU_dr, g.data(), g.size() * sizeof(double));
+  if (dU_dr) memcpy(dU_dr, g, 3 * (size_t)n * sizeof(double));
   if (dU_dq) {
     std::vector<int> off(c->nspecies + 1, 0);
     for (int is = 0; is < c->nspecies; ++is) off[is + 1] = off[is] + (c->sp[is].defined ? c->sp[is].natoms : 0);

@@ -1,6 +1,6 @@
 // k_widom.cu -- batched CBMC Widom insertion on the GPU.
 //
-//   k_cell_count / k_cell_scan / k_cell_scatter / k_cell_sort
+//   k_cell_count / k_cell_scan / k_cell_scatter / k_cell_place
 //       per-box cell lists (counting sort, deterministic order inside a cell);
 //       the GPU counterpart of Sector_Setup / CBMC_Cell_List_Setup
 //       (sector_routines.f90:39-374).  Cells only accelerate the search:
@@ -138,15 +138,30 @@ __global__ void k_cell_scan(const BoxDev* boxes, const int* count, int* cstart, 
   if (threadIdx.x == 0) cs[nc] = carry;
 }
 
-__global__ void k_cell_scatter(const BoxSrc* src, const BoxDev* boxes, const int* cell_of, const int* cstart,
-                               int* fill, double4_32a* c64, float4* c32, int* ctype, float* cq32, int* corig) {
+// the packed indices of each cell's atoms, in any order
+__global__ void k_cell_scatter(const BoxDev* boxes, const int* cell_of, const int* cstart, int* fill, int* list) {
   int k = blockIdx.y;
   const BoxDev& b = boxes[k];
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= b.natoms) return;
   int c = cell_of[b.atom_off + i];
-  int pos = cstart[b.cell_off + k + c] + atomicAdd(&fill[b.cell_off + c], 1);
-  int g = b.atom_off + pos;
+  list[b.atom_off + cstart[b.cell_off + k + c] + atomicAdd(&fill[b.cell_off + c], 1)] = i;
+}
+
+// The cell-sorted copies: an atom stands in its cell behind those of smaller packed
+// index, a deterministic order.  A thread per atom counts them; a thread per cell that
+// sorted its cell took 281 us for the 27 cells of 256 waters.
+__global__ void k_cell_place(const BoxSrc* src, const BoxDev* boxes, const int* cell_of, const int* cstart,
+                             const int* list, double4_32a* c64, float4* c32, int* ctype, float* cq32, int* corig) {
+  int k = blockIdx.y;
+  const BoxDev& b = boxes[k];
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= b.natoms) return;
+  const int c = cell_of[b.atom_off + i];
+  const int first = cstart[b.cell_off + k + c], end = cstart[b.cell_off + k + c + 1];
+  int rank = 0;
+  for (int q = first; q < end; ++q) rank += list[b.atom_off + q] < i ? 1 : 0;
+  const int g = b.atom_off + first + rank;
   // the copies hold the positions their cells were chosen from, wrapped into
   // [-L/2, L/2) (an atom of a molecule folded by its COM may stick out of the
   // box), so that a query's per-row image shift is the whole periodic shift
@@ -160,40 +175,6 @@ __global__ void k_cell_scatter(const BoxSrc* src, const BoxDev* boxes, const int
   ctype[g] = src[k].meta[i].y;
   cq32[g] = (float)p.w;
   corig[g] = i;
-}
-
-// insertion sort of each cell by packed index: a deterministic order
-__global__ void k_cell_sort(const BoxDev* boxes, int nb, const int* cstart, double4_32a* c64, float4* c32, int* ctype,
-                            float* cq32, int* corig) {
-  int k = blockIdx.y;
-  if (k >= nb) return;
-  const BoxDev& b = boxes[k];
-  int nc = b.nc[0] * b.nc[1] * b.nc[2];
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= nc) return;
-  const int* cs = cstart + b.cell_off + k;
-  int s = b.atom_off + cs[c], e = b.atom_off + cs[c + 1];
-  for (int i = s + 1; i < e; ++i) {
-    int key = corig[i];
-    double4_32a a64 = c64[i];
-    float4 a32 = c32[i];
-    int at = ctype[i];
-    float aq = cq32[i];
-    int j = i - 1;
-    while (j >= s && corig[j] > key) {
-      corig[j + 1] = corig[j];
-      c64[j + 1] = c64[j];
-      c32[j + 1] = c32[j];
-      ctype[j + 1] = ctype[j];
-      cq32[j + 1] = cq32[j];
-      --j;
-    }
-    corig[j + 1] = key;
-    c64[j + 1] = a64;
-    c32[j + 1] = a32;
-    ctype[j + 1] = at;
-    cq32[j + 1] = aq;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1034,6 +1015,8 @@ struct CoopBox {
   const float4* p32;  // global (SMEM false)
   const float* q32;
   const int* cstart;
+  const double4_32a* c64;  // FP64 kernel
+  const PairTable* T;
   unsigned off_cells, off_atoms;
 };
 extern __shared__ __align__(32) unsigned char smem[];
@@ -2433,6 +2416,726 @@ __global__ void __launch_bounds__(128) k_widom(WidomSpecies S, PairTable T, Spec
   }
 }
 
+// ---------------------------------------------------------------------------
+// Warp-wide queries of the FP64 kernel.
+//
+// GB300 takes 16 cycles of an SM for a warp's FP64 instruction however many lanes need
+// it, so the FP64 work is done for full warps: a query's voxel list is gone through by
+// all lanes in FP32 with a margin far above its rounding, the pairs that pass are
+// queued, and 32 of them at a time are decided and evaluated in FP64.  (A thread per
+// insertion had 8.5 of 32 lanes at work and formed every visited pair in FP64.)
+constexpr int kHits64 = 256;  // queued pairs of a warp
+constexpr int kThreads64 = 384;
+
+struct Coop64 {
+  double4_32a pos[32];  // query points and charges
+  double sum[32], sabs[32];
+  double e[kHits64];
+  float4 posf[32];
+  unsigned hit[kHits64];  // atom | image code << 17 | query << 24 | image to be checked << 29
+  int type[32], ov[32], first[33];
+};
+struct Head64 {
+  BoxDev b;
+  BoxF f;
+  VoxGrid vox[2];
+  float4 shift[125];
+  double4_32a shift64[125];
+  double2 lj[kMaxTypes * kMaxTypes];  // eps, sigma^2
+  float pre[2];                       // FP32 bound of r^2 beyond the CBMC and the full cutoffs
+  float low_sure, low_pre;            // FP32 r^2 below / above which a pair surely is / is not an overlap
+  float edge_lo[3], edge_hi[3];       // |d| about half a box edge: surely this image / surely another
+};
+__device__ __forceinline__ Head64& head64() { return *reinterpret_cast<Head64*>(smem); }
+constexpr unsigned kHead64Bytes = (sizeof(Head64) + 31) & ~31u;
+__device__ __forceinline__ Coop64& coop64() { return reinterpret_cast<Coop64*>(smem + kHead64Bytes)[threadIdx.x >> 5]; }
+
+// FP64 separation of query point p and cell-sorted atom a through image code c
+__device__ __forceinline__ double sep64(const Head64& H, const double4_32a& p, const double4_32a& a, int c, double d[3]) {
+  const double4_32a sh = H.shift64[c];
+  d[0] = (p.x - a.x) + sh.x;
+  d[1] = (p.y - a.y) + sh.y;
+  d[2] = (p.z - a.z) + sh.z;
+  return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+}
+
+// Core overlap of a CBMC query point, decided in FP64 where FP32 cannot tell
+template <bool SMEM>
+__device__ __forceinline__ bool vox_overlap64(const CoopBox& B, const Head64& H, const double4_32a* c64,
+                                              const double4_32a& p) {
+  const float4* p32;
+  if constexpr (SMEM) p32 = reinterpret_cast<const float4*>(smem + B.off_atoms);
+  else p32 = B.p32;
+  if (!H.vox[0].on) return false;
+  float x = (float)p.x, y = (float)p.y, z = (float)p.z;
+  int code;
+  const uint4 rec = vox_record(H.f, H.vox[0], B.vrec, x, y, z, code);
+  const unsigned* list = reinterpret_cast<const unsigned*>(B.vlist + rec.x);
+  bool ov = false;
+  for (int t = 0; t < (int)rec.y && !ov; ++t) {
+    const unsigned e = __ldg(&list[t]);
+    const int j = (int)(e & kVoxAtomMask), c = (int)(e >> kVoxAtomBits) + code;
+    const float4 a = p32[j], sh = H.shift[c];
+    const float dx = (x + sh.x) - a.x, dy = (y + sh.y) - a.y, dz = (z + sh.z) - a.z;
+    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    if (r2 > H.low_pre) continue;
+    double d[3];
+    ov = r2 < H.low_sure || sep64(H, p, c64[j], c, d) < H.b.rcut_lowsq;
+  }
+  return ov;
+}
+
+// The energies of the nq queries of the warp's scratch, left in sum (sabs: of |terms|,
+// FULL only) and ov (FULL only; CBMC queries come without an overlap)
+template <bool SMEM, bool FULL>
+__device__ __noinline__ void coop_eval64(const CoopBox B, int nq, bool want_qq, PairCount& pc) {
+  const Head64& H = head64();
+  const double4_32a* __restrict__ c64 = B.c64;
+  const PairTable& T = *B.T;
+  const BoxDev& b = H.b;
+  Coop64& W = coop64();
+  const float4* p32;
+  if constexpr (SMEM) p32 = reinterpret_cast<const float4*>(smem + B.off_atoms);
+  else p32 = B.p32;
+  const int lane = threadIdx.x & 31;
+  const VoxGrid& g = H.vox[FULL ? 1 : 0];
+  const bool qq_on = want_qq && b.charge_style == CASS_CHARGE_COUL, lj = lj_plain_style(b);
+  const bool ewald = b.charge_sum_style == CASS_QQ_EWALD;
+  const float pre = H.pre[FULL ? 1 : 0];
+  if (lane < nq) W.sum[lane] = W.sabs[lane] = 0.0;
+  int cnt = 0;
+  double acc = 0.0, aabs = 0.0;  // FULL: this lane's share of the current query
+  // queued pair h in FP64
+  auto pair = [&](unsigned h, double& e, double& ea) {
+    const int q = (int)(h >> 24) & 31, j = (int)(h & kVoxAtomMask);
+    const double4_32a p = W.pos[q], a = c64[j];
+    double d[3];
+    const double r2 = sep64(H, p, a, (int)(h >> kVoxAtomBits) & 127, d);
+    e = 0.0;
+    ea = 0.0;
+    if (h >> 29)  // near half a box edge: this atom's other image may be the nearer one
+      for (int k = 0; k < 3; ++k)
+        if (fabs(d[k]) > b.hL[k]) return;
+    if (FULL && r2 < b.rcut_lowsq) {
+      W.ov[q] = 1;
+      return;
+    }
+    int m = cutoff_mask(b, r2, !FULL);
+    if (!qq_on) m &= 1;
+    if (m) ++pc.in_cut;
+    const int ta = W.type[q], tj = __float_as_int(p32[j].w);
+    if ((m & 1) && ta >= 0 && tj >= 0) {
+      double ev;
+      if (lj) {
+        const double2 es = H.lj[ta * kMaxTypes + tj];
+        const double s2 = es.y * (1.0 / r2), s6 = s2 * s2 * s2;
+        ev = 4.0 * es.x * (s6 * s6 - s6);
+      } else {
+        ev = vdw_pair(T, b, ta, tj, r2, 1.0);
+      }
+      e += ev;
+      if (FULL) ea += fabs(ev);
+    }
+    if (m & 2) {
+      double eq;
+      if (ewald) {
+        const double ri = rsqrt(r2);
+        eq = p.w * a.w * kCHARGE_FACTOR * ri * erfc_as(b.alpha * (r2 * ri));
+      } else {
+        eq = qq_pair_inter(b, p.w * a.w, r2);
+      }
+      e += eq;
+      if (FULL) ea += fabs(eq);
+    }
+  };
+  // evaluates the queue; q: the query being listed
+  auto flush = [&](int q) {
+    __syncwarp();
+    for (int t = lane; t < cnt; t += 32) {
+      double e, ea;
+      pair(W.hit[t], e, ea);
+      if (FULL) {
+        acc += e;
+        aabs += ea;
+      } else {
+        W.e[t] = e;
+      }
+    }
+    __syncwarp();
+    if (!FULL && lane <= q) {  // each query's pairs stand together, in their order
+      const int t1 = lane < q ? W.first[lane + 1] : cnt;
+      double e = W.sum[lane];
+      for (int t = W.first[lane]; t < t1; ++t) e += W.e[t];
+      W.sum[lane] = e;
+    }
+    __syncwarp();
+    if (!FULL && lane <= q) W.first[lane] = 0;
+    cnt = 0;
+    __syncwarp();
+  };
+  for (int q = 0; q < nq; ++q) {
+    if (!FULL && lane == 0) W.first[q] = cnt;
+    const float4 p = W.posf[q];
+    float x = p.x, y = p.y, z = p.z;
+    int code = 0, n = 0;
+    const unsigned* list = nullptr;
+    if (g.on) {
+      const uint4 rec = vox_record(H.f, g, B.vrec, x, y, z, code);
+      list = reinterpret_cast<const unsigned*>(B.vlist + rec.x);
+      n = (int)rec.z;
+    }
+    if (lane == 0) pc.visited += (unsigned long long)n;
+    for (int t0 = 0; t0 < n; t0 += 32) {
+      bool hit = false;
+      unsigned h = 0;
+      if (t0 + lane < n) {
+        const unsigned e = __ldg(&list[t0 + lane]);
+        const int j = (int)(e & kVoxAtomMask), c = (int)(e >> kVoxAtomBits) + code;
+        const float4 a = p32[j], sh = H.shift[c];
+        const float dx = fabsf((x + sh.x) - a.x), dy = fabsf((y + sh.y) - a.y), dz = fabsf((z + sh.z) - a.z);
+        hit = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > pre) && dx <= H.edge_hi[0] && dy <= H.edge_hi[1] &&
+              dz <= H.edge_hi[2];
+        const unsigned check = dx > H.edge_lo[0] || dy > H.edge_lo[1] || dz > H.edge_lo[2];
+        h = (unsigned)j | (unsigned)c << kVoxAtomBits | (unsigned)q << 24 | check << 29;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (hit) W.hit[cnt + __popc(m & ((1u << lane) - 1u))] = h;
+      cnt += __popc(m);
+      if (cnt > kHits64 - 32) flush(q);
+    }
+    if (FULL) {
+      flush(q);
+      for (int o = 16; o > 0; o >>= 1) {
+        acc += __shfl_down_sync(0xffffffffu, acc, o);
+        aabs += __shfl_down_sync(0xffffffffu, aabs, o);
+      }
+      if (lane == 0) {
+        W.sum[q] = acc;
+        W.sabs[q] = aabs;
+      }
+      acc = aabs = 0.0;
+    }
+  }
+  if (!FULL) flush(nq - 1);
+  __syncwarp();
+}
+
+// Energy of the atoms ids[0..nat) of every lane that is `on` (all atoms in order where
+// ids is NULL) at r, or r - old + cen, against the box: added to e (and eabs), ov set on
+// core overlap
+template <bool SMEM, bool FULL>
+__device__ __forceinline__ void coop_atoms64(const CoopBox& B, const WidomSpecies& S, bool on, const double* r,
+                                             const signed char* ids, int nat, const double* old, const double* cen,
+                                             bool want_qq, double& e, double* eabs, bool& ov, PairCount& pc) {
+  const Head64& H = head64();
+  Coop64& W = coop64();
+  const int lane = threadIdx.x & 31;
+  on = on && !ov;
+  auto place = [&](int i) {
+    const int a = ids ? ids[i] : i;
+    double x = r[3 * a], y = r[3 * a + 1], z = r[3 * a + 2];
+    if (old) {
+      x = x - old[0] + cen[0];
+      y = y - old[1] + cen[1];
+      z = z - old[2] + cen[2];
+    }
+    return make_double4_32a(x, y, z, S.q[a]);
+  };
+  if (!FULL && on)
+    for (int i = 0; i < nat && !ov; ++i) ov = vox_overlap64<SMEM>(B, H, B.c64, place(i));
+  const int most = __reduce_max_sync(0xffffffffu, on ? nat : 0);
+  for (int i0 = 0; i0 < most;) {
+    const bool mine = on && !ov && i0 < nat;
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (!m) break;
+    const int per = min(32 / __popc(m), most - i0);  // atoms of a lane in this batch
+    // the lanes' atoms that exist, packed
+    const int cnt = mine ? min(per, nat - i0) : 0;
+    int s0 = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, s0, o);
+      if (lane >= o) s0 += t;
+    }
+    const int nq = __shfl_sync(0xffffffffu, s0, 31);
+    s0 -= cnt;
+    for (int k = 0; k < cnt; ++k) {
+      const double4_32a p = place(i0 + k);
+      W.pos[s0 + k] = p;
+      W.posf[s0 + k] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.0f);
+      W.type[s0 + k] = S.type[ids ? ids[i0 + k] : i0 + k];
+      W.ov[s0 + k] = 0;
+    }
+    __syncwarp();
+    coop_eval64<SMEM, FULL>(B, nq, want_qq, pc);
+    for (int k = 0; k < cnt; ++k) {
+      if (W.ov[s0 + k]) ov = true;
+      e += W.sum[s0 + k];
+      if (eabs) *eabs += W.sabs[s0 + k];
+    }
+    __syncwarp();
+    i0 += per;
+  }
+}
+
+// One Widom insertion per lane that is `on`, as run_insertion in FP64: the queries are
+// the warp's, everything else is a lane's own.  The whole warp calls it.
+template <bool SMEM>
+__device__ void run_insertion_w(const WidomSpecies& S, const SpeciesPools& P, const PairTable& T, const CoopBox& B,
+                                bool on, const double* __restrict__ lib, Lfsr rng, WRec& rec, int& status,
+                                double* xyz_out, CassWidomTrace* tr, PairCount& pc) {
+  const BoxDev& b = head64().b;
+  const SpeciesDevHdr& H = P.hdr[S.is0];
+  const int n = S.natoms;
+  const double beta = b.beta;
+  double r[3 * kMaxAtoms];
+  unsigned exist = 0u;
+  double ln_pbias = 0.0, ln_pseq;
+  double first_sum = 0.0;
+  int selected = 0;
+  bool cbmc_overlap = !on;
+
+  // Step 1: first fragment and growth order (fragment_growth.f90:218-253, 1317-1446)
+  double u = rng.next();
+  int fstart = 0;
+  while (fstart < S.nfrag && !(u < S.cum_prob_ins[fstart])) ++fstart;
+  if (fstart >= S.nfrag) fstart = S.nfrag - 1;
+  ln_pseq = S.ln_prob_ins[fstart];
+  int order[kMaxFrags];
+  int norder = 1;
+  order[0] = fstart;
+  unsigned live = 1u << fstart;
+  if (S.nfrag > 1) {
+    int hang[kMaxFrags];
+    int nh = 0;
+    for (int k = 0; k < S.frag_nconnect[fstart]; ++k) {
+      int f = S.frag_connect[fstart][k];
+      if (!((live >> f) & 1u)) hang[nh++] = f;
+    }
+    while (nh > 0) {
+      double prob[kMaxFrags], cum[kMaxFrags];
+      for (int k = 0; k < nh; ++k) {
+        prob[k] = (double)(S.frag_natoms[hang[k]] - 2);
+        cum[k] = (k == 0 ? 0.0 : cum[k - 1]) + prob[k];
+      }
+      double tot = cum[nh - 1];
+      for (int k = 0; k < nh; ++k) {
+        prob[k] = prob[k] / tot;
+        cum[k] = cum[k] / tot;
+      }
+      double uu = rng.next();
+      int k = 0;
+      while (k < nh && !(uu < cum[k])) ++k;
+      if (k >= nh) k = nh - 1;
+      int f = hang[k];
+      ln_pseq = ln_pseq + log(prob[k]);
+      order[norder++] = f;
+      live |= 1u << f;
+      for (int q = k; q + 1 < nh; ++q) hang[q] = hang[q + 1];
+      --nh;
+      for (int q = 0; q < S.frag_nconnect[f]; ++q) {
+        int g = S.frag_connect[f][q];
+        if (!((live >> g) & 1u) && nh < kMaxFrags) hang[nh++] = g;
+      }
+    }
+  }
+
+  // Step 2: library conformation of the first fragment (:274-304)
+  const int nfa = S.frag_natoms[fstart];
+  {
+    int nconf = S.nconfig[fstart];
+    int conf = (int)(rng.next() * nconf);
+    if (conf >= nconf) conf = nconf - 1;
+    const double* L0 = lib + S.lib_off[fstart] + (size_t)conf * nfa * 3;
+    for (int i = 0; i < nfa; ++i) {
+      int a = S.frag_atoms[fstart][i];
+      r[3 * a] = L0[3 * i];
+      r[3 * a + 1] = L0[3 * i + 1];
+      r[3 * a + 2] = L0[3 * i + 2];
+      exist |= 1u << a;
+    }
+  }
+
+  // Step 3: Get_COM + Rotate_Molecule_Eulerian (rotation_routines.f90:41-137)
+  double com[3];
+  get_com(S, r, exist, com);
+  {
+    double theta = acos(1.0 - 2.0 * rng.next());
+    double phi = (1.0 - 2.0 * rng.next()) * kPI;
+    double psi = (1.0 - 2.0 * rng.next()) * kPI;
+    double st, ct, sp, cp, ss, cs;
+    sincos(theta, &st, &ct);
+    sincos(phi, &sp, &cp);
+    sincos(psi, &ss, &cs);
+    double r11 = cs * cp - ct * sp * ss, r12 = cs * sp + ct * cp * ss, r13 = ss * st;
+    double r21 = -ss * cp - ct * sp * cs, r22 = -ss * sp + ct * cp * cs, r23 = cs * st;
+    double r31 = st * sp, r32 = -st * cp, r33 = ct;
+    for (int i = 0; i < nfa; ++i) {
+      int a = S.frag_atoms[fstart][i];
+      double x = r[3 * a] - com[0], y = r[3 * a + 1] - com[1], z = r[3 * a + 2] - com[2];
+      r[3 * a] = (r11 * x + r12 * y + r13 * z) + com[0];
+      r[3 * a + 1] = (r21 * x + r22 * y + r23 * z) + com[1];
+      r[3 * a + 2] = (r31 * x + r32 * y + r33 * z) + com[2];
+    }
+  }
+
+  // Step 4: kappa_ins trial positions of the first fragment (:383-620)
+  const int ki = S.kappa_ins;
+  double nrg[kMaxKappa], w[kMaxKappa];
+  unsigned ovm = 0u;
+  double r0[3 * kMaxAtoms];
+  for (int i = 0; i < 3 * n; ++i) r0[i] = r[i];
+  const double com_old[3] = {com[0], com[1], com[2]};
+  Lfsr replay = rng;
+  for (int it = 0; it < ki; ++it) {
+    double ax = (0.5 - rng.next()) * b.L[0];
+    double ay = (0.5 - rng.next()) * b.L[1];
+    double az = (0.5 - rng.next()) * b.L[2];
+    double e = 0.0;
+    bool ov = false;
+    const double cen[3] = {ax, ay, az};
+    coop_atoms64<SMEM, false>(B, S, on, r0, S.frag_atoms[fstart], nfa, com_old, cen, S.want_qq_cbmc != 0, e, nullptr, ov,
+                              pc);
+    nrg[it] = e;
+    w[it] = 0.0;
+    if (ov) {
+      ovm |= 1u << it;
+    } else {
+      double nk = beta * nrg[it];
+      if (nk >= kMAX_KBT) {
+        ovm |= 1u << it;
+      } else {
+        w[it] = exp(-nk);
+        first_sum += nrg[it];
+      }
+    }
+    if (it > 0) w[it] = w[it - 1] + w[it];
+  }
+  int sel = -1;
+  if (!on || ovm == ((ki >= 32) ? 0xffffffffu : ((1u << ki) - 1u))) {
+    cbmc_overlap = true;
+  } else {
+    double rn = rng.next() * w[ki - 1];
+    int i = 0;
+    while (i < ki && !(rn < w[i])) ++i;
+    if (i == ki) cbmc_overlap = true;
+    else sel = i;
+  }
+  if (!cbmc_overlap) {
+    ln_pbias = ln_pbias - beta * nrg[sel] - log(w[ki - 1]);
+    double ax = 0, ay = 0, az = 0;
+    for (int k = 0; k <= sel; ++k) {
+      ax = (0.5 - replay.next()) * b.L[0];
+      ay = (0.5 - replay.next()) * b.L[1];
+      az = (0.5 - replay.next()) * b.L[2];
+    }
+    for (int i = 0; i < nfa; ++i) {
+      int a = S.frag_atoms[fstart][i];
+      r[3 * a] = r0[3 * a] - com_old[0] + ax;
+      r[3 * a + 1] = r0[3 * a + 1] - com_old[1] + ay;
+      r[3 * a + 2] = r0[3 * a + 2] - com_old[2] + az;
+    }
+    selected = sel + 1;
+  }
+
+  // Step 5: Fragment_Placement (:1449-2132)
+  if (S.nfrag > 1) {
+    double e_prev = cbmc_overlap ? 0.0 : dihedral_masked(H, P, r, exist);
+    unsigned placed = 1u << fstart;
+    const int kd = S.kappa_dih;
+    double dn[kMaxKappa], dd[kMaxKappa];
+    for (int oi = 1; oi < S.nfrag; ++oi) {
+      bool grow = !cbmc_overlap && oi < norder;  // this lane places a fragment
+      if (!__any_sync(0xffffffffu, grow)) break;
+      const int f = order[grow ? oi : 0];
+      const int nf = S.frag_natoms[f];
+      unsigned grown = exist;
+      int nconf = S.nconfig[f];
+      int cf = 0;
+      if (grow) {
+        rng.next();
+        cf = (int)(rng.next() * nconf);  // the duplicated draw of fragment_growth.f90:1578,1584
+        if (cf >= nconf) cf = nconf - 1;
+      }
+      double cfg[3 * kMaxAtoms];
+      const double* Lf = lib + S.lib_off[f] + (size_t)cf * nf * 3;
+      for (int j = 0; j < nf; ++j) {
+        int a = S.frag_atoms[f][j];
+        if (grow) exist |= 1u << a;
+        cfg[3 * a] = Lf[3 * j];
+        cfg[3 * a + 1] = Lf[3 * j + 1];
+        cfg[3 * a + 2] = Lf[3 * j + 2];
+      }
+      const unsigned combined = exist;
+      signed char newids[kMaxAtoms];
+      int nnew = 0;
+      for (int a = 0; a < n; ++a)
+        if (((combined & ~grown) >> a) & 1u) newids[nnew++] = (signed char)a;
+      int fc = -1;
+      for (int q = 0; q < S.frag_nconnect[f]; ++q) {
+        int g = S.frag_connect[f][q];
+        if ((placed >> g) & 1u) {
+          fc = g;
+          break;
+        }
+      }
+      if (fc < 0) {  // no placed neighbour: the fragment graph is not connected
+        if (grow) cbmc_overlap = true;
+        grow = false;
+        fc = f;
+      }
+      const int anc_i = S.frag_atoms[f][0], anc_c = S.frag_atoms[fc][0];
+      int ids[kMaxAtoms], nid = 0;
+      for (int j = 0; j < nf; ++j) {
+        int a = S.frag_atoms[f][j];
+        if (a != anc_i && a != anc_c) ids[nid++] = a;
+      }
+      unsigned idmask = 0u;
+      for (int j = 0; j < nid; ++j) idmask |= 1u << ids[j];
+      int atom_ifrag = nid > 0 ? ids[0] : S.frag_atoms[f][nf - 1];
+      int atom_fc = S.frag_atoms[fc][S.frag_natoms[fc] - 1];
+      for (int j = 0; j < S.frag_natoms[fc]; ++j) {
+        int a = S.frag_atoms[fc][j];
+        if (a != anc_i && a != anc_c) {
+          atom_fc = a;
+          break;
+        }
+      }
+      double v1[3], v2[3], al_i[9], hg_i[9], al_c[9], hg_c[9];
+      for (int d = 0; d < 3; ++d) {
+        v1[d] = cfg[3 * anc_i + d] - cfg[3 * anc_c + d];
+        v2[d] = cfg[3 * atom_ifrag + d] - cfg[3 * anc_c + d];
+      }
+      aligner_hanger(v1, v2, al_i, hg_i);
+      for (int d = 0; d < 3; ++d) {
+        v1[d] = r[3 * anc_i + d] - r[3 * anc_c + d];
+        v2[d] = r[3 * atom_fc + d] - r[3 * anc_c + d];
+      }
+      aligner_hanger(v1, v2, al_c, hg_c);
+      const double tx = cfg[3 * anc_c], ty = cfg[3 * anc_c + 1], tz = cfg[3 * anc_c + 2];
+      for (int j = 0; j < nf; ++j) {
+        int a = S.frag_atoms[f][j];
+        double x = cfg[3 * a] - tx, y = cfg[3 * a + 1] - ty, z = cfg[3 * a + 2] - tz;
+        cfg[3 * a] = x * al_i[0] + y * al_i[1] + z * al_i[2];
+        cfg[3 * a + 1] = x * al_i[3] + y * al_i[4] + z * al_i[5];
+        cfg[3 * a + 2] = x * al_i[6] + y * al_i[7] + z * al_i[8];
+      }
+      const double theta0 = grow ? kTWOPI * rng.next() : 0.0;
+      const double dtheta = kTWOPI / (double)kd;
+      unsigned dov = 0u;
+      double dw[kMaxKappa];
+      double theta = theta0;
+      for (int ii = 0; ii < kd; ++ii) {
+        if (ii > 0) theta = theta + dtheta;
+        double sth, cth;
+        sincos(theta, &sth, &cth);
+        for (int j = 0; grow && j < nid; ++j) {
+          int a = ids[j];
+          double x = cfg[3 * a], y = cfg[3 * a + 1], z = cfg[3 * a + 2];
+          double yr = cth * y + sth * z, zr = -sth * y + cth * z;
+          r[3 * a] = (x * hg_c[0] + yr * hg_c[1] + zr * hg_c[2]) + r[3 * anc_c];
+          r[3 * a + 1] = (x * hg_c[3] + yr * hg_c[4] + zr * hg_c[5]) + r[3 * anc_c + 1];
+          r[3 * a + 2] = (x * hg_c[6] + yr * hg_c[7] + zr * hg_c[8]) + r[3 * anc_c + 2];
+        }
+        dn[ii] = 0.0;
+        dd[ii] = 0.0;
+        double niv = 0.0, niq = 0.0, noq = 0.0;
+        bool ov = !grow;
+        if (grow) exist &= ~idmask;
+        for (int j = 0; j < nid && !ov; ++j) {
+          exist |= 1u << ids[j];
+          double eiv, eiq, eoq;
+          if (atom_intra(H, P, b, T, ids[j], r, exist, eiv, eiq, eoq)) {
+            ov = true;
+            break;
+          }
+          niv += eiv;
+          niq += eiq;
+          noq += eoq;
+        }
+        double einter = 0.0;
+        coop_atoms64<SMEM, false>(B, S, grow, r, newids, nnew, nullptr, nullptr, S.want_qq_cbmc != 0, einter, nullptr, ov,
+                                  pc);
+        exist = combined;
+        if (ov) {
+          dw[ii] = 0.0;
+          dov |= 1u << ii;
+        } else {
+          double ed = dihedral_masked(H, P, r, exist);
+          dd[ii] = ed;
+          dn[ii] = ed + niv + niq + einter + noq - e_prev;
+          double nk = beta * dn[ii];
+          if (nk >= kMAX_KBT) {
+            dw[ii] = 0.0;
+            dov |= 1u << ii;
+          } else {
+            dw[ii] = exp(-nk);
+          }
+        }
+        if (ii > 0) dw[ii] = dw[ii - 1] + dw[ii];
+      }
+      if (!grow) continue;
+      if (dov == ((kd >= 32) ? 0xffffffffu : ((1u << kd) - 1u))) {
+        cbmc_overlap = true;
+        continue;
+      }
+      double pp = rng.next() * dw[kd - 1];
+      int trl = 0;
+      while (trl < kd && !(pp < dw[trl])) ++trl;
+      if (trl == kd) {
+        cbmc_overlap = true;
+        continue;
+      }
+      ln_pbias = ln_pbias - beta * dn[trl] - log(dw[kd - 1]);
+      theta = theta0;
+      for (int ii = 1; ii <= trl; ++ii) theta = theta + dtheta;
+      double sth, cth;
+      sincos(theta, &sth, &cth);
+      for (int j = 0; j < nid; ++j) {
+        int a = ids[j];
+        double x = cfg[3 * a], y = cfg[3 * a + 1], z = cfg[3 * a + 2];
+        double yr = cth * y + sth * z, zr = -sth * y + cth * z;
+        r[3 * a] = (x * hg_c[0] + yr * hg_c[1] + zr * hg_c[2]) + r[3 * anc_c];
+        r[3 * a + 1] = (x * hg_c[3] + yr * hg_c[4] + zr * hg_c[5]) + r[3 * anc_c + 1];
+        r[3 * a + 2] = (x * hg_c[6] + yr * hg_c[7] + zr * hg_c[8]) + r[3 * anc_c + 2];
+      }
+      e_prev = dd[trl];
+      placed |= 1u << f;
+    }
+    if (!cbmc_overlap) get_com(S, r, exist, com);
+  }
+
+  // widom_insert.f90:350-447
+  ln_pbias = ln_pbias + ln_pseq;
+  ln_pbias = ln_pbias + S.ln_kappa_ins;
+  ln_pbias = ln_pbias + S.ln_kappa_dih_term;
+  if (on && tr) {
+    tr->ln_pbias = ln_pbias;
+    tr->e_first_trial_sum = first_sum;
+    tr->selected_trial = selected;
+    tr->e_inter = 0.0;
+    tr->e_inter_abs = 0.0;
+  }
+  rec = make_double4_32a(0.0, 0.0, 0.0, ln_pbias);
+  if (!cbmc_overlap && S.nfrag > 1) {  // Fold_Molecule, orthorhombic branch
+    for (int d = 0; d < 3; ++d) {
+      if (com[d] > b.hL[d]) {
+        com[d] = com[d] - b.L[d];
+        for (int a = 0; a < n; ++a) r[3 * a + d] -= b.L[d];
+      } else if (com[d] < -b.hL[d]) {
+        com[d] = com[d] + b.L[d];
+        for (int a = 0; a < n; ++a) r[3 * a + d] += b.L[d];
+      }
+    }
+  }
+  double e_inter = 0.0, e_abs = 0.0;
+  bool ov = false;
+  coop_atoms64<SMEM, true>(B, S, !cbmc_overlap, r, nullptr, n, nullptr, nullptr, true, e_inter, &e_abs, ov, pc);
+  if (cbmc_overlap || ov) {
+    status = cbmc_overlap ? 1 : 2;
+    return;
+  }
+  IntraOut io = molecule_intra(P, S.is0, b, T, r);
+  if (io.overlap) {
+    status = 3;
+    return;
+  }
+  e_inter = e_inter + io.pqq;
+  double dE_inter = e_inter + b.e_inter_constant;
+  double dE_intra = io.ivdw + io.iqq;
+  dE_intra = dE_intra + io.bond + io.angle + io.dih + io.imp;
+  rec = make_double4_32a(dE_intra, dE_inter, io.angle, ln_pbias);
+  status = 0;
+  if (tr) {
+    tr->e_inter = e_inter;
+    tr->e_inter_abs = e_abs;
+  }
+  if (xyz_out)
+    for (int i = 0; i < 3 * n; ++i) xyz_out[i] = r[i];
+}
+
+// FP64 kernel, a lane per insertion and the warp's queries together (the reference's
+// arithmetic); per_warp: insertions a warp works on at a time.
+// 16 boxes x 1,000 butane insertions: 2.2 ms against 21.4 ms with a thread per
+// insertion (k_widom, which remains for what the lists do not serve: CBMC options, the
+// molecule-pair cutoff, styles without a cutoff).
+template <bool SMEM>
+__global__ void __launch_bounds__(kThreads64, 1) k_widom_w(const __grid_constant__ WidomSpecies S,
+                                                        const __grid_constant__ PairTable T,
+                                                        const __grid_constant__ SpeciesPools P, const BoxDev* boxes,
+                                                        const int* box_ids, const double4_32a* c64, const float4* c32,
+                                                        const VoxGrid* vox, const uint4* vrec, const uint4* vlist,
+                                                        const double* __restrict__ lib, long long n_ins, uint64_t seed,
+                                                        int per_warp, WRec* rec, signed char* status, double* xyz,
+                                                        int want_xyz, CassWidomTrace* trace,
+                                                        unsigned long long* pair_counts) {
+  Head64& H = head64();
+  const int k = blockIdx.y;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    H.b = boxes[k];
+    const BoxDev& b = H.b;
+    widom_boxf(H.f, b, 1.0);
+    const double lmax = fmax(b.L[0], fmax(b.L[1], b.L[2]));
+    auto above = [&](double r2) { return (float)(r2 * (1.0 + 1.0e-4) + 1.0e-3 + 2.0e-6 * lmax * sqrt(r2)); };
+    H.pre[0] = above(fmax(b.rcut_cbmcsq, b.rcut_lowsq));
+    double full = fmax(fmax(b.rcut_vdwsq, b.rcut_coulsq), b.rcut_lowsq);
+    if (b.vdw_sum_style == CASS_VDW_SUM_CUT_SWITCH) full = fmax(full, b.roff_switch_sq);
+    H.pre[1] = above(full);
+    H.low_pre = above(b.rcut_lowsq);
+    H.low_sure = (float)(2.0 * b.rcut_lowsq) - H.low_pre;
+    for (int d = 0; d < 3; ++d) {
+      H.edge_lo[d] = (float)(b.hL[d] * (1.0 - 1.0e-5));
+      H.edge_hi[d] = (float)(b.hL[d] * (1.0 + 1.0e-5));
+    }
+  }
+  if (threadIdx.x < 2) H.vox[threadIdx.x] = vox[2 * k + threadIdx.x];
+  for (int q = threadIdx.x; q < 125; q += blockDim.x) {
+    const double4_32a v = make_double4_32a((q % 5 - 2) * boxes[k].L[0], (q / 5 % 5 - 2) * boxes[k].L[1],
+                                           (q / 25 - 2) * boxes[k].L[2], 0.0);
+    H.shift64[q] = v;
+    H.shift[q] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.0f);
+  }
+  for (int i = threadIdx.x; i < kMaxTypes * kMaxTypes; i += blockDim.x) {
+    const int a = i / kMaxTypes, c = i % kMaxTypes;
+    const bool ok = a < T.ntypes && c < T.ntypes;
+    H.lj[i] = ok ? make_double2(T.eps[pidx(a, c, T.ntypes)], T.sig2[pidx(a, c, T.ntypes)]) : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  CoopBox B;
+  B.vrec = vrec;
+  B.vlist = vlist;
+  B.p32 = c32 + H.b.atom_off;
+  B.c64 = c64 + H.b.atom_off;
+  B.T = &T;
+  B.off_atoms = kHead64Bytes + (blockDim.x >> 5) * (unsigned)sizeof(Coop64);
+  if (SMEM) {
+    float4* s32 = reinterpret_cast<float4*>(smem + B.off_atoms);
+    for (int j = threadIdx.x; j < H.b.natoms; j += blockDim.x) s32[j] = B.p32[j];
+    __syncthreads();
+  }
+  PairCount pc;
+  const long long warps = blockDim.x >> 5;
+  for (long long first = (blockIdx.x * warps + (threadIdx.x >> 5)) * per_warp; first < n_ins;
+       first += gridDim.x * warps * per_warp) {
+    const long long i = first + lane;
+    const bool on = lane < per_warp && i < n_ins;
+    const size_t g = (size_t)k * n_ins + i;
+    WRec rr;
+    int st = 0;
+    run_insertion_w<SMEM>(S, P, T, B, on, lib, seed_stream(seed, box_ids[k], i), rr, st,
+                          want_xyz && on ? xyz + g * 3 * S.natoms : nullptr, trace && on ? trace + g : nullptr, pc);
+    __syncwarp();
+    if (!on) continue;
+    rec[g] = rr;
+    status[g] = (signed char)st;
+    if (trace) trace[g].overlap = st;
+  }
+  if (pair_counts) {
+    atomicAdd(&pair_counts[0], pc.visited);
+    atomicAdd(&pair_counts[1], pc.in_cut);
+  }
+}
+
 // E_recip of each surviving insertion (absolute, as the reference computes it)
 __global__ void __launch_bounds__(256) k_widom_recip(const BoxDev* boxes, const double4_32a* kvec_all,
                                                      const double* cos_all, const double* sin_all,
@@ -2651,6 +3354,73 @@ int pack_box_ext(cass_ctx* c, int ibox);
 const std::vector<int>& members_ext(cass_ctx* c, int ibox);
 }  // namespace cassgpu
 
+namespace {
+
+// The voxel grid `which` (0 CBMC, 1 full) of box b for queries of radius rc: record
+// offset off; room: entries it can need.  False where an entry cannot describe the box.
+bool vox_grid(const BoxDev& b, int which, double rc, int off, VoxGrid& g, double& nvox, double& room) {
+  memset(&g, 0, sizeof(g));
+  if (b.natoms < 1 || b.natoms > (int)kVoxAtomMask || !(rc > 0.0)) return false;
+  const double edge = rc / (which ? kVoxPerCutoffFull : kVoxPerCutoffCbmc);
+  const double lmax = std::max(b.L[0], std::max(b.L[1], b.L[2])), lmin = std::min(b.L[0], std::min(b.L[1], b.L[2]));
+  double diag2 = 0.0, most = 1.0;
+  nvox = 1.0;
+  for (int d = 0; d < 3; ++d) {
+    g.nv[d] = (int)std::min(1024.0, std::ceil(b.L[d] / edge));
+    g.inv[d] = (float)(g.nv[d] / b.L[d]);
+    g.edge[d] = (float)(b.L[d] / g.nv[d]);
+    diag2 += (double)g.edge[d] * g.edge[d];
+    nvox *= g.nv[d];
+  }
+  // half a diagonal, with a margin above the FP32 rounding of the coordinates
+  const double half = 0.5 * std::sqrt(diag2) + 2.0e-3 + 4.0e-6 * lmax, R = rc + half;
+  for (int d = 0; d < 3; ++d) most *= 2.0 * (R + half) / g.edge[d] + 1.0;
+  // entries of an atom: at most the voxels in the sphere of R and another half diagonal
+  const double per_atom = std::min(most, 4.18879021 * std::pow(R + half, 3.0) * nvox / b.volume);
+  room = b.natoms * per_atom + 3.0 * nvox;
+  g.R2 = (float)(R * R);
+  const double near = std::sqrt(b.rcut_lowsq) + half;
+  g.near2 = (float)(near * near);
+  g.off = off;
+  // images of the neighbouring boxes only; a list of 2e4 atoms is no neighbour list
+  return R < 0.95 * lmin && nvox <= 1.0e8 && 4.18879021 * R * R * R * b.natoms / b.volume <= 2.0e4;
+}
+
+double full_radius(const BoxDev& b) {
+  double r2 = std::max(b.rcut_vdwsq, b.rcut_coulsq);
+  if (b.vdw_sum_style == CASS_VDW_SUM_CUT_SWITCH) r2 = std::max(r2, b.roff_switch_sq);
+  return std::sqrt(std::max(r2, b.rcut_lowsq));
+}
+
+// True where the FP64 insertions run on the voxel lists (k_widom_w): every style has a
+// cutoff, no CBMC option and no molecule-pair cutoff asks for more than the atoms within
+// it, and the boxes can be listed
+bool lists64(cass_ctx* c, int nboxes, const int32_t* iboxes) {
+  if (c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap) return false;
+  double total = 0.0;
+  for (int k = 0; k < nboxes; ++k) {
+    const BoxH& B = c->box[iboxes[k] - 1];
+    const CassBoxDesc& d = B.desc;
+    if (B.comcut || (d.vdw_style != CASS_VDW_NONE &&
+                     (d.vdw_sum_style == CASS_VDW_SUM_MINIMUM || d.vdw_sum_style == CASS_VDW_SUM_CHARMM)) ||
+        (d.charge_style == CASS_CHARGE_COUL && d.charge_sum_style == CASS_QQ_MINIMUM))
+      return false;
+    BoxDev b = B.dev;
+    b.natoms = B.npacked;
+    if (b.natoms == 0) continue;
+    if (!(b.rcut_cbmcsq >= b.rcut_lowsq)) return false;
+    for (int w = 0; w < 2; ++w) {
+      VoxGrid g;
+      double nvox, room;
+      if (!vox_grid(b, w, w ? full_radius(b) : std::sqrt(b.rcut_cbmcsq), 0, g, nvox, room)) return false;
+      total += room;
+    }
+  }
+  return total * sizeof(unsigned) <= kVoxMaxBytes;
+}
+
+}  // namespace
+
 static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
                                  int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
                                  CassWidomTrace* trace) {
@@ -2694,14 +3464,20 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   // the FP32 warp kernel covers LJ cut / cut_tail with no charges or Ewald
   bool fast_mixed = c->pt.ntypes <= kMaxTypes;
   for (int k = 0; k < nboxes; ++k) {
+    if ((rc = pack_box_ext(c, iboxes[k] - 1))) return rc;
+    const CassBoxDesc& d = c->box[iboxes[k] - 1].desc;
+    fast_mixed = fast_mixed && d.vdw_style == CASS_VDW_LJ &&
+                 (d.vdw_sum_style == CASS_VDW_SUM_CUT || d.vdw_sum_style == CASS_VDW_SUM_CUT_TAIL) &&
+                 (d.charge_style == CASS_CHARGE_NONE || d.charge_sum_style == CASS_QQ_EWALD);
+  }
+  SpeciesF SF;
+  const bool f32 = mixed && fast_mixed && species_f(s, SF);
+  const bool warp64 = !f32 && lists64(c, nboxes, iboxes);
+  for (int k = 0; k < nboxes; ++k) {
     int ib = iboxes[k] - 1;
-    if ((rc = pack_box_ext(c, ib))) return rc;
     BoxH& B = c->box[ib];
     BoxDev v = B.dev;
-    // cells of about half the CBMC cutoff: the row-trimmed stencils then visit
-    // little more than the cutoff sphere
-    const double cpc = c->widom_cells > 0.0 ? c->widom_cells
-                                             : (c->precision == CASS_PREC_MIXED ? kCellsPerCutoffMixed : kCellsPerCutoffFP64);
+    const double cpc = c->widom_cells > 0.0 ? c->widom_cells : (f32 || warp64 ? kCellsPerCutoffMixed : kCellsPerCutoffFP64);
     double rcell = (B.desc.rcut_cbmc > 0.0 ? B.desc.rcut_cbmc : B.rcut_max) / cpc;
     int ncell = 1;
     for (int d = 0; d < 3; ++d) {
@@ -2743,9 +3519,6 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
       e_recip_in = B.energy.reciprocal;
     }
     v.e_inter_constant = lrc_diff + e_self - e_recip_in;
-    fast_mixed = fast_mixed && B.desc.vdw_style == CASS_VDW_LJ &&
-                 (B.desc.vdw_sum_style == CASS_VDW_SUM_CUT || B.desc.vdw_sum_style == CASS_VDW_SUM_CUT_TAIL) &&
-                 (B.desc.charge_style == CASS_CHARGE_NONE || B.desc.charge_sum_style == CASS_QQ_EWALD);
     if (B.desc.charge_style == CASS_CHARGE_COUL && B.desc.charge_sum_style == CASS_QQ_EWALD && s.has_charge &&
         B.nvecs > 0) {
       has_ew[k] = 1;
@@ -2778,7 +3551,7 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   if ((rc = c->d_cq32.reserve((size_t)total_atoms * sizeof(float)))) return rc;
   if ((rc = c->d_cell_start.reserve(((size_t)total_cells + nboxes) * sizeof(int)))) return rc;
   if ((rc = c->d_cell_count.reserve(((size_t)total_cells * 2 + 64) * sizeof(int)))) return rc;
-  if ((rc = c->d_cell_of.reserve((size_t)total_atoms * sizeof(int)))) return rc;
+  if ((rc = c->d_cell_of.reserve((size_t)total_atoms * 2 * sizeof(int)))) return rc;
   float4* d_c32 = c->d_c32.as<float4>();
   int* d_ctype = reinterpret_cast<int*>(d_c32 + total_atoms);
   int* d_corig = d_ctype + total_atoms;
@@ -2796,13 +3569,10 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     dim3 g((max_na + 255) / 256, nboxes);
     k_cell_count<<<g, 256, 0, c->stream>>>(d_src, d_bd, c->d_cell_of.as<int>(), d_count);
     k_cell_scan<<<nboxes, 1024, 0, c->stream>>>(d_bd, d_count, c->d_cell_start.as<int>(), d_fill);
-    k_cell_scatter<<<g, 256, 0, c->stream>>>(d_src, d_bd, c->d_cell_of.as<int>(), c->d_cell_start.as<int>(), d_fill,
-                                             c->d_c64.as<double4_32a>(), d_c32, d_ctype, c->d_cq32.as<float>(), d_corig);
-    int maxc = 1;
-    for (int k = 0; k < nboxes; ++k) maxc = std::max(maxc, bd[k].nc[0] * bd[k].nc[1] * bd[k].nc[2]);
-    dim3 gs((maxc + 127) / 128, nboxes);
-    k_cell_sort<<<gs, 128, 0, c->stream>>>(d_bd, nboxes, c->d_cell_start.as<int>(), c->d_c64.as<double4_32a>(), d_c32,
-                                           d_ctype, c->d_cq32.as<float>(), d_corig);
+    int* d_cell_of = c->d_cell_of.as<int>();
+    k_cell_scatter<<<g, 256, 0, c->stream>>>(d_bd, d_cell_of, c->d_cell_start.as<int>(), d_fill, d_cell_of + total_atoms);
+    k_cell_place<<<g, 256, 0, c->stream>>>(d_src, d_bd, d_cell_of, c->d_cell_start.as<int>(), d_cell_of + total_atoms,
+                                           c->d_c64.as<double4_32a>(), d_c32, d_ctype, c->d_cq32.as<float>(), d_corig);
   } else {
     k_cell_scan<<<nboxes, 1024, 0, c->stream>>>(d_bd, d_count, c->d_cell_start.as<int>(), d_fill);
   }
@@ -2832,8 +3602,6 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   if (d_pairs) CASS_CUDA(cudaMemsetAsync(d_pairs, 0, 2 * sizeof(unsigned long long), c->stream));
   // K8 launch shape: 128-thread CTAs, enough CTAs per box to fill every SM;
   // the box is staged in shared memory when it fits
-  SpeciesF SF;
-  const bool f32 = mixed && fast_mixed && species_f(s, SF);
   const size_t max_smem = max_smem64;
   const bool use_smem = max_smem <= (size_t)200 * 1024;
   int dev_sms = 0;
@@ -2865,62 +3633,116 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   // queued (both inside the kernel timing)
   int* d_fixn = nullptr;
   FixEntry* d_fixq = nullptr;
-  // Voxel lists: per box and radius, where the query's stencil never spans the box (the
-  // cell search then sees every pair through one image shift, as an entry does) and the
-  // insertions' queries are worth the lists: a list costs about as much as the cell
-  // search of a query, and 32 of an insertion's queries (4 full-cutoff ones) use them
+  // Voxel lists per box and radius.  FP64: everywhere.  Mixed: where the query's stencil
+  // never spans the box (the cell search then sees every pair through one image shift, as
+  // an entry does) and the insertions' queries are worth the lists: a list costs about as
+  // much as the cell search of a query, and 32 of an insertion's queries (4 full-cutoff
+  // ones) use them
   std::vector<VoxGrid> vox(2 * nboxes);
   size_t vox_records = 0;
   double vox_entries = 0.0;
   int vox_most[2] = {0, 0};
+  memset(vox.data(), 0, vox.size() * sizeof(VoxGrid));
   const bool opt_cbmc = c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap;
-  if (f32 && !opt_cbmc && n_ins > 0)
+  if (((f32 && !opt_cbmc) || warp64) && n_ins > 0)
     for (int k = 0; k < nboxes; ++k) {
       const BoxDev& b = bd[k];
       const double rfull2 = std::max(b.rcut_vdwsq, b.rcut_coulsq);
-      // the full-cutoff pass also looks at the pairs of the bands (widom_boxf) outside its cutoffs
+      // the mixed full-cutoff pass also looks at the pairs of the bands (widom_boxf) outside its cutoffs
       const double band = 3.5 * std::sqrt(rfull2) * 5.0e-7 * (std::max(b.L[0], std::max(b.L[1], b.L[2])) + 20.0) *
                               c->widom_band + 1.0e-6 * rfull2;
-      const double rcs[2] = {std::sqrt(b.rcut_cbmcsq), std::sqrt(rfull2 + band)};
+      const double rcs[2] = {std::sqrt(b.rcut_cbmcsq), f32 ? std::sqrt(rfull2 + band) : full_radius(b)};
       for (int w = 0; w < 2; ++w) {
-        VoxGrid& g = vox[2 * k + w];
-        memset(&g, 0, sizeof(g));
-        if (b.natoms < 1 || b.natoms > (int)kVoxAtomMask || !(rcs[w] > 0.0)) continue;
-        const double edge = rcs[w] / (w ? kVoxPerCutoffFull : kVoxPerCutoffCbmc);
-        bool open = true;
-        double diag2 = 0.0, nvox = 1.0, most = 1.0;
-        for (int d = 0; d < 3; ++d) {
-          g.nv[d] = (int)std::min(1024.0, std::ceil(b.L[d] / edge));
-          g.inv[d] = (float)(g.nv[d] / b.L[d]);
-          g.edge[d] = (float)(b.L[d] / g.nv[d]);
-          diag2 += (double)g.edge[d] * g.edge[d];
-          nvox *= g.nv[d];
-          open = open && std::floor(2.0 * rcs[w] * b.cell_inv[d] + 8.0e-3) + 2.0 < b.nc[d];
+        VoxGrid g;
+        double nvox, room;
+        if (!vox_grid(b, w, rcs[w], (int)vox_records, g, nvox, room)) continue;
+        if (f32) {
+          bool open = (double)n_ins * (w ? 2.0 : 32.0) >= nvox;
+          for (int d = 0; d < 3; ++d)
+            open = open && std::floor(2.0 * rcs[w] * b.cell_inv[d] + 8.0e-3) + 2.0 < b.nc[d];
+          if (!open || (vox_entries + room) * sizeof(unsigned) > kVoxMaxBytes) continue;
         }
-        // half a diagonal, with a margin above the FP32 rounding of the coordinates
-        const double lmax = std::max(b.L[0], std::max(b.L[1], b.L[2]));
-        const double half = 0.5 * std::sqrt(diag2) + 2.0e-3 + 4.0e-6 * lmax, R = rcs[w] + half;
-        for (int d = 0; d < 3; ++d) {
-          open = open && R < 0.5 * b.L[d] + 0.25 * rcs[w];
-          most *= 2.0 * (R + half) / g.edge[d] + 1.0;
-        }
-        // entries of an atom: at most the voxels in the sphere of R and another half diagonal
-        const double per_atom = std::min(most, 4.18879021 * std::pow(R + half, 3.0) * nvox / b.volume);
-        const double room = b.natoms * per_atom + 3.0 * nvox;
-        const double rho_list = 4.18879021 * R * R * R * b.natoms / b.volume;
-        if (!open || nvox > 1.0e8 || rho_list > 2.0e4 || (double)n_ins * (w ? 2.0 : 32.0) < nvox ||
-            (vox_entries + room) * sizeof(unsigned) > kVoxMaxBytes)
-          continue;
-        g.R2 = (float)(R * R);
-        const double near = std::sqrt(b.rcut_lowsq) + half;
-        g.near2 = (float)(near * near);
-        g.off = (int)vox_records;
         g.on = 1;
+        vox[2 * k + w] = g;
         vox_records += (size_t)nvox;
         vox_entries += room;
         vox_most[w] = std::max(vox_most[w], (int)nvox);
       }
     }
+  // their device arrays, built from the cell lists; `need`: an error where there is no room
+  VoxGrid* d_vox = nullptr;
+  uint4* d_vrec = nullptr;
+  unsigned* d_vlist = nullptr;
+  auto build_lists = [&](bool need) -> int {
+    const size_t vox_head = ((2 * (size_t)nboxes * sizeof(VoxGrid) + sizeof(unsigned long long) + 255) & ~(size_t)255);
+    const size_t vox_rec = (vox_records * sizeof(uint4) + 255) & ~(size_t)255;
+    int rc2 = c->d_vox.reserve(vox_head + vox_rec + (size_t)vox_entries * sizeof(unsigned) + 256);
+    if (rc2) {
+      cudaGetLastError();  // no room for the lists: the cell search serves every query
+      if (need) return rc2;
+      for (VoxGrid& g : vox) g.on = 0;
+      vox_most[0] = vox_most[1] = 0;
+      if ((rc2 = c->d_vox.reserve(vox_head))) return rc2;
+    }
+    unsigned char* vb = c->d_vox.as<unsigned char>();
+    d_vox = reinterpret_cast<VoxGrid*>(vb);
+    unsigned long long* d_cursor = reinterpret_cast<unsigned long long*>(vb + 2 * (size_t)nboxes * sizeof(VoxGrid));
+    d_vrec = reinterpret_cast<uint4*>(vb + vox_head);
+    d_vlist = reinterpret_cast<unsigned*>(vb + vox_head + vox_rec);
+    CASS_CUDA(h2d(c, d_vox, vox.data(), vox.size() * sizeof(VoxGrid)));
+    CASS_CUDA(cudaMemsetAsync(d_cursor, 0, sizeof(unsigned long long), c->stream));
+    CASS_CUDA(cudaEventRecord(c->ev[1], c->stream));
+    for (int w = 0; w < 2; ++w)
+      if (vox_most[w] > 0) {
+        k_vox_lists<<<dim3((vox_most[w] + 127) / 128, nboxes), 128, 0, c->stream>>>(
+            d_bd, d_vox, w, d_c32, c->d_cell_start.as<int>(), d_vrec, d_vlist, d_cursor);
+        CASS_CUDA(cudaGetLastError());
+        count_launch(c);
+      }
+    return CASS_OK;
+  };
+  // The launch of a warp-wide kernel: insertions per warp, as few as give every warp of
+  // the GPU work at once, up to one per lane; then one group of insertions per warp: a
+  // CTA is as long as its slowest warp and the hardware hands out the CTAs; in very
+  // large calls several, to stage the box less often
+  int per_warp = 1, wthreads = 32;
+  auto warp_grid = [&](int warps) {
+    while (per_warp < 32 && (n_ins + per_warp - 1) / per_warp * nboxes > (long long)dev_sms * warps) per_warp *= 2;
+    const long long groups = (n_ins + per_warp - 1) / per_warp;
+    wthreads = 32 * (int)std::min<long long>(warps, std::max<long long>(1, (groups * nboxes + dev_sms - 1) / dev_sms));
+    const long long need = (groups + wthreads / 32 - 1) / (wthreads / 32);
+    const long long most = std::max<long long>(1, (long long)dev_sms * kF32Waves / nboxes);
+    const long long turns = (need + most - 1) / most;
+    const int chunks = (int)std::max<long long>(1, (need + turns - 1) / turns);
+    c->stats.widom_grid_x = chunks;
+    c->stats.widom_grid_y = nboxes;
+    c->stats.widom_block = wthreads;
+    return dim3(chunks, nboxes);
+  };
+  // FP64 kernel on the lists; no room for them: a negative status, and the thread-per-insertion kernel serves the call
+  auto launch_w64 = [&]() -> int {
+    int rc2 = build_lists(true);
+    if (rc2) return rc2;
+    const size_t box = (size_t)std::max(1, max_na) * sizeof(float4);
+    auto dyn_of = [&](int warps, bool staged) { return kHead64Bytes + warps * sizeof(Coop64) + (staged ? box : 0); };
+    int warps = kThreads64 / 32;
+    while (warps > 4 && dyn_of(warps, true) > kSmemMax) warps /= 2;
+    const bool staged = dyn_of(warps, true) <= kSmemMax;
+    if (!staged) warps = kThreads64 / 32;
+    const size_t dyn = dyn_of(warps, staged);
+    auto kern = staged ? k_widom_w<true> : k_widom_w<false>;
+    CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    const dim3 g = warp_grid(warps);
+    c->stats.widom_smem_bytes = (int)dyn;
+    kern<<<g, wthreads, dyn, c->stream>>>(S, c->pt, c->pools, d_bd, d_ids, c->d_c64.as<double4_32a>(), d_c32, d_vox,
+                                          d_vrec, reinterpret_cast<const uint4*>(d_vlist), s.d_library.as<double>(),
+                                          (long long)n_ins, seed, per_warp, d_rec, d_status, d_xyz, any_recip ? 1 : 0,
+                                          d_trace, d_pairs);
+    CASS_CUDA(cudaGetLastError());
+    CASS_CUDA(cudaEventRecord(c->ev[2], c->stream));
+    count_launch(c);
+    return CASS_OK;
+  };
   // warps per CTA: as many as fit beside the staged box
   auto smem_f32 = [&](int warps, bool box) { return kCoopHeadBytes + warps * sizeof(CoopWarp) + (box ? max_smem32 : 0); };
   int warps32 = kF32Threads / 32;
@@ -2934,47 +3756,12 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     d_fixn = c->d_widom_fix.as<int>();
     d_fixq = reinterpret_cast<FixEntry*>(c->d_widom_fix.as<unsigned char>() + fix_off);
     CASS_CUDA(cudaMemsetAsync(d_fixn, 0, (size_t)nboxes * sizeof(int), c->stream));
-    const size_t vox_head = ((2 * (size_t)nboxes * sizeof(VoxGrid) + sizeof(unsigned long long) + 255) & ~(size_t)255);
-    const size_t vox_rec = (vox_records * sizeof(uint4) + 255) & ~(size_t)255;
-    if (c->d_vox.reserve(vox_head + vox_rec + (size_t)vox_entries * sizeof(unsigned) + 256)) {
-      cudaGetLastError();  // no room for the lists: the cell search serves every query
-      for (VoxGrid& g : vox) g.on = 0;
-      vox_most[0] = vox_most[1] = 0;
-      if ((rc2 = c->d_vox.reserve(vox_head))) return rc2;
-    }
-    unsigned char* vb = c->d_vox.as<unsigned char>();
-    VoxGrid* d_vox = reinterpret_cast<VoxGrid*>(vb);
-    unsigned long long* d_cursor = reinterpret_cast<unsigned long long*>(vb + 2 * (size_t)nboxes * sizeof(VoxGrid));
-    uint4* d_vrec = reinterpret_cast<uint4*>(vb + vox_head);
-    unsigned* d_vlist = reinterpret_cast<unsigned*>(vb + vox_head + vox_rec);
-    CASS_CUDA(h2d(c, d_vox, vox.data(), vox.size() * sizeof(VoxGrid)));
-    CASS_CUDA(cudaMemsetAsync(d_cursor, 0, sizeof(unsigned long long), c->stream));
-    CASS_CUDA(cudaEventRecord(c->ev[1], c->stream));
-    for (int w = 0; w < 2; ++w)
-      if (vox_most[w] > 0) {
-        k_vox_lists<<<dim3((vox_most[w] + 127) / 128, nboxes), 128, 0, c->stream>>>(
-            d_bd, d_vox, w, d_c32, c->d_cell_start.as<int>(), d_vrec, d_vlist, d_cursor);
-        CASS_CUDA(cudaGetLastError());
-        count_launch(c);
-      }
+    if ((rc2 = build_lists(false))) return rc2;
     const size_t dyn = smem_f32(warps32, smem32);
     CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    // insertions per warp: as few as give every warp of the GPU work at once, up to one per lane
-    int per_warp = 1;
-    while (per_warp < 32 && (n_ins + per_warp - 1) / per_warp * nboxes > (long long)dev_sms * warps32) per_warp *= 2;
-    // one group of insertions per warp: a CTA is as long as its slowest warp, and the
-    // hardware hands out the CTAs; in very large calls several, to stage the box less often
-    const long long groups = (n_ins + per_warp - 1) / per_warp;
-    const int nthreads = 32 * (int)std::min<long long>(warps32, std::max<long long>(1, (groups * nboxes + dev_sms - 1) / dev_sms));
-    const long long need = (groups + nthreads / 32 - 1) / (nthreads / 32);
-    const long long most = std::max<long long>(1, (long long)dev_sms * kF32Waves / nboxes);
-    const int chunks = (int)std::max<long long>(1, (need + (need + most - 1) / most - 1) / ((need + most - 1) / most));
-    dim3 g(chunks, nboxes);
-    c->stats.widom_grid_x = chunks;
-    c->stats.widom_grid_y = nboxes;
-    c->stats.widom_block = nthreads;
+    const dim3 g = warp_grid(warps32);
     c->stats.widom_smem_bytes = (int)dyn;
-    kern<<<g, nthreads, dyn, c->stream>>>(
+    kern<<<g, wthreads, dyn, c->stream>>>(
         S, SF, c->pt, d_bd, d_ids, d_c32, c->d_cq32.as<float>(), c->d_cell_start.as<int>(), s.d_library_f.as<float>(),
         (long long)n_ins, seed, d_rec, d_status, d_xyz, any_recip ? 1 : 0, d_trace, d_fixq, d_fixn, per_warp,
         d_vox, d_vrec, reinterpret_cast<const uint4*>(d_vlist), c->widom_band, d_pairs);
@@ -2996,7 +3783,8 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     if (f32 && opt) rc = smem32 ? launch_f32(k_widom_f32<true, false, true>, SF) : launch_f32(k_widom_f32<false, false, true>, SF);
     else if (f32 && d_pairs) rc = smem32 ? launch_f32(k_widom_f32<true, true, false>, SF) : launch_f32(k_widom_f32<false, true, false>, SF);
     else if (f32) rc = smem32 ? launch_f32(k_widom_f32<true, false, false>, SF) : launch_f32(k_widom_f32<false, false, false>, SF);
-    else rc = use_smem ? launch(k_widom<true>) : launch(k_widom<false>);
+    else if (warp64) rc = launch_w64();
+    if (!f32 && (!warp64 || rc == CASS_ENOMEM)) rc = use_smem ? launch(k_widom<true>) : launch(k_widom<false>);
     if (rc) return rc;
     if (any_recip) {
       // k-vectors and structure factors of the batch boxes, concatenated
@@ -3056,7 +3844,7 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   return CASS_OK;
 }
 
-// The cell-edge autotuner of the FP64 kernel: the first call with a new batch
+// The cell-edge autotuner of the thread-per-insertion FP64 kernel: the first call with a new batch
 // signature (species, boxes, CBMC options, order of magnitude of the insertion count)
 // times the kernel with each candidate edge on a sample of the insertions with its own
 // seed (the faster of two runs after a first that sizes the buffers), keeps the faster
@@ -3067,8 +3855,12 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
 extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
                                  int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
                                  CassWidomTrace* trace) {
-  if (!c || c->precision == CASS_PREC_MIXED || !iboxes || nboxes < 1 || !out || n_ins < 64 || !c->widom_autotune ||
-      c->widom_cells > 0.0)
+  bool tune = c && c->precision != CASS_PREC_MIXED && iboxes && nboxes >= 1 && out && n_ins >= 64 && c->widom_autotune &&
+              !(c->widom_cells > 0.0);
+  for (int k = 0; tune && k < nboxes; ++k) tune = iboxes[k] >= 1 && iboxes[k] <= c->nboxes;
+  for (int k = 0; tune && k < nboxes; ++k)
+    if (pack_box_ext(c, iboxes[k] - 1)) tune = false;  // the call itself says why
+  if (!tune || lists64(c, nboxes, iboxes))
     return widom_insert_impl(c, is1, nboxes, iboxes, n_ins, kappa_ins, kappa_dih, seed, out, trace);
   std::vector<long long> key = {is1, c->precision, kappa_ins, kappa_dih, c->cbmc_opt.energy_table_res,
                                 c->cbmc_opt.sector_overlap, (long long)std::log2((double)n_ins)};

@@ -58,3 +58,29 @@ def test_widom_warp_queries(boxes, n_ins):
     ok = to["overlap"] == 0
     assert (np.abs(tm["e_inter"] - to["e_inter"])[ok] <= 2e-5 * to["e_inter_abs"][ok] + 1e-7).all()
     assert [r["n_overlaps"] for r in rm] == [r["n_overlaps"] for r in ro]
+
+
+@pytest.mark.parametrize("n_ins", [1, 33, 400])
+@pytest.mark.parametrize("boxes", [
+    [(180, (20.0, 20.0, 20.0), 1.0), (0, (30.0, 30.0, 30.0), 1.0)],    # cutoff of half the edge: two images listed; no atoms
+    [(1300, (48.3, 48.3, 48.3), 1.0), (1, (40.0, 40.0, 40.0), 1.0)],
+    [(500, (60.0, 50.0, 50.0), 0.4), (700, (30.0, 45.0, 52.0), 1.0)],
+])
+def test_widom_warp_queries_fp64(boxes, n_ins):
+    """The FP64 kernel: equal decisions, energies to the rounding of FP64 sums."""
+    s = _system(boxes)
+    ids = list(range(1, len(boxes) + 1))
+    with oracle.open_system(s) as o, cg.open_system(s, precision=abi.PREC_FP64) as g:
+        for b in ids:
+            o.system_total_energy(b)
+            g.system_total_energy(b)
+        ro, to = o.widom_insert(2, ids, n_ins, 12, 7, seed=78, trace=True)
+        rg, tg = g.widom_insert(2, ids, n_ins, 12, 7, seed=78, trace=True)
+        again, ta = g.widom_insert(2, ids, n_ins, 12, 7, seed=78, trace=True)
+    assert again == rg and ta.tobytes() == tg.tobytes()
+    assert np.array_equal(to["overlap"], tg["overlap"])
+    assert np.array_equal(to["selected_trial"], tg["selected_trial"])
+    ok = to["overlap"] == 0
+    assert np.allclose(tg["widom_var"][ok], to["widom_var"][ok], rtol=1e-8, atol=0)
+    assert (np.abs(tg["e_inter"] - to["e_inter"])[ok] <= 1e-11 * to["e_inter_abs"][ok] + 1e-9).all()
+    assert np.allclose(tg["e_inter_abs"][ok], to["e_inter_abs"][ok], rtol=1e-11)

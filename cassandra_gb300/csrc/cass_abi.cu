@@ -556,11 +556,12 @@ __global__ void __launch_bounds__(128) k_sfac(const double4_32a* __restrict__ kv
 // a k-vector costs one complex product and sum per atom (4 FP64 operations) and no phase
 // of its own; threads take consecutive k, so the rows are written in whole lines.  12,288
 // atoms of water and 13,190 k-vectors: 4.25 ms with a thread per (row, molecule), which
-// spent most of its FP64 time on the two sincos that started each row, 3.53 ms now.
+// spent most of its FP64 time on the two sincos that started each row, 2.1 ms now.
 constexpr int kSfacRowAtoms = 4;   // molecules of up to this many atoms
 constexpr int kSfacRows = 480;     // k-vector rows of a CTA
 __global__ void __launch_bounds__(kBlock) k_sfac_rows(const double4_32a* __restrict__ kvec, const int2* __restrict__ rows,
-                                                      int nrows, int rows_per_cta, double hx1, double hy1, double hz1,
+                                                      int nrows, int rows_per_cta, int kmax, double hx1, double hy1,
+                                                      double hz1,
                                                       const double4_32a* __restrict__ p64,
                                                       const MolInfo* __restrict__ mols, const int* __restrict__ charged,
                                                       double* cos_mol, double* sin_mol, int stride) {
@@ -570,8 +571,9 @@ __global__ void __launch_bounds__(kBlock) k_sfac_rows(const double4_32a* __restr
   const MolInfo mi = mols[blockIdx.x];
   if (!charged[mi.y]) return;
   const int r0 = blockIdx.y * rows_per_cta, nr = min(rows_per_cta, nrows - r0);
-  for (int e = threadIdx.x; e < 3 * mi.w * kMaxKRow; e += blockDim.x) {
-    const int k = e % kMaxKRow, a = e / kMaxKRow % mi.w, d = e / (kMaxKRow * mi.w);
+  const double ix1 = 1.0 / hx1, iy1 = 1.0 / hy1, iz1 = 1.0 / hz1;
+  for (int e = threadIdx.x; e < 3 * mi.w * kmax; e += blockDim.x) {  // kmax <= kMaxKRow
+    const int k = e % kmax, a = e / kmax % mi.w, d = e / (kmax * mi.w);
     const double4_32a p = p64[mi.z + a];
     const double h = (double)k * (d == 0 ? hx1 : d == 1 ? hy1 : hz1);
     double s, c;
@@ -583,9 +585,9 @@ __global__ void __launch_bounds__(kBlock) k_sfac_rows(const double4_32a* __restr
   for (int e = threadIdx.x; e < nr * mi.w; e += blockDim.x) {
     const int a = e / nr, r = e - a * nr;
     const double4_32a h = kvec[srow[r].x], p = p64[mi.z + a];
-    const int nx = (int)rint(h.x / hx1), ny = (int)rint(h.y / hy1), nz = (int)rint(h.z / hz1);  // of the row's first k
+    const int nx = __double2int_rn(h.x * ix1), ny = __double2int_rn(h.y * iy1), nz = __double2int_rn(h.z * iz1);  // of the row's first k
     double c, s;
-    if (nx == 0 && abs(ny) < kMaxKRow && abs(nz) < kMaxKRow) {
+    if (nx == 0 && abs(ny) < kmax && abs(nz) < kmax) {
       const double2 y = T[1][a][abs(ny)], z = T[2][a][abs(nz)];
       const double ys = ny < 0 ? -y.y : y.y, zs = nz < 0 ? -z.y : z.y;
       c = y.x * z.x - ys * zs;
@@ -612,8 +614,8 @@ __global__ void __launch_bounds__(kBlock) k_sfac_rows(const double4_32a* __restr
     for (int a = 0; a < kSfacRowAtoms; ++a)
       if (a < mi.w) {
         const double2 x = T[0][a][j], q = YZ[a][r];
-        c += q.x * x.x - q.y * x.y;
-        s += q.x * x.y + q.y * x.x;
+        c = fma(q.x, x.x, fma(-q.y, x.y, c));
+        s = fma(q.x, x.y, fma(q.y, x.x, s));
       }
     cm[k] = c;
     sm[k] = s;
@@ -1581,6 +1583,11 @@ int cass_set_box(cass_ctx* c, int32_t ibox, const CassBoxDesc* d) {
     double const_val = 1.0 / (4.0 * v.alpha * v.alpha), hcutsq = hcut * hcut;
     int kz = (int)((hcut * v.L[2]) / kTWOPI) + 1, ky = (int)((hcut * v.L[1]) / kTWOPI) + 1,
         kx = (int)((hcut * v.L[0]) / kTWOPI) + 1;
+    std::vector<int> kint;  // their integers, for phase tables
+    B.kn[0] = kx + 1;
+    B.kn[1] = ky + 1;
+    B.kn[2] = kz + 1;
+    B.kint_ok = kx < 512 && ky < 512 && kz < 512;
     for (int nz = -kz; nz <= kz; ++nz)
       for (int ny = -ky; ny <= ky; ++ny)
         for (int nx = 0; nx <= kx; ++nx) {
@@ -1592,6 +1599,7 @@ int cass_set_box(cass_ctx* c, int32_t ibox, const CassBoxDesc* d) {
             double cn = kTWOPI / v.volume * std::exp(-h2 * const_val) / h2;
             if (nx != 0) cn = 2.0 * kTWOPI / v.volume * std::exp(-h2 * const_val) / h2;
             B.kvec.insert(B.kvec.end(), {hx, hy, hz, cn});
+            kint.push_back(nx | (ny + 512) << 10 | (nz + 512) << 20);
             ++B.nvecs;
           }
         }
@@ -1614,6 +1622,8 @@ int cass_set_box(cass_ctx* c, int32_t ibox, const CassBoxDesc* d) {
     }
     if ((rc = B.d_krow.reserve(std::max<size_t>(1, B.krow.size()) * sizeof(int2)))) return rc;
     CASS_CUDA(h2d(c, B.d_krow.p, B.krow.data(), B.krow.size() * sizeof(int2)));
+    if ((rc = B.d_kint.reserve(std::max<size_t>(1, kint.size()) * sizeof(int)))) return rc;
+    CASS_CUDA(h2d(c, B.d_kint.p, kint.data(), kint.size() * sizeof(int)));
     CASS_CUDA(cudaMemsetAsync(B.d_cos_sum.p, 0, nb, c->stream));
     CASS_CUDA(cudaMemsetAsync(B.d_sin_sum.p, 0, nb, c->stream));
     CASS_CUDA(cudaStreamSynchronize(c->stream));
@@ -2038,7 +2048,8 @@ static int box_reciprocal(cass_ctx* c, int ibox, double* e_recip) {
     const int nrows = (int)B.krow.size();
     const int groups = (nrows + kSfacRows - 1) / kSfacRows, per = (nrows + groups - 1) / groups;
     k_sfac_rows<<<dim3(B.npacked_mols, (nrows + per - 1) / per), kBlock, 0, c->stream>>>(
-        B.d_kvec.as<double4_32a>(), B.d_krow.as<int2>(), nrows, per, kTWOPI / B.dev.L[0], kTWOPI / B.dev.L[1],
+        B.d_kvec.as<double4_32a>(), B.d_krow.as<int2>(), nrows, per,
+        std::min(kMaxKRow, std::max(B.kn[0], std::max(B.kn[1], B.kn[2]))), kTWOPI / B.dev.L[0], kTWOPI / B.dev.L[1],
         kTWOPI / B.dev.L[2], B.d_p64.as<double4_32a>(), B.d_molinfo.as<int4>(), dch.as<int>(),
         c->d_cos_mol.as<double>(), c->d_sin_mol.as<double>(), c->cos_mol_stride);
     CASS_CUDA(cudaGetLastError());
@@ -2090,7 +2101,8 @@ int cass_system_total_energy(cass_ctx* c, int32_t ibox1, int32_t intra_flag, Cas
   // copy with the overlap flag: result[0..7) intra, [8..10) pairs, the flag at [10].
   // Boxes of single atoms have no intramolecular part.
   const bool intra = intra_flag && B.npacked_mols > 0 && n > B.npacked_mols;
-  const int nblk_intra = std::max(1, std::min(296, (B.npacked_mols + kBlock - 1) / kBlock));
+  // a warp per CTA: a molecule is a long FP64 chain, and the SMs' FP64 units are what bounds it
+  const int nblk_intra = std::max(1, std::min(1216, (B.npacked_mols + 31) / 32));
   const bool fast = c->precision == CASS_PREC_MIXED && B.desc.vdw_style == CASS_VDW_LJ &&
                     (B.desc.vdw_sum_style == CASS_VDW_SUM_CUT || B.desc.vdw_sum_style == CASS_VDW_SUM_CUT_TAIL) &&
                     (B.desc.charge_style == CASS_CHARGE_NONE || B.desc.charge_sum_style == CASS_QQ_EWALD);
@@ -2106,7 +2118,7 @@ int cass_system_total_energy(cass_ctx* c, int32_t ibox1, int32_t intra_flag, Cas
   int* d_ov = reinterpret_cast<int*>(d_res + 10);
   CASS_CUDA(cudaMemsetAsync(d_res, 0, 11 * sizeof(double), c->stream));
   if (intra) {
-    k_intra_total<<<nblk_intra, kBlock, 0, c->stream>>>(B.dev, c->pt, c->pools, B.d_p64.as<double4_32a>(),
+    k_intra_total<<<nblk_intra, 32, 0, c->stream>>>(B.dev, c->pt, c->pools, B.d_p64.as<double4_32a>(),
                                                         B.d_molinfo.as<int4>(), B.npacked_mols,
                                                         c->d_partial.as<double>(), c->d_counter.as<unsigned>(), d_res,
                                                         d_ov);

@@ -153,6 +153,10 @@ struct BoxH {
   // nx rising by one, at most kMaxKRow long, for the FP64 rebuild and the adjoint
   std::vector<int2> krow;
   DevBuf d_krow;
+  // integers of the k-vectors (nx | (ny + 512) << 10 | (nz + 512) << 20) and the largest |n| + 1
+  DevBuf d_kint;
+  int kn[3] = {1, 1, 1};
+  bool kint_ok = false;
   bool cell_dirty = true;
   // Check_MoleculePair_Cutoff decides which molecule pairs interact when a
   // style has no atom cutoff (LJ CHARMM, minimum-image charges) and the vdW sum

@@ -17,7 +17,13 @@
 //      bookkeeping, step-size adaptation (move_translate.f90:330-352,
 //      move_rotate.f90:307-326)
 //   E  on acceptance: coordinates, COM and structure factors are committed.
-// FP64 kernel: the reference arithmetic.  Mixed kernel: FP32 positions for the
+// FP64 kernel: the reference arithmetic, done for full warps.  GB300 takes 16 cycles of
+// an SM for a warp's FP64 instruction however many lanes need it, so B tests the pairs
+// in FP32 (with a margin far above its rounding), queues those within reach and forms 32
+// at a time in FP64, pairs with a vdW term apart from those without; and C takes its
+// phases from tables of the powers of e^{i 2 pi x / L} of the trial atoms (8 FP64
+// operations per k-vector and atom instead of a cosine and a sine).  One chain of 256
+// waters: 39 us a move before, 33 us after.  Mixed kernel: FP32 positions for the
 // pair loop, FP32 phases for the structure factors and the FP32 change of the
 // reciprocal energy, Cn [dc (2 S_c + dc) + ds (2 S_s + ds)] summed per thread
 // with compensation; the master coordinates, the running structure factors, the
@@ -26,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -40,6 +47,7 @@ constexpr int kMcWarps = kMcThreads / 32;
 constexpr int kMcThreadsG = 512;  // boxes in global memory: more lanes for their longer loops
 constexpr int kMaxSpeciesMC = 8;
 constexpr size_t kMcSmemLimit = 200 * 1024;
+constexpr int kMcTab = 512;  // entries of the FP64 kernel's phase tables
 
 struct McSpecies {
   int natoms, linear, has_charge;
@@ -74,10 +82,13 @@ struct McBox {
   double* new_cos;  // scratch [nvecs]
   double* new_sin;
   int nvecs, ewald;
+  const int* kint;  // nx | (ny + 512) << 10 | (nz + 512) << 20 of each k-vector (NULL: some |n| > 511)
+  int kn[3];        // largest |n| + 1 per dimension
   // Check_MoleculePair_Cutoff decides which molecule pairs interact (LJ CHARMM,
   // minimum-image charges): COM distance against rmax + both max_dcom
   int comcut;
   double rmax;
+  float pre2, pre2_none;  // FP64 kernel: FP32 bounds of r^2 beyond every cutoff, with and without a vdW term
   double* max_disp;   // [nspecies] in/out
   double* max_rot;
   CassEnergy* energy;  // in/out
@@ -89,7 +100,7 @@ struct McBox {
 
 // the move thread 0 prepared for the block
 struct McMove {
-  int skip, stop, kind, is, pm, na, first, slot, accept, ewald;
+  int skip, stop, kind, is, pm, na, first, slot, accept, ewald, tab;
   double old_r[3 * kMaxAtoms], trial[3 * kMaxAtoms], q[kMaxAtoms];
   int type[kMaxAtoms];
   float old_f[3 * kMaxAtoms], trial_f[3 * kMaxAtoms];
@@ -230,6 +241,8 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
   __shared__ double cd[2][4];  // this CTA's partial sums for the cluster (alternating buffers)
   __shared__ int ci[2][2];
   __shared__ McBox G;  // the box descriptor, read by the serial steps of every move
+  __shared__ double2 tab[MIXED ? 1 : kMcTab];
+  __shared__ unsigned queue[MIXED ? 1 : NW][2][64];  // FP64 pairs, without and with a vdW term: j | a << 26 | trial << 30
   const int crank = (int)(blockIdx.x % (unsigned)csize);
   int cbuf = 0;
   if (threadIdx.x == 0) {
@@ -452,8 +465,10 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
           mv.com_new[1] = c1;
           mv.com_new[2] = c2;
         }
-        if (MIXED)
-          for (int i = 0; i < 3 * mv.na; ++i) mv.trial_f[i] = (float)mv.trial[i];
+        for (int i = 0; i < 3 * mv.na; ++i) mv.trial_f[i] = (float)mv.trial[i];
+        if (!MIXED)
+          for (int i = 0; i < 3 * mv.na; ++i) mv.old_f[i] = (float)mv.old_r[i];
+        mv.tab = !MIXED && mv.ewald && G.kint && mv.na * (G.kn[0] + G.kn[1] + G.kn[2]) <= kMcTab;
       }
     }
     __syncthreads();
@@ -503,6 +518,91 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
       }
       pv2 = make_float2(kv.s, kv.c);
       pq2 = make_float2(kq.s, kq.c);
+    } else if (!G.comcut) {
+      if (mv.tab) {  // the trial atoms' phase tables, read in C
+        const int nx = G.kn[0] * na, ny = G.kn[1] * na, nz = G.kn[2] * na;
+        for (int e = threadIdx.x; e < nx + ny + nz; e += blockDim.x) {
+          const int d = e < nx ? 0 : (e < nx + ny ? 1 : 2), f = e - (d > 0 ? nx : 0) - (d > 1 ? ny : 0);
+          const int a = f / G.kn[d], k = f - a * G.kn[d];
+          double sn, cs;
+          sincos((double)k * (kTWOPI / b.L[d]) * mv.trial[3 * a + d], &sn, &cs);
+          const double q = d == 0 ? mv.q[a] : 1.0;
+          tab[e] = make_double2(q * cs, q * sn);
+        }
+      }
+      const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+      const bool ewald = b.charge_style == CASS_CHARGE_COUL && b.charge_sum_style == CASS_QQ_EWALD;
+      const bool lj = lj_plain_style(b);
+      int cnt[2] = {0, 0};
+      // queued pair e; V: it may have a vdW term
+      auto pair = [&](unsigned e, bool V) {
+        const int j = (int)(e & 0x3ffffffu), a = (int)(e >> 26) & 15, w = (int)(e >> 30);
+        const double* r = (w ? mv.trial : mv.old_r) + 3 * a;
+        double d[3] = {r[0] - sx[j], r[1] - sy[j], r[2] - sz[j]};
+#pragma unroll
+        for (int k = 0; k < 3; ++k) d[k] = fold(d[k], b.hL[k], b.L[k]);
+        const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+        if (r2 < b.rcut_lowsq) {
+          if (w) pn = 1;
+          else po = 1;
+          return;
+        }
+        const int m = cutoff_mask(b, r2, false);
+        double ev = 0.0, eq = 0.0;
+        const double ri = ewald ? rsqrt(r2) : 0.0;
+        if (V && (m & 1)) {
+          if (lj && ewald) {
+            const int k = pidx(mv.type[a], stype[j], T.ntypes);
+            const double s2 = T.sig2[k] * (ri * ri), s6 = s2 * s2 * s2;
+            ev = 4.0 * T.eps[k] * (s6 * s6 - s6);
+          } else {
+            ev = vdw_pair(T, b, mv.type[a], stype[j], r2, 1.0);
+          }
+        }
+        if (m & 2)
+          eq = ewald ? mv.q[a] * sq[j] * kCHARGE_FACTOR * ri * erfc_as(b.alpha * (r2 * ri))
+                     : qq_pair_inter(b, mv.q[a] * sq[j], r2);
+        pdv += w ? ev : -ev;
+        pdq += w ? eq : -eq;
+      };
+      for (int base = (threadIdx.x & ~31) + crank * blockDim.x; base < N; base += jstep) {
+        const int j = base + lane;
+        const bool live = j < N && smol[min(j, N - 1)] != pm;
+        const int jj = min(j, N - 1);
+        const float xj = (float)sx[jj], yj = (float)sy[jj], zj = (float)sz[jj];
+        const int tj = stype[jj];
+        for (int a = 0; a < na; ++a) {
+          const int ta = mv.type[a];
+          const bool V = ta >= 0 && tj >= 0 && T.eps[pidx(max(ta, 0), max(tj, 0), T.ntypes)] != 0.0;
+          const float pre = V ? G.pre2 : G.pre2_none;
+#pragma unroll
+          for (int w = 0; w < 2; ++w) {
+            const float* r = (w ? mv.trial_f : mv.old_f) + 3 * a;
+            const float dx = fold(r[0] - xj, b.hLf[0], b.Lf[0]), dy = fold(r[1] - yj, b.hLf[1], b.Lf[1]),
+                        dz = fold(r[2] - zj, b.hLf[2], b.Lf[2]);
+            const bool hit = live && !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > pre);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              const unsigned m = __ballot_sync(0xffffffffu, hit && V == (c == 1));
+              if (!m) continue;
+              if ((m >> lane) & 1u)
+                queue[wq][c][cnt[c] + __popc(m & ((1u << lane) - 1u))] = (unsigned)j | (unsigned)a << 26 | (unsigned)w << 30;
+              cnt[c] += __popc(m);
+              if (cnt[c] >= 32) {
+                __syncwarp();
+                cnt[c] -= 32;
+                pair(queue[wq][c][cnt[c] + lane], c == 1);
+                __syncwarp();
+              }
+            }
+          }
+        }
+      }
+      __syncwarp();
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+        if (lane < cnt[c]) pair(queue[wq][c][lane], c == 1);
+      __syncwarp();
     } else {
       for (int j = j0; j < N; j += jstep) {
         const int mj = smol[j];
@@ -510,15 +610,15 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
         const double xj = sx[j], yj = sy[j], zj = sz[j], qj = sq[j];
         const int tj = stype[j];
         bool in[2] = {true, true};
-        if (G.comcut)  // Check_MoleculePair_Cutoff (energy_routines.f90:3027-3088), old and trial COM
+        // Check_MoleculePair_Cutoff (energy_routines.f90:3027-3088), old and trial COM
 #pragma unroll
-          for (int w = 0; w < 2; ++w) {
-            const double* cw = w ? mv.com_new : com + 3 * pm;
-            const double dx = fold(cw[0] - com[3 * mj], b.hL[0], b.L[0]);
-            const double dy = fold(cw[1] - com[3 * mj + 1], b.hL[1], b.L[1]);
-            const double dz = fold(cw[2] - com[3 * mj + 2], b.hL[2], b.L[2]);
-            in[w] = !(sqrt(dx * dx + dy * dy + dz * dz) > G.rmax + dcom[pm] + dcom[mj]);
-          }
+        for (int w = 0; w < 2; ++w) {
+          const double* cw = w ? mv.com_new : com + 3 * pm;
+          const double dx = fold(cw[0] - com[3 * mj], b.hL[0], b.L[0]);
+          const double dy = fold(cw[1] - com[3 * mj + 1], b.hL[1], b.L[1]);
+          const double dz = fold(cw[2] - com[3 * mj + 2], b.hL[2], b.L[2]);
+          in[w] = !(sqrt(dx * dx + dy * dy + dz * dz) > G.rmax + dcom[pm] + dcom[mj]);
+        }
         for (int a = 0; a < na; ++a) {
 #pragma unroll
           for (int w = 0; w < 2; ++w) {
@@ -639,6 +739,17 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
           }
           cn = (double)cf;
           sn = (double)sf;
+        } else if (mv.tab) {
+          const int v = G.kint[k], kx = v & 1023, ky = ((v >> 10) & 1023) - 512, kz = ((v >> 20) & 1023) - 512;
+          const double2* ty = tab + na * G.kn[0] + abs(ky);
+          const double2* tz = tab + na * (G.kn[0] + G.kn[1]) + abs(kz);
+          for (int a = 0; a < na; ++a) {
+            const double2 x = tab[a * G.kn[0] + kx], y = ty[a * G.kn[1]], z = tz[a * G.kn[2]];
+            const double ys = ky < 0 ? -y.y : y.y, zs = kz < 0 ? -z.y : z.y;
+            const double c = y.x * z.x - ys * zs, sv = y.x * zs + ys * z.x;
+            cn = fma(x.x, c, fma(-x.y, sv, cn));
+            sn = fma(x.x, sv, fma(x.y, c, sn));
+          }
         } else {
           for (int a = 0; a < na; ++a) {
             const double hdotr = h.x * mv.trial[3 * a] + h.y * mv.trial[3 * a + 1] + h.z * mv.trial[3 * a + 2];
@@ -916,6 +1027,23 @@ extern "C" int cass_mc_sweeps(cass_ctx* c, int32_t nboxes, const int32_t* iboxes
     g.ewald = B.desc.charge_style == CASS_CHARGE_COUL && B.desc.charge_sum_style == CASS_QQ_EWALD && B.nvecs > 0;
     g.nvecs = g.ewald ? B.nvecs : 0;
     g.kvec = B.d_kvec.as<double4_32a>();
+    g.kint = B.kint_ok ? B.d_kint.as<int>() : nullptr;
+    for (int d = 0; d < 3; ++d) g.kn[d] = B.kn[d];
+    {  // beyond every cutoff of cutoff_mask, by far more than FP32 rounds
+      const CassBoxDesc& d = B.desc;
+      const double lmax = std::max(d.length[0], std::max(d.length[1], d.length[2]));
+      auto above = [&](double r2) { return (float)(r2 * (1.0 + 1.0e-4) + 1.0e-3 + 2.0e-6 * lmax * std::sqrt(r2)); };
+      double r2 = B.dev.rcut_lowsq, q2 = B.dev.rcut_lowsq;
+      bool bounded = true;
+      if (d.vdw_style != CASS_VDW_NONE) {
+        if (d.vdw_sum_style == CASS_VDW_SUM_MINIMUM || d.vdw_sum_style == CASS_VDW_SUM_CHARMM) bounded = false;
+        r2 = std::max(r2, d.vdw_sum_style == CASS_VDW_SUM_CUT_SWITCH ? B.dev.roff_switch_sq : B.dev.rcut_vdwsq);
+      }
+      if (d.charge_style == CASS_CHARGE_COUL) q2 = std::max(q2, B.dev.rcut_coulsq);
+      const bool open = d.charge_style == CASS_CHARGE_COUL && d.charge_sum_style == CASS_QQ_MINIMUM;
+      g.pre2 = bounded && !open ? above(std::max(r2, q2)) : FLT_MAX;
+      g.pre2_none = open ? FLT_MAX : above(q2);
+    }
     g.cos_sum = B.d_cos_sum.as<double>();
     g.sin_sum = B.d_sin_sum.as<double>();
     g.new_cos = d_scr + 2 * (size_t)k * max_nv;

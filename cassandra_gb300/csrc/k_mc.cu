@@ -1,29 +1,34 @@
 // k_mc.cu -- NVT Monte Carlo sweeps on the device (translation / rotation).
 //
-// One CTA runs one box's Markov chain for the whole call: the box's atoms,
-// charges, types and molecule table live in shared memory, thread 0 owns the
-// lfsr258 stream and makes every random choice in the reference's order, and
-// the block evaluates each move's energies cooperatively:
-//   A  thread 0: move kind (nvtmc_driver.f90:107-134), species and molecule
+// One CTA (or a cluster) runs one box's Markov chain for the whole call: the box's
+// atoms, charges, types and molecule table live in shared memory, warp 0 owns the
+// lfsr258 stream (every lane holds it and draws alike) and makes every random choice in
+// the reference's order, and the block evaluates each move's energies cooperatively:
+//   A  warp 0: move kind (nvtmc_driver.f90:107-134), species and molecule
 //      (move_translate.f90:150-185), trial coordinates (:205-215 and Fold_Molecule,
-//      or Rotate_Molecule_Axis / Rotate_Molecule_Eulerian, move_rotate.f90:362-536)
+//      or Rotate_Molecule_Axis / Rotate_Molecule_Eulerian, move_rotate.f90:362-536),
+//      a coordinate per lane: one lane after the other coordinate took 3,250 cycles of
+//      a 500-sphere move and 12,300 of a move of 4,096 waters in global memory
 //   B  all threads: the moved molecule's old and trial energies against every
 //      other atom in one pass (Compute_Molecule_Nonbond_Inter_Energy twice,
-//      energy_routines.f90:1088-1206), block reduction
+//      energy_routines.f90:1088-1206)
 //   C  all threads, charged species in Ewald boxes: the molecule's new
 //      cos/sin sums per k-vector and the new reciprocal energy
-//      (Update_System_Ewald_Reciprocal_Energy, :2384-2431)
-//   D  thread 0: accept_or_reject (accept_or_reject.f90:22-65), energy
+//      (Update_System_Ewald_Reciprocal_Energy, :2384-2431), before B's outcome is
+//      known, so that both sums cross the block (and the cluster) together
+//   D  warp 0: accept_or_reject (accept_or_reject.f90:22-65), energy
 //      bookkeeping, step-size adaptation (move_translate.f90:330-352,
-//      move_rotate.f90:307-326)
-//   E  on acceptance: coordinates, COM and structure factors are committed.
+//      move_rotate.f90:307-326), coordinates and COM on acceptance
+//   E  all threads, on acceptance: structure factors are committed.
+// Two move records alternate, so that warp 0 goes on with the next move's A while the
+// other warps finish E.  Two block barriers a move, three with an Ewald sum.
 // FP64 kernel: the reference arithmetic, done for full warps.  GB300 takes 16 cycles of
 // an SM for a warp's FP64 instruction however many lanes need it, so B tests the pairs
 // in FP32 (with a margin far above its rounding), queues those within reach and forms 32
 // at a time in FP64, pairs with a vdW term apart from those without; and C takes its
 // phases from tables of the powers of e^{i 2 pi x / L} of the trial atoms (8 FP64
 // operations per k-vector and atom instead of a cosine and a sine).  One chain of 256
-// waters: 39 us a move before, 33 us after.  Mixed kernel: FP32 positions for the
+// waters: 39 us a move before, 27 us now.  Mixed kernel: FP32 positions for the
 // pair loop, FP32 phases for the structure factors and the FP32 change of the
 // reciprocal energy, Cn [dc (2 S_c + dc) + ds (2 S_s + ds)] summed per thread
 // with compensation; the master coordinates, the running structure factors, the
@@ -42,9 +47,8 @@
 
 namespace cassgpu {
 
-constexpr int kMcThreads = 128;
-constexpr int kMcWarps = kMcThreads / 32;
-constexpr int kMcThreadsG = 512;  // boxes in global memory: more lanes for their longer loops
+constexpr int kMcThreads = 512;  // at most; 128 or 256 where chains fill the GPU or a box is small
+constexpr int kMcClusterMax = 16;
 constexpr int kMaxSpeciesMC = 8;
 constexpr size_t kMcSmemLimit = 200 * 1024;
 constexpr int kMcTab = 512;  // entries of the FP64 kernel's phase tables
@@ -188,34 +192,9 @@ __device__ __forceinline__ float2 warp_sum2(float2 v) {
 }
 
 template <class V>
-__device__ __forceinline__ V block_sum_mc(V v, V* red, int slot) {
+__device__ __forceinline__ V warp_sum_mc(V v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red[(threadIdx.x >> 5) * 8 + slot] = v;
   return v;
-}
-
-// Sums over the CTAs of a box's cluster, in rank order, of the nd doubles and
-// ni ints that thread 0 of every CTA placed in cd[buf] / ci[buf]; the results
-// land in the same arrays of every CTA's thread 0 view.  Two buffers alternate,
-// so a buffer is written again only after every CTA passed the barrier that
-// followed its last read.  Thread 0 only reads; all threads take the barrier.
-__device__ __forceinline__ void cluster_sum(int csize, double (*cd)[4], int (*ci)[2], int buf, int nd, int ni,
-                                            double* od, int* oi) {
-  namespace cgr = cooperative_groups;
-  cgr::cluster_group cl = cgr::this_cluster();
-  cl.sync();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < nd; ++k) {
-      double v = 0.0;
-      for (int r = 0; r < csize; ++r) v += *cl.map_shared_rank(&cd[buf][k], r);
-      od[k] = v;
-    }
-    for (int k = 0; k < ni; ++k) {
-      int v = 0;
-      for (int r = 0; r < csize; ++r) v |= *cl.map_shared_rank(&ci[buf][k], r);
-      oi[k] = v;
-    }
-  }
 }
 
 // GMEM: the box layout lives in a per-box global buffer (L2-resident) instead
@@ -227,19 +206,20 @@ __device__ __forceinline__ void cluster_sum(int csize, double (*cd)[4], int (*ci
 // added in rank order through distributed shared memory, and each CTA commits
 // the structure factors of its own k-vectors.
 template <bool MIXED, bool GMEM>
-__global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(McArgs A, McBox* boxes, PairTable T,
-                                                                           int csize) {
-  constexpr int NW = (GMEM ? kMcThreadsG : kMcThreads) / 32;
-  const int nwarps = blockDim.x >> 5;  // <= NW
+__global__ void __launch_bounds__(kMcThreads) k_mc_sweeps(const __grid_constant__ McArgs A, McBox* boxes,
+                                                          const __grid_constant__ PairTable T, int csize) {
+  constexpr int NW = kMcThreads / 32;
+  const int nwarps = blockDim.x >> 5;  // 4, 8 or 16
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
   extern __shared__ __align__(16) unsigned char dsmem[];
   __shared__ BoxDev b;
-  __shared__ McMove mv;
-  __shared__ double red[NW * 8];
+  __shared__ McMove mvs[2];
+  __shared__ double red[NW * 4];  // FP64 sums per warp: vdW, Coulomb, reciprocal
   __shared__ float redf[NW * 4];  // mixed kernel: compensated FP32 pair sums per warp
-  __shared__ int redi[NW * 2];
+  __shared__ int redi[NW];
   __shared__ float2 ljp[kMaxTypes * kMaxTypes];
   __shared__ double cd[2][4];  // this CTA's partial sums for the cluster (alternating buffers)
-  __shared__ int ci[2][2];
+  __shared__ unsigned ci[2];
   __shared__ McBox G;  // the box descriptor, read by the serial steps of every move
   __shared__ double2 tab[MIXED ? 1 : kMcTab];
   __shared__ unsigned queue[MIXED ? 1 : NW][2][64];  // FP64 pairs, without and with a vdW term: j | a << 26 | trial << 30
@@ -314,7 +294,7 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
     }
     dcom[m] = sqrt(dmax);
   }
-  // thread 0 state
+  // state of warp 0, alike in its lanes (E and R: lane 0)
   Lfsr rng;
   CassEnergy E;
   CassMCResult R;
@@ -323,16 +303,13 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
   int nt_d[kMaxSpeciesMC], ns_d[kMaxSpeciesMC], nt_r[kMaxSpeciesMC], ns_r[kMaxSpeciesMC];
   int last_d = 0, last_r = 0;
   bool any_d = false, any_r = false;
-  double dv = 0, dq = 0;
-  // mixed kernel, one CTA and no k-space work: the move's energy change as
-  // compensated FP32 pairs and its acceptance decided in FP32 (FP64 only for
-  // the bookkeeping of an accepted move)
-  float2 dv2 = make_float2(0.f, 0.f), dq2 = make_float2(0.f, 0.f);
-  bool fast = false;
   float ptf = 1.0f, betaf = 0.0f;
-  if (threadIdx.x == 0) {
+  double e_rec = 0.0;  // the box's reciprocal energy
+  const bool lead = threadIdx.x < 32;
+  if (lead) {
     rng = seed_stream(A.seed, G.ibox1, 0);
     E = *G.energy;
+    e_rec = E.reciprocal;
     memset(&R, 0, sizeof(R));
     for (int is = 0; is < A.nspecies; ++is) {
       md[is] = G.max_disp[is];
@@ -355,133 +332,136 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
   int status = 0;
   __syncthreads();
   for (long long step = 0; step < steps; ++step) {
+    McMove& mv = mvs[step & 1];
     // ---- A: the move
-    if (threadIdx.x == 0) {
-      mv.skip = 0;
-      mv.stop = 0;
-      mv.accept = 0;
-      const bool tr = MIXED ? draw_f(rng) <= ptf : rng.next() <= A.prob_translate;
-      mv.kind = tr ? 0 : 1;
-      int is = -1;
-      if (tr ? any_d : any_r)
-        is = MIXED ? mc_pick_species_f(A.nspecies, tr ? xdf : xrf, tr ? last_d : last_r, rng)
-                   : mc_pick_species(A.nspecies, tr ? xd : xr, tr ? last_d : last_r, rng);
-      if (is < 0) {
-        mv.skip = 1;
-      } else {
-        // INT(rranf() * nmols) + 1, kept in range when rranf() rounds to 1.0
-        const int im = MIXED ? min((int)(draw_f(rng) * (float)G.nmol_sp[is]) + 1, G.nmol_sp[is])
-                             : min((int)(rng.next() * G.nmol_sp[is]) + 1, G.nmol_sp[is]);
-        const int pm = G.first_sp[is] + im - 1;
-        const McSpecies& s = A.sp[is];
-        mv.is = is;
-        mv.pm = pm;
-        mv.na = mnat[pm];
-        mv.first = mfirst[pm];
-        mv.slot = mslot[pm];
-        mv.ewald = G.ewald && s.has_charge;
-        for (int a = 0; a < mv.na; ++a) {
-          const int j = mv.first + a;
-          mv.old_r[3 * a] = sx[j];
-          mv.old_r[3 * a + 1] = sy[j];
-          mv.old_r[3 * a + 2] = sz[j];
-          if (MIXED) {  // (float) of the FP64 position, kept so at every commit
-            const float4 f = s32[j];
-            mv.old_f[3 * a] = f.x;
-            mv.old_f[3 * a + 1] = f.y;
-            mv.old_f[3 * a + 2] = f.z;
+    if (lead) {
+      bool skip = false;
+      if (!status) {
+        const bool tr = MIXED ? draw_f(rng) <= ptf : rng.next() <= A.prob_translate;
+        int is = -1;
+        if (tr ? any_d : any_r)
+          is = MIXED ? mc_pick_species_f(A.nspecies, tr ? xdf : xrf, tr ? last_d : last_r, rng)
+                     : mc_pick_species(A.nspecies, tr ? xd : xr, tr ? last_d : last_r, rng);
+        skip = is < 0;
+        if (!skip) {
+          // INT(rranf() * nmols) + 1, kept in range when rranf() rounds to 1.0
+          const int im = MIXED ? min((int)(draw_f(rng) * (float)G.nmol_sp[is]) + 1, G.nmol_sp[is])
+                               : min((int)(rng.next() * G.nmol_sp[is]) + 1, G.nmol_sp[is]);
+          const int pm = G.first_sp[is] + im - 1;
+          const McSpecies& s = A.sp[is];
+          const int na = mnat[pm], first = mfirst[pm], slot = mslot[pm];
+          const double c[3] = {com[3 * pm], com[3 * pm + 1], com[3 * pm + 2]};
+          for (int e = lane; e < 3 * na; e += 32) {
+            const int a = e / 3, k = e - 3 * a;
+            const double v = (k == 0 ? sx : k == 1 ? sy : sz)[first + a];
+            mv.old_r[e] = v;
+            if (MIXED) mv.old_f[e] = reinterpret_cast<const float*>(&s32[first + a])[k];  // (float) of it, kept at every commit
+            else mv.old_f[e] = (float)v;
           }
-          mv.q[a] = sq[j];
-          mv.type[a] = stype[j];
-        }
-        const double c0 = com[3 * pm], c1 = com[3 * pm + 1], c2 = com[3 * pm + 2];
-        if (tr) {
-          ++R.n_translate;
-          if (A.nupdate > 0) ++nt_d[is];
-          double d[3];
-          if (MIXED)
-            for (int k = 0; k < 3; ++k) d[k] = (double)((2.0f * draw_f(rng) - 1.0f) * mdf[is]);
-          else
-            for (int k = 0; k < 3; ++k) d[k] = (2.0 * rng.next() - 1.0) * md[is];
-          double cn[3] = {c0 + d[0], c1 + d[1], c2 + d[2]};
-          double sh[3];
-          for (int k = 0; k < 3; ++k) {  // Fold_Molecule
-            sh[k] = cn[k] > b.hL[k] ? -b.L[k] : (cn[k] < -b.hL[k] ? b.L[k] : 0.0);
-            cn[k] = cn[k] + sh[k];
+          if (lane < na) {
+            mv.q[lane] = sq[first + lane];
+            mv.type[lane] = stype[first + lane];
           }
-          for (int a = 0; a < mv.na; ++a)
+          if (lane == 0) {
+            mv.kind = tr ? 0 : 1;
+            mv.is = is;
+            mv.pm = pm;
+            mv.na = na;
+            mv.first = first;
+            mv.slot = slot;
+            mv.ewald = G.ewald && s.has_charge;
+            mv.tab = !MIXED && !G.comcut && mv.ewald && G.kint && na * (G.kn[0] + G.kn[1] + G.kn[2]) <= kMcTab;
+          }
+          if (tr) {
+            ++R.n_translate;
+            if (A.nupdate > 0) ++nt_d[is];
+            float uf[3];
+            double ud[3];
             for (int k = 0; k < 3; ++k) {
-              double v = mv.old_r[3 * a + k] + d[k];
-              if (sh[k] != 0.0) v = v + sh[k];
-              mv.trial[3 * a + k] = v;
+              if (MIXED) uf[k] = draw_f(rng);
+              else ud[k] = rng.next();
             }
-          for (int k = 0; k < 3; ++k) mv.com_new[k] = cn[k];
-        } else {
-          ++R.n_rotate;
-          if (A.nupdate > 0) ++nt_r[is];
-          double Rm[9];
-          if (s.linear) {
-            const double theta = acos(1.0 - 2.0 * mc_u<MIXED>(rng));
-            const double phi = (1.0 - 2.0 * mc_u<MIXED>(rng)) * kPI;
-            const double psi = (1.0 - 2.0 * mc_u<MIXED>(rng)) * kPI;
-            Rm[0] = cos(psi) * cos(phi) - cos(theta) * sin(phi) * sin(psi);
-            Rm[1] = cos(psi) * sin(phi) + cos(theta) * cos(phi) * sin(psi);
-            Rm[2] = sin(psi) * sin(theta);
-            Rm[3] = -sin(psi) * cos(phi) - cos(theta) * sin(phi) * cos(psi);
-            Rm[4] = -sin(psi) * sin(phi) + cos(theta) * cos(phi) * cos(psi);
-            Rm[5] = cos(psi) * sin(theta);
-            Rm[6] = sin(theta) * sin(phi);
-            Rm[7] = -sin(theta) * cos(phi);
-            Rm[8] = cos(theta);
+            for (int e = lane; e < 3 * na; e += 32) {
+              const int k = e % 3;
+              double d;
+              if (MIXED) d = (double)((2.0f * (k == 0 ? uf[0] : k == 1 ? uf[1] : uf[2]) - 1.0f) * mdf[is]);
+              else d = (2.0 * (k == 0 ? ud[0] : k == 1 ? ud[1] : ud[2]) - 1.0) * md[is];
+              const double cn = (k == 0 ? c[0] : k == 1 ? c[1] : c[2]) + d;
+              const double sh = cn > b.hL[k] ? -b.L[k] : (cn < -b.hL[k] ? b.L[k] : 0.0);  // Fold_Molecule
+              double v = mv.old_r[e] + d;
+              if (sh != 0.0) v = v + sh;
+              mv.trial[e] = v;
+              mv.trial_f[e] = (float)v;
+              if (e < 3) mv.com_new[k] = cn + sh;
+            }
           } else {
-            double p1 = 0.0, p2 = 0.0, p3 = 0.0;
-            const int axis = (int)(3.0 * mc_u<MIXED>(rng)) + 1;
-            const double ang = (2.0 * mc_u<MIXED>(rng) - 1.0) * mr[is];
-            if (axis == 1) p1 = ang;
-            else if (axis == 2) p2 = ang;
-            else p3 = ang;
-            // DCOS / DSIN of the two zero angles are exactly 1 and 0
-            double k1 = 1.0, k2 = 1.0, k3 = 1.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
-            if (axis == 1) sincos(p1, &s1, &k1);
-            else if (axis == 2) sincos(p2, &s2, &k2);
-            else sincos(p3, &s3, &k3);
-            Rm[0] = k1 * k3 - s1 * k2 * s3;
-            Rm[1] = s1 * k3 + k1 * k2 * s3;
-            Rm[2] = s2 * s3;
-            Rm[3] = -k1 * s3 - s1 * k2 * k3;
-            Rm[4] = -s1 * s3 + k1 * k2 * k3;
-            Rm[5] = s2 * k3;
-            Rm[6] = s1 * s2;
-            Rm[7] = -k1 * s2;
-            Rm[8] = k2;
+            ++R.n_rotate;
+            if (A.nupdate > 0) ++nt_r[is];
+            double Rm[9];
+            if (s.linear) {
+              const double theta = acos(1.0 - 2.0 * mc_u<MIXED>(rng));
+              const double phi = (1.0 - 2.0 * mc_u<MIXED>(rng)) * kPI;
+              const double psi = (1.0 - 2.0 * mc_u<MIXED>(rng)) * kPI;
+              double st, ct, sp, cp, ss, cs;
+              sincos(theta, &st, &ct);
+              sincos(phi, &sp, &cp);
+              sincos(psi, &ss, &cs);
+              Rm[0] = cs * cp - ct * sp * ss;
+              Rm[1] = cs * sp + ct * cp * ss;
+              Rm[2] = ss * st;
+              Rm[3] = -ss * cp - ct * sp * cs;
+              Rm[4] = -ss * sp + ct * cp * cs;
+              Rm[5] = cs * st;
+              Rm[6] = st * sp;
+              Rm[7] = -st * cp;
+              Rm[8] = ct;
+            } else {
+              // one Euler angle, the cosines and sines of the other two exactly 1 and 0:
+              // the first and the third turn about z, the second about x
+              const int axis = (int)(3.0 * mc_u<MIXED>(rng)) + 1;
+              const double ang = (2.0 * mc_u<MIXED>(rng) - 1.0) * mr[is];
+              double sn, cs;
+              sincos(ang, &sn, &cs);
+              const bool z = axis != 2;
+              Rm[0] = z ? cs : 1.0;
+              Rm[1] = z ? sn : 0.0;
+              Rm[2] = 0.0;
+              Rm[3] = z ? -sn : 0.0;
+              Rm[4] = cs;
+              Rm[5] = z ? 0.0 : sn;
+              Rm[6] = 0.0;
+              Rm[7] = z ? 0.0 : -sn;
+              Rm[8] = z ? 1.0 : cs;
+            }
+            __syncwarp();
+            for (int e = lane; e < 3 * na; e += 32) {
+              const int a = e / 3, k = e - 3 * a;
+              const double x = mv.old_r[3 * a] - c[0], y = mv.old_r[3 * a + 1] - c[1], z = mv.old_r[3 * a + 2] - c[2];
+              const double r0 = k == 0 ? Rm[0] : k == 1 ? Rm[3] : Rm[6], r1 = k == 0 ? Rm[1] : k == 1 ? Rm[4] : Rm[7],
+                           r2 = k == 0 ? Rm[2] : k == 1 ? Rm[5] : Rm[8];
+              const double v = (r0 * x + r1 * y + r2 * z) + (k == 0 ? c[0] : k == 1 ? c[1] : c[2]);
+              mv.trial[e] = v;
+              mv.trial_f[e] = (float)v;
+              if (e < 3) mv.com_new[k] = k == 0 ? c[0] : k == 1 ? c[1] : c[2];
+            }
           }
-          for (int a = 0; a < mv.na; ++a) {
-            const double x = mv.old_r[3 * a] - c0, y = mv.old_r[3 * a + 1] - c1, z = mv.old_r[3 * a + 2] - c2;
-            mv.trial[3 * a] = (Rm[0] * x + Rm[1] * y + Rm[2] * z) + c0;
-            mv.trial[3 * a + 1] = (Rm[3] * x + Rm[4] * y + Rm[5] * z) + c1;
-            mv.trial[3 * a + 2] = (Rm[6] * x + Rm[7] * y + Rm[8] * z) + c2;
-          }
-          mv.com_new[0] = c0;
-          mv.com_new[1] = c1;
-          mv.com_new[2] = c2;
         }
-        for (int i = 0; i < 3 * mv.na; ++i) mv.trial_f[i] = (float)mv.trial[i];
-        if (!MIXED)
-          for (int i = 0; i < 3 * mv.na; ++i) mv.old_f[i] = (float)mv.old_r[i];
-        mv.tab = !MIXED && mv.ewald && G.kint && mv.na * (G.kn[0] + G.kn[1] + G.kn[2]) <= kMcTab;
+      }
+      if (lane == 0) {
+        mv.stop = status;
+        mv.skip = skip;
       }
     }
     __syncthreads();
-    if (mv.skip) {  // uniform: no species can make this kind of move
-      __syncthreads();
-      continue;
-    }
+    if (mv.stop) break;  // the last move's molecule overlapped another before it moved
+    if (mv.skip) continue;  // no species can make this kind of move
     // ---- B: old and trial energies of the molecule against the other atoms
     const int pm = mv.pm, na = mv.na;
     double pdv = 0, pdq = 0;  // this thread's share of E_new - E_old
     float2 pv2 = make_float2(0.f, 0.f), pq2 = make_float2(0.f, 0.f);  // the same, mixed kernel
     int po = 0, pn = 0;
-    const int j0 = threadIdx.x + crank * blockDim.x, jstep = blockDim.x * csize;
+    // warps of all CTAs take 32 atoms in turn, so that no CTA is left without
+    const int jbase = (wq * csize + crank) * 32, j0 = jbase + lane, jstep = blockDim.x * csize;
     if (MIXED) {
       KahanF kv, kq;
       const float rv2 = (float)b.rcut_vdwsq, rq2 = (float)b.rcut_coulsq, low2 = (float)b.rcut_lowsq;
@@ -530,7 +510,6 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
           tab[e] = make_double2(q * cs, q * sn);
         }
       }
-      const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
       const bool ewald = b.charge_style == CASS_CHARGE_COUL && b.charge_sum_style == CASS_QQ_EWALD;
       const bool lj = lj_plain_style(b);
       int cnt[2] = {0, 0};
@@ -540,7 +519,11 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
         const double* r = (w ? mv.trial : mv.old_r) + 3 * a;
         double d[3] = {r[0] - sx[j], r[1] - sy[j], r[2] - sz[j]};
 #pragma unroll
-        for (int k = 0; k < 3; ++k) d[k] = fold(d[k], b.hL[k], b.L[k]);
+        for (int k = 0; k < 3; ++k) {  // the high word of |d| tells the image, unless it is that of L / 2
+          const int hd = __double2hiint(d[k]) & 0x7fffffff, hl = __double2hiint(b.hL[k]);
+          if (hd == hl) d[k] = fold(d[k], b.hL[k], b.L[k]);
+          else if (hd > hl) d[k] += __double2hiint(d[k]) > 0 ? -b.L[k] : b.L[k];
+        }
         const double r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
         if (r2 < b.rcut_lowsq) {
           if (w) pn = 1;
@@ -565,7 +548,7 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
         pdv += w ? ev : -ev;
         pdq += w ? eq : -eq;
       };
-      for (int base = (threadIdx.x & ~31) + crank * blockDim.x; base < N; base += jstep) {
+      for (int base = jbase; base < N; base += jstep) {
         const int j = base + lane;
         const bool live = j < N && smol[min(j, N - 1)] != pm;
         const int jj = min(j, N - 1);
@@ -641,182 +624,206 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
         }
       }
     }
+    // ---- C: reciprocal-space energy after the move
+    double part = 0.0;
+    if (mv.ewald) {
+      if (!MIXED && mv.tab) __syncthreads();  // the tables
+      const double* cm = A.cos_mol + (size_t)mv.slot * A.stride;
+      const double* smv = A.sin_mol + (size_t)mv.slot * A.stride;
+      KahanF partf;
+      constexpr int U = 2;  // k-vectors in flight per thread: their loads come before the phases
+      for (int k0 = threadIdx.x + crank * blockDim.x; k0 < G.nvecs; k0 += U * jstep) {
+        double4_32a h[U];
+        double ocm[U], osm[U], ocs[U], oss[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int k = min(k0 + u * jstep, G.nvecs - 1);
+          h[u] = G.kvec[k];
+          ocm[u] = cm[k];
+          osm[u] = smv[k];
+          ocs[u] = G.cos_sum[k];
+          oss[u] = G.sin_sum[k];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int k = k0 + u * jstep;
+          if (k >= G.nvecs) break;
+          double cn = 0.0, sn = 0.0;
+          if (MIXED) {
+            float cf = 0.0f, sf = 0.0f;
+            const float hx = (float)h[u].x, hy = (float)h[u].y, hz = (float)h[u].z;
+            for (int a = 0; a < na; ++a) {
+              float s_, c_;
+              sincosf(hx * mv.trial_f[3 * a] + hy * mv.trial_f[3 * a + 1] + hz * mv.trial_f[3 * a + 2], &s_, &c_);
+              cf += (float)mv.q[a] * c_;
+              sf += (float)mv.q[a] * s_;
+            }
+            cn = (double)cf;
+            sn = (double)sf;
+            // the change of Cn (S_c^2 + S_s^2) in FP32: dc (2 S_c + dc) + ds (2 S_s + ds)
+            const float dc = (float)cn - (float)ocm[u], ds = (float)sn - (float)osm[u];
+            const float sc = (float)ocs[u], ss = (float)oss[u];
+            partf.add((float)h[u].w * (dc * (2.0f * sc + dc) + ds * (2.0f * ss + ds)));
+          } else {
+            if (mv.tab) {
+              const int v = G.kint[k], kx = v & 1023, ky = ((v >> 10) & 1023) - 512, kz = ((v >> 20) & 1023) - 512;
+              const double2* ty = tab + na * G.kn[0] + abs(ky);
+              const double2* tz = tab + na * (G.kn[0] + G.kn[1]) + abs(kz);
+              for (int a = 0; a < na; ++a) {
+                const double2 x = tab[a * G.kn[0] + kx], y = ty[a * G.kn[1]], z = tz[a * G.kn[2]];
+                const double ys = ky < 0 ? -y.y : y.y, zs = kz < 0 ? -z.y : z.y;
+                const double cc = y.x * z.x - ys * zs, sv = y.x * zs + ys * z.x;
+                cn = fma(x.x, cc, fma(-x.y, sv, cn));
+                sn = fma(x.x, sv, fma(x.y, cc, sn));
+              }
+            } else {
+              for (int a = 0; a < na; ++a) {
+                const double hdotr = h[u].x * mv.trial[3 * a] + h[u].y * mv.trial[3 * a + 1] + h[u].z * mv.trial[3 * a + 2];
+                cn = cn + mv.q[a] * cos(hdotr);
+                sn = sn + mv.q[a] * sin(hdotr);
+              }
+            }
+            const double cc = ocs[u] + (cn - ocm[u]), ss = oss[u] + (sn - osm[u]);
+            part += h[u].w * (cc * cc + ss * ss);
+          }
+          G.new_cos[k] = cn;
+          G.new_sin[k] = sn;
+        }
+      }
+      if (MIXED) part = partf.value();
+    }
+    // ---- the sums of the warps, of the block and of the cluster
+    const bool qq = b.charge_style == CASS_CHARGE_COUL;
     if (MIXED) {  // compensated FP32 warp sums (no FP64 instructions in any warp)
       pv2 = warp_sum2(pv2);
-      pq2 = warp_sum2(pq2);
-      if ((threadIdx.x & 31) == 0) {
-        const int w = threadIdx.x >> 5;
-        redf[4 * w] = pv2.x;
-        redf[4 * w + 1] = pv2.y;
-        redf[4 * w + 2] = pq2.x;
-        redf[4 * w + 3] = pq2.y;
+      if (qq) pq2 = warp_sum2(pq2);
+      if (lane == 0) {
+        redf[4 * wq] = pv2.x;
+        redf[4 * wq + 1] = pv2.y;
+        redf[4 * wq + 2] = pq2.x;
+        redf[4 * wq + 3] = pq2.y;
       }
     } else {
-      block_sum_mc(pdv, red, 0);
-      block_sum_mc(pdq, red, 1);
+      pdv = warp_sum_mc(pdv);
+      if (qq) pdq = warp_sum_mc(pdq);
+      if (lane == 0) {
+        red[4 * wq] = pdv;
+        red[4 * wq + 1] = pdq;
+      }
+    }
+    if (mv.ewald) {
+      part = warp_sum_mc(part);
+      if (lane == 0) red[4 * wq + 2] = part;
     }
     {
       const int o = __any_sync(0xffffffffu, po), n = __any_sync(0xffffffffu, pn);
-      if ((threadIdx.x & 31) == 0) {
-        redi[(threadIdx.x >> 5) * 2] = o;
-        redi[(threadIdx.x >> 5) * 2 + 1] = n;
-      }
+      if (lane == 0) redi[wq] = o | n << 1;
     }
     __syncthreads();
-    int o = 0, n = 0;
-    if (threadIdx.x == 0) {
+    // warp 0, alike in all lanes
+    double dv = 0.0, dq = 0.0, er = 0.0;
+    float2 dv2 = make_float2(0.f, 0.f), dq2 = make_float2(0.f, 0.f);
+    unsigned flags = 0;
+    // mixed kernel, one CTA and no k-space work: the move's energy change as compensated
+    // FP32 pairs and its acceptance decided in FP32 (FP64 only for an accepted move)
+    const bool fast = MIXED && csize == 1 && !mv.ewald;
+    if (lead) {
+      const int w = lane & (nwarps - 1);
+      flags = __reduce_or_sync(0xffffffffu, (unsigned)redi[w]);
       if (MIXED) {
-        dv2 = dq2 = make_float2(0.f, 0.f);
-        for (int w = 0; w < nwarps; ++w) {
-          two_sum_add(dv2, make_float2(redf[4 * w], redf[4 * w + 1]));
-          two_sum_add(dq2, make_float2(redf[4 * w + 2], redf[4 * w + 3]));
-          o |= redi[2 * w];
-          n |= redi[2 * w + 1];
-        }
-        fast = csize == 1 && !mv.ewald;
-        if (!fast) {
-          dv = (double)dv2.x + (double)dv2.y;
-          dq = (double)dq2.x + (double)dq2.y;
-        }
+        dv2 = make_float2(redf[4 * w], redf[4 * w + 1]);
+        dq2 = make_float2(redf[4 * w + 2], redf[4 * w + 3]);
       } else {
-        dv = dq = 0.0;
-        for (int w = 0; w < nwarps; ++w) {
-          dv += red[w * 8];
-          dq += red[w * 8 + 1];
-          o |= redi[2 * w];
-          n |= redi[2 * w + 1];
-        }
+        dv = red[4 * w];
+        dq = red[4 * w + 1];
       }
-      if (csize > 1) {
+      if (mv.ewald) er = red[4 * w + 2];
+      for (int o = nwarps >> 1; o > 0; o >>= 1) {
+        if (MIXED) {
+          two_sum_add(dv2, make_float2(__shfl_xor_sync(0xffffffffu, dv2.x, o), __shfl_xor_sync(0xffffffffu, dv2.y, o)));
+          if (qq)
+            two_sum_add(dq2, make_float2(__shfl_xor_sync(0xffffffffu, dq2.x, o), __shfl_xor_sync(0xffffffffu, dq2.y, o)));
+        } else {
+          dv += __shfl_xor_sync(0xffffffffu, dv, o);
+          if (qq) dq += __shfl_xor_sync(0xffffffffu, dq, o);
+        }
+        if (mv.ewald) er += __shfl_xor_sync(0xffffffffu, er, o);
+      }
+      if (MIXED && !fast) {
+        dv = (double)dv2.x + (double)dv2.y;
+        dq = (double)dq2.x + (double)dq2.y;
+      }
+      if (csize > 1 && lane == 0) {
         cd[cbuf][0] = dv;
         cd[cbuf][1] = dq;
-        ci[cbuf][0] = o;
-        ci[cbuf][1] = n;
+        cd[cbuf][2] = er;
+        ci[cbuf] = flags;
       }
     }
     if (csize > 1) {
-      double sums[2];
-      int flags[2];
-      cluster_sum(csize, cd, ci, cbuf, 2, 2, sums, flags);
+      // Two buffers alternate: one is written again only after every CTA has passed the
+      // barrier that followed its last read
+      namespace cgr = cooperative_groups;
+      cgr::cluster_group cl = cgr::this_cluster();
+      cl.sync();
+      if (lead) {
+        dv = dq = er = 0.0;
+        flags = 0;
+        if (lane < csize) {
+          const double* r = cl.map_shared_rank(&cd[cbuf][0], lane);
+          dv = r[0];
+          dq = r[1];
+          er = r[2];
+          flags = *cl.map_shared_rank(&ci[cbuf], lane);
+        }
+        flags = __reduce_or_sync(0xffffffffu, flags);
+        dv = warp_sum_mc(dv);
+        if (qq) dq = warp_sum_mc(dq);
+        if (mv.ewald) er = warp_sum_mc(er);
+      }
       cbuf ^= 1;
-      if (threadIdx.x == 0) {
-        dv = sums[0];
-        dq = sums[1];
-        o = flags[0];
-        n = flags[1];
-      }
-    }
-    if (threadIdx.x == 0) {
-      if (o) {
-        mv.stop = 1;
-        status = 1;
-      } else if (n) {
-        ++R.n_overlap;
-        mv.ewald = 0;
-      }
-      mv.accept = (!o && !n) ? 1 : 0;  // provisional: energies valid
-    }
-    __syncthreads();
-    if (mv.stop) break;
-    // ---- C: reciprocal-space energy after the move
-    double e_recip = 0.0;
-    if (mv.ewald) {
-      const double* cm = A.cos_mol + (size_t)mv.slot * A.stride;
-      const double* smv = A.sin_mol + (size_t)mv.slot * A.stride;
-      double part = 0.0;
-      KahanF partf;
-      for (int k = threadIdx.x + crank * blockDim.x; k < G.nvecs; k += blockDim.x * csize) {
-        const double4_32a h = G.kvec[k];
-        double cn = 0.0, sn = 0.0;
-        if (MIXED) {
-          float cf = 0.0f, sf = 0.0f;
-          const float hx = (float)h.x, hy = (float)h.y, hz = (float)h.z;
-          for (int a = 0; a < na; ++a) {
-            float s_, c_;
-            sincosf(hx * mv.trial_f[3 * a] + hy * mv.trial_f[3 * a + 1] + hz * mv.trial_f[3 * a + 2], &s_, &c_);
-            cf += (float)mv.q[a] * c_;
-            sf += (float)mv.q[a] * s_;
-          }
-          cn = (double)cf;
-          sn = (double)sf;
-        } else if (mv.tab) {
-          const int v = G.kint[k], kx = v & 1023, ky = ((v >> 10) & 1023) - 512, kz = ((v >> 20) & 1023) - 512;
-          const double2* ty = tab + na * G.kn[0] + abs(ky);
-          const double2* tz = tab + na * (G.kn[0] + G.kn[1]) + abs(kz);
-          for (int a = 0; a < na; ++a) {
-            const double2 x = tab[a * G.kn[0] + kx], y = ty[a * G.kn[1]], z = tz[a * G.kn[2]];
-            const double ys = ky < 0 ? -y.y : y.y, zs = kz < 0 ? -z.y : z.y;
-            const double c = y.x * z.x - ys * zs, sv = y.x * zs + ys * z.x;
-            cn = fma(x.x, c, fma(-x.y, sv, cn));
-            sn = fma(x.x, sv, fma(x.y, c, sn));
-          }
-        } else {
-          for (int a = 0; a < na; ++a) {
-            const double hdotr = h.x * mv.trial[3 * a] + h.y * mv.trial[3 * a + 1] + h.z * mv.trial[3 * a + 2];
-            cn = cn + mv.q[a] * cos(hdotr);
-            sn = sn + mv.q[a] * sin(hdotr);
-          }
-        }
-        if (MIXED) {
-          // the change of Cn (S_c^2 + S_s^2) in FP32: dc (2 S_c + dc) + ds (2 S_s + ds)
-          const float dc = (float)cn - (float)cm[k], ds = (float)sn - (float)smv[k];
-          const float sc = (float)G.cos_sum[k], ss = (float)G.sin_sum[k];
-          partf.add((float)h.w * (dc * (2.0f * sc + dc) + ds * (2.0f * ss + ds)));
-        } else {
-          const double c = G.cos_sum[k] + (cn - cm[k]);
-          const double s = G.sin_sum[k] + (sn - smv[k]);
-          part += h.w * (c * c + s * s);
-        }
-        G.new_cos[k] = cn;
-        G.new_sin[k] = sn;
-      }
-      if (MIXED) part = partf.value();
-      block_sum_mc(part, red, 4);
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        for (int w = 0; w < nwarps; ++w) e_recip += red[w * 8 + 4];
-        if (csize > 1) cd[cbuf][0] = e_recip;
-      }
-      if (csize > 1) {
-        double sums[1];
-        cluster_sum(csize, cd, ci, cbuf, 1, 0, sums, nullptr);
-        cbuf ^= 1;
-        if (threadIdx.x == 0) e_recip = sums[0];
-      }
-      if (threadIdx.x == 0)  // mixed: the previous reciprocal energy plus the FP32 change (FP64 sum)
-        e_recip = MIXED ? E.reciprocal + e_recip * kCHARGE_FACTOR : e_recip * kCHARGE_FACTOR;
     }
     // ---- D: acceptance
-    if (threadIdx.x == 0) {
+    if (lead) {
+      const bool o = flags & 1u, n = flags & 2u;
+      if (o) status = 1;
+      else if (n) ++R.n_overlap;
       bool acc = false;
-      if (mv.accept && MIXED && fast) {
-        // accept_or_reject in FP32 (the rule of accept_or_reject.f90:22-65 with
-        // a 23-bit draw); the bookkeeping of an accepted move in FP64
-        const float lnf = betaf * ((dv2.x + dq2.x) + (dv2.y + dq2.y));
-        acc = lnf <= 0.0f || (lnf < (float)kMAX_KBT && draw_f(rng) <= expf(-lnf));
-        if (acc) {
-          dv = (double)dv2.x + (double)dv2.y;
-          dq = (double)dq2.x + (double)dq2.y;
-          const double dE = dv + dq;
-          E.total = E.total + dE;
-          E.inter = E.inter + dE;
-          E.inter_vdw = E.inter_vdw + dv;
-          E.inter_q = E.inter_q + dq;
-        }
-      } else if (mv.accept) {
-        double dE = 0.0;
-        if (mv.ewald) dE = e_recip - E.reciprocal;
-        dE = dE + dv + dq;
-        acc = accept_or_reject_d(b.beta * dE, rng);
-        if (acc) {
-          E.total = E.total + dE;
-          E.inter = E.inter + dE;
-          E.inter_vdw = E.inter_vdw + dv;
-          E.inter_q = E.inter_q + dq;
-          if (mv.ewald) E.reciprocal = e_recip;
+      if (!o && !n) {
+        if (fast) {
+          // accept_or_reject in FP32 (the rule of accept_or_reject.f90:22-65 with
+          // a 23-bit draw); the bookkeeping of an accepted move in FP64
+          const float lnf = betaf * ((dv2.x + dq2.x) + (dv2.y + dq2.y));
+          acc = lnf <= 0.0f || (lnf < (float)kMAX_KBT && draw_f(rng) <= expf(-lnf));
+          if (acc && lane == 0) {
+            dv = (double)dv2.x + (double)dv2.y;
+            dq = (double)dq2.x + (double)dq2.y;
+            const double dE = dv + dq;
+            E.total = E.total + dE;
+            E.inter = E.inter + dE;
+            E.inter_vdw = E.inter_vdw + dv;
+            E.inter_q = E.inter_q + dq;
+          }
+        } else {
+          double dE = 0.0, e_new = e_rec;
+          if (mv.ewald) {  // mixed: the previous reciprocal energy plus the FP32 change (FP64 sum)
+            e_new = MIXED ? e_rec + er * kCHARGE_FACTOR : er * kCHARGE_FACTOR;
+            dE = e_new - e_rec;
+          }
+          dE = dE + dv + dq;
+          acc = accept_or_reject_d(b.beta * dE, rng);
+          if (acc) {
+            e_rec = e_new;
+            E.total = E.total + dE;
+            E.inter = E.inter + dE;
+            E.inter_vdw = E.inter_vdw + dv;
+            E.inter_q = E.inter_q + dq;
+            if (mv.ewald) E.reciprocal = e_rec;
+          }
         }
       }
-      mv.accept = acc ? 1 : 0;
+      if (lane == 0) mv.accept = acc ? 1 : 0;
+      if (!o) {
       const int is = mv.is;
       if (mv.kind == 0) {
         if (acc) {
@@ -847,46 +854,44 @@ __global__ void __launch_bounds__(GMEM ? kMcThreadsG : kMcThreads) k_mc_sweeps(M
           else mr[is] = fmin(kPI, 1.05 * mr[is]);
         }
       }
+      }
       if (acc) {  // commit the coordinates and the COM
-        for (int a = 0; a < na; ++a) {
-          const int j = mv.first + a;
-          sx[j] = mv.trial[3 * a];
-          sy[j] = mv.trial[3 * a + 1];
-          sz[j] = mv.trial[3 * a + 2];
-          if (MIXED) s32[j] = make_float4(mv.trial_f[3 * a], mv.trial_f[3 * a + 1], mv.trial_f[3 * a + 2], s32[j].w);
+        for (int e = lane; e < 3 * na; e += 32) {
+          const int a = e / 3, k = e - 3 * a;
+          (k == 0 ? sx : k == 1 ? sy : sz)[mv.first + a] = mv.trial[e];
+          if (MIXED) reinterpret_cast<float*>(&s32[mv.first + a])[k] = mv.trial_f[e];
         }
-        if (mv.kind == 0) {
-          for (int k = 0; k < 3; ++k) com[3 * pm + k] = mv.com_new[k];
-        } else {  // Get_COM on acceptance of a rotation
-          const McSpecies& s = A.sp[is];
-          double tm = 0, x = 0, y = 0, z = 0;
-          for (int a = 0; a < na; ++a) {
-            tm += s.mass[a];
-            x += s.mass[a] * mv.trial[3 * a];
-            y += s.mass[a] * mv.trial[3 * a + 1];
-            z += s.mass[a] * mv.trial[3 * a + 2];
+        if (lane < 3) {
+          double v = mv.com_new[lane];
+          if (mv.kind != 0) {  // Get_COM on acceptance of a rotation
+            const McSpecies& s = A.sp[mv.is];
+            double tm = 0, x = 0;
+            for (int a = 0; a < na; ++a) {
+              tm += s.mass[a];
+              x += s.mass[a] * mv.trial[3 * a + lane];
+            }
+            v = x / tm;
           }
-          com[3 * pm] = x / tm;
-          com[3 * pm + 1] = y / tm;
-          com[3 * pm + 2] = z / tm;
+          com[3 * pm + lane] = v;
+        }
+      }
+      __syncwarp();
+    }
+    // ---- E: commit the structure factors
+    if (mv.ewald) {
+      __syncthreads();
+      if (mv.accept) {
+        double* cm = A.cos_mol + (size_t)mv.slot * A.stride;
+        double* smv = A.sin_mol + (size_t)mv.slot * A.stride;
+        for (int k = threadIdx.x + crank * blockDim.x; k < G.nvecs; k += jstep) {
+          const double cn = G.new_cos[k], sn = G.new_sin[k];
+          G.cos_sum[k] = G.cos_sum[k] + (cn - cm[k]);
+          G.sin_sum[k] = G.sin_sum[k] + (sn - smv[k]);
+          cm[k] = cn;
+          smv[k] = sn;
         }
       }
     }
-    __syncthreads();
-    // ---- E: commit the structure factors
-    if (mv.accept && mv.ewald) {
-      double* cm = A.cos_mol + (size_t)mv.slot * A.stride;
-      double* smv = A.sin_mol + (size_t)mv.slot * A.stride;
-      for (int k = threadIdx.x + crank * blockDim.x; k < G.nvecs; k += blockDim.x * csize) {
-        const double cn = G.new_cos[k], sn = G.new_sin[k];
-        G.cos_sum[k] = G.cos_sum[k] + (cn - cm[k]);
-        G.sin_sum[k] = G.sin_sum[k] + (sn - smv[k]);
-        cm[k] = cn;
-        smv[k] = sn;
-      }
-    }
-    // the next move's thread-0 phase reads committed shared data only
-    __syncthreads();
   }
   __syncthreads();
   if (csize > 1) cooperative_groups::this_cluster().sync();  // no CTA leaves while its shared memory may be read
@@ -1065,21 +1070,31 @@ extern "C" int cass_mc_sweeps(cass_ctx* c, int32_t nboxes, const int32_t* iboxes
                    : (mixed ? k_mc_sweeps<true, false> : k_mc_sweeps<false, false>);
   if (gmem) dyn = 0;
   CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-  const int threads = gmem ? kMcThreadsG : kMcThreads;
   // CTAs per chain: a cluster splits the pair and k-vector loops of a move when
   // SMs would otherwise stay idle (few chains); every cluster must be resident.
-  // Measured on single chains (sweeps/s, 1 -> best cluster): FP64 LJ-500
-  // 117 -> 218 at 4 CTAs, FP64 water-256 with Ewald 20 -> 100 at 8, mixed
-  // water-256 143 -> 288 at 8, while mixed LJ-500 (FP32 pairs, no k-space) is
-  // bound by the serial steps of a move and loses a little (307 -> 278-292).
-  int csize = 1;
+  // Clusters of 16 (beyond the portable 8) for Ewald boxes: one mixed chain of 256 waters
+  // 3.02 ms a sweep at 8 CTAs before, 2.18 ms at 16 now.  An uncharged mixed box is bound
+  // by the serial steps of a move and stays on one CTA, as does an FP64 box of up to 128
+  // atoms (110 atoms: 3.3 ms on one CTA, 3.7 ms on two).  Threads per CTA: 512 while chains
+  // are few, no more than the box's atoms or k-vectors need; 128 once they fill the SMs.
+  int csize = 1, threads = 128;
   {
     int sms = 0, nmax = 1;
     CASS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    for (const McBox& g : hb) nmax = std::max(nmax, g.natoms);
-    int want = c->mc_cluster > 0 ? c->mc_cluster : std::min(8, std::max(1, sms / nboxes));
-    if (c->mc_cluster <= 0) want = std::min(want, any_ewald ? 8 : (mixed ? 1 : std::max(1, (nmax + 127) / 128)));
-    for (int cs = std::min(8, want); cs >= 2; --cs) {
+    CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (const McBox& g : hb) nmax = std::max(nmax, std::max(g.natoms, g.nvecs));
+    auto threads_of = [&](int cs) {
+      if (gmem) return kMcThreads;
+      if ((long long)nboxes * cs > sms) return 128;
+      const int per = (nmax + cs - 1) / cs;
+      return per > 256 ? 512 : (per > 128 ? 256 : 128);
+    };
+    int want = c->mc_cluster > 0 ? c->mc_cluster : std::min(kMcClusterMax, std::max(1, sms / nboxes));
+    if (c->mc_cluster <= 0)
+      want = std::min(want, any_ewald ? kMcClusterMax : (mixed || nmax <= 128 ? 1 : (nmax + 63) / 64));
+    threads = threads_of(1);
+    for (int cs = want; cs >= 2; --cs) {
+      if (cs > 8 && cs < kMcClusterMax) continue;
       cudaLaunchConfig_t q = {};
       cudaLaunchAttribute qa[1];
       qa[0].id = cudaLaunchAttributeClusterDimension;
@@ -1087,13 +1102,14 @@ extern "C" int cass_mc_sweeps(cass_ctx* c, int32_t nboxes, const int32_t* iboxes
       qa[0].val.clusterDim.y = 1;
       qa[0].val.clusterDim.z = 1;
       q.gridDim = dim3(nboxes * cs);
-      q.blockDim = dim3(threads);
+      q.blockDim = dim3(threads_of(cs));
       q.dynamicSmemBytes = dyn;
       q.attrs = qa;
       q.numAttrs = 1;
       int nclusters = 0;
       if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &q) == cudaSuccess && nclusters >= nboxes) {
         csize = cs;
+        threads = threads_of(cs);
         break;
       }
       (void)cudaGetLastError();

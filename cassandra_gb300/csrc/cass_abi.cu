@@ -218,16 +218,20 @@ template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_trial_energy(BoxDev b, PairTable t, const double4_32a* __restrict__ p64,
                                                          const int4* __restrict__ meta, int n, int skip_slot,
                                                          const double4_32a* __restrict__ trial, const int* ttype,
-                                                         int nat, int cbmc, int want_qq, const double4_32a* __restrict__ tcom,
+                                                         int nat, int cbmc, int want_qq, const float4* __restrict__ p32,
+                                                         float pre2, const double4_32a* __restrict__ tcom,
                                                          const double4_32a* __restrict__ com, double rmax, double* e,
                                                          int* overlap) {
   __shared__ double4_32a qa[kTrialMaxAtoms];
+  __shared__ float4 qf[kTrialMaxAtoms];
   __shared__ int qt[kTrialMaxAtoms];
   __shared__ double sh[32];
   __shared__ int ovs;
   const double4_32a* tr = trial + (size_t)blockIdx.x * nat;
   for (int a = threadIdx.x; a < nat; a += blockDim.x) {
-    qa[a] = tr[a];
+    const double4_32a p = tr[a];
+    qa[a] = p;
+    qf[a] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.0f);
     qt[a] = ttype[a];
   }
   if (threadIdx.x == 0) ovs = 0;
@@ -241,7 +245,12 @@ __global__ void __launch_bounds__(kBlock) k_trial_energy(BoxDev b, PairTable t, 
     if (mj.x == skip_slot) continue;
     if (tcom && !molpair_in(b, rmax, tcom[blockIdx.x], com[j])) continue;
     const double4_32a pj = p64[j];
+    const float4 fj = p32[j];
     for (int a = 0; a < nat; ++a) {
+      // beyond every cutoff (and overlap radius) by far more than FP32 rounds: most pairs
+      const float ex = fold(qf[a].x - fj.x, b.hLf[0], b.Lf[0]), ey = fold(qf[a].y - fj.y, b.hLf[1], b.Lf[1]),
+                  ez = fold(qf[a].z - fj.z, b.hLf[2], b.Lf[2]);
+      if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) > pre2) continue;
       const double dx = fold(qa[a].x - pj.x, b.hL[0], b.L[0]);
       const double dy = fold(qa[a].y - pj.y, b.hL[1], b.L[1]);
       const double dz = fold(qa[a].z - pj.z, b.hL[2], b.L[2]);
@@ -1928,8 +1937,14 @@ int cass_cbmc_trial_energies(cass_ctx* c, int32_t ibox1, int32_t is, int32_t ski
   if ((rc = set_device(c)) || (rc = pack_box(c, ib))) return rc;
   if (cbmc && (rc = ensure_cbmc(c))) return rc;
   BoxH& B = c->box[ib];
-  std::vector<double4_32a> tr((size_t)ntrial * nat);
-  std::vector<int> tt(nat);
+  // Page-locked staging of one upload (positions, COMs, types) and one read-back
+  // (energies, overlaps): five small copies from pageable memory were a third of a call
+  const size_t ntr = (size_t)ntrial * nat, ncom = B.comcut ? (size_t)ntrial : 0;
+  const size_t up = (ntr + ncom) * sizeof(double4_32a) + (((size_t)nat * sizeof(int) + 31) & ~(size_t)31);
+  const size_t down = (size_t)ntrial * (sizeof(double) + sizeof(int));
+  if ((rc = c->d_trial.reserve(up + down + 64)) || (rc = c->h_read.reserve(up + down + 64))) return rc;
+  double4_32a* tr = c->h_read.as<double4_32a>();
+  int* tt = reinterpret_cast<int*>(tr + ntr + ncom);
   for (int a = 0; a < nat; ++a) tt[a] = s.type[atoms[a] - 1];
   for (int k = 0; k < ntrial; ++k)
     for (int a = 0; a < nat; ++a) {
@@ -1938,7 +1953,7 @@ int cass_cbmc_trial_energies(cass_ctx* c, int32_t ibox1, int32_t is, int32_t ski
     }
   // Check_MoleculePair_Cutoff where a style has no atom cutoff: the COM and
   // max_dcom of each trial's atoms (get_com.f90:45-105, 220-295)
-  std::vector<double4_32a> tcom;
+  double4_32a* tcom = tr + ntr;
   if (B.comcut)
     for (int k = 0; k < ntrial; ++k) {
       double tm = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
@@ -1959,37 +1974,49 @@ int cass_cbmc_trial_energies(cass_ctx* c, int32_t ibox1, int32_t is, int32_t ski
         const double dx = p.x - cx, dy = p.y - cy, dz = p.z - cz;
         dmax = std::max(dmax, dx * dx + dy * dy + dz * dz);
       }
-      tcom.push_back(make_double4_32a(cx, cy, cz, std::sqrt(dmax)));
+      tcom[k] = make_double4_32a(cx, cy, cz, std::sqrt(dmax));
     }
-  const size_t tb = tr.size() * sizeof(double4_32a);
-  const size_t cb = tcom.size() * sizeof(double4_32a);
-  if ((rc = c->d_trial.reserve(tb + cb + (size_t)nat * sizeof(int) + (size_t)ntrial * (sizeof(double) + sizeof(int)) + 64)))
-    return rc;
   double4_32a* d_tr = c->d_trial.as<double4_32a>();
-  double4_32a* d_tcom = B.comcut ? d_tr + tr.size() : nullptr;
-  int* d_tt = reinterpret_cast<int*>(d_tr + tr.size() + tcom.size());
-  double* d_e = reinterpret_cast<double*>(reinterpret_cast<char*>(d_tt) + (((size_t)nat * sizeof(int) + 7) & ~(size_t)7));
+  double4_32a* d_tcom = B.comcut ? d_tr + ntr : nullptr;
+  int* d_tt = reinterpret_cast<int*>(d_tr + ntr + ncom);
+  double* d_e = reinterpret_cast<double*>(c->d_trial.as<unsigned char>() + up);
   int* d_ov = reinterpret_cast<int*>(d_e + ntrial);
-  CASS_CUDA(h2d(c, d_tr, tr.data(), tb));
-  if (B.comcut) CASS_CUDA(h2d(c, d_tcom, tcom.data(), cb));
-  CASS_CUDA(h2d(c, d_tt, tt.data(), (size_t)nat * sizeof(int)));
+  CASS_CUDA(h2d(c, d_tr, tr, up));
+  // beyond every cutoff of cutoff_mask and the overlap radius
+  double r2 = std::max(B.dev.rcut_lowsq, B.dev.rcut_cbmcsq);
+  bool bounded = true;
+  if (!cbmc) {
+    const CassBoxDesc& d = B.desc;
+    r2 = std::max(B.dev.rcut_lowsq, d.charge_style == CASS_CHARGE_COUL ? B.dev.rcut_coulsq : 0.0);
+    if (d.vdw_style != CASS_VDW_NONE) {
+      bounded = d.vdw_sum_style != CASS_VDW_SUM_MINIMUM && d.vdw_sum_style != CASS_VDW_SUM_CHARMM;
+      r2 = std::max(r2, d.vdw_sum_style == CASS_VDW_SUM_CUT_SWITCH ? B.dev.roff_switch_sq : B.dev.rcut_vdwsq);
+    }
+  }
+  if (B.desc.charge_style == CASS_CHARGE_COUL && B.desc.charge_sum_style == CASS_QQ_MINIMUM) bounded = false;
+  const double lmax = std::max(B.dev.L[0], std::max(B.dev.L[1], B.dev.L[2]));
+  const float pre2 = bounded ? (float)(r2 * (1.0 + 1.0e-4) + 1.0e-3 + 2.0e-6 * lmax * std::sqrt(r2)) : FLT_MAX;
   const double4_32a* d_com = B.comcut ? B.d_com.as<double4_32a>() : nullptr;
   const double rmax = cbmc ? B.desc.rcut_cbmc : B.rcut_max;
   const int skip_slot = skip_im > 0 ? mol_slot(c, skip_im, is) : -1;
   const int want_qq = (cbmc && !s.l_coul_cbmc) ? 0 : 1;  // Compute_MoleculePair_Energy, energy_routines.f90:1684-1686
   if (c->precision == CASS_PREC_MIXED)
     k_trial_energy<true><<<ntrial, kBlock, 0, c->stream>>>(B.dev, c->pt, B.d_p64.as<double4_32a>(), B.d_meta.as<int4>(),
-                                                           B.npacked, skip_slot, d_tr, d_tt, nat, cbmc, want_qq, d_tcom,
+                                                           B.npacked, skip_slot, d_tr, d_tt, nat, cbmc, want_qq,
+                                                           B.d_p32.as<float4>(), pre2, d_tcom,
                                                            d_com, rmax, d_e, d_ov);
   else
     k_trial_energy<false><<<ntrial, kBlock, 0, c->stream>>>(B.dev, c->pt, B.d_p64.as<double4_32a>(), B.d_meta.as<int4>(),
-                                                            B.npacked, skip_slot, d_tr, d_tt, nat, cbmc, want_qq, d_tcom,
+                                                            B.npacked, skip_slot, d_tr, d_tt, nat, cbmc, want_qq,
+                                                            B.d_p32.as<float4>(), pre2, d_tcom,
                                                             d_com, rmax, d_e, d_ov);
   CASS_CUDA(cudaGetLastError());
   count_launch(c);
-  CASS_CUDA(d2h(c, e, d_e, (size_t)ntrial * sizeof(double)));
-  CASS_CUDA(d2h(c, overlap, d_ov, (size_t)ntrial * sizeof(int)));
+  // the staging may be written again: the kernel has read its upload before this copy starts
+  CASS_CUDA(d2h(c, tr, d_e, down));
   CASS_CUDA(cudaStreamSynchronize(c->stream));
+  memcpy(e, tr, (size_t)ntrial * sizeof(double));
+  memcpy(overlap, reinterpret_cast<const char*>(tr) + (size_t)ntrial * sizeof(double), (size_t)ntrial * sizeof(int));
   return CASS_OK;
 }
 

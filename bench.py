@@ -68,7 +68,7 @@ def parse():
     p.add_argument("--npt-blocks", type=int, default=32, help="production blocks (configurations per chain)")
     p.add_argument("--profile-case", choices=["mixed", "fp64", "mc"], default=None,
                    help="only the small case a kernel profile uses: the Widom kernel on 16 of the benchmark boxes, "
-                        "16,000 (mixed) or 4,096 (FP64) insertions per box, fixed cell edge, three launches; or (mc) "
+                        "16,000 (mixed) or 4,096 (FP64) insertions per box, three launches; or (mc) "
                         "single MC chains: FP64 water-256 (warm-up and 2 sweeps), then mixed LJ-500 (warm-up and 20 "
                         "sweeps)")
     return p.parse_args()
@@ -608,8 +608,6 @@ def profile_case(args):
     with cg.open_system(s, precision=abi.PREC_MIXED if mixed else abi.PREC_FP64) as g:
         for b in boxes:
             g.system_total_energy(b)
-        g.set_widom_autotune(False)
-        g.set_widom_cells(1.0 if mixed else 4.0)
         for r in range(3):
             g.widom_insert(2, boxes, n, args.kappa, args.kappa, seed=1 + r)
             st = g.stats()
@@ -809,7 +807,7 @@ def main():
            "widom_launch": {"ctas_per_box": st["widom_grid_x"], "threads": st["widom_block"],
                             "smem_bytes": st["widom_smem_bytes"], "fp64_fixups": int(st["widom_fixups"]),
                             "fp64_fixup_fraction": st["widom_fixups"] / float(n_per_box * len(boxes)),
-                            "note": "shape chosen by the library's launch autotuner on its first call"},
+                            "note": "shape chosen by the library from the insertion count"},
            "gpu_launches": int(launches),
            "wall_s": t_wall,
            "mu_ex_per_box": {"unit": "kJ/mol", "definition": "-kT ln <widom_var> (widom_insert.f90:445-447), "
@@ -825,8 +823,8 @@ def main():
                         "frac": achieved_tf / fp32_peak, "traffic": traffic,
                         "pairs_visited": st["widom_pairs_visited"], "pairs_in_cutoff": st["widom_pairs_in_cutoff"],
                         "in_cutoff_only": {"achieved": achieved_alg_tf, "frac": achieved_alg_tf / fp32_peak},
-                        "note": "the Widom kernels (k_widom_f32, one thread per insertion, then k_widom_fix for the "
-                                "insertions it queues; kernel_ms spans both); 15 FP32 ops per visited candidate pair "
+                        "note": "the Widom kernels (k_vox_lists, k_widom_f32, then k_widom_fix for the insertions it "
+                                "queues; kernel_ms spans them); 15 FP32 ops per visited candidate pair "
                                 "+ 8 per in-cutoff LJ pair, pairs counted by the kernel in an extra untimed pass; "
                                 "peak is nominal (SMs x 128 FP32 lanes x 2 x max SM clock): the measured-peak file "
                                 "has no FP32 figure; traffic = DRAM bytes per launch scaled from the ncu capture "
@@ -834,7 +832,7 @@ def main():
            "hbm_roofline": {"bound": "hbm", "achieved": achieved_gbs, "peak": hbm_peak, "unit": "GB/s",
                             "frac": achieved_gbs / hbm_peak,
                             "note": "algorithmic bytes = 33 B record per insertion + box staged once per CTA; "
-                                    "peak of measured; the kernel keeps its box in shared memory, so HBM is idle"},
+                                    "peak of measured; the boxes sit in shared memory, the neighbour lists in L2"},
            "kernel_ms": kern_ms, "clocks": clk}
 
     # end to end through the public API with host buffers (frame upload, energies, Widom, results back)

@@ -541,11 +541,11 @@ int cass_set_count_pairs(cass_ctx* ctx, int32_t count_pairs);
  * edge is rcut_cbmc / cells_per_cutoff (0 restores the default of the
  * context's precision).  Results do not depend on it beyond summation order. */
 int cass_set_widom_cells(cass_ctx* ctx, double cells_per_cutoff);
-/* on != 0 (the default): the first cass_widom_insert of each batch signature
- * times a few launch shapes (cell edge, CTAs per resident slot) on a sample of
- * insertions and the context keeps the fastest; a cell edge set with
- * cass_set_widom_cells disables it.  Results do not depend on the shape beyond
- * summation order. */
+/* on != 0 (the default): the first FP64 cass_widom_insert of each batch signature
+ * whose boxes have no neighbour lists (CBMC options, molecule-pair cutoff, styles
+ * without a cutoff) times two cell edges on a sample of insertions and the context
+ * keeps the faster; a cell edge set with cass_set_widom_cells disables it.  Results
+ * do not depend on the edge beyond summation order. */
 int cass_set_widom_autotune(cass_ctx* ctx, int32_t on);
 /* CTAs (a thread-block cluster) that run each chain of cass_mc_sweeps: 0 (the
  * default) chooses per call -- several when few chains leave SMs idle, so a

@@ -1,7 +1,8 @@
 // cass_abi.cu -- C-ABI entry points of libcassgpu.so and the energy kernels
 // that back them:
 //   k_mol_inter      Compute_Molecule_Nonbond_Inter_Energy   (energy_routines.f90:1088-1206)
-//   k_pair_total     inter-molecular part of Compute_System_Total_Energy (:2775-2917)
+//   k_pair_total / k_pair_hits  inter-molecular part of Compute_System_Total_Energy
+//                    (:2775-2917), mixed / FP64
 //   k_intra_total    intra + bonded part of Compute_System_Total_Energy  (:2697-2769)
 //   k_sfac / k_sfac_reduce  Compute_System_Ewald_Reciprocal_Energy     (:4111-4231)
 //   k_ewald_update   Update_System_Ewald_Reciprocal_Energy   (:2326-2497)

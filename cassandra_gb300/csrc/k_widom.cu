@@ -7,13 +7,21 @@
 //       every pair with r <= cutoff is visited exactly once, whatever the cell
 //       count, so the energies are those of the molecule loop of
 //       Compute_Molecule_Nonbond_Inter_Energy_Widom (energy_routines.f90:1266-1297).
-//   k_widom
-//       one thread per Widom insertion: Build_Molecule with kappa_ins first-
-//       fragment trials and Fragment_Placement with kappa_dih dihedral trials
+//   k_vox_lists
+//       neighbour lists on a grid of voxels, from the cell lists.
+//   k_widom_f32 / k_widom_w (mixed / FP64)
+//       a lane per Widom insertion: Build_Molecule with kappa_ins first-fragment
+//       trials and Fragment_Placement with kappa_dih dihedral trials
 //       (fragment_growth.f90:72-707, 1449-2132), then the full-cutoff energy,
 //       intramolecular and bonded energies of the grown molecule
-//       (widom_insert.f90:320-447).  The CTA's box (cell-sorted atoms and cell
-//       offsets) is staged in shared memory when it fits.
+//       (widom_insert.f90:320-447); the neighbour queries of a warp's insertions
+//       are worked through by the whole warp.  The CTA's box (cell-sorted atoms)
+//       is staged in shared memory when it fits.
+//   k_widom_fix
+//       the FP64 cutoff decisions of the mixed path.
+//   k_widom
+//       FP64, one thread per insertion through the cell lists: CBMC options, the
+//       molecule-pair cutoff, styles without a cutoff.
 //   k_widom_recip
 //       Update_System_Ewald_Reciprocal_Energy_Widom (energy_routines.f90:2500-2550)
 //       for the insertions that survived, when the box carries an Ewald sum.
@@ -738,7 +746,7 @@ __device__ void run_insertion(const WidomSpecies& S, const SpeciesPools& P, cons
 }
 
 // ---------------------------------------------------------------------------
-// Mixed-precision Widom kernel: one insertion per thread, FP32 throughout.
+// Mixed-precision Widom kernel: a lane per insertion, FP32 throughout.
 //
 // GB300 issues FP64 at 1/64 of its FP32 rate, so this kernel reads only FP32
 // tables (species, box constants, fragment libraries, cell-sorted atoms) and
@@ -2354,7 +2362,7 @@ __global__ void __launch_bounds__(128) k_widom_fix(WidomSpecies S, SpeciesF SF, 
   }
 }
 
-// FP64 kernel: one insertion per thread (the reference's arithmetic)
+// FP64 kernel: one insertion per thread through the cell lists
 template <bool SMEM>
 __global__ void __launch_bounds__(128) k_widom(WidomSpecies S, PairTable T, SpeciesPools P, const BoxDev* boxes,
                                                const int* box_ids, const double4_32a* c64, const int* ctype,

@@ -1188,8 +1188,10 @@ __device__ __noinline__ void coop_eval(const CoopBox B, int nq, bool want_qq, Qu
                   ov = true;
                 } else if (f.tab_res > 0) {
                   float et = 0.0f;
+                  // the table's charges count whatever want_qq says (energy_routines.f90:1563-1583)
                   const int k = table_pair_f(f.tab_v, f.tab_f2, f.tab_res, f.tab_shift, f.tab_rcs, f.tab_step,
-                                             f.tab_inv_step, f.ntypes, r2, ta, tj, qicf, qq_on ? B.q32[j] : 0.0f, et);
+                                             f.tab_inv_step, f.ntypes, r2, ta, tj, qicf,
+                                             f.charge_on ? B.q32[j] : 0.0f, et);
                   if (k == 2) ov = true;
                   if (k == 1) {
                     e.add(et);

@@ -1005,13 +1005,24 @@ struct VoxGrid {
 };
 constexpr unsigned kVoxAtomBits = 17;
 constexpr unsigned kVoxAtomMask = (1u << kVoxAtomBits) - 1u;
+// An entry's image code is kImage0 + sx + 7 sy + 49 sz, a query point's own shift is added to
+// it.  Minimum_Image_Separation (minimum_image_separation.f90:35-112) moves a separation by
+// one box edge at most, so a sum beyond that is no pair: its shift is out of every reach.
+constexpr int kImages = 343, kImage0 = 171;
+constexpr float kNoImage = 1.0e15f;
+__device__ __forceinline__ int image_of(int code, int d) {  // shift in dimension d, in box edges
+  return (d == 0 ? code % 7 : d == 1 ? code / 7 % 7 : code / 49) - 3;
+}
+__device__ __forceinline__ bool image_valid(int code) {
+  return abs(image_of(code, 0)) <= 1 && abs(image_of(code, 1)) <= 1 && abs(image_of(code, 2)) <= 1;
+}
 
 // Dynamic shared memory of a CTA: the head, one CoopWarp per warp, then (with
 // SMEM) the box's cell starts and atoms at the offsets of its CoopBox.
 struct CoopHead {
   BoxF f;
   VoxGrid vox[2];                     // neighbour lists of the CBMC and the full-cutoff radius
-  float4 shift[125];                  // (sx Lx, sy Ly, sz Lz) at 62 + sx + 5 sy + 25 sz
+  float4 shift[kImages];              // (sx Lx, sy Ly, sz Lz) of an image code
   float2 ljp[kMaxTypes * kMaxTypes];  // (eps, sigma^2)
   double ec;
   int atom_off, cell_off, natoms;
@@ -1248,26 +1259,24 @@ __device__ __noinline__ void coop_eval(const CoopBox B, int nq, bool want_qq, Qu
   }
 }
 
-// the voxel record of point (x, y, z), which is moved by whole box edges where it
-// lies beyond the neighbouring images; code: its own image shift as an entry has it
-__device__ __forceinline__ uint4 vox_record(const BoxF& f, const VoxGrid& g, const uint4* vrec, float& x, float& y,
-                                            float& z, int& code) {
-  float p[3] = {x, y, z};
+// the voxel record of point (x, y, z); code: its own image shift, to be added to an entry's
+__device__ __forceinline__ uint4 vox_record(const BoxF& f, const VoxGrid& g, const uint4* vrec, float x, float y,
+                                            float z, int& code) {
+  const float p[3] = {x, y, z};
   int w[3], s[3];
+  bool far = false;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     const int i = (int)floorf(fminf(fmaxf((p[d] + f.hL[d]) * g.inv[d], -1.0e6f), 1.0e6f));
     s[d] = cell_image(i, g.nv[d]);
     w[d] = i + s[d] * g.nv[d];
-    if (s[d] > 1 || s[d] < -1) {
-      p[d] += (float)s[d] * f.L[d];
-      s[d] = 0;
-    }
+    far = far || s[d] > 2 || s[d] < -2;
   }
-  x = p[0];
-  y = p[1];
-  z = p[2];
-  code = s[0] + 5 * s[1] + 25 * s[2];
+  code = s[0] + 7 * s[1] + 49 * s[2];
+  if (far) {  // no image of an atom is one box edge away
+    code = 0;
+    return make_uint4(0u, 0u, 0u, 0u);
+  }
   return __ldg(&vrec[g.off + (w[2] * g.nv[1] + w[1]) * g.nv[0] + w[0]]);
 }
 
@@ -2115,7 +2124,7 @@ __global__ void __launch_bounds__(128) k_vox_lists(const BoxDev* boxes, const Vo
           const int sx = cell_image(cx, nc[0]);
           const int wx = cx + sx * nc[0], run = min(xhi - cx, nc[0] - 1 - wx) + 1;
           const float qx = c[0] + (float)sx * L[0];
-          const int code = 62 + sx + 5 * sy + 25 * sz;
+          const int code = kImage0 + sx + 7 * sy + 49 * sz;
           for (int j = cs[row + wx]; j < cs[row + wx + run]; ++j) {
             const float4 a = p32[j];
             const float dx = qx - a.x, dy = qy - a.y, dz = qz - a.z;
@@ -2182,9 +2191,11 @@ __global__ void __launch_bounds__(kF32Threads, 1) k_widom_f32(WidomSpecies S, Sp
   if (OPT) boxf_options(H.f, boxes[k], T.ntypes);
   widom_ljp(H.ljp, T);
   if (threadIdx.x < 2) H.vox[threadIdx.x] = vox[2 * k + threadIdx.x];
-  for (int q = threadIdx.x; q < 125; q += blockDim.x)
-    H.shift[q] = make_float4((float)(q % 5 - 2) * (float)boxes[k].L[0], (float)(q / 5 % 5 - 2) * (float)boxes[k].L[1],
-                             (float)(q / 25 - 2) * (float)boxes[k].L[2], 0.0f);
+  for (int q = threadIdx.x; q < kImages; q += blockDim.x)
+    H.shift[q] = image_valid(q) ? make_float4((float)image_of(q, 0) * (float)boxes[k].L[0],
+                                              (float)image_of(q, 1) * (float)boxes[k].L[1],
+                                              (float)image_of(q, 2) * (float)boxes[k].L[2], 0.0f)
+                                : make_float4(kNoImage, kNoImage, kNoImage, 0.0f);
   __syncthreads();
   const int ncell = H.f.nc[0] * H.f.nc[1] * H.f.nc[2];
   CoopBox B;
@@ -2442,15 +2453,15 @@ struct Coop64 {
   double sum[32], sabs[32];
   double e[kHits64];
   float4 posf[32];
-  unsigned hit[kHits64];  // atom | image code << 17 | query << 24 | image to be checked << 29
+  unsigned hit[kHits64];  // atom | image code << 17 | query << 26 | image to be checked << 31
   int type[32], ov[32], first[33];
 };
 struct Head64 {
   BoxDev b;
   BoxF f;
   VoxGrid vox[2];
-  float4 shift[125];
-  double4_32a shift64[125];
+  float4 shift[kImages];
+  double4_32a shift64[kImages];
   double2 lj[kMaxTypes * kMaxTypes];  // eps, sigma^2
   float pre[2];                       // FP32 bound of r^2 beyond the CBMC and the full cutoffs
   float low_sure, low_pre;            // FP32 r^2 below / above which a pair surely is / is not an overlap
@@ -2517,15 +2528,17 @@ __device__ __noinline__ void coop_eval64(const CoopBox B, int nq, bool want_qq, 
   double acc = 0.0, aabs = 0.0;  // FULL: this lane's share of the current query
   // queued pair h in FP64
   auto pair = [&](unsigned h, double& e, double& ea) {
-    const int q = (int)(h >> 24) & 31, j = (int)(h & kVoxAtomMask);
+    const int q = (int)(h >> 26) & 31, j = (int)(h & kVoxAtomMask), c = (int)(h >> kVoxAtomBits) & 511;
     const double4_32a p = W.pos[q], a = c64[j];
     double d[3];
-    const double r2 = sep64(H, p, a, (int)(h >> kVoxAtomBits) & 127, d);
+    const double r2 = sep64(H, p, a, c, d);
     e = 0.0;
     ea = 0.0;
-    if (h >> 29)  // near half a box edge: this atom's other image may be the nearer one
+    if (h >> 31) {  // the image that Minimum_Image_Separation takes, and no other
+      const double d0[3] = {p.x - a.x, p.y - a.y, p.z - a.z};
       for (int k = 0; k < 3; ++k)
-        if (fabs(d[k]) > b.hL[k]) return;
+        if (image_of(c, k) != (d0[k] > b.hL[k] ? -1 : d0[k] < -b.hL[k] ? 1 : 0)) return;
+    }
     if (FULL && r2 < b.rcut_lowsq) {
       W.ov[q] = 1;
       return;
@@ -2603,10 +2616,11 @@ __device__ __noinline__ void coop_eval64(const CoopBox B, int nq, bool want_qq, 
         const int j = (int)(e & kVoxAtomMask), c = (int)(e >> kVoxAtomBits) + code;
         const float4 a = p32[j], sh = H.shift[c];
         const float dx = fabsf((x + sh.x) - a.x), dy = fabsf((y + sh.y) - a.y), dz = fabsf((z + sh.z) - a.z);
-        hit = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > pre) && dx <= H.edge_hi[0] && dy <= H.edge_hi[1] &&
-              dz <= H.edge_hi[2];
-        const unsigned check = dx > H.edge_lo[0] || dy > H.edge_lo[1] || dz > H.edge_lo[2];
-        h = (unsigned)j | (unsigned)c << kVoxAtomBits | (unsigned)q << 24 | check << 29;
+        // a point outside the box may have its pairs through another image than the nearest
+        hit = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > pre) &&
+              (code != 0 || (dx <= H.edge_hi[0] && dy <= H.edge_hi[1] && dz <= H.edge_hi[2]));
+        const unsigned check = code != 0 || dx > H.edge_lo[0] || dy > H.edge_lo[1] || dz > H.edge_lo[2];
+        h = (unsigned)j | (unsigned)c << kVoxAtomBits | (unsigned)q << 26 | check << 31;
       }
       const unsigned m = __ballot_sync(0xffffffffu, hit);
       if (hit) W.hit[cnt + __popc(m & ((1u << lane) - 1u))] = h;
@@ -3099,11 +3113,12 @@ __global__ void __launch_bounds__(kThreads64, 1) k_widom_w(const __grid_constant
     }
   }
   if (threadIdx.x < 2) H.vox[threadIdx.x] = vox[2 * k + threadIdx.x];
-  for (int q = threadIdx.x; q < 125; q += blockDim.x) {
-    const double4_32a v = make_double4_32a((q % 5 - 2) * boxes[k].L[0], (q / 5 % 5 - 2) * boxes[k].L[1],
-                                           (q / 25 - 2) * boxes[k].L[2], 0.0);
+  for (int q = threadIdx.x; q < kImages; q += blockDim.x) {
+    const double4_32a v = make_double4_32a(image_of(q, 0) * boxes[k].L[0], image_of(q, 1) * boxes[k].L[1],
+                                           image_of(q, 2) * boxes[k].L[2], 0.0);
     H.shift64[q] = v;
-    H.shift[q] = make_float4((float)v.x, (float)v.y, (float)v.z, 0.0f);
+    H.shift[q] = image_valid(q) ? make_float4((float)v.x, (float)v.y, (float)v.z, 0.0f)
+                                : make_float4(kNoImage, kNoImage, kNoImage, 0.0f);
   }
   for (int i = threadIdx.x; i < kMaxTypes * kMaxTypes; i += blockDim.x) {
     const int a = i / kMaxTypes, c = i % kMaxTypes;

@@ -4,6 +4,7 @@ import pytest
 
 import cassandra_gb300 as cg
 from cassandra_gb300 import abi, workloads
+from cassandra_gb300.system import Atom, BoxSpec, ForceField, MoleculeSet, Species, System
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -29,3 +30,36 @@ def test_energy_table_counts_the_charges(l_coul_cbmc):
     # FP32 sums are within 1e-5 of the terms; the odd pair of the neighbouring bin stays out of the median
     first = np.abs(tm["e_first_trial_sum"] / np.where(both, to["e_first_trial_sum"], 1.0) - 1.0)[both]
     assert np.median(first) < 1e-4
+
+
+def _rod_system(length=9.6, sites=12, spacing=2.5):
+    """Spheres in a small box and a rigid rod that reaches past the neighbouring images."""
+    ball = Species(atoms=[Atom("B", 20.0, 0.0, ("LJ", 60.0, 1.6))], scale_vdw=(0, 0, 0, 0), scale_qq=(0, 0, 0, 0),
+                   fragments=[[1]], libraries=[np.zeros((1, 1, 3))])
+    site = np.zeros((sites, 3))
+    site[:, 0] = spacing * np.arange(sites)
+    rod = Species(atoms=[Atom("R", 15.0, 0.0, ("LJ", 40.0, 1.4)) for _ in range(sites)], scale_vdw=(0, 0, 0, 0),
+                  scale_qq=(0, 0, 0, 0), fragments=[list(range(1, sites + 1))], libraries=[site[None]])
+    ms = MoleculeSet()
+    for k, p in enumerate(workloads.lj_fluid_box(12, length, 2.0, np.random.default_rng(4))):
+        ms.add(k + 1, 1, 1, p[None])
+    box = BoxSpec(length=(length,) * 3, rcut_vdw=4.0, rcut_cbmc=3.0, rcut_low=0.7, temperature=200.0)
+    return System([ball, rod], [box], ms, ForceField([ball, rod]), [12, 1])
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64])
+def test_atoms_beyond_the_neighbouring_images(prec):
+    """A test molecule longer than the box: Minimum_Image_Separation moves a separation by one
+    box edge at most, so its far atoms see no box atom, or an image that is not the nearest."""
+    s = _rod_system()
+    with oracle.open_system(s) as o, cg.open_system(s, precision=prec) as g:
+        o.system_total_energy(1)
+        g.system_total_energy(1)
+        to = o.widom_insert(2, [1], 400, 12, 12, seed=8, trace=True)[1]
+        tg = g.widom_insert(2, [1], 400, 12, 12, seed=8, trace=True)[1]
+    assert np.array_equal(to["overlap"], tg["overlap"])
+    assert np.array_equal(to["selected_trial"], tg["selected_trial"])
+    ok = to["overlap"] == 0
+    assert ok.sum() > 50
+    tol = 1e-11 if prec == abi.PREC_FP64 else 2e-5  # sums of FP64 terms; FP32 coordinates of a few ulps of 2 box edges
+    assert (np.abs(tg["e_inter"] - to["e_inter"])[ok] <= tol * to["e_inter_abs"][ok] + 1e-7).all()

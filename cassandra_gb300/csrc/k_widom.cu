@@ -914,10 +914,10 @@ __device__ bool query_f_exact(const BoxViewF& V, QueryAcc& A, float px, float py
     const int wz = cz + sz * nc2;
     const float qz = pz + (float)sz * f.L[2];
     const float dz2 = full[2] ? 0.0f : slab_d2_f(cz, f.ch[2], f.hL[2], pz);
-    if (dz2 > rc2) continue;
+    if (dz2 > rc2 || abs(sz) > 1) continue;  // a separation moves by one box edge at most
     for (int cy = lo[1]; cy <= hi[1]; ++cy) {
       const float d2 = full[1] ? dz2 : dz2 + slab_d2_f(cy, f.ch[1], f.hL[1], py);
-      if (d2 > rc2) continue;
+      if (d2 > rc2 || abs(cell_image(cy, nc1)) > 1) continue;
       int xlo, xhi;
       bool fl[3] = {false, full[1], full[2]};
       row_x_cells_f(f, px, rc2 - d2, xlo, xhi, fl[0]);
@@ -932,7 +932,7 @@ __device__ bool query_f_exact(const BoxViewF& V, QueryAcc& A, float px, float py
         const int wx = cx + sx * nc0;
         const int run = min(xhi - cx, nc0 - 1 - wx) + 1;
         const float qx = px + (float)sx * f.L[0];
-        const int j0 = V.cstart[row + wx], j1 = V.cstart[row + wx + run];
+        const int j0 = V.cstart[row + wx], j1 = abs(sx) <= 1 ? V.cstart[row + wx + run] : j0;
         for (int j = j0; j < j1; ++j) {
           const float4 a = V.p32[j];
           const float r2 = pair_r2(f, fl, fold_any, qx, qy, qz, a);
@@ -1150,8 +1150,9 @@ __device__ __noinline__ void coop_eval(const CoopBox B, int nq, bool want_qq, Qu
           const int cz = lo2 + iz, cy = lo1 + rr - iz * ny;
           const float dz2 = fullz ? 0.0f : slab_d2_f(cz, f.ch[2], f.hL[2], p.z);
           const float d2 = fully ? dz2 : dz2 + slab_d2_f(cy, f.ch[1], f.hL[1], p.y);
-          if (dz2 <= rc2 && d2 <= rc2) {
-            const int sz = cell_image(cz, nc2), sy = cell_image(cy, nc1);
+          const int sz = cell_image(cz, nc2), sy = cell_image(cy, nc1);
+          // a separation moves by one box edge at most
+          if (dz2 <= rc2 && d2 <= rc2 && abs(sz) <= 1 && abs(sy) <= 1) {
             qz = p.z + (float)sz * f.L[2];
             qy = p.y + (float)sy * f.L[1];
             int xlo, xhi;
@@ -1162,8 +1163,8 @@ __device__ __noinline__ void coop_eval(const CoopBox B, int nq, bool want_qq, Qu
             const int run = min(xhi - xlo, nc0 - 1 - wx) + 1;
             qxa = p.x + (float)sx * f.L[0];
             ja = cs[wx];
-            n = na = cs[wx + run] - ja;
-            if (xlo + run <= xhi) {
+            n = na = abs(sx) <= 1 ? cs[wx + run] - ja : 0;
+            if (xlo + run <= xhi && abs(sx - 1) <= 1) {
               qxb = p.x + (float)(sx - 1) * f.L[0];
               jb = cs[0];
               n += cs[xhi + (sx - 1) * nc0 + 1] - jb;

@@ -63,3 +63,16 @@ def test_atoms_beyond_the_neighbouring_images(prec):
     assert ok.sum() > 50
     tol = 1e-11 if prec == abi.PREC_FP64 else 2e-5  # sums of FP64 terms; FP32 coordinates of a few ulps of 2 box edges
     assert (np.abs(tg["e_inter"] - to["e_inter"])[ok] <= tol * to["e_inter_abs"][ok] + 1e-7).all()
+
+
+def test_far_atoms_in_the_mixed_kernels_rows():
+    """The same box with the mixed kernel, whose stencils span it: equal decisions.  (Its FP32
+    coordinates of two box edges are too coarse for energies of pairs this steep.)"""
+    s = _rod_system()
+    with oracle.open_system(s) as o, cg.open_system(s, precision=abi.PREC_MIXED) as m:
+        o.system_total_energy(1)
+        m.system_total_energy(1)
+        to = o.widom_insert(2, [1], 400, 12, 12, seed=8, trace=True)[1]
+        tm = m.widom_insert(2, [1], 400, 12, 12, seed=8, trace=True)[1]
+    assert np.array_equal(to["overlap"], tm["overlap"])
+    assert (to["selected_trial"] == tm["selected_trial"]).mean() >= 0.995

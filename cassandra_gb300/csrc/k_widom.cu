@@ -1301,8 +1301,42 @@ __device__ __forceinline__ bool vox_overlap(const CoopBox& B, const CoopHead& H,
   return ov;
 }
 
+// A compensated sum of the even and the odd entries of a list, and its sum of |terms|
+struct PairSum {
+  float2 s = make_float2(0.0f, 0.0f), c = make_float2(0.0f, 0.0f);
+  float a = 0.0f;
+  __device__ __forceinline__ void first(float2 v) {  // the first term
+    s = v;
+    c = make_float2(0.0f, 0.0f);
+  }
+  __device__ __forceinline__ void add(float2 v) {  // TwoSum: the rounding error of the addition, exactly
+    const float2 t = __fadd2_rn(s, v);
+    const float2 m1 = make_float2(-1.0f, -1.0f);
+    const float2 w = __ffma2_rn(s, m1, t);                      // t - s
+    const float2 d = __fadd2_rn(__ffma2_rn(__ffma2_rn(w, m1, t), m1, s), __ffma2_rn(w, m1, v));
+    c = __fadd2_rn(c, d);
+    s = t;
+  }
+  __device__ __forceinline__ void add(const PairSum& o) {
+    add(o.s);
+    c = __fadd2_rn(c, o.c);
+    a += o.a;
+  }
+  __device__ __forceinline__ PairSum down(int o, bool with_abs) const {  // that of the lane o further
+    PairSum r;
+    r.s.x = __shfl_down_sync(0xffffffffu, s.x, o);
+    r.s.y = __shfl_down_sync(0xffffffffu, s.y, o);
+    r.c.x = __shfl_down_sync(0xffffffffu, c.x, o);
+    r.c.y = __shfl_down_sync(0xffffffffu, c.y, o);
+    if (with_abs) r.a = __shfl_down_sync(0xffffffffu, a, o);
+    return r;
+  }
+};
+
 // coop_eval through the voxel lists: a query per lane, or per 2, 4 ... 32 lanes where
-// the queue is short.  CBMC queries (not DETECT) come without an overlap.
+// the queue is short.  CBMC queries (not DETECT) come without an overlap.  Each word of a
+// list (four entries) is summed by itself and the words in their order, whatever lanes
+// have them: an insertion's bits do not depend on what else its warp works on.
 template <bool SMEM, bool COUNT, bool DETECT>
 __device__ __noinline__ void coop_eval_list(const CoopBox B, int nq, bool want_qq, QueryAcc& cnt) {
   const CoopHead& H = coop_head();
@@ -1337,87 +1371,81 @@ __device__ __noinline__ void coop_eval_list(const CoopBox B, int nq, bool want_q
   }
   // half of the entries lie within the cutoff, so every entry's energy is formed, two
   // at a time on the packed FP32 pipe, and those outside add zero
-  float2 es = make_float2(0.0f, 0.0f), ec = es;  // compensated sums of the even and the odd entries
-  float eabs = 0.0f;
+  PairSum sum;
   bool ov = false;
-  auto add2 = [&](float2 v) {  // TwoSum: the rounding error of the addition, exactly
-    const float2 t = __fadd2_rn(es, v);
-    const float2 m1 = make_float2(-1.0f, -1.0f);
-    const float2 w = __ffma2_rn(es, m1, t);                      // t - es
-    const float2 d = __fadd2_rn(__ffma2_rn(__ffma2_rn(w, m1, t), m1, es), __ffma2_rn(w, m1, v));
-    ec = __fadd2_rn(ec, d);
-    es = t;
-  };
   if (COUNT && sub == 0) cnt.visited += (unsigned long long)n;
-  for (int g = sub; 4 * g < n && !ov; g += 1 << lb) {
-    const uint4 E = __ldg(&list[g]);
+  // with several lanes per query all go through the words of the longest list, one each
+  const int most = lb > 0 ? __reduce_max_sync(0xffffffffu, (n + 3) >> 2) : 1;
+  for (int g0 = 0; g0 < most; g0 += 1 << lb) {
+    PairSum w;
+    const int end = lb > 0 ? min(n, 4 * (g0 + (1 << lb))) : n;
+    for (int g = g0 + sub; 4 * g < end && !ov; g += 1 << lb) {
+      const uint4 E = __ldg(&list[g]);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int left = n - 4 * g - 2 * k;
-      if (left <= 0) break;
-      const unsigned e0 = k ? E.z : E.x, e1 = left > 1 ? (k ? E.w : E.y) : e0;
-      const int j0 = (int)(e0 & kVoxAtomMask), j1 = (int)(e1 & kVoxAtomMask);
-      const float4 a0 = p32[j0], a1 = p32[j1];
-      const float4 s0 = H.shift[(int)(e0 >> kVoxAtomBits) + code], s1 = H.shift[(int)(e1 >> kVoxAtomBits) + code];
-      const float2 m1 = make_float2(-1.0f, -1.0f);
-      const float2 dx = __ffma2_rn(make_float2(a0.x, a1.x), m1, __fadd2_rn(make_float2(x, x), make_float2(s0.x, s1.x)));
-      const float2 dy = __ffma2_rn(make_float2(a0.y, a1.y), m1, __fadd2_rn(make_float2(y, y), make_float2(s0.y, s1.y)));
-      const float2 dz = __ffma2_rn(make_float2(a0.z, a1.z), m1, __fadd2_rn(make_float2(z, z), make_float2(s0.z, s1.z)));
-      const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-      const bool in0 = r2.x <= rsel2, in1 = left > 1 && r2.y <= rsel2;
-      if (COUNT) cnt.in_cut += (int)in0 + (int)in1;
-      if (DETECT) {
-        const float rmin = fminf(r2.x, left > 1 ? r2.y : r2.x);
-        if (rmin < low2q) {
-          if (rmin < f.low2 - f.band_low) {
-            ov = true;  // a certain overlap
-          } else {
-            if (r2.x < low2q) coop_note(W, W.own[qi], j0, r2.x, 1);
-            if (left > 1 && r2.y < low2q) coop_note(W, W.own[qi], j1, r2.y, 1);
+      for (int k = 0; k < 2; ++k) {
+        const int left = n - 4 * g - 2 * k;
+        if (left <= 0) break;
+        const unsigned e0 = k ? E.z : E.x, e1 = left > 1 ? (k ? E.w : E.y) : e0;
+        const int j0 = (int)(e0 & kVoxAtomMask), j1 = (int)(e1 & kVoxAtomMask);
+        const float4 a0 = p32[j0], a1 = p32[j1];
+        const float4 s0 = H.shift[(int)(e0 >> kVoxAtomBits) + code], s1 = H.shift[(int)(e1 >> kVoxAtomBits) + code];
+        const float2 m1 = make_float2(-1.0f, -1.0f);
+        const float2 dx = __ffma2_rn(make_float2(a0.x, a1.x), m1, __fadd2_rn(make_float2(x, x), make_float2(s0.x, s1.x)));
+        const float2 dy = __ffma2_rn(make_float2(a0.y, a1.y), m1, __fadd2_rn(make_float2(y, y), make_float2(s0.y, s1.y)));
+        const float2 dz = __ffma2_rn(make_float2(a0.z, a1.z), m1, __fadd2_rn(make_float2(z, z), make_float2(s0.z, s1.z)));
+        const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        const bool in0 = r2.x <= rsel2, in1 = left > 1 && r2.y <= rsel2;
+        if (COUNT) cnt.in_cut += (int)in0 + (int)in1;
+        if (DETECT) {
+          const float rmin = fminf(r2.x, left > 1 ? r2.y : r2.x);
+          if (rmin < low2q) {
+            if (rmin < f.low2 - f.band_low) {
+              ov = true;  // a certain overlap
+            } else {
+              if (r2.x < low2q) coop_note(W, W.own[qi], j0, r2.x, 1);
+              if (left > 1 && r2.y < low2q) coop_note(W, W.own[qi], j1, r2.y, 1);
+            }
           }
+          if (in0 && r2.x >= rlo) coop_note(W, W.own[qi], j0, r2.x, 0);
+          if (in1 && r2.y >= rlo) coop_note(W, W.own[qi], j1, r2.y, 0);
         }
-        if (in0 && r2.x >= rlo) coop_note(W, W.own[qi], j0, r2.x, 0);
-        if (in1 && r2.y >= rlo) coop_note(W, W.own[qi], j1, r2.y, 0);
+        if (vdw_on) {
+          const int t0 = __float_as_int(a0.w), t1 = __float_as_int(a1.w);
+          const float2 l0 = lrow[max(t0, 0)], l1 = lrow[max(t1, 0)];
+          float2 ev = make_float2(lj_pair_f(l0.x, l0.y, r2.x), lj_pair_f(l1.x, l1.y, r2.y));
+          if (!(t0 >= 0 && r2.x <= rv2)) ev.x = 0.0f;
+          if (!(t1 >= 0 && left > 1 && r2.y <= rv2)) ev.y = 0.0f;
+          if (k == 0) w.first(ev);
+          else w.add(ev);
+          if (DETECT) w.a += fabsf(ev.x) + fabsf(ev.y);
+        }
+        if (qq_on) {
+          float2 eq = make_float2(0.0f, 0.0f);
+          if (r2.x <= rq2) eq.x = qq_ewald_inter_f(f.alpha, qa * B.q32[j0], r2.x);
+          if (left > 1 && r2.y <= rq2) eq.y = qq_ewald_inter_f(f.alpha, qa * B.q32[j1], r2.y);
+          w.add(eq);
+          if (DETECT) w.a += fabsf(eq.x) + fabsf(eq.y);
+        }
       }
-      if (vdw_on) {
-        const int t0 = __float_as_int(a0.w), t1 = __float_as_int(a1.w);
-        const float2 l0 = lrow[max(t0, 0)], l1 = lrow[max(t1, 0)];
-        float2 ev = make_float2(lj_pair_f(l0.x, l0.y, r2.x), lj_pair_f(l1.x, l1.y, r2.y));
-        if (!(t0 >= 0 && r2.x <= rv2)) ev.x = 0.0f;
-        if (!(t1 >= 0 && left > 1 && r2.y <= rv2)) ev.y = 0.0f;
-        add2(ev);
-        if (DETECT) eabs += fabsf(ev.x) + fabsf(ev.y);
-      }
-      if (qq_on) {
-        float2 eq = make_float2(0.0f, 0.0f);
-        if (r2.x <= rq2) eq.x = qq_ewald_inter_f(f.alpha, qa * B.q32[j0], r2.x);
-        if (left > 1 && r2.y <= rq2) eq.y = qq_ewald_inter_f(f.alpha, qa * B.q32[j1], r2.y);
-        add2(eq);
-        if (DETECT) eabs += fabsf(eq.x) + fabsf(eq.y);
+      if (lb == 0) {
+        sum.add(w);
+        w.a = 0.0f;
+        if (!vdw_on) w.first(make_float2(0.0f, 0.0f));  // the next word's first term is a Coulomb one
       }
     }
+    if (lb > 0) {  // the lanes' words in their order; those beyond a list's end are zero, which adds exactly
+      sum.add(w);
+      for (int o = 1; o < min(1 << lb, most - g0); ++o) sum.add(w.down(o, DETECT));
+    }
   }
+  if (DETECT && ov) W.ov[qi] = 1;
   KahanF e;
-  e.s = es.x;
-  e.c = ec.x;
-  e.add(es.y);
-  e.c += ec.y;
+  e.s = sum.s.x;
+  e.c = sum.c.x;
+  e.add(sum.s.y);
+  e.c += sum.c.y;
   __syncwarp();
-  for (int o = 1 << lb >> 1; o > 0; o >>= 1) {
-    const float s = __shfl_down_sync(0xffffffffu, e.s, o), c = __shfl_down_sync(0xffffffffu, e.c, o);
-    e.add(s);
-    e.c += c;
-    if (DETECT) {
-      eabs += __shfl_down_sync(0xffffffffu, eabs, o);
-      const int other = __shfl_down_sync(0xffffffffu, (int)ov, o);
-      ov = ov || other;
-    }
-  }
-  __syncwarp();
-  if (valid && sub == 0) {
-    W.pos[qi] = make_float4(e.s, e.c, eabs, 0.0f);
-    if (DETECT && ov) W.ov[qi] = 1;
-  }
+  if (valid && sub == 0) W.pos[qi] = make_float4(e.s, e.c, sum.a, 0.0f);
   __syncwarp();
 }
 

@@ -76,3 +76,28 @@ def test_far_atoms_in_the_mixed_kernels_rows():
         tm = m.widom_insert(2, [1], 400, 12, 12, seed=8, trace=True)[1]
     assert np.array_equal(to["overlap"], tm["overlap"])
     assert (to["selected_trial"] == tm["selected_trial"]).mean() >= 0.995
+
+
+def _alone_and_together(s, prec, is_, n_ins, pick, band=1.0, **opts):
+    """Records of box `pick` from a call for it alone and from one for all boxes."""
+    ids = list(range(1, len(s.boxes) + 1))
+    with cg.open_system(s, precision=prec) as g:
+        for b in ids:
+            g.system_total_energy(b)
+        if opts:
+            g.set_cbmc_options(**opts)
+        g.set_widom_band(band)
+        g.set_widom_autotune(False)
+        one, t1 = g.widom_insert(is_, [pick], n_ins, 12, 12, seed=5, trace=True)
+        every, ta = g.widom_insert(is_, ids, n_ins, 12, 12, seed=5, trace=True)
+    return one[0], t1[0], every[pick - 1], ta[pick - 1]
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("sizes", [[250] * 40, [1000, 300, 600] * 10])
+def test_an_insertion_does_not_depend_on_the_other_boxes(prec, sizes):
+    """One insertion per warp in the call for one box, 16 and more in that for all of them."""
+    s = workloads.widom_batch_system(nboxes=len(sizes), sizes=sizes, seed=6, nconfig=100)
+    one, t1, among, ta = _alone_and_together(s, prec, 2, 2400, 1)
+    assert t1.tobytes() == ta.tobytes()
+    assert one == among

@@ -1213,6 +1213,9 @@ int ensure_cbmc(cass_ctx_impl* c) {
       if (B.defined)
         for (double r2 : rmin)
           if (r2 > B.dev.rcut_cbmcsq) return set_error(CASS_EUNSUPPORTED, "r_min exceeds rcut_cbmc");
+  c->rminsq_most = 0.0;
+  if (o.sector_overlap)
+    for (double r2 : rmin) c->rminsq_most = std::max(c->rminsq_most, r2);
   // host image of the device buffer
   const size_t nn = (size_t)nt * nt;
   const size_t per_box = res > 0 ? (nn * res + res) * (sizeof(double) + sizeof(float)) : 0;

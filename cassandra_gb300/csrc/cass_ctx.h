@@ -229,6 +229,7 @@ struct cass_ctx_impl {
   std::vector<int> widom_boxes;
   // CBMC options and the tables they derive (energy table per box, r_min^2)
   CassCBMCOptions cbmc_opt{};
+  double rminsq_most = 0.0;  // the largest r_min^2 of check_overlap (0 without it)
   bool cbmc_dirty = true;
   DevBuf d_cbmc_tab;
   // pinned staging of the packed-box uploads

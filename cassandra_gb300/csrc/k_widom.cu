@@ -1281,9 +1281,11 @@ __device__ __forceinline__ uint4 vox_record(const BoxF& f, const VoxGrid& g, con
   return __ldg(&vrec[g.off + (w[2] * g.nv[1] + w[1]) * g.nv[0] + w[0]]);
 }
 
-// Core overlap of a CBMC query point: only the first entries of its list can be that near
-template <bool SMEM>
-__device__ __forceinline__ bool vox_overlap(const CoopBox& B, const CoopHead& H, float x, float y, float z) {
+// Core overlap of a CBMC query point of type ta: only the first entries of its list can be
+// that near.  OPT: check_overlap (sector_routines.f90:160-233) and the energy table's rule.
+template <bool SMEM, bool OPT>
+__device__ __forceinline__ bool vox_overlap(const CoopBox& B, const CoopHead& H, float x, float y, float z, int ta) {
+  const BoxF& f = H.f;
   const float4* p32;
   if constexpr (SMEM) p32 = reinterpret_cast<const float4*>(smem + B.off_atoms);
   else p32 = B.p32;
@@ -1296,7 +1298,12 @@ __device__ __forceinline__ bool vox_overlap(const CoopBox& B, const CoopHead& H,
     const unsigned e = __ldg(&list[t]);
     const float4 a = p32[e & kVoxAtomMask], sh = H.shift[(int)(e >> kVoxAtomBits) + code];
     const float dx = (x + sh.x) - a.x, dy = (y + sh.y) - a.y, dz = (z + sh.z) - a.z;
-    ov = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < H.f.low2;
+    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+    ov = OPT && f.tab_res > 0 ? r2 - f.tab_shift < f.tab_step : r2 < f.low2;
+    if (OPT && f.sector) {
+      const int tj = __float_as_int(a.w);
+      ov = ov || r2 < (ta >= 0 && tj >= 0 ? f.rmin2[ta * kMaxTypes + tj] : f.low2);
+    }
   }
   return ov;
 }
@@ -1337,7 +1344,7 @@ struct PairSum {
 // the queue is short.  CBMC queries (not DETECT) come without an overlap.  Each word of a
 // list (four entries) is summed by itself and the words in their order, whatever lanes
 // have them: an insertion's bits do not depend on what else its warp works on.
-template <bool SMEM, bool COUNT, bool DETECT>
+template <bool SMEM, bool COUNT, bool OPT, bool DETECT>
 __device__ __noinline__ void coop_eval_list(const CoopBox B, int nq, bool want_qq, QueryAcc& cnt) {
   const CoopHead& H = coop_head();
   const BoxF& f = H.f;
@@ -1409,6 +1416,18 @@ __device__ __noinline__ void coop_eval_list(const CoopBox B, int nq, bool want_q
           if (in0 && r2.x >= rlo) coop_note(W, W.own[qi], j0, r2.x, 0);
           if (in1 && r2.y >= rlo) coop_note(W, W.own[qi], j1, r2.y, 0);
         }
+        if (OPT && f.tab_res > 0) {  // Estimate_MoleculePair_Energy, its charges whatever want_qq says
+          const float qic = qa * (float)kCHARGE_FACTOR;
+          float2 et = make_float2(0.0f, 0.0f);
+          table_pair_f(f.tab_v, f.tab_f2, f.tab_res, f.tab_shift, f.tab_rcs, f.tab_step, f.tab_inv_step, f.ntypes, r2.x,
+                       ta, __float_as_int(a0.w), qic, f.charge_on ? B.q32[j0] : 0.0f, et.x);
+          if (left > 1)
+            table_pair_f(f.tab_v, f.tab_f2, f.tab_res, f.tab_shift, f.tab_rcs, f.tab_step, f.tab_inv_step, f.ntypes, r2.y,
+                         ta, __float_as_int(a1.w), qic, f.charge_on ? B.q32[j1] : 0.0f, et.y);
+          if (k == 0) w.first(et);
+          else w.add(et);
+          continue;
+        }
         if (vdw_on) {
           const int t0 = __float_as_int(a0.w), t1 = __float_as_int(a1.w);
           const float2 l0 = lrow[max(t0, 0)], l1 = lrow[max(t1, 0)];
@@ -1461,12 +1480,12 @@ __device__ __forceinline__ void coop_atoms(const CoopBox& B, const SpeciesF& S, 
   CoopWarp& W = coop_warp();
   const int lane = threadIdx.x & 31;
   const float rc = DETECT ? f.rc_full : f.rc_cbmc;
-  const bool lists = !OPT && coop_head().vox[DETECT ? 1 : 0].on;
+  const bool lists = coop_head().vox[DETECT ? 1 : 0].on;
   on = on && !ov;
   if (lists && !DETECT && on)  // the trials with a core overlap end here, before their energies
     for (int i = 0; i < nat && !ov; ++i) {
       const int at = ids[i];
-      ov = vox_overlap<SMEM>(B, coop_head(), r[3 * at] + sx, r[3 * at + 1] + sy, r[3 * at + 2] + sz);
+      ov = vox_overlap<SMEM, OPT>(B, coop_head(), r[3 * at] + sx, r[3 * at + 1] + sy, r[3 * at + 2] + sz, S.type[at]);
     }
   const int most = __reduce_max_sync(0xffffffffu, on ? nat : 0);
   for (int i0 = 0; i0 < most;) {
@@ -1498,7 +1517,7 @@ __device__ __forceinline__ void coop_atoms(const CoopBox& B, const SpeciesF& S, 
         }
       }
     __syncwarp();
-    if (lists) coop_eval_list<SMEM, COUNT, DETECT>(B, __popc(m) * per, want_qq, cnt);
+    if (lists) coop_eval_list<SMEM, COUNT, OPT, DETECT>(B, __popc(m) * per, want_qq, cnt);
     else coop_eval<SMEM, COUNT, OPT, DETECT>(B, __popc(m) * per, want_qq, cnt);
     if (mine)
       for (int a = 0; a < per && i0 + a < nat; ++a) {
@@ -3445,9 +3464,10 @@ const std::vector<int>& members_ext(cass_ctx* c, int ibox);
 
 namespace {
 
-// The voxel grid `which` (0 CBMC, 1 full) of box b for queries of radius rc: record
-// offset off; room: entries it can need.  False where an entry cannot describe the box.
-bool vox_grid(const BoxDev& b, int which, double rc, int off, VoxGrid& g, double& nvox, double& room) {
+// The voxel grid `which` (0 CBMC, 1 full) of box b for queries of radius rc whose core
+// overlaps lie within lowsq: record offset off; room: entries it can need.  False where an
+// entry cannot describe the box.
+bool vox_grid(const BoxDev& b, int which, double rc, double lowsq, int off, VoxGrid& g, double& nvox, double& room) {
   memset(&g, 0, sizeof(g));
   if (b.natoms < 1 || b.natoms > (int)kVoxAtomMask || !(rc > 0.0)) return false;
   const double edge = rc / (which ? kVoxPerCutoffFull : kVoxPerCutoffCbmc);
@@ -3468,7 +3488,7 @@ bool vox_grid(const BoxDev& b, int which, double rc, int off, VoxGrid& g, double
   const double per_atom = std::min(most, 4.18879021 * std::pow(R + half, 3.0) * nvox / b.volume);
   room = b.natoms * per_atom + 3.0 * nvox;
   g.R2 = (float)(R * R);
-  const double near = std::sqrt(b.rcut_lowsq) + half;
+  const double near = std::sqrt(lowsq) + half;
   g.near2 = (float)(near * near);
   g.off = off;
   // images of the neighbouring boxes only; a list of 2e4 atoms is no neighbour list
@@ -3501,7 +3521,8 @@ bool lists64(cass_ctx* c, int nboxes, const int32_t* iboxes) {
     for (int w = 0; w < 2; ++w) {
       VoxGrid g;
       double nvox, room;
-      if (!vox_grid(b, w, w ? full_radius(b) : std::sqrt(b.rcut_cbmcsq), 0, g, nvox, room)) return false;
+      if (!vox_grid(b, w, w ? full_radius(b) : std::sqrt(b.rcut_cbmcsq), b.rcut_lowsq, 0, g, nvox, room))
+        return false;
       total += room;
     }
   }
@@ -3727,7 +3748,7 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   int vox_most[2] = {0, 0};
   memset(vox.data(), 0, vox.size() * sizeof(VoxGrid));
   const bool opt_cbmc = c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap;
-  if (((f32 && !opt_cbmc) || warp64) && n_ins > 0)
+  if ((f32 || warp64) && n_ins > 0)
     for (int k = 0; k < nboxes; ++k) {
       const BoxDev& b = bd[k];
       const double rfull2 = std::max(b.rcut_vdwsq, b.rcut_coulsq);
@@ -3738,7 +3759,9 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
       for (int w = 0; w < 2; ++w) {
         VoxGrid g;
         double nvox, room;
-        if (!vox_grid(b, w, rcs[w], (int)vox_records, g, nvox, room)) continue;
+        // check_overlap of the CBMC options reaches to r_min
+        const double lowsq = opt_cbmc && w == 0 ? std::max(b.rcut_lowsq, c->rminsq_most) : b.rcut_lowsq;
+        if (!vox_grid(b, w, rcs[w], lowsq, (int)vox_records, g, nvox, room)) continue;
         if (f32) {
           bool open = (double)n_ins * (w ? 2.0 : 32.0) >= nvox;
           for (int d = 0; d < 3; ++d)

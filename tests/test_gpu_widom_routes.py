@@ -101,3 +101,25 @@ def test_an_insertion_does_not_depend_on_the_other_boxes(prec, sizes):
     one, t1, among, ta = _alone_and_together(s, prec, 2, 2400, 1)
     assert t1.tobytes() == ta.tobytes()
     assert one == among
+
+
+@pytest.mark.parametrize("opts", [{"energy_table_res": 1000}, {"sector_overlap": True, "rmin_u_max": 300.0},
+                                  {"energy_table_res": 1000, "sector_overlap": True, "rmin_u_max": 300.0}])
+def test_cbmc_options_in_the_mixed_kernel(opts):
+    """The options' queries on the neighbour lists, per insertion: FP32 may put a pair into the
+    neighbouring bin of the table or across an r_min, everything else is the oracle's."""
+    s = workloads.widom_batch_system(nboxes=2, sizes=[1300, 220], seed=3, nconfig=100)
+    with oracle.open_system(s) as o, cg.open_system(s, precision=abi.PREC_MIXED) as m:
+        for c in (o, m):
+            for b in (1, 2):
+                c.system_total_energy(b)
+            c.set_cbmc_options(**opts)
+        to = o.widom_insert(2, [1, 2], 300, 12, 12, seed=21, trace=True)[1]
+        tm = m.widom_insert(2, [1, 2], 300, 12, 12, seed=21, trace=True)[1]
+        alone = m.widom_insert(2, [2], 300, 12, 12, seed=21, trace=True)[1]
+    assert (to["overlap"] == tm["overlap"]).mean() > 0.98
+    assert (to["selected_trial"] == tm["selected_trial"]).mean() > 0.95
+    both = (to["overlap"] == 0) & (tm["overlap"] == 0)
+    near = np.abs(tm["e_inter"] - to["e_inter"]) <= 2e-5 * to["e_inter_abs"] + 1e-7
+    assert near[both].mean() > 0.9 and both.sum() > 100
+    assert alone[0].tobytes() == tm[1].tobytes()

@@ -63,6 +63,11 @@ constexpr size_t kSmemMax = 227 * 1024;  // dynamic shared memory of a CTA
 // 15.4, 15.2 and 15.8 ms, 3, 4 and 5 for the full one 15.2, 15.2 and 15.5 ms
 constexpr double kVoxPerCutoffCbmc = 3.25;
 constexpr double kVoxPerCutoffFull = 4.0;
+// Most voxels per atom of a box: a voxel costs its search even where it is empty.  500
+// atoms in a box of 400 A had 8e6 voxels of the CBMC radius: one FP64 insertion 1.62 ms,
+// 0.37 ms now (1.30 ms without lists); 1e5 mixed ones, which went without lists, 2.70 ms,
+// 1.02 ms now.  Liquids have 1 to 11.
+constexpr double kVoxPerAtom = 16.0;
 constexpr double kVoxMaxBytes = 4.0e9;      // most device memory for them
 
 __device__ __forceinline__ int wrapc(int c, int n) {
@@ -1003,7 +1008,7 @@ struct VoxGrid {
   int off;         // first record of the box
   int on;
 };
-constexpr unsigned kVoxAtomBits = 17;
+constexpr unsigned kVoxAtomBits = 23;
 constexpr unsigned kVoxAtomMask = (1u << kVoxAtomBits) - 1u;
 // An entry's image code is kImage0 + sx + 7 sy + 49 sz, a query point's own shift is added to
 // it.  Minimum_Image_Separation (minimum_image_separation.f90:35-112) moves a separation by
@@ -2494,6 +2499,7 @@ __global__ void __launch_bounds__(128) k_widom(WidomSpecies S, PairTable T, Spec
 // queued, and 32 of them at a time are decided and evaluated in FP64.  (A thread per
 // insertion had 8.5 of 32 lanes at work and formed every visited pair in FP64.)
 constexpr int kHits64 = 256;  // queued pairs of a warp
+constexpr unsigned kHitAtomBits = 17;  // a box on the FP64 lists has fewer than 2^17 atoms
 constexpr int kThreads64 = 384;
 
 struct Coop64 {
@@ -2501,7 +2507,7 @@ struct Coop64 {
   double sum[32], sabs[32];
   double e[kHits64];
   float4 posf[32];
-  unsigned hit[kHits64];  // atom | image code << 17 | query << 26 | image to be checked << 31
+  unsigned hit[kHits64];  // atom | image code << kHitAtomBits | query << 26 | image to be checked << 31
   int type[32], ov[32], first[33];
 };
 struct Head64 {
@@ -2576,7 +2582,7 @@ __device__ __noinline__ void coop_eval64(const CoopBox B, int nq, bool want_qq, 
   double acc = 0.0, aabs = 0.0;  // FULL: this lane's share of the current query
   // queued pair h in FP64
   auto pair = [&](unsigned h, double& e, double& ea) {
-    const int q = (int)(h >> 26) & 31, j = (int)(h & kVoxAtomMask), c = (int)(h >> kVoxAtomBits) & 511;
+    const int q = (int)(h >> 26) & 31, j = (int)(h & ((1u << kHitAtomBits) - 1u)), c = (int)(h >> kHitAtomBits) & 511;
     const double4_32a p = W.pos[q], a = c64[j];
     double d[3];
     const double r2 = sep64(H, p, a, c, d);
@@ -2668,7 +2674,7 @@ __device__ __noinline__ void coop_eval64(const CoopBox B, int nq, bool want_qq, 
         hit = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > pre) &&
               (code != 0 || (dx <= H.edge_hi[0] && dy <= H.edge_hi[1] && dz <= H.edge_hi[2]));
         const unsigned check = code != 0 || dx > H.edge_lo[0] || dy > H.edge_lo[1] || dz > H.edge_lo[2];
-        h = (unsigned)j | (unsigned)c << kVoxAtomBits | (unsigned)q << 26 | check << 31;
+        h = (unsigned)j | (unsigned)c << kHitAtomBits | (unsigned)q << 26 | check << 31;
       }
       const unsigned m = __ballot_sync(0xffffffffu, hit);
       if (hit) W.hit[cnt + __popc(m & ((1u << lane) - 1u))] = h;
@@ -3467,11 +3473,14 @@ namespace {
 // The voxel grid `which` (0 CBMC, 1 full) of box b for queries of radius rc whose core
 // overlaps lie within lowsq: record offset off; room: entries it can need.  False where an
 // entry cannot describe the box.
-bool vox_grid(const BoxDev& b, int which, double rc, double lowsq, int off, VoxGrid& g, double& nvox, double& room) {
+bool vox_grid(const BoxDev& b, int which, double rc, double lowsq, bool f32, int off, VoxGrid& g, double& nvox,
+              double& room) {
   memset(&g, 0, sizeof(g));
-  if (b.natoms < 1 || b.natoms > (int)kVoxAtomMask || !(rc > 0.0)) return false;
-  const double edge = rc / (which ? kVoxPerCutoffFull : kVoxPerCutoffCbmc);
+  if (b.natoms < 1 || b.natoms >= 1 << (f32 ? kVoxAtomBits : kHitAtomBits) || !(rc > 0.0)) return false;
   const double lmax = std::max(b.L[0], std::max(b.L[1], b.L[2])), lmin = std::min(b.L[0], std::min(b.L[1], b.L[2]));
+  // a fraction of the radius; in a dilute box no more than kVoxPerAtom voxels an atom
+  const double edge = std::max(rc / (which ? kVoxPerCutoffFull : kVoxPerCutoffCbmc),
+                               std::min(std::cbrt(b.volume / (kVoxPerAtom * b.natoms)), 0.25 * lmin));
   double diag2 = 0.0, most = 1.0;
   nvox = 1.0;
   for (int d = 0; d < 3; ++d) {
@@ -3521,7 +3530,8 @@ bool lists64(cass_ctx* c, int nboxes, const int32_t* iboxes) {
     for (int w = 0; w < 2; ++w) {
       VoxGrid g;
       double nvox, room;
-      if (!vox_grid(b, w, w ? full_radius(b) : std::sqrt(b.rcut_cbmcsq), b.rcut_lowsq, 0, g, nvox, room))
+      if (!vox_grid(b, w, w ? full_radius(b) : std::sqrt(b.rcut_cbmcsq), b.rcut_lowsq, false, 0, g, nvox,
+                    room))
         return false;
       total += room;
     }
@@ -3589,6 +3599,8 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     BoxDev v = B.dev;
     const double cpc = c->widom_cells > 0.0 ? c->widom_cells : (f32 || warp64 ? kCellsPerCutoffMixed : kCellsPerCutoffFP64);
     double rcell = (B.desc.rcut_cbmc > 0.0 ? B.desc.rcut_cbmc : B.rcut_max) / cpc;
+    // an atom a cell at least, for what goes through the cells of a dilute box
+    if ((f32 || warp64) && !(c->widom_cells > 0.0)) rcell = std::max(rcell, std::cbrt(v.volume / std::max(1, B.npacked)));
     int ncell = 1;
     for (int d = 0; d < 3; ++d) {
       v.nc[d] = std::max(1, (int)std::floor(v.L[d] / rcell));
@@ -3761,7 +3773,7 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
         double nvox, room;
         // check_overlap of the CBMC options reaches to r_min
         const double lowsq = opt_cbmc && w == 0 ? std::max(b.rcut_lowsq, c->rminsq_most) : b.rcut_lowsq;
-        if (!vox_grid(b, w, rcs[w], lowsq, (int)vox_records, g, nvox, room)) continue;
+        if (!vox_grid(b, w, rcs[w], lowsq, f32, (int)vox_records, g, nvox, room)) continue;
         if (f32) {
           bool open = (double)n_ins * (w ? 2.0 : 32.0) >= nvox;
           for (int d = 0; d < 3; ++d)

@@ -123,3 +123,124 @@ def test_cbmc_options_in_the_mixed_kernel(opts):
     near = np.abs(tm["e_inter"] - to["e_inter"]) <= 2e-5 * to["e_inter_abs"] + 1e-7
     assert near[both].mean() > 0.9 and both.sum() > 100
     assert alone[0].tobytes() == tm[1].tobytes()
+
+
+def _spheres(edges, n, rng, jitter=0.3):
+    """n spheres on a jittered lattice of the box."""
+    edges = np.asarray(edges, dtype=float)
+    step = (np.prod(edges) / n) ** (1.0 / 3.0)
+    sides = np.maximum(1, np.ceil(edges / step - 1e-9)).astype(int)
+    grid = np.array(np.meshgrid(*[np.arange(k) for k in sides], indexing="ij")).reshape(3, -1).T
+    grid = grid[np.sort(rng.choice(len(grid), min(n, len(grid)), replace=False))]
+    return ((grid + 0.5) / sides - 0.5) * edges + rng.uniform(-jitter, jitter, (len(grid), 3))
+
+
+def _sphere_system(boxes, rcut=14.0, seed=2):
+    """boxes: (edges, spheres); butane as the test molecule."""
+    rng = np.random.default_rng(seed)
+    ball, but = workloads.lj_sphere_species(), workloads.butane_species(150.0, 200, 8)
+    ms, specs, k = MoleculeSet(), [], 1
+    for b, (edges, n) in enumerate(boxes):
+        for p in _spheres(edges, n, rng):
+            ms.add(k, 1, b + 1, p[None])
+            k += 1
+        specs.append(BoxSpec(length=tuple(edges), rcut_vdw=min(rcut, 0.5 * min(edges)), rcut_cbmc=6.5, rcut_low=2.0,
+                             temperature=150.0))
+    return System([ball, but], specs, ms, ForceField([ball, but]), [k - 1, 1])
+
+
+def _against_the_oracle(s, prec, n_ins, n_ref, is_=2, seed=31):
+    """The first n_ref insertions of every box against the oracle's, the rest unseen."""
+    ids = list(range(1, len(s.boxes) + 1))
+    with oracle.open_system(s) as o, cg.open_system(s, precision=prec) as g:
+        for b in ids:
+            g.system_total_energy(b)
+            o.system_total_energy(b)
+        to = o.widom_insert(is_, ids, n_ref, 12, 12, seed=seed, trace=True)[1]
+        tg = g.widom_insert(is_, ids, n_ins, 12, 12, seed=seed, trace=True)[1][:, :n_ref]
+    assert np.array_equal(to["overlap"], tg["overlap"])
+    same = to["selected_trial"] == tg["selected_trial"]
+    assert same.all() if prec == abi.PREC_FP64 else same.mean() >= 0.99  # FP32 weights at a boundary
+    ok = (to["overlap"] == 0) & same
+    assert ok.sum() >= 0.1 * ok.size
+    tol = 1e-11 if prec == abi.PREC_FP64 else 2e-5
+    far = np.abs(tg["e_inter"] - to["e_inter"]) > tol * to["e_inter_abs"] + 1e-7
+    assert far[ok].mean() <= (0.0 if prec == abi.PREC_FP64 else 0.01)  # another dihedral trial
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("boxes", [
+    [((24.0, 60.0, 50.0), 900)],                         # two full radii span x and no other edge
+    [((28.5, 28.5, 28.5), 300), ((13.5, 30.0, 13.2), 60)],  # just above two radii; two CBMC radii just fit
+    [((12.4, 12.4, 40.0), 80), ((9.0, 9.0, 9.0), 9)],    # the CBMC radius spans too
+])
+def test_boxes_of_about_two_radii(prec, boxes):
+    _against_the_oracle(_sphere_system(boxes), prec, 300, 300)
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("boxes", [
+    [((400.0, 400.0, 400.0), 500), ((300.0, 60.0, 90.0), 40)],  # voxels wider than a fraction of the radius
+    [((1000.0, 1000.0, 30.0), 300), ((60.0, 60.0, 60.0), 1)],
+])
+def test_dilute_boxes(prec, boxes):
+    _against_the_oracle(_sphere_system(boxes), prec, 400, 400)
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("n", [8000, 14000])
+def test_large_boxes(prec, n):
+    """A box that leaves room for fewer warps, and one that stays in global memory."""
+    edge = (n / 0.6) ** (1.0 / 3.0) * 3.73
+    _against_the_oracle(_sphere_system([((edge,) * 3, n)]), prec, 30, 30)
+
+
+def test_more_than_2_to_the_17_atoms():
+    """The mixed kernel on lists against the FP64 one on cells."""
+    n = 135000
+    edge = (n / 0.6) ** (1.0 / 3.0) * 3.73
+    s = _sphere_system([((edge,) * 3, n)])
+    t = []
+    for prec in (abi.PREC_FP64, abi.PREC_MIXED):
+        with cg.open_system(s, precision=prec) as g:
+            g.system_total_energy(1)
+            t.append(g.widom_insert(2, [1], 50000 if prec == abi.PREC_MIXED else 500, 12, 12, seed=3, trace=True)[1][0, :500])
+    assert np.array_equal(t[0]["overlap"], t[1]["overlap"])
+    same = t[0]["selected_trial"] == t[1]["selected_trial"]
+    ok = (t[0]["overlap"] == 0) & same
+    assert same.mean() >= 0.99 and ok.sum() > 50
+    far = np.abs(t[1]["e_inter"] - t[0]["e_inter"]) > 5e-5 * t[0]["e_inter_abs"] + 1e-7  # coordinates of 230 A in FP32
+    assert far[ok].mean() <= 0.01
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
+@pytest.mark.parametrize("edges, n", [((30.0, 34.0, 32.0), 380), ((20.0, 19.0, 21.0), 90), ((45.0, 45.0, 45.0), 1000)])
+def test_full_warps(prec, edges, n):
+    """A call of 32 insertions per warp: the records of the oracle, and the bits of a short call."""
+    s = _sphere_system([(edges, n)])
+    n_ins = 130000 if prec == abi.PREC_MIXED else 60000
+    _against_the_oracle(s, prec, n_ins, 300)
+    with cg.open_system(s, precision=prec) as g:
+        g.system_total_energy(1)
+        few = g.widom_insert(2, [1], 2500, 12, 12, seed=4, trace=True)[1][0]
+        many = g.widom_insert(2, [1], n_ins, 12, 12, seed=4, trace=True)[1][0][:2500]
+    assert few.tobytes() == many.tobytes()
+
+
+def test_full_warps_of_charged_insertions():
+    """Charges with a Coulomb cutoff other than the vdW one, in a box that has lists for both
+    radii: the charged band notes and terms of the lists."""
+    s = workloads.water_nvt_system(nboxes=1, nmol=1100, length=33.0, rcut=9.0)
+    s.boxes[0].rcut_vdw = 8.2
+    s.max_molecules = [1101]
+    _against_the_oracle(s, abi.PREC_MIXED, 2000, 250, is_=1)
+    with cg.open_system(s, precision=abi.PREC_MIXED) as g:
+        g.system_total_energy(1)
+        few = g.widom_insert(1, [1], 1500, 12, 12, seed=4, trace=True)[1][0]
+        assert g.stats()["widom_fixups"] > 10
+        g.set_widom_band(30.0)
+        wide = g.widom_insert(1, [1], 1500, 12, 12, seed=4, trace=True)[1][0]
+        assert g.stats()["widom_fixups"] > 500
+    ok = few["overlap"] == 0
+    assert np.array_equal(few["overlap"], wide["overlap"])
+    assert (np.abs(few["e_inter"] - wide["e_inter"])[ok] <= 1e-6 * few["e_inter_abs"][ok] + 1e-7).all()

@@ -965,7 +965,6 @@ __device__ bool query_f_exact(const BoxViewF& V, QueryAcc& A, float px, float py
 // lane whose candidate happens to be near.
 constexpr int kCoopItems = 128;  // rows of one batch of queries
 constexpr int kCoopHits = 8;     // listed pairs per lane
-constexpr int kCoopBand = 64;    // band pairs of a warp's insertions
 
 // Scratch of one warp
 struct CoopWarp {
@@ -978,8 +977,9 @@ struct CoopWarp {
   float pabs[kCoopItems];    // its sum of |terms|
   float2 hit[kCoopHits][32]; // r^2 and box atom of the listed pairs of a lane
   int nband[32];             // band pairs met by an owner's full-cutoff pass
-  BandPair band[kCoopBand];  // the noted ones; pad0: owner lane
-  int nnote;
+  float band_r2[32][kMaxBand];  // the first of them: r^2, box atom, atom | kind << 7
+  int band_j[32][kMaxBand];
+  unsigned char band_at[32][kMaxBand];
 };
 
 // cells of dimension d within rc of p, as a query's stencil spans them
@@ -1057,11 +1057,11 @@ __device__ __forceinline__ int stencil_max(const BoxF& f, int d, float rc) {
 
 // a band pair of owner lane `own`, atom `atom` noted in W (all lanes of a warp may call it at once)
 __device__ __forceinline__ void coop_note(CoopWarp& W, int own, int j, float r2, int kind) {
-  const int lane = own & 0xff;
-  if (atomicAdd(&W.nband[lane], 1) >= kMaxBand) return;
-  const int s = atomicAdd(&W.nnote, 1);
-  if (s < kCoopBand) W.band[s] = BandPair{j, r2, (unsigned char)(own >> 8), (unsigned char)kind, (unsigned char)lane, 0};
-  else atomicAdd(&W.nband[lane], kMaxBand);  // no room: k_widom_fix redoes the pass
+  const int lane = own & 0xff, s = atomicAdd(&W.nband[lane], 1);
+  if (s >= kMaxBand) return;  // k_widom_fix redoes the pass
+  W.band_r2[lane][s] = r2;
+  W.band_j[lane][s] = j;
+  W.band_at[lane][s] = (unsigned char)(own >> 8 | kind << 7);
 }
 
 // The energies of the nq queries of W (pos, q, own, st filled, ov cleared): sums
@@ -2017,7 +2017,6 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
   CoopWarp& W = coop_warp();
   const int lane = threadIdx.x & 31;
   W.nband[lane] = 0;
-  if (lane == 0) W.nnote = 0;
   __syncwarp();
   QueryAcc A;
   bool ov = false;
@@ -2030,11 +2029,10 @@ __device__ RecF run_insertion_f(const WidomSpecies& S, const SpeciesF& SF, const
   if (!ov && A.nband > 0) {  // pairs within FP32 rounding of a cutoff: k_widom_fix decides them in FP64
     out.fix = true;
     fe.nband = A.nband;
-    int nn = 0;  // this insertion's notes, by atom and box atom
-    for (int q = 0; q < min(W.nnote, kCoopBand) && A.nband <= kMaxBand; ++q) {
-      if (W.band[q].pad0 != lane) continue;
-      const BandPair bp = W.band[q];
-      int at = nn++;
+    for (int q = 0; q < A.nband && A.nband <= kMaxBand; ++q) {  // the notes, by atom and box atom
+      const unsigned char ak = W.band_at[lane][q];
+      const BandPair bp{W.band_j[lane][q], W.band_r2[lane][q], (unsigned char)(ak & 127), (unsigned char)(ak >> 7), 0, 0};
+      int at = q;
       for (; at > 0 && (fe.band[at - 1].atom > bp.atom || (fe.band[at - 1].atom == bp.atom && fe.band[at - 1].j > bp.j)); --at)
         fe.band[at] = fe.band[at - 1];
       fe.band[at] = bp;

@@ -244,3 +244,11 @@ def test_full_warps_of_charged_insertions():
     ok = few["overlap"] == 0
     assert np.array_equal(few["overlap"], wide["overlap"])
     assert (np.abs(few["e_inter"] - wide["e_inter"])[ok] <= 1e-6 * few["e_inter_abs"][ok] + 1e-7).all()
+
+
+def test_band_notes_do_not_depend_on_the_other_boxes():
+    """Bands so wide that a full warp meets more pairs in them than it had room for."""
+    s = workloads.widom_batch_system(nboxes=30, sizes=[1000, 300, 600] * 10, seed=6, nconfig=100)
+    one, t1, among, ta = _alone_and_together(s, abi.PREC_MIXED, 2, 4000, 1, band=60.0)
+    assert t1.tobytes() == ta.tobytes()
+    assert one == among

@@ -68,7 +68,7 @@ constexpr double kVoxPerCutoffFull = 4.0;
 // 0.37 ms now (1.30 ms without lists); 1e5 mixed ones, which went without lists, 2.70 ms,
 // 1.02 ms now.  Liquids have 1 to 11.
 constexpr double kVoxPerAtom = 16.0;
-constexpr double kVoxMaxBytes = 4.0e9;      // most device memory for them
+constexpr double kVoxMaxBytes = 4.0e9;      // most device memory for them, records and entries
 
 __device__ __forceinline__ int wrapc(int c, int n) {
   c %= n;
@@ -3469,9 +3469,9 @@ const std::vector<int>& members_ext(cass_ctx* c, int ibox);
 namespace {
 
 // The voxel grid `which` (0 CBMC, 1 full) of box b for queries of radius rc whose core
-// overlaps lie within lowsq: record offset off; room: entries it can need.  False where an
+// overlaps lie within lowsq; room: entries it can need.  False where an
 // entry cannot describe the box.
-bool vox_grid(const BoxDev& b, int which, double rc, double lowsq, bool f32, int off, VoxGrid& g, double& nvox,
+bool vox_grid(const BoxDev& b, int which, double rc, double lowsq, bool f32, VoxGrid& g, double& nvox,
               double& room) {
   memset(&g, 0, sizeof(g));
   if (b.natoms < 1 || b.natoms >= 1 << (f32 ? kVoxAtomBits : kHitAtomBits) || !(rc > 0.0)) return false;
@@ -3497,9 +3497,17 @@ bool vox_grid(const BoxDev& b, int which, double rc, double lowsq, bool f32, int
   g.R2 = (float)(R * R);
   const double near = std::sqrt(lowsq) + half;
   g.near2 = (float)(near * near);
-  g.off = off;
   // images of the neighbouring boxes only; a list of 2e4 atoms is no neighbour list
   return R < 0.95 * lmin && nvox <= 1.0e8 && 4.18879021 * R * R * R * b.natoms / b.volume <= 2.0e4;
+}
+
+// Cells of a box in dimension d for the warp-wide kernels, or the thread-per-insertion one
+int widom_cells(const cass_ctx* c, const BoxH& B, int d, bool warp_wide) {
+  const double cpc = c->widom_cells > 0.0 ? c->widom_cells : (warp_wide ? kCellsPerCutoffMixed : kCellsPerCutoffFP64);
+  double rcell = (B.desc.rcut_cbmc > 0.0 ? B.desc.rcut_cbmc : B.rcut_max) / cpc;
+  // an atom a cell at least, for what goes through the cells of a dilute box
+  if (warp_wide && !(c->widom_cells > 0.0)) rcell = std::max(rcell, std::cbrt(B.dev.volume / std::max(1, B.npacked)));
+  return std::min(std::max(1, (int)std::floor(B.dev.L[d] / rcell)), 64);
 }
 
 double full_radius(const BoxDev& b) {
@@ -3508,33 +3516,82 @@ double full_radius(const BoxDev& b) {
   return std::sqrt(std::max(r2, b.rcut_lowsq));
 }
 
-// True where the FP64 insertions run on the voxel lists (k_widom_w): every style has a
-// cutoff, no CBMC option and no molecule-pair cutoff asks for more than the atoms within
-// it, and the boxes can be listed
-bool lists64(cass_ctx* c, int nboxes, const int32_t* iboxes) {
-  if (c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap) return false;
-  double total = 0.0;
-  for (int k = 0; k < nboxes; ++k) {
-    const BoxH& B = c->box[iboxes[k] - 1];
-    const CassBoxDesc& d = B.desc;
-    if (B.comcut || (d.vdw_style != CASS_VDW_NONE &&
-                     (d.vdw_sum_style == CASS_VDW_SUM_MINIMUM || d.vdw_sum_style == CASS_VDW_SUM_CHARMM)) ||
-        (d.charge_style == CASS_CHARGE_COUL && d.charge_sum_style == CASS_QQ_MINIMUM))
-      return false;
-    BoxDev b = B.dev;
-    b.natoms = B.npacked;
-    if (b.natoms == 0) continue;
-    if (!(b.rcut_cbmcsq >= b.rcut_lowsq)) return false;
-    for (int w = 0; w < 2; ++w) {
-      VoxGrid g;
-      double nvox, room;
-      if (!vox_grid(b, w, w ? full_radius(b) : std::sqrt(b.rcut_cbmcsq), b.rcut_lowsq, false, 0, g, nvox,
-                    room))
-        return false;
-      total += room;
+// The lists of a box (g[w].on) and the device memory they may take.  FP64: both radii or
+// none.  Mixed: each where a query's stencil never spans the box (the cell search then
+// sees every pair through one image shift, as an entry does) and the insertions' queries
+// are worth it: a list costs about as much as the cell search of a query, and 32 of an
+// insertion's queries (4 full-cutoff ones) use them.  A matter of the box and of n_ins
+// alone, so that an insertion does not depend on the other boxes of its call.
+struct BoxLists {
+  VoxGrid g[2];
+  double nvox[2] = {0.0, 0.0}, room[2] = {0.0, 0.0};
+  double bytes() const { return (room[0] + room[1]) * sizeof(unsigned) + (nvox[0] + nvox[1]) * sizeof(uint4); }
+};
+BoxLists box_lists(cass_ctx* c, const BoxH& B, bool f32, int64_t n_ins) {
+  BoxLists P;
+  memset(P.g, 0, sizeof(P.g));
+  BoxDev b = B.dev;
+  b.natoms = B.npacked;
+  const double rfull2 = std::max(b.rcut_vdwsq, b.rcut_coulsq);
+  // the mixed full-cutoff pass also looks at the pairs of the bands (widom_boxf) outside its cutoffs
+  const double band = 3.5 * std::sqrt(rfull2) * 5.0e-7 * (std::max(b.L[0], std::max(b.L[1], b.L[2])) + 20.0) *
+                          c->widom_band + 1.0e-6 * rfull2;
+  const double rcs[2] = {std::sqrt(b.rcut_cbmcsq), f32 ? std::sqrt(rfull2 + band) : full_radius(b)};
+  const bool opt = c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap;
+  for (int w = 0; w < 2; ++w) {
+    // check_overlap of the CBMC options reaches to r_min
+    const double lowsq = opt && w == 0 ? std::max(b.rcut_lowsq, c->rminsq_most) : b.rcut_lowsq;
+    VoxGrid g;
+    double nvox, room;
+    if (!vox_grid(b, w, rcs[w], lowsq, f32, g, nvox, room)) continue;
+    if (f32) {
+      bool open = (double)n_ins * (w ? 2.0 : 32.0) >= nvox;
+      for (int d = 0; d < 3; ++d) {
+        const int nc = widom_cells(c, B, d, true);
+        open = open && std::floor(2.0 * rcs[w] * ((double)nc / b.L[d]) + 8.0e-3) + 2.0 < nc;
+      }
+      if (!open) continue;
     }
+    if (P.bytes() + room * sizeof(unsigned) + nvox * sizeof(uint4) > kVoxMaxBytes) continue;
+    P.g[w] = g;
+    P.g[w].on = 1;
+    P.nvox[w] = nvox;
+    P.room[w] = room;
   }
-  return total * sizeof(unsigned) <= kVoxMaxBytes;
+  if (!f32 && !(P.g[0].on && P.g[1].on)) P = BoxLists(), memset(P.g, 0, sizeof(P.g));
+  return P;
+}
+
+// True where the FP64 insertions into a box run on the voxel lists (k_widom_w): every
+// style has a cutoff, no CBMC option and no molecule-pair cutoff asks for more than the
+// atoms within it, and the box can be listed
+bool lists64(cass_ctx* c, const BoxH& B) {
+  const CassBoxDesc& d = B.desc;
+  if (c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap || B.comcut ||
+      (d.vdw_style != CASS_VDW_NONE &&
+       (d.vdw_sum_style == CASS_VDW_SUM_MINIMUM || d.vdw_sum_style == CASS_VDW_SUM_CHARMM)) ||
+      (d.charge_style == CASS_CHARGE_COUL && d.charge_sum_style == CASS_QQ_MINIMUM))
+    return false;
+  return B.npacked == 0 || (B.dev.rcut_cbmcsq >= B.dev.rcut_lowsq && box_lists(c, B, false, 1).g[0].on);
+}
+
+bool lists64(cass_ctx* c, int nboxes, const int32_t* iboxes) {
+  for (int k = 0; k < nboxes; ++k)
+    if (!lists64(c, c->box[iboxes[k] - 1])) return false;
+  return true;
+}
+
+// True where the mixed kernel serves the call: LJ cut / cut_tail with no charges or Ewald
+bool mixed_f32(cass_ctx* c, const SpeciesH& s, int nboxes, const int32_t* iboxes, SpeciesF& SF) {
+  if (c->precision != CASS_PREC_MIXED || c->pt.ntypes > kMaxTypes) return false;
+  for (int k = 0; k < nboxes; ++k) {
+    const CassBoxDesc& d = c->box[iboxes[k] - 1].desc;
+    if (d.vdw_style != CASS_VDW_LJ ||
+        (d.vdw_sum_style != CASS_VDW_SUM_CUT && d.vdw_sum_style != CASS_VDW_SUM_CUT_TAIL) ||
+        (d.charge_style != CASS_CHARGE_NONE && d.charge_sum_style != CASS_QQ_EWALD))
+      return false;
+  }
+  return species_f(s, SF);
 }
 
 }  // namespace
@@ -3577,32 +3634,19 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   std::vector<char> has_ew(nboxes, 0);
   int atom_off = 0, cell_off = 0, max_na = 0;
   size_t max_smem32 = 0, max_smem64 = 0;
-  const bool mixed = c->precision == CASS_PREC_MIXED;
   bool any_recip = false;
-  // the FP32 warp kernel covers LJ cut / cut_tail with no charges or Ewald
-  bool fast_mixed = c->pt.ntypes <= kMaxTypes;
-  for (int k = 0; k < nboxes; ++k) {
+  for (int k = 0; k < nboxes; ++k)
     if ((rc = pack_box_ext(c, iboxes[k] - 1))) return rc;
-    const CassBoxDesc& d = c->box[iboxes[k] - 1].desc;
-    fast_mixed = fast_mixed && d.vdw_style == CASS_VDW_LJ &&
-                 (d.vdw_sum_style == CASS_VDW_SUM_CUT || d.vdw_sum_style == CASS_VDW_SUM_CUT_TAIL) &&
-                 (d.charge_style == CASS_CHARGE_NONE || d.charge_sum_style == CASS_QQ_EWALD);
-  }
   SpeciesF SF;
-  const bool f32 = mixed && fast_mixed && species_f(s, SF);
+  const bool f32 = mixed_f32(c, s, nboxes, iboxes, SF);
   const bool warp64 = !f32 && lists64(c, nboxes, iboxes);
   for (int k = 0; k < nboxes; ++k) {
     int ib = iboxes[k] - 1;
     BoxH& B = c->box[ib];
     BoxDev v = B.dev;
-    const double cpc = c->widom_cells > 0.0 ? c->widom_cells : (f32 || warp64 ? kCellsPerCutoffMixed : kCellsPerCutoffFP64);
-    double rcell = (B.desc.rcut_cbmc > 0.0 ? B.desc.rcut_cbmc : B.rcut_max) / cpc;
-    // an atom a cell at least, for what goes through the cells of a dilute box
-    if ((f32 || warp64) && !(c->widom_cells > 0.0)) rcell = std::max(rcell, std::cbrt(v.volume / std::max(1, B.npacked)));
     int ncell = 1;
     for (int d = 0; d < 3; ++d) {
-      v.nc[d] = std::max(1, (int)std::floor(v.L[d] / rcell));
-      v.nc[d] = std::min(v.nc[d], 64);
+      v.nc[d] = widom_cells(c, B, d, f32 || warp64);
       v.cell_inv[d] = (double)v.nc[d] / v.L[d];
       ncell *= v.nc[d];
     }
@@ -3747,42 +3791,22 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
   // queued (both inside the kernel timing)
   int* d_fixn = nullptr;
   FixEntry* d_fixq = nullptr;
-  // Voxel lists per box and radius.  FP64: everywhere.  Mixed: where the query's stencil
-  // never spans the box (the cell search then sees every pair through one image shift, as
-  // an entry does) and the insertions' queries are worth the lists: a list costs about as
-  // much as the cell search of a query, and 32 of an insertion's queries (4 full-cutoff
-  // ones) use them
+  // Voxel lists per box and radius
   std::vector<VoxGrid> vox(2 * nboxes);
   size_t vox_records = 0;
   double vox_entries = 0.0;
   int vox_most[2] = {0, 0};
   memset(vox.data(), 0, vox.size() * sizeof(VoxGrid));
-  const bool opt_cbmc = c->cbmc_opt.energy_table_res > 0 || c->cbmc_opt.sector_overlap;
   if ((f32 || warp64) && n_ins > 0)
     for (int k = 0; k < nboxes; ++k) {
-      const BoxDev& b = bd[k];
-      const double rfull2 = std::max(b.rcut_vdwsq, b.rcut_coulsq);
-      // the mixed full-cutoff pass also looks at the pairs of the bands (widom_boxf) outside its cutoffs
-      const double band = 3.5 * std::sqrt(rfull2) * 5.0e-7 * (std::max(b.L[0], std::max(b.L[1], b.L[2])) + 20.0) *
-                              c->widom_band + 1.0e-6 * rfull2;
-      const double rcs[2] = {std::sqrt(b.rcut_cbmcsq), f32 ? std::sqrt(rfull2 + band) : full_radius(b)};
+      const BoxLists P = box_lists(c, c->box[iboxes[k] - 1], f32, n_ins);
       for (int w = 0; w < 2; ++w) {
-        VoxGrid g;
-        double nvox, room;
-        // check_overlap of the CBMC options reaches to r_min
-        const double lowsq = opt_cbmc && w == 0 ? std::max(b.rcut_lowsq, c->rminsq_most) : b.rcut_lowsq;
-        if (!vox_grid(b, w, rcs[w], lowsq, f32, (int)vox_records, g, nvox, room)) continue;
-        if (f32) {
-          bool open = (double)n_ins * (w ? 2.0 : 32.0) >= nvox;
-          for (int d = 0; d < 3; ++d)
-            open = open && std::floor(2.0 * rcs[w] * b.cell_inv[d] + 8.0e-3) + 2.0 < b.nc[d];
-          if (!open || (vox_entries + room) * sizeof(unsigned) > kVoxMaxBytes) continue;
-        }
-        g.on = 1;
-        vox[2 * k + w] = g;
-        vox_records += (size_t)nvox;
-        vox_entries += room;
-        vox_most[w] = std::max(vox_most[w], (int)nvox);
+        if (!P.g[w].on) continue;
+        vox[2 * k + w] = P.g[w];
+        vox[2 * k + w].off = (int)vox_records;
+        vox_records += (size_t)P.nvox[w];
+        vox_entries += P.room[w];
+        vox_most[w] = std::max(vox_most[w], (int)P.nvox[w]);
       }
     }
   // their device arrays, built from the cell lists; `need`: an error where there is no room
@@ -3972,9 +3996,9 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
 // insertions' random streams nor the per-box sums (fixed order over insertions), only
 // the order of each query's pair sum.  The mixed kernel has one shape: its queries
 // hardly use the cells, and the lists' own edge does not matter within a tenth.
-extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
-                                 int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
-                                 CassWidomTrace* trace) {
+static int widom_insert_tuned(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
+                              int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
+                              CassWidomTrace* trace) {
   bool tune = c && c->precision != CASS_PREC_MIXED && iboxes && nboxes >= 1 && out && n_ins >= 64 && c->widom_autotune &&
               !(c->widom_cells > 0.0);
   for (int k = 0; tune && k < nboxes; ++k) tune = iboxes[k] >= 1 && iboxes[k] <= c->nboxes;
@@ -4012,4 +4036,66 @@ extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const
   }
   c->widom_tuned.push_back({key, best});
   return run_with(best, n_ins, 0, out, trace);
+}
+
+// A batch whose lists need more than kVoxMaxBytes together is worked off in pieces, box
+// after box as they fit.
+extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
+                                 int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
+                                 CassWidomTrace* trace) {
+  bool ok = c && iboxes && out && nboxes > 1 && is1 >= 1 && is1 <= c->nspecies && n_ins > 0;
+  for (int k = 0; ok && k < nboxes; ++k) {
+    const int ib = iboxes[k] - 1;
+    ok = ib >= 0 && ib < c->nboxes && (c->box[ib].energy_valid || c->box[ib].frame_ready) && !pack_box_ext(c, ib);
+  }
+  std::vector<int> piece(ok ? nboxes : 0, 0);
+  int npieces = 1;
+  if (ok) {
+    if (int rc = ensure_cbmc(c)) return rc;
+    SpeciesF SF;
+    const bool f32 = c->sp[is1 - 1].defined && mixed_f32(c, c->sp[is1 - 1], nboxes, iboxes, SF);
+    double bytes = 0.0;
+    if (f32 || lists64(c, nboxes, iboxes))
+      for (int k = 0; k < nboxes; ++k) {
+        const double need = box_lists(c, c->box[iboxes[k] - 1], f32, n_ins).bytes();
+        if (bytes > 0.0 && bytes + need > kVoxMaxBytes) {
+          ++npieces;
+          bytes = 0.0;
+        }
+        bytes += need;
+        piece[k] = npieces - 1;
+      }
+  }
+  if (npieces == 1)  // also whatever is wrong with the call: the reason comes from there
+    return widom_insert_tuned(c, is1, nboxes, iboxes, n_ins, kappa_ins, kappa_dih, seed, out, trace);
+  CassStats sum{};
+  for (int p = 0; p < npieces; ++p) {
+    std::vector<int> at;
+    std::vector<int32_t> ids;
+    for (int k = 0; k < nboxes; ++k)
+      if (piece[k] == p) {
+        at.push_back(k);
+        ids.push_back(iboxes[k]);
+      }
+    std::vector<CassWidomResult> o(at.size());
+    std::vector<CassWidomTrace> t(trace ? at.size() * (size_t)n_ins : 0);
+    if (int rc = widom_insert_tuned(c, is1, (int)ids.size(), ids.data(), n_ins, kappa_ins, kappa_dih, seed, o.data(),
+                                    trace ? t.data() : nullptr))
+      return rc;
+    for (size_t q = 0; q < at.size(); ++q) {
+      out[at[q]] = o[q];
+      if (trace) memcpy(trace + (size_t)at[q] * n_ins, t.data() + q * n_ins, n_ins * sizeof(CassWidomTrace));
+    }
+    sum.widom_ms += c->stats.widom_ms;
+    sum.widom_kernel_ms += c->stats.widom_kernel_ms;
+    sum.widom_pairs_visited += c->stats.widom_pairs_visited;
+    sum.widom_pairs_in_cutoff += c->stats.widom_pairs_in_cutoff;
+    sum.widom_fixups += c->stats.widom_fixups;
+  }
+  c->stats.widom_ms = sum.widom_ms;
+  c->stats.widom_kernel_ms = sum.widom_kernel_ms;
+  c->stats.widom_pairs_visited = sum.widom_pairs_visited;
+  c->stats.widom_pairs_in_cutoff = sum.widom_pairs_in_cutoff;
+  c->stats.widom_fixups = sum.widom_fixups;
+  return CASS_OK;
 }

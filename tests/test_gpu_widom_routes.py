@@ -252,3 +252,24 @@ def test_band_notes_do_not_depend_on_the_other_boxes():
     one, t1, among, ta = _alone_and_together(s, abi.PREC_MIXED, 2, 4000, 1, band=60.0)
     assert t1.tobytes() == ta.tobytes()
     assert one == among
+
+
+def test_batches_of_more_lists_than_fit():
+    """40 boxes of 20,000 atoms need more than 4 GB of lists: worked off in pieces, every box as alone."""
+    edge = (20000 / 0.6) ** (1.0 / 3.0) * 3.73
+    spots = _spheres((edge,) * 3, 20000, np.random.default_rng(1))
+    ball, but = workloads.lj_sphere_species(), workloads.butane_species(150.0, 200, 8)
+    nb = 40
+    box = BoxSpec(length=(edge,) * 3, rcut_vdw=14.0, rcut_cbmc=6.5, rcut_low=2.0, temperature=150.0)
+    s = System([ball, but], [box] * nb, MoleculeSet(), ForceField([ball, but]), [nb * len(spots), 1])
+    n_ins = 22000
+    with cg.open_system(s, precision=abi.PREC_MIXED) as g:
+        g.set_molecules(np.arange(1, nb * len(spots) + 1), np.ones(nb * len(spots)), np.repeat(np.arange(1, nb + 1), len(spots)),
+                        np.tile(spots.ravel(), nb))
+        for b in range(1, nb + 1):
+            g.system_total_energy(b)
+        every, ta = g.widom_insert(2, list(range(1, nb + 1)), n_ins, 4, 4, seed=5, trace=True)
+        for b in (1, 21, nb):
+            one, t1 = g.widom_insert(2, [b], n_ins, 4, 4, seed=5, trace=True)
+            assert t1[0].tobytes() == ta[b - 1].tobytes()
+            assert one[0] == every[b - 1]

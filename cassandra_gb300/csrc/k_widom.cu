@@ -4039,7 +4039,9 @@ static int widom_insert_tuned(cass_ctx* c, int32_t is1, int32_t nboxes, const in
 }
 
 // A batch whose lists need more than kVoxMaxBytes together is worked off in pieces, box
-// after box as they fit.
+// after box as they fit; in FP64 the boxes without lists (k_widom) are a piece of their
+// own, so that one of them does not send the others there (17 boxes x 1,000 butane
+// insertions, one of them without lists: 20.1 ms together, 18.7 ms so, 16.5 ms of it the one).
 extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
                                  int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
                                  CassWidomTrace* trace) {
@@ -4055,16 +4057,26 @@ extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const
     SpeciesF SF;
     const bool f32 = c->sp[is1 - 1].defined && mixed_f32(c, c->sp[is1 - 1], nboxes, iboxes, SF);
     double bytes = 0.0;
-    if (f32 || lists64(c, nboxes, iboxes))
-      for (int k = 0; k < nboxes; ++k) {
-        const double need = box_lists(c, c->box[iboxes[k] - 1], f32, n_ins).bytes();
-        if (bytes > 0.0 && bytes + need > kVoxMaxBytes) {
-          ++npieces;
-          bytes = 0.0;
-        }
-        bytes += need;
-        piece[k] = npieces - 1;
+    bool any = false, rest = false;
+    npieces = 0;
+    for (int k = 0; k < nboxes; ++k) {
+      const BoxH& B = c->box[iboxes[k] - 1];
+      piece[k] = -1;
+      if (!f32 && !lists64(c, B)) {
+        rest = true;
+        continue;
       }
+      const double need = box_lists(c, B, f32, n_ins).bytes();
+      if (!any || (bytes > 0.0 && bytes + need > kVoxMaxBytes)) {
+        ++npieces;
+        bytes = 0.0;
+      }
+      any = true;
+      bytes += need;
+      piece[k] = npieces - 1;
+    }
+    if (rest) ++npieces;  // the boxes without lists
+    for (int& q : piece) q = q < 0 ? npieces - 1 : q;
   }
   if (npieces == 1)  // also whatever is wrong with the call: the reason comes from there
     return widom_insert_tuned(c, is1, nboxes, iboxes, n_ins, kappa_ins, kappa_dih, seed, out, trace);

@@ -273,3 +273,15 @@ def test_batches_of_more_lists_than_fit():
             one, t1 = g.widom_insert(2, [b], n_ins, 4, 4, seed=5, trace=True)
             assert t1[0].tobytes() == ta[b - 1].tobytes()
             assert one[0] == every[b - 1]
+
+
+@pytest.mark.parametrize("prec", [abi.PREC_FP64, abi.PREC_MIXED])
+def test_a_box_without_lists_beside_others(prec):
+    """The last box is too small for lists (a radius reaches beyond the neighbouring images): the
+    others keep theirs, and every box its own bits."""
+    s = _sphere_system([((40.0, 40.0, 40.0), 700), ((9.0, 9.0, 9.0), 9), ((30.0, 50.0, 30.0), 500)])
+    _against_the_oracle(s, prec, 300, 300)
+    for pick in (1, 2, 3):
+        one, t1, among, ta = _alone_and_together(s, prec, 2, 300, pick)
+        assert t1.tobytes() == ta.tobytes()
+        assert one == among

@@ -1390,7 +1390,7 @@ int cass_set_widom_band(cass_ctx* c, double scale) {
 }
 
 int cass_set_mc_cluster(cass_ctx* c, int32_t ctas) {
-  if (!c || ctas < 0 || ctas > 8) return set_error(CASS_EINVAL, "ctas must be in [0, 8]");
+  if (!c || ctas < 0 || (ctas > 8 && ctas != 16)) return set_error(CASS_EINVAL, "ctas must be in [0, 8] or 16");
   c->mc_cluster = ctas;
   return CASS_OK;
 }

@@ -549,9 +549,10 @@ int cass_set_widom_cells(cass_ctx* ctx, double cells_per_cutoff);
 int cass_set_widom_autotune(cass_ctx* ctx, int32_t on);
 /* CTAs (a thread-block cluster) that run each chain of cass_mc_sweeps: 0 (the
  * default) chooses per call -- several when few chains leave SMs idle, so a
- * single chain's pair and k-vector loops spread over up to 8 multiprocessors;
- * 1..8 fixes it (boxes kept in global memory always run on one CTA).  Results
- * do not depend on it beyond summation order.  cass_get_stats reports the
+ * single chain's pair and k-vector loops spread over up to 16 multiprocessors;
+ * 1..8 or 16 asks for that many, and fewer run where so many do not fit at once
+ * (boxes kept in global memory have one copy per CTA).  Results do not depend on
+ * it beyond summation order.  cass_get_stats reports the
  * choice in gcmc_cluster. */
 int cass_set_mc_cluster(cass_ctx* ctx, int32_t ctas);
 /* Mixed precision: the full-cutoff pass of each Widom insertion notes the pairs

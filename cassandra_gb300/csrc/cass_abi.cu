@@ -383,7 +383,6 @@ __global__ void __launch_bounds__(kBlock) k_pair_total(BoxDev b, PairTable t, co
 // 2,250 atoms of water: 2.83 ms with a thread per i and its pairs as they came, 0.14 ms
 // now; 12,288 atoms: 6.3 ms and 0.74 ms.
 constexpr int kPairWarps = 4;
-constexpr int kPairSms = 152;  // the SMs a launch is sized for
 
 __global__ void __launch_bounds__(32 * kPairWarps) k_pair_hits(BoxDev b, PairTable t, const double4_32a* __restrict__ p64,
                                                                const float4* __restrict__ p32,
@@ -2140,7 +2139,9 @@ int cass_system_total_energy(cass_ctx* c, int32_t ibox1, int32_t intra_flag, Cas
   // FP64 pairs: tiles of j per warp so that about 24 warps per SM share the box's tile pairs
   const int nt = (n + 31) / 32;
   const long long tile_pairs = (long long)nt * (nt + 1) / 2;
-  const int tiles = (int)std::max<long long>(1, std::min<long long>(16, tile_pairs / (24LL * kPairSms)));
+  int sms = 0;
+  CASS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  const int tiles = (int)std::max<long long>(1, std::min<long long>(16, tile_pairs / (24LL * sms)));
   const dim3 grid = fast ? dim3((n + kBlock - 1) / kBlock, (n + kTileJ - 1) / kTileJ)
                          : dim3(nt, (nt + kPairWarps * tiles - 1) / (kPairWarps * tiles));
   if ((rc = ensure_scratch(c, std::max(7 * nblk_intra, n > 1 ? 2 * (int)(grid.x * grid.y) : 1), 1))) return rc;

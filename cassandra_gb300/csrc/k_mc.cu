@@ -102,7 +102,7 @@ struct McBox {
   size_t gbox_stride;  // one copy per CTA of the box's cluster, this many bytes apart
 };
 
-// the move thread 0 prepared for the block
+// the move warp 0 prepared for the block
 struct McMove {
   int skip, stop, kind, is, pm, na, first, slot, accept, ewald, tab;
   double old_r[3 * kMaxAtoms], trial[3 * kMaxAtoms], q[kMaxAtoms];
@@ -823,9 +823,10 @@ __global__ void __launch_bounds__(kMcThreads) k_mc_sweeps(const __grid_constant_
         }
       }
       if (lane == 0) mv.accept = acc ? 1 : 0;
-      if (!o) {
       const int is = mv.is;
-      if (mv.kind == 0) {
+      if (o) {
+        // the chain stops: no counts and no adaptation
+      } else if (mv.kind == 0) {
         if (acc) {
           ++R.n_translate_accepted;
           ++ns_d[is];
@@ -853,7 +854,6 @@ __global__ void __launch_bounds__(kMcThreads) k_mc_sweeps(const __grid_constant_
           if (ratio < 0.5) mr[is] = fmax(0.01, 0.95 * mr[is]);
           else mr[is] = fmin(kPI, 1.05 * mr[is]);
         }
-      }
       }
       if (acc) {  // commit the coordinates and the COM
         for (int e = lane; e < 3 * na; e += 32) {

@@ -3373,8 +3373,6 @@ double lrc_host(cass_ctx* c, const BoxH& B, const std::vector<double>& nb) {
   return e;
 }
 
-// FP32 tables of the test species for k_widom_mixed; false when the species
-// does not fit them (the FP64-geometry kernel runs instead)
 }  // namespace
 
 namespace cassgpu {

@@ -66,7 +66,7 @@ constexpr double kVoxPerCutoffFull = 4.0;
 // Most voxels per atom of a box: a voxel costs its search even where it is empty.  500
 // atoms in a box of 400 A had 8e6 voxels of the CBMC radius: one FP64 insertion 1.62 ms,
 // 0.37 ms now (1.30 ms without lists); 1e5 mixed ones, which went without lists, 2.70 ms,
-// 1.02 ms now.  Liquids have 1 to 11.
+// 1.09 ms now.  Liquids have 1 to 11.
 constexpr double kVoxPerAtom = 16.0;
 constexpr double kVoxMaxBytes = 4.0e9;      // most device memory for them, records and entries
 
@@ -3840,12 +3840,15 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     return CASS_OK;
   };
   // The launch of a warp-wide kernel: insertions per warp, as few as give every warp of
-  // the GPU work at once, up to one per lane; then one group of insertions per warp: a
-  // CTA is as long as its slowest warp and the hardware hands out the CTAs; in very
-  // large calls several, to stage the box less often
+  // the GPU work at once (`waves` times), up to one per lane; then one group of insertions
+  // per warp: a CTA is as long as its slowest warp and the hardware hands out the CTAs; in
+  // very large calls several, to stage the box less often.  Cell rows fill the lanes
+  // whatever a warp's insertions are, and a half-empty wave of long groups costs more than
+  // the shorter ones: two waves where they serve (64 boxes of 180 x 1,000: 5.9 ms with one,
+  // 4.2 with two, 4.0 with four; one box of 180 x 100,000: 4.4, 4.9, 5.8).
   int per_warp = 1, wthreads = 32;
-  auto warp_grid = [&](int warps) {
-    while (per_warp < 32 && (n_ins + per_warp - 1) / per_warp * nboxes > (long long)dev_sms * warps) per_warp *= 2;
+  auto warp_grid = [&](int warps, int waves) {
+    while (per_warp < 32 && (n_ins + per_warp - 1) / per_warp * nboxes > (long long)dev_sms * warps * waves) per_warp *= 2;
     const long long groups = (n_ins + per_warp - 1) / per_warp;
     wthreads = 32 * (int)std::min<long long>(warps, std::max<long long>(1, (groups * nboxes + dev_sms - 1) / dev_sms));
     const long long need = (groups + wthreads / 32 - 1) / (wthreads / 32);
@@ -3870,7 +3873,7 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     const size_t dyn = dyn_of(warps, staged);
     auto kern = staged ? k_widom_w<true> : k_widom_w<false>;
     CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    const dim3 g = warp_grid(warps);
+    const dim3 g = warp_grid(warps, 1);
     c->stats.widom_smem_bytes = (int)dyn;
     kern<<<g, wthreads, dyn, c->stream>>>(S, c->pt, c->pools, d_bd, d_ids, c->d_c64.as<double4_32a>(), d_c32, d_vox,
                                           d_vrec, reinterpret_cast<const uint4*>(d_vlist), s.d_library.as<double>(),
@@ -3897,7 +3900,9 @@ static int widom_insert_impl(cass_ctx* c, int32_t is1, int32_t nboxes, const int
     if ((rc2 = build_lists(false))) return rc2;
     const size_t dyn = smem_f32(warps32, smem32);
     CASS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    const dim3 g = warp_grid(warps32);
+    bool rows = false;
+    for (int k = 0; k < nboxes; ++k) rows = rows || !vox[2 * k].on || !vox[2 * k + 1].on;
+    const dim3 g = warp_grid(warps32, rows ? 2 : 1);
     c->stats.widom_smem_bytes = (int)dyn;
     kern<<<g, wthreads, dyn, c->stream>>>(
         S, SF, c->pt, d_bd, d_ids, d_c32, c->d_cq32.as<float>(), c->d_cell_start.as<int>(), s.d_library_f.as<float>(),

@@ -2518,6 +2518,7 @@ struct Head64 {
   float pre[2];                       // FP32 bound of r^2 beyond the CBMC and the full cutoffs
   float low_sure, low_pre;            // FP32 r^2 below / above which a pair surely is / is not an overlap
   float edge_lo[3], edge_hi[3];       // |d| about half a box edge: surely this image / surely another
+  int wide[2];                        // the cutoffs reach half a box edge: more than one image may be within them
 };
 __device__ __forceinline__ Head64& head64() { return *reinterpret_cast<Head64*>(smem); }
 constexpr unsigned kHead64Bytes = (sizeof(Head64) + 31) & ~31u;
@@ -2575,6 +2576,7 @@ __device__ __noinline__ void coop_eval64(const CoopBox B, int nq, bool want_qq, 
   const bool qq_on = want_qq && b.charge_style == CASS_CHARGE_COUL, lj = lj_plain_style(b);
   const bool ewald = b.charge_sum_style == CASS_QQ_EWALD;
   const float pre = H.pre[FULL ? 1 : 0];
+  const bool wide = H.wide[FULL ? 1 : 0];
   if (lane < nq) W.sum[lane] = W.sabs[lane] = 0.0;
   int cnt = 0;
   double acc = 0.0, aabs = 0.0;  // FULL: this lane's share of the current query
@@ -2668,10 +2670,12 @@ __device__ __noinline__ void coop_eval64(const CoopBox B, int nq, bool want_qq, 
         const int j = (int)(e & kVoxAtomMask), c = (int)(e >> kVoxAtomBits) + code;
         const float4 a = p32[j], sh = H.shift[c];
         const float dx = fabsf((x + sh.x) - a.x), dy = fabsf((y + sh.y) - a.y), dz = fabsf((z + sh.z) - a.z);
-        // a point outside the box may have its pairs through another image than the nearest
-        hit = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > pre) &&
-              (code != 0 || (dx <= H.edge_hi[0] && dy <= H.edge_hi[1] && dz <= H.edge_hi[2]));
-        const unsigned check = code != 0 || dx > H.edge_lo[0] || dy > H.edge_lo[1] || dz > H.edge_lo[2];
+        hit = !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > pre);
+        unsigned check = 0u;
+        if (wide) {  // a point outside the box may have its pairs through another image than the nearest
+          hit = hit && (code != 0 || (dx <= H.edge_hi[0] && dy <= H.edge_hi[1] && dz <= H.edge_hi[2]));
+          check = code != 0 || dx > H.edge_lo[0] || dy > H.edge_lo[1] || dz > H.edge_lo[2];
+        }
         h = (unsigned)j | (unsigned)c << kHitAtomBits | (unsigned)q << 26 | check << 31;
       }
       const unsigned m = __ballot_sync(0xffffffffu, hit);
@@ -3163,6 +3167,8 @@ __global__ void __launch_bounds__(kThreads64, 1) k_widom_w(const __grid_constant
       H.edge_lo[d] = (float)(b.hL[d] * (1.0 - 1.0e-5));
       H.edge_hi[d] = (float)(b.hL[d] * (1.0 + 1.0e-5));
     }
+    const float edge = fminf(H.edge_lo[0], fminf(H.edge_lo[1], H.edge_lo[2]));
+    for (int w = 0; w < 2; ++w) H.wide[w] = !(H.pre[w] < edge * edge);
   }
   if (threadIdx.x < 2) H.vox[threadIdx.x] = vox[2 * k + threadIdx.x];
   for (int q = threadIdx.x; q < kImages; q += blockDim.x) {

@@ -33,6 +33,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <vector>
 
 #include "cass_ctx.h"
@@ -4054,6 +4056,7 @@ static int widom_insert_tuned(cass_ctx* c, int32_t is1, int32_t nboxes, const in
 extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const int32_t* iboxes, int64_t n_ins,
                                  int32_t kappa_ins, int32_t kappa_dih, uint64_t seed, CassWidomResult* out,
                                  CassWidomTrace* trace) {
+  if (c) CASS_CUDA(cudaSetDevice(c->device));  // the boxes are packed to tell how they are worked off
   bool ok = c && iboxes && out && nboxes > 1 && is1 >= 1 && is1 <= c->nspecies && n_ins > 0;
   for (int k = 0; ok && k < nboxes; ++k) {
     const int ib = iboxes[k] - 1;
@@ -4099,13 +4102,17 @@ extern "C" int cass_widom_insert(cass_ctx* c, int32_t is1, int32_t nboxes, const
         ids.push_back(iboxes[k]);
       }
     std::vector<CassWidomResult> o(at.size());
-    std::vector<CassWidomTrace> t(trace ? at.size() * (size_t)n_ins : 0);
+    std::unique_ptr<CassWidomTrace[]> t;
+    if (trace) {
+      t.reset(new (std::nothrow) CassWidomTrace[at.size() * (size_t)n_ins]);
+      if (!t) return set_error(CASS_ENOMEM, "no room for the records of a piece of the batch");
+    }
     if (int rc = widom_insert_tuned(c, is1, (int)ids.size(), ids.data(), n_ins, kappa_ins, kappa_dih, seed, o.data(),
-                                    trace ? t.data() : nullptr))
+                                    t.get()))
       return rc;
     for (size_t q = 0; q < at.size(); ++q) {
       out[at[q]] = o[q];
-      if (trace) memcpy(trace + (size_t)at[q] * n_ins, t.data() + q * n_ins, n_ins * sizeof(CassWidomTrace));
+      if (trace) memcpy(trace + (size_t)at[q] * n_ins, t.get() + q * n_ins, n_ins * sizeof(CassWidomTrace));
     }
     sum.widom_ms += c->stats.widom_ms;
     sum.widom_kernel_ms += c->stats.widom_kernel_ms;

@@ -1350,7 +1350,10 @@ struct PairSum {
 // coop_eval through the voxel lists: a query per lane, or per 2, 4 ... 32 lanes where
 // the queue is short.  CBMC queries (not DETECT) come without an overlap.  Each word of a
 // list (four entries) is summed by itself and the words in their order, whatever lanes
-// have them: an insertion's bits do not depend on what else its warp works on.
+// have them: an insertion's bits do not depend on what else its warp works on.  A sum per
+// lane and a tree over the lanes, whose order did, took 2 % less (64 boxes x 15,625
+// insertions 13.06 ms against 13.39, 250 in one box 350 us against 356); all terms through
+// one lane took 13.71 ms and 369 us.
 template <bool SMEM, bool COUNT, bool OPT, bool DETECT>
 __device__ __noinline__ void coop_eval_list(const CoopBox B, int nq, bool want_qq, QueryAcc& cnt) {
   const CoopHead& H = coop_head();
